@@ -308,6 +308,26 @@ typedef struct MkbStatus {
 int mkb_launch(const MkbGlobals *g, void *cuda_stream);
 
 /*
+ * A prompt's tokens at once (no counterpart in the reference, whose prompts go through its torch model,
+ * scripts/generate.py:125-137): `tokens` rows of embeddings, the first at position `pos0` of sequence 0, whose
+ * earlier positions are in the caches.  Writes their keys and values into the caches and, with `want_logits`, the
+ * last token's logits.  `g` is that of mkb_launch; batch and tensor-parallel launches, residual_scale > 1 and a
+ * head_dim other than 64 or 128 are MKB_ERR_UNSUPPORTED.  Instructions, barriers, accumulators and the
+ * activation vectors of `g` are not touched.  `workspace`: mkb_prompt_bytes(g, tokens) bytes, 256-byte aligned.
+ */
+typedef struct MkbPrompt {
+    uint32_t struct_bytes;
+    int32_t tokens;
+    int32_t pos0;
+    int32_t want_logits;
+    const void *hidden;   /* bf16 [tokens, hidden_size], 16-byte aligned */
+    void *workspace;
+    size_t workspace_bytes;
+} MkbPrompt;
+size_t mkb_prompt_bytes(const MkbGlobals *g, int32_t tokens);
+int mkb_prompt(const MkbGlobals *g, const MkbPrompt *p, void *cuda_stream);
+
+/*
  * Synchronise `cuda_stream` and copy the device status record to `out`.
  * Returns out->code (MKB_OK when the last launches ran clean).  The reference
  * has no counterpart: its device waits are unbounded and a bad opcode traps

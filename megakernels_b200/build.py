@@ -48,8 +48,10 @@ class Library:
 LIBRARIES = {
     "llama": Library(
         "libmkb200.so",
-        ("megakernel.cu", "megakernel_batched.cu", "megakernel_gemm.cu", "host.cu", "no_alloc.cu", "peer.cu"),
-        ("mk_common.cuh", "megakernel.cu", "../../include/mkb200.h"),
+        ("megakernel.cu", "megakernel_batched.cu", "megakernel_gemm.cu", "host.cu", "no_alloc.cu", "peer.cu",
+         "llama_prompt.cu", "hybrid_gemm_bf16.cu", "hybrid_flash.cu"),
+        ("mk_common.cuh", "megakernel.cu", "llama_prompt.h", "../../include/mkb200.h", "hybrid_common.cuh", "hybrid_kernels.h", "hybrid_tcgen05.cuh",
+         "../../include/mkb200_hybrid.h"),
     ),
     "hybrid": Library(
         "libmkb200_hybrid.so",

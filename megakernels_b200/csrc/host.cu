@@ -9,6 +9,7 @@
 #include <mutex>
 #include <vector>
 
+#include "llama_prompt.h"
 #include "mk_common.cuh"
 
 namespace mkb {
@@ -538,6 +539,29 @@ int mkb_launch(const MkbGlobals* g, void* cuda_stream) {
 }
 
 
+
+size_t mkb_prompt_bytes(const MkbGlobals* g, int32_t tokens) { return g && tokens > 0 ? mkb::PromptBuffers(*g, tokens, nullptr).total : 0; }
+
+int mkb_prompt(const MkbGlobals* g, const MkbPrompt* p, void* cuda_stream) {
+    if (!p || p->struct_bytes != sizeof(MkbPrompt)) return fail(MKB_ERR_INVALID_ARGUMENT, "prompt: NULL or another struct size");
+    int* status = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        DeviceState* ds = nullptr;
+        int rc = device_state(&ds);
+        if (rc || (rc = validate(g))) return rc;
+        status = g->status ? g->status : ds->status;
+    }
+    if (g->batch > 1 || g->tp.size > 1 || g->residual_scale > 1.f || (g->head_dim != 64 && g->head_dim != 128))
+        return fail(MKB_ERR_UNSUPPORTED, "prompt: one sequence on one GPU, head_dim 64 or 128");
+    if (p->tokens < 1 || p->pos0 < 0 || (int64_t)p->pos0 + p->tokens > g->kv_max_len)
+        return fail(MKB_ERR_INVALID_ARGUMENT, "prompt: %d tokens from position %d on, cache length %d", p->tokens, p->pos0, g->kv_max_len);
+    if (!p->hidden || !aligned16(p->hidden) || !p->workspace || ((uintptr_t)p->workspace & 255) ||
+        p->workspace_bytes < mkb_prompt_bytes(g, p->tokens))
+        return fail(MKB_ERR_INVALID_ARGUMENT, "prompt: hidden or workspace missing, unaligned or too small");
+    MKB_CUDA(mkb::prompt_launch(*g, *p, status, (cudaStream_t)cuda_stream));
+    return MKB_OK;
+}
 
 int mkb_sync_status(const MkbGlobals* g, void* cuda_stream, MkbStatus* out) {
     if (!out) return fail(MKB_ERR_INVALID_ARGUMENT, "status output pointer is NULL");

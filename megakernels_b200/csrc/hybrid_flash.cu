@@ -383,4 +383,19 @@ cudaError_t flash_tc(const MkbhGlobals& g, const MkbhLayer& L, bf16* out, int64_
     return s.v_slabs == 1 ? launch<64>(m, s, stream) : launch<128>(m, s, stream);
 }
 
+cudaError_t flash_cache(const CacheAttention& a, cudaStream_t stream) {
+    const int slabs = a.dim / 64, rows = a.pos0 + a.n;
+    FlashMaps m;
+    cudaError_t e;
+    // rows that nobody has written yet lie outside the maps: they read as zero
+    if ((e = tc_map(&m.q, a.q, a.heads * a.dim, a.n, a.heads * a.dim, 64, kRows)) != cudaSuccess) return e;
+    if ((e = tc_map(&m.k, a.k, a.kv_heads * a.dim, rows, a.kv_heads * a.dim, 64, kTile)) != cudaSuccess) return e;
+    if ((e = tc_map(&m.v, a.v, a.kv_heads * a.dim, rows, a.kv_heads * a.dim, 64, kTile)) != cudaSuccess) return e;
+    m.k_rest = m.k;
+    constexpr int kAll = 1 << 30;
+    FlashShape s{a.n, a.pos0, a.heads, a.heads / a.kv_heads, slabs, 0, slabs, stages_for(slabs, slabs), a.dim, a.dim, 0, 0, 0, kAll, 0, kAll,
+                 a.dim, a.scale, nullptr, nullptr, nullptr, a.out, (int64_t)a.heads * a.dim, 2000000000ull, a.status};
+    return slabs == 1 ? launch<64>(m, s, stream) : launch<128>(m, s, stream);
+}
+
 }  // namespace mkbh

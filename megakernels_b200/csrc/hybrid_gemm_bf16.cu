@@ -5,7 +5,8 @@
 // (tcgen05.mma, M = 128 tokens, N = kBN features), four epilogue warps that read one of two
 // accumulators back while the other is being filled.  The epilogue goes through shared memory so
 // that stores are row segments: plus the bias, times the layer scale into the 32-bit residual stream,
-// in bf16, or the gated unit of neighbouring columns in bf16.
+// in bf16, the gated unit of neighbouring columns in bf16, the gated unit of two matrices (a tile is then
+// as many rows of either), or rotated into the queries and the key/value cache.
 #include "hybrid_kernels.h"
 #include "hybrid_tcgen05.cuh"
 
@@ -35,10 +36,14 @@ struct Shape {
     int* status;
 };
 
-template <int kBN>
+// What the epilogue can do: a build per group of results, so that one group's code does not cost the others registers.
+enum class Group { kPlain, kSilu, kRope };  // kSilu: two weight matrices, kBN / 2 columns of each per tile
+constexpr Group group_of(Result r) { return r == Result::kSilu ? Group::kSilu : r == Result::kRope ? Group::kRope : Group::kPlain; }
+
+template <int kBN, Group kGroup>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap, const Shape s,
-                 const GemmEpilogue e) {
+gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap,
+                 const __grid_constant__ CUtensorMap wmap2, const Shape s, const GemmEpilogue e) {
     using G = Geo<kBN>;
     extern __shared__ uint8_t raw[];
     const uint32_t raw32 = mkb::smem_u32(raw), base = (raw32 + 1023u) & ~1023u;
@@ -73,13 +78,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = (uint32_t)ctl[1];
+    constexpr bool kDual = kGroup == Group::kSilu;
+    constexpr int wide = kDual ? kBN / 2 : kBN;
     const int ksteps = (s.K + kBK - 1) / kBK;
 
     if (warp == 0 && lane == 0) {
         uint32_t it = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < s.tiles && ok; tile += gridDim.x) {
-            const int m0 = (tile % s.tiles_m) * kBM, n0 = (tile / s.tiles_m) * kBN;
+            const int m0 = (tile % s.tiles_m) * kBM, n0 = (tile / s.tiles_m) * wide;
             for (int k = 0; k < ksteps; ++k, ++it) {
                 const int st = it % G::kStages;
                 if (!tc_wait(empty(st), ((it / G::kStages) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 0)) {
@@ -90,6 +97,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                 mkb::mbar_expect_tx(full(st), G::kStageBytes);
                 tc_tma_2d(dst, &amap, k * kBK, m0, full(st));
                 tc_tma_2d(dst + kBM * kBK * 2, &wmap, k * kBK, n0, full(st));
+                if (kDual) tc_tma_2d(dst + (kBM + kBN / 2) * kBK * 2, &wmap2, k * kBK, n0, full(st));
             }
         }
         // no copy may be in flight when the CTA's shared memory goes away
@@ -122,20 +130,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         float* tr = reinterpret_cast<float*>(gbase + G::kEpi) + (warp - 2) * 32 * kEpiStride;
         uint32_t acc = 0;
         for (int tile = blockIdx.x; tile < s.tiles; tile += gridDim.x, ++acc) {
-            const int m0 = (tile % s.tiles_m) * kBM + q * 32, n0 = (tile / s.tiles_m) * kBN;
+            const int m0 = (tile % s.tiles_m) * kBM + q * 32, n0 = (tile / s.tiles_m) * wide;
             const uint32_t buf = acc & 1u;
             const bool ok = tc_wait(acc_full(buf), (acc >> 1) & 1u, ctl, s.timeout_ns, s.status, 2);
             if (!__all_sync(0xffffffffu, ok)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int rows = min(32, s.T - m0);
-            for (int c0 = 0; c0 < kBN; c0 += 32) {
+            for (int c0 = 0; c0 < wide; c0 += 32) {
                 if (n0 + c0 >= s.N || rows <= 0) break;  // uniform over the warp
                 uint32_t r[32];
                 tc_load32(tmem + ((uint32_t)(q * 32) << 16) + buf * kBN + c0, r);
+                if constexpr (kDual) {
+                    uint32_t u[32];
+                    tc_load32(tmem + ((uint32_t)(q * 32) << 16) + buf * kBN + kBN / 2 + c0, u);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const float g = __uint_as_float(r[j]);
+                        r[j] = __float_as_uint(g * sigmoid_f(g) * __uint_as_float(u[j]));
+                    }
+                }
 #pragma unroll
                 for (int j = 0; j < 32; ++j) tr[lane * kEpiStride + j] = __uint_as_float(r[j]);
                 __syncwarp();
-                if (e.what == Result::kCast) {  // two rows at a time, two columns per lane
+                if (kDual || (kGroup == Group::kPlain && e.what == Result::kCast)) {  // two rows at a time, two columns per lane
                     const int col = 2 * (lane & 15), n = n0 + c0 + col;
                     bf16* o = static_cast<bf16*>(e.cast) + (size_t)m0 * e.ld + n;
                     for (int i = lane >> 4; i < rows; i += 2) {
@@ -143,7 +160,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                         if (n + 1 < s.N) *reinterpret_cast<uint32_t*>(o + (size_t)i * e.ld) = mkb::pack_bf16x2(v[0], v[1]);
                         else if (n < s.N) o[(size_t)i * e.ld] = __float2bfloat16_rn(v[0]);
                     }
-                } else if (e.what == Result::kGlu) {  // 16 units of a row per half warp
+                } else if (kGroup == Group::kPlain && e.what == Result::kGlu) {  // 16 units of a row per half warp
                     const int col = 2 * (lane & 15), n = n0 + c0 + col;
                     bf16* o = static_cast<bf16*>(e.cast) + (size_t)m0 * e.ld + n / 2;
                     if (n < s.N)  // (N is even)
@@ -151,9 +168,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                             const float* v = tr + i * kEpiStride + col;
                             o[(size_t)i * e.ld] = __float2bfloat16_rn(clamped_glu(v[0], v[1], e.limit, e.alpha));
                         }
+                } else if (kGroup == Group::kRope) {  // (boundaries are multiples of 64: a chunk has one target)
+                    const int col = 2 * (lane & 15), n = n0 + c0 + col;
+                    const RopeTarget& p = e.rope;
+                    const int at = n - p.q_cols;  // column of [keys | values]
+                    bf16* o = at < 0 ? p.q + n : at < p.k_cols ? p.k + at : p.v + (at - p.k_cols);
+                    const int64_t ld = at < 0 ? p.q_cols : p.k_cols;
+                    const int row0 = at < 0 ? m0 : p.pos0 + m0;
+                    for (int i = lane >> 4; i < rows; i += 2) {
+                        float x = tr[i * kEpiStride + col], y = tr[i * kEpiStride + col + 1];
+                        if (at < p.k_cols) {
+                            const size_t z = (size_t)(p.pos0 + m0 + i) * p.dim + n % p.dim;
+                            const float2 c = __ldg(reinterpret_cast<const float2*>(p.cos + z)), d = __ldg(reinterpret_cast<const float2*>(p.sin + z));
+                            const float turned = x * c.x - y * d.x;
+                            y = y * c.y + x * d.y;
+                            x = turned;
+                        }
+                        *reinterpret_cast<uint32_t*>(o + (size_t)(row0 + i) * ld) = mkb::pack_bf16x2(x, y);
+                    }
                 }
                 const int n = n0 + c0 + lane;
-                if (n < s.N && e.what <= Result::kAdd) {
+                if (kGroup == Group::kPlain && n < s.N && e.what <= Result::kAdd) {
                     float* o = e.out + (size_t)m0 * e.ld + n;
                     if (e.what == Result::kAdd) {
                         const float f = e.scale ? __ldg(e.scale + n) : 1.f;
@@ -179,32 +214,51 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * kBN)) : "memory");
 }
 
-template <int kBN>
-cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, Shape s, const GemmEpilogue& e, int sms,
-                   cudaStream_t st) {
+template <int kBN, Group kGroup>
+cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, Shape s, const GemmEpilogue& e,
+                   int sms, cudaStream_t st) {
     using G = Geo<kBN>;
     static bool set[64] = {};
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
     if (!set[dev & 63]) {
-        err = cudaFuncSetAttribute(gemm_bf16_kernel<kBN>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kAlloc);
+        err = cudaFuncSetAttribute(gemm_bf16_kernel<kBN, kGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kAlloc);
         if (err != cudaSuccess) return err;
         set[dev & 63] = true;
     }
-    CUtensorMap amap, wmap;
+    CUtensorMap amap, wmap, wmap2;
+    constexpr bool kDual = kGroup == Group::kSilu;
+    constexpr int wide = kDual ? kBN / 2 : kBN;
     if ((err = tc_map(&amap, A, s.K, s.T, lda, kBK, kBM)) != cudaSuccess) return err;
-    if ((err = tc_map(&wmap, W, s.K, s.N, ldw, kBK, kBN)) != cudaSuccess) return err;
+    if ((err = tc_map(&wmap, W, s.K, s.N, ldw, kBK, wide)) != cudaSuccess) return err;
+    wmap2 = wmap;
+    if (kDual && (err = tc_map(&wmap2, W2, s.K, s.N, ldw, kBK, wide)) != cudaSuccess) return err;
     s.tiles_m = (s.T + kBM - 1) / kBM;
-    s.tiles = s.tiles_m * ((s.N + kBN - 1) / kBN);
-    gemm_bf16_kernel<kBN><<<s.tiles < sms ? s.tiles : sms, kGemmThreads, G::kAlloc, st>>>(amap, wmap, s, e);
+    s.tiles = s.tiles_m * ((s.N + wide - 1) / wide);
+    gemm_bf16_kernel<kBN, kGroup><<<s.tiles < sms ? s.tiles : sms, kGemmThreads, G::kAlloc, st>>>(amap, wmap, wmap2, s, e);
     return cudaGetLastError();
+}
+
+template <Group kGroup>
+cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, const Shape& s, const GemmEpilogue& e, int sms,
+                   cudaStream_t st) {
+    // the tile width with the shortest estimated time: full waves of tiles, wide tiles being cheaper per column
+    const int tm = (s.T + kBM - 1) / kBM;
+    auto cost = [&](int bn, float per_tile) {
+        const int wide = kGroup == Group::kSilu ? bn / 2 : bn, tiles = tm * ((s.N + wide - 1) / wide);
+        return ((tiles + sms - 1) / sms) * per_tile;
+    };
+    const float c256 = cost(256, 1.f), c128 = cost(128, 0.56f), c64 = cost(64, 0.36f);
+    if (c256 <= c128 && c256 <= c64) return launch<256, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    if (c128 <= c64) return launch<128, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    return launch<64, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
 }
 
 }  // namespace
 
 cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, int T, int N, int K, const GemmEpilogue& e,
-                      int* status, cudaStream_t st) {
+                      int* status, cudaStream_t st, const bf16* W2) {
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;
@@ -212,17 +266,12 @@ cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, in
         if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (err != cudaSuccess) return err;
     }
-    Shape s{T, N, K, 0, 0, 2000000000ull, status};
-    // the tile width with the shortest estimated time: full waves of tiles, wide tiles being cheaper per column
-    const int tm = (T + kBM - 1) / kBM;
-    auto cost = [&](int bn, float per_tile) {
-        const int tiles = tm * ((N + bn - 1) / bn);
-        return ((tiles + sms - 1) / sms) * per_tile;
-    };
-    const float c256 = cost(256, 1.f), c128 = cost(128, 0.56f), c64 = cost(64, 0.36f);
-    if (c256 <= c128 && c256 <= c64) return launch<256>(A, lda, W, ldw, s, e, sms, st);
-    if (c128 <= c64) return launch<128>(A, lda, W, ldw, s, e, sms, st);
-    return launch<64>(A, lda, W, ldw, s, e, sms, st);
+    const Shape s{T, N, K, 0, 0, 2000000000ull, status};
+    switch (group_of(e.what)) {
+        case Group::kSilu: return choose<Group::kSilu>(A, lda, W, W2, ldw, s, e, sms, st);
+        case Group::kRope: return choose<Group::kRope>(A, lda, W, W2, ldw, s, e, sms, st);
+        default: return choose<Group::kPlain>(A, lda, W, W2, ldw, s, e, sms, st);
+    }
 }
 
 }  // namespace mkbh

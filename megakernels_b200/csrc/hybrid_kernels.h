@@ -10,6 +10,15 @@ enum class Result {
     kAdd,    // out[t, n] += scale[n] * acc (the residual stream)
     kCast,   // cast[t, n] = acc in the model dtype
     kGlu,    // cast[t, n / 2] = clamped gated unit of columns n (gate) and n + 1
+    kSilu,   // cast[t, n] = silu(gate[n]) * up[n], two weight matrices (bf16 only)
+    kRope,   // queries, keys and values to their places, the first two rotated (bf16 only)
+};
+// Where kRope puts a row of [queries | keys | values]: the keys and values of token t are row pos0 + t of
+// caches [position, key columns].  Neighbours (2i, 2i + 1) of a head are turned by the tables [position, dim].
+struct RopeTarget {
+    bf16 *q, *k, *v;
+    int q_cols, k_cols, dim, pos0;
+    const float *cos, *sin;
 };
 struct GemmEpilogue {
     Result what;
@@ -19,17 +28,31 @@ struct GemmEpilogue {
     const float* bias;   // kStore; may be NULL
     const float* scale;  // kAdd; NULL: 1
     float limit, alpha;  // kGlu
+    RopeTarget rope;     // kRope
     static GemmEpilogue store(float* out, int64_t ld, const float* bias) { return {Result::kStore, out, nullptr, ld, bias, nullptr, 0.f, 0.f}; }
     static GemmEpilogue add(float* out, int64_t ld, const float* scale) { return {Result::kAdd, out, nullptr, ld, nullptr, scale, 0.f, 0.f}; }
     static GemmEpilogue to(void* out, int64_t ld) { return {Result::kCast, nullptr, out, ld, nullptr, nullptr, 0.f, 0.f}; }
     static GemmEpilogue glu(void* out, int64_t ld, float limit, float alpha) { return {Result::kGlu, nullptr, out, ld, nullptr, nullptr, limit, alpha}; }
+    static GemmEpilogue silu(void* out, int64_t ld) { return {Result::kSilu, nullptr, out, ld, nullptr, nullptr, 0.f, 0.f}; }
+    static GemmEpilogue rotate(const RopeTarget& r) { return {Result::kRope, nullptr, nullptr, 0, nullptr, nullptr, 0.f, 0.f, r}; }
 };
 
 // out[T, N] from A [T, lda] and W [N, ldw], K columns of both (rows 16-byte aligned)
 cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int T, int N, int K,
                      const GemmEpilogue& e, cudaStream_t s);
 cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, int T, int N, int K,
-                      const GemmEpilogue& e, int* status, cudaStream_t s);
+                      const GemmEpilogue& e, int* status, cudaStream_t s, const bf16* W2 = nullptr);  // W2: kSilu's up rows
+
+// Causal attention of `n` queries from position pos0 on over a cache [position, kv head, dim] that holds
+// their own rows too; dim 64 or 128.  Nothing beyond row pos0 + n - 1 is read.
+struct CacheAttention {
+    const bf16 *q, *k, *v;  // q [n, heads, dim]
+    bf16* out;              // [n, heads, dim]
+    int n, pos0, heads, kv_heads, dim;
+    float scale;
+    int* status;
+};
+cudaError_t flash_cache(const CacheAttention& a, cudaStream_t s);
 
 // prefill kernels (template argument: element type of the model)
 template <typename T>

@@ -67,3 +67,12 @@ def interpret_with_mk(globs: Globals, mk_func, stream=None, **kwargs):
 class LatencyMK_Interpreter(MK_Interpreter):
     def interpret(self, globs: Globals, **kwargs):
         return interpret_with_mk(globs, self.mk_func, **kwargs)
+
+    def prompt(self, globs: Globals, hidden: torch.Tensor, pos0: int, want_logits: bool):
+        """The tokens whose embeddings are ``hidden`` at once, from position ``pos0`` on; no counterpart in the reference."""
+        globs.pos_id = pos0 + hidden.shape[0] - 1
+
+        def call(*args, **kwargs):
+            return self.module.mk_llama_prompt(*args, hidden=hidden, pos0=pos0, want_logits=want_logits, **kwargs)
+
+        return interpret_with_mk(globs, call)

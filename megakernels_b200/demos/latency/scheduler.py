@@ -511,3 +511,27 @@ def split_at_collectives(instructions: list[Instruction]) -> list[tuple[list[Ins
         last = cur[-1].opcode()
         segments.append((cur, last in (O_ProjResidual.opcode(), DownProjResidual.opcode())))
     return segments
+
+
+def covers_model(globs: Globals, instructions: list[Instruction]) -> bool:
+    """Whether a single-sequence instruction list is the model's whole step: every block of every layer and the head."""
+    blocks: dict[tuple[int, int], int] = {}
+    for ins in instructions:
+        op, layer = ins.opcode(), getattr(ins, "layer_idx", 0)
+        if isinstance(ins, LayerNormDoubleMatVecSiLU):
+            n = len(ins.block_idxs)
+        elif isinstance(ins, (O_ProjResidual, DownProjResidual)):
+            n = ins.end_block_idx - ins.start_block_idx
+        elif isinstance(ins, (LayerNorm_QKV_MatVecRopeAppend, RMS_LM_Head)):
+            n = ins.end_output_block_idx - ins.start_output_block_idx
+        else:
+            continue
+        blocks[op, layer] = blocks.get((op, layer), 0) + n
+    rows = (globs.num_attention_heads + 2 * globs.num_kv_heads) * globs.head_dim
+    want = {(RMS_LM_Head.opcode(), 0): globs.vocab_size // globs.lm_head_block_size}
+    for layer in range(globs.num_hidden_layers):
+        want[LayerNorm_QKV_MatVecRopeAppend.opcode(), layer] = rows // globs.qkv_block_size
+        want[O_ProjResidual.opcode(), layer] = globs.hidden_size // globs.o_proj_block_size * globs.num_o_proj_col_splits()
+        want[LayerNormDoubleMatVecSiLU.opcode(), layer] = globs.intermediate_size // globs.up_gate_proj_block_size
+        want[DownProjResidual.opcode(), layer] = globs.hidden_size // globs.down_proj_block_size * globs.num_down_proj_col_splits()
+    return blocks == want

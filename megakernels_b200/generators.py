@@ -12,6 +12,8 @@ from __future__ import annotations
 import torch
 from torch import Tensor
 
+from megakernels_b200.demos.latency.mk import LatencyMK_Interpreter
+from megakernels_b200.demos.latency.scheduler import covers_model
 from megakernels_b200.mk import MK_Interpreter
 from megakernels_b200.model_types import BatchState
 from megakernels_b200.scheduler import Schedule
@@ -92,6 +94,9 @@ class MK_Generator(Generator):
                 globs.batch_size, dtype=torch.int32, device=globs.hidden_states.device
             )
 
+        # prompts need not go token by token when the schedule is the model's whole step
+        self._whole = has_head and globs.batch_size == 1 and covers_model(globs, schedule.get_linear_instructions())
+
     def fill(self):
         """Reset the per-token VM state: barrier counters and residual accumulators."""
         globs = self.schedule.globs
@@ -104,6 +109,7 @@ class MK_Generator(Generator):
 
     def replace_with_noops(self):
         self.schedule.globs.instructions.zero_()
+        self._whole = False
 
     # -- CUDA-graph replay of one decode step -------------------------------- #
     def enable_cuda_graph(self, warmup_pos: int = 0):
@@ -203,15 +209,65 @@ class MK_Generator(Generator):
             output_ids = self.run(input_ids, pos_id=pos_id)
             output_tokens[:, in_pos + 1] = output_ids.reshape(-1)
 
-    def prefill(self, prompt_ids: Tensor) -> Tensor:
-        """Run the prompt through the decode kernel one token at a time.
+    # Tokens of a prompt that go through the layers together: the activations of a portion, 60 KB a token
+    # at the 8B widths, are a workspace of this many tokens.
+    prompt_portion = 2048
 
-        The reference prefills with its torch model (scripts/generate.py:125-137);
-        here the KV cache is filled by the megakernel itself, so no second
-        implementation of the forward pass exists in the product.  Returns the
-        first generated token ``[1]``.
+    def _takes_prompts(self, count: int) -> bool:
+        """Whether a prompt of ``count`` tokens goes through the layers at once (``mkb_prompt``).
+
+        Only where that is the same as a step per token: the whole model's schedule on the library's own
+        interpreter, one sequence on one GPU, no part of a step left out or replaced, every position inside
+        cache and tables.  Shorter prompts cost less as steps.
+        """
+        globs, interp = self.schedule.globs, self.interpreter
+        own = lambda f, cls, name: getattr(f, "__func__", None) is getattr(cls, name)  # noqa: E731
+        return (
+            count >= self.shortest_prompt
+            and self._whole
+            and not (self.skip_mk or self.skip_rest)
+            and self.barrier_fill_val == 0
+            and globs.tp is None
+            and globs.residual_scale == 1.0
+            and globs.residual_acc is not None
+            and globs.hidden_states.is_cuda
+            and count <= globs.k_cache.shape[2]
+            and count <= globs.rope_cos.shape[0]
+            and own(self.run, MK_Generator, "run")
+            and own(self._step, MK_Generator, "_step")
+            and isinstance(interp, LatencyMK_Interpreter)
+            and own(interp.interpret, LatencyMK_Interpreter, "interpret")
+            and hasattr(interp.module, "mk_llama_prompt")
+            and interp.mk_func is interp.module.mk_llama
+        )
+
+    # A step per token costs what the weights' traffic costs, the layers at once that and their launches.
+    shortest_prompt = 4
+
+    def _prompt(self, ids: Tensor) -> Tensor:
+        globs, count = self.schedule.globs, ids.shape[1]
+        for a in range(0, count, self.prompt_portion):
+            b = min(count, a + self.prompt_portion)
+            hidden = self.model.model.embed_tokens(BatchState(input_ids=ids[:, a:b])).hidden_states.reshape(b - a, -1)
+            self.last_call = self.interpreter.prompt(globs, hidden, a, b == count)
+        globs.hidden_states[:] = hidden[-1]
+        if globs.pos_id_device is not None:
+            globs.pos_id_device.fill_(count - 1)
+        token = torch.argmax(globs.logits, dim=-1).reshape(1)
+        if globs.argmax_out is not None:
+            globs.argmax_out.copy_(token)
+        return token
+
+    def prefill(self, prompt_ids: Tensor) -> Tensor:
+        """Fill the KV cache with a prompt; returns the first generated token ``[1]``.
+
+        The reference prefills with its torch model (scripts/generate.py:125-137).  Here the tokens go
+        through the layers at once, in portions, or where that does not apply (``_takes_prompts``) through
+        the decode kernel one at a time.
         """
         ids = prompt_ids.reshape(1, -1)
+        if self._takes_prompts(ids.shape[1]):
+            return self._prompt(ids)
         out = None
         for pos in range(ids.shape[1]):
             out = self.run(ids[:, pos : pos + 1], pos_id=pos)
@@ -248,6 +304,7 @@ class Hybrid_Generator(MK_Generator):
         self.model, self.interpreter, self.schedule = model, interpreter, schedule
         self.skip_mk, self.skip_rest = kw.get("skip_mk", False), kw.get("skip_rest", False)
         self.last_call = None
+        self._whole = False  # (prefill and feed are this class's own)
 
     def fill(self):
         """Nothing to reset: counters are cleared by the launch, recurrent state at position 0."""

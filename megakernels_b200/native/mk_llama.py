@@ -109,6 +109,18 @@ class MkbGlobals(ctypes.Structure):
     ]
 
 
+class MkbPrompt(ctypes.Structure):
+    _fields_ = [
+        ("struct_bytes", ctypes.c_uint32),
+        ("tokens", ctypes.c_int32),
+        ("pos0", ctypes.c_int32),
+        ("want_logits", ctypes.c_int32),
+        ("hidden", ctypes.c_void_p),
+        ("workspace", ctypes.c_void_p),
+        ("workspace_bytes", ctypes.c_size_t),
+    ]
+
+
 class MkbStatus(ctypes.Structure):
     _fields_ = [
         ("code", ctypes.c_int32),
@@ -146,6 +158,10 @@ def load_library() -> ctypes.CDLL:
     lib.mkb_launch.restype = ctypes.c_int
     lib.mkb_launch_no_alloc.argtypes = [ctypes.POINTER(MkbGlobals), ctypes.c_void_p]
     lib.mkb_launch_no_alloc.restype = ctypes.c_int
+    lib.mkb_prompt.argtypes = [ctypes.POINTER(MkbGlobals), ctypes.POINTER(MkbPrompt), ctypes.c_void_p]
+    lib.mkb_prompt.restype = ctypes.c_int
+    lib.mkb_prompt_bytes.argtypes = [ctypes.POINTER(MkbGlobals), ctypes.c_int32]
+    lib.mkb_prompt_bytes.restype = ctypes.c_size_t
     lib.mkb_sync_status.argtypes = [
         ctypes.POINTER(MkbGlobals),
         ctypes.c_void_p,
@@ -458,6 +474,30 @@ def mk_llama(
         normed_states=normed_states,
     )
     rc = lib.mkb_launch(ctypes.byref(g), ctypes.c_void_p(_stream_handle(stream)))
+    if rc != 0:
+        raise MegakernelError(rc, lib.mkb_last_error().decode())
+    return g
+
+
+def mk_llama_prompt(*args, hidden, pos0, want_logits, stream=None, **kw):
+    """Enqueue a prompt's tokens at once (``mkb_prompt``); other arguments as :func:`mk_llama`.
+
+    ``hidden`` holds their embeddings ``[tokens, H]``, the first of position ``pos0``; ``pos_id`` is the
+    last one's position.  Keys and values go to the caches, the last token's logits (``want_logits``) to ``logits``.
+    """
+    lib = load_library()
+    g = pack_globals(*args, **kw)
+    p = MkbPrompt()
+    p.struct_bytes = ctypes.sizeof(MkbPrompt)
+    p.hidden = _check_tensor("hidden", hidden, torch.bfloat16, 2)
+    if hidden.shape[1] != g.hidden_size:
+        raise ValueError(f"hidden must be [tokens, {g.hidden_size}], got {tuple(hidden.shape)}")
+    p.tokens, p.pos0, p.want_logits = hidden.shape[0], pos0, int(want_logits)
+    p.workspace_bytes = lib.mkb_prompt_bytes(ctypes.byref(g), p.tokens)
+    # (allocated on the current stream, which has to be the one that is launched on)
+    workspace = torch.empty(p.workspace_bytes, dtype=torch.uint8, device=hidden.device)
+    p.workspace = workspace.data_ptr()
+    rc = lib.mkb_prompt(ctypes.byref(g), ctypes.byref(p), ctypes.c_void_p(_stream_handle(stream)))
     if rc != 0:
         raise MegakernelError(rc, lib.mkb_last_error().decode())
     return g
