@@ -408,7 +408,7 @@ struct ScanToken {
 };
 
 template <int M>
-__global__ void __launch_bounds__(kScanThreads, 1)
+__global__ void __launch_bounds__(kScanThreads, M <= 2 ? 2 : 1)
 delta_scan_kernel(const float* __restrict__ proj, int64_t ld, int n, int heads, int dim, const float* __restrict__ decay,
                   const float* __restrict__ ab, float* __restrict__ state, int fresh, float* __restrict__ out) {
     constexpr int DP = 32 * M, TC = scan_tokens<M>(), BUF = scan_buf<M>();
