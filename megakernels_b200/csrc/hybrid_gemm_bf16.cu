@@ -2,7 +2,7 @@
 // out[token, feature] = sum_k A[token, k] * W[feature, k], fp32 accumulation in tensor memory.
 //
 // Persistent, warp-specialised: one producer thread (TMA, 128-byte swizzle), one MMA thread
-// (tcgen05.mma, M = 128 tokens, N = kBN features), four epilogue warps that read one of two
+// (tcgen05.mma, M = 128 tokens per CTA, N = kBN features), four epilogue warps that read one of two
 // accumulators back while the other is being filled.  The epilogue goes through shared memory so
 // that stores are row segments: plus the bias, times the layer scale into the 32-bit residual stream,
 // in bf16, the gated unit of neighbouring columns in bf16, the gated unit of two matrices (a tile is then
@@ -17,10 +17,12 @@ constexpr int kBM = 128, kBK = 64;
 constexpr int kGemmThreads = 192;
 constexpr int kEpiStride = 33;  // floats per row of a warp's 32 x 32 transpose buffer
 
-template <int kBN>
+// kPair CTAs work on one tile: 128 tokens each, the features' operand halved between them.
+template <int kBN, int kPair>
 struct Geo {
-    static constexpr int kStageBytes = (kBM + kBN) * kBK * 2;
-    static constexpr int kStages = kBN == 256 ? 4 : kBN == 128 ? 6 : 8;
+    static constexpr int kRowsW = kBN / kPair;
+    static constexpr int kStageBytes = (kBM + kRowsW) * kBK * 2;
+    static constexpr int kStages = kRowsW == 256 ? 4 : kRowsW == 128 ? 6 : 8;
     static constexpr int kEpi = kStages * kStageBytes;
     static constexpr int kBars = kEpi + 4 * 32 * kEpiStride * 4;
     static constexpr int kNumBars = 2 * kStages + 4;
@@ -40,16 +42,18 @@ struct Shape {
 enum class Group { kPlain, kSilu, kRope };  // kSilu: two weight matrices, kBN / 2 columns of each per tile
 constexpr Group group_of(Result r) { return r == Result::kSilu ? Group::kSilu : r == Result::kRope ? Group::kRope : Group::kPlain; }
 
-template <int kBN, Group kGroup>
+template <int kBN, int kPair, Group kGroup>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap,
                  const __grid_constant__ CUtensorMap wmap2, const Shape s, const GemmEpilogue e) {
-    using G = Geo<kBN>;
+    using G = Geo<kBN, kPair>;
     extern __shared__ uint8_t raw[];
     const uint32_t raw32 = mkb::smem_u32(raw), base = (raw32 + 1023u) & ~1023u;
     uint8_t* gbase = raw + (base - raw32);
     volatile int* ctl = reinterpret_cast<volatile int*>(gbase + G::kCtl);  // [0] dead, [1] tensor-memory base
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = kPair == 2 ? tc_rank() : 0u;
+    const int worker = blockIdx.x / kPair, workers = gridDim.x / kPair;  // (a pair's CTAs are neighbours)
     auto full = [&](int i) { return base + G::kBars + i * 8; };
     auto empty = [&](int i) { return base + G::kBars + (G::kStages + i) * 8; };
     auto acc_full = [&](int i) { return base + G::kBars + (2 * G::kStages + i) * 8; };
@@ -62,20 +66,28 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         }
         for (int i = 0; i < 2; ++i) {
             mkb::mbar_init(acc_full(i), 1);
-            mkb::mbar_init(acc_empty(i), 4);
+            mkb::mbar_init(acc_empty(i), 4 * kPair);
         }
         ctl[0] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(base + G::kCtl + 4),
-                     "r"((uint32_t)(2 * kBN))
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (kPair == 2) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(base + G::kCtl + 4),
+                         "r"((uint32_t)(2 * kBN))
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(base + G::kCtl + 4),
+                         "r"((uint32_t)(2 * kBN))
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (kPair == 2) tc_cluster_sync();  // (the other CTA's barriers are there)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = (uint32_t)ctl[1];
     constexpr bool kDual = kGroup == Group::kSilu;
@@ -85,29 +97,39 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     if (warp == 0 && lane == 0) {
         uint32_t it = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < s.tiles && ok; tile += gridDim.x) {
-            const int m0 = (tile % s.tiles_m) * kBM, n0 = (tile / s.tiles_m) * wide;
+        for (int tile = worker; tile < s.tiles && ok; tile += workers) {
+            const int m0 = ((tile % s.tiles_m) * kPair + rank) * kBM, n0 = (tile / s.tiles_m) * wide;
             for (int k = 0; k < ksteps; ++k, ++it) {
                 const int st = it % G::kStages;
                 if (!tc_wait(empty(st), ((it / G::kStages) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 0)) {
                     ok = false;
                     break;
                 }
-                const uint32_t dst = base + st * G::kStageBytes;
-                mkb::mbar_expect_tx(full(st), G::kStageBytes);
-                tc_tma_2d(dst, &amap, k * kBK, m0, full(st));
-                tc_tma_2d(dst + kBM * kBK * 2, &wmap, k * kBK, n0, full(st));
-                if (kDual) tc_tma_2d(dst + (kBM + kBN / 2) * kBK * 2, &wmap2, k * kBK, n0, full(st));
+                const uint32_t dst = base + st * G::kStageBytes, dw = dst + kBM * kBK * 2;
+                if (rank == 0) mkb::mbar_expect_tx(full(st), kPair * G::kStageBytes);
+                if constexpr (kPair == 2) {  // both CTAs' copies count on the first one's barrier
+                    const uint32_t bar = tc_peer(full(st), 0);
+                    tc_tma_2d_pair(dst, &amap, k * kBK, m0, bar);
+                    if (kDual) tc_tma_2d_pair(dw, rank ? &wmap2 : &wmap, k * kBK, n0, bar);
+                    else tc_tma_2d_pair(dw, &wmap, k * kBK, n0 + rank * G::kRowsW, bar);
+                } else {
+                    tc_tma_2d(dst, &amap, k * kBK, m0, full(st));
+                    tc_tma_2d(dw, &wmap, k * kBK, n0, full(st));
+                    if (kDual) tc_tma_2d(dw + kBN / 2 * kBK * 2, &wmap2, k * kBK, n0, full(st));
+                }
             }
         }
-        // no copy may be in flight when the CTA's shared memory goes away
-        for (uint32_t i = it > (uint32_t)G::kStages ? it - G::kStages : 0u; i < it; ++i)
-            tc_wait(full(i % G::kStages), (i / G::kStages) & 1u, nullptr, s.timeout_ns, s.status, 0);
-    } else if (warp == 1 && lane == 0) {
-        const uint32_t idesc = tc_idesc(kBM, kBN);
+        // no copy may be in flight when the CTA's shared memory goes away, nor an arrival from the pair's first CTA
+        const uint32_t last = it > (uint32_t)G::kStages ? it - G::kStages : 0u;
+        for (uint32_t i = last; i < it; ++i) {
+            if (ok) tc_wait(empty(i % G::kStages), (i / G::kStages) & 1u, ctl, s.timeout_ns, s.status, 0);
+            else if (rank == 0) tc_wait(full(i % G::kStages), (i / G::kStages) & 1u, nullptr, s.timeout_ns, s.status, 0);
+        }
+    } else if (warp == 1 && lane == 0 && rank == 0) {
+        const uint32_t idesc = tc_idesc(kPair * kBM, kBN);
         uint32_t it = 0, acc = 0;
         bool ok = true;
-        for (int tile = blockIdx.x; tile < s.tiles && ok; tile += gridDim.x, ++acc) {
+        for (int tile = worker; tile < s.tiles && ok; tile += workers, ++acc) {
             const uint32_t buf = acc & 1u;
             ok = tc_wait(acc_empty(buf), ((acc >> 1) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 1);
             if (!ok) break;
@@ -120,17 +142,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                 const uint32_t a = base + st * G::kStageBytes, w = a + kBM * kBK * 2;
 #pragma unroll
                 for (int kk = 0; kk < kBK / 16; ++kk)
-                    tc_mma(tmem + buf * kBN, tc_desc(a + kk * 32), tc_desc(w + kk * 32), idesc, (uint32_t)((k | kk) != 0));
-                tc_commit(empty(st));
+                    if constexpr (kPair == 2) tc_mma_pair(tmem + buf * kBN, tc_desc(a + kk * 32), tc_desc(w + kk * 32), idesc, (uint32_t)((k | kk) != 0));
+                    else tc_mma(tmem + buf * kBN, tc_desc(a + kk * 32), tc_desc(w + kk * 32), idesc, (uint32_t)((k | kk) != 0));
+                if constexpr (kPair == 2) tc_commit_pair(empty(st));
+                else tc_commit(empty(st));
             }
-            if (ok) tc_commit(acc_full(buf));
+            if (!ok) break;
+            if constexpr (kPair == 2) tc_commit_pair(acc_full(buf));
+            else tc_commit(acc_full(buf));
         }
     } else if (warp >= 2) {
         const int q = warp & 3;  // the quarter of tensor memory's lanes this warp may read
         float* tr = reinterpret_cast<float*>(gbase + G::kEpi) + (warp - 2) * 32 * kEpiStride;
         uint32_t acc = 0;
-        for (int tile = blockIdx.x; tile < s.tiles; tile += gridDim.x, ++acc) {
-            const int m0 = (tile % s.tiles_m) * kBM + q * 32, n0 = (tile / s.tiles_m) * wide;
+        for (int tile = worker; tile < s.tiles; tile += workers, ++acc) {
+            const int m0 = ((tile % s.tiles_m) * kPair + rank) * kBM + q * 32, n0 = (tile / s.tiles_m) * wide;
             const uint32_t buf = acc & 1u;
             const bool ok = tc_wait(acc_full(buf), (acc >> 1) & 1u, ctl, s.timeout_ns, s.status, 2);
             if (!__all_sync(0xffffffffu, ok)) break;
@@ -205,54 +231,77 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mkb::mbar_arrive(acc_empty(buf));
+            if (lane == 0) {
+                if constexpr (kPair == 2) tc_arrive_cluster(tc_peer(acc_empty(buf), 0));
+                else mkb::mbar_arrive(acc_empty(buf));
+            }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 1)
+    if constexpr (kPair == 2) {
+        tc_cluster_sync();
+        if (warp == 1)
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * kBN)) : "memory");
+    } else if (warp == 1) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)(2 * kBN)) : "memory");
+    }
 }
 
-template <int kBN, Group kGroup>
+template <int kBN, int kPair, Group kGroup>
 cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, Shape s, const GemmEpilogue& e,
                    int sms, cudaStream_t st) {
-    using G = Geo<kBN>;
+    using G = Geo<kBN, kPair>;
     static bool set[64] = {};
+    const auto kernel = gemm_bf16_kernel<kBN, kPair, kGroup>;
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
     if (!set[dev & 63]) {
-        err = cudaFuncSetAttribute(gemm_bf16_kernel<kBN, kGroup>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kAlloc);
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kAlloc);
         if (err != cudaSuccess) return err;
         set[dev & 63] = true;
     }
     CUtensorMap amap, wmap, wmap2;
     constexpr bool kDual = kGroup == Group::kSilu;
-    constexpr int wide = kDual ? kBN / 2 : kBN;
+    constexpr int wide = kDual ? kBN / 2 : kBN, box = kPair == 2 ? kBN / 2 : wide;
     if ((err = tc_map(&amap, A, s.K, s.T, lda, kBK, kBM)) != cudaSuccess) return err;
-    if ((err = tc_map(&wmap, W, s.K, s.N, ldw, kBK, wide)) != cudaSuccess) return err;
+    if ((err = tc_map(&wmap, W, s.K, s.N, ldw, kBK, box)) != cudaSuccess) return err;
     wmap2 = wmap;
-    if (kDual && (err = tc_map(&wmap2, W2, s.K, s.N, ldw, kBK, wide)) != cudaSuccess) return err;
-    s.tiles_m = (s.T + kBM - 1) / kBM;
+    if (kDual && (err = tc_map(&wmap2, W2, s.K, s.N, ldw, kBK, box)) != cudaSuccess) return err;
+    s.tiles_m = (s.T + kPair * kBM - 1) / (kPair * kBM);
     s.tiles = s.tiles_m * ((s.N + wide - 1) / wide);
-    gemm_bf16_kernel<kBN, kGroup><<<s.tiles < sms ? s.tiles : sms, kGemmThreads, G::kAlloc, st>>>(amap, wmap, wmap2, s, e);
-    return cudaGetLastError();
+    const int workers = s.tiles < sms / kPair ? s.tiles : sms / kPair;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(workers * kPair);
+    c.blockDim = dim3(kGemmThreads);
+    c.dynamicSmemBytes = G::kAlloc;
+    c.stream = st;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = kPair;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    c.attrs = &cluster;
+    c.numAttrs = kPair > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, amap, wmap, wmap2, s, e);
 }
 
 template <Group kGroup>
 cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, const Shape& s, const GemmEpilogue& e, int sms,
                    cudaStream_t st) {
-    // the tile width with the shortest estimated time: full waves of tiles, wide tiles being cheaper per column
-    const int tm = (s.T + kBM - 1) / kBM;
-    auto cost = [&](int bn, float per_tile) {
-        const int wide = kGroup == Group::kSilu ? bn / 2 : bn, tiles = tm * ((s.N + wide - 1) / wide);
-        return ((tiles + sms - 1) / sms) * per_tile;
+    // the tile with the shortest estimated time: full waves of tiles, wide tiles being cheaper per column
+    auto cost = [&](int bn, int pair, float per_tile) {
+        const int wide = kGroup == Group::kSilu ? bn / 2 : bn, tm = (s.T + pair * kBM - 1) / (pair * kBM);
+        const int tiles = tm * ((s.N + wide - 1) / wide), workers = sms / pair;
+        return ((tiles + workers - 1) / workers) * per_tile;
     };
-    const float c256 = cost(256, 1.f), c128 = cost(128, 0.56f), c64 = cost(64, 0.36f);
-    if (c256 <= c128 && c256 <= c64) return launch<256, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
-    if (c128 <= c64) return launch<128, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
-    return launch<64, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    const float p256 = cost(256, 2, 0.7f), p128 = cost(128, 2, 0.46f);
+    const float c256 = cost(256, 1, 1.f), c128 = cost(128, 1, 0.56f), c64 = cost(64, 1, 0.36f), least = fminf(fminf(c256, c128), c64);
+    if (p256 <= p128 && p256 <= least) return launch<256, 2, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    if (p128 <= least) return launch<128, 2, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    if (c256 <= c128 && c256 <= c64) return launch<256, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    if (c128 <= c64) return launch<128, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    return launch<64, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
 }
 
 }  // namespace

@@ -255,6 +255,34 @@ int mkb_hybrid_decode(const MkbhGlobals* gp, void* stream) {
     return MKBH_OK;
 }
 
+int mkb_hybrid_product(const MkbhProduct* p, void* stream) {
+    REQUIRE(p && p->struct_bytes == sizeof(MkbhProduct), "product: NULL or another struct size");
+    const bool f32 = p->dtype == MKBH_F32;
+    const int64_t unit = f32 ? 4 : 8;  // elements of 16 bytes
+    REQUIRE(f32 || p->dtype == MKBH_BF16, "product: unknown dtype %d", p->dtype);
+    REQUIRE(p->tokens > 0 && p->features > 0 && p->inner > 0 && p->tokens <= 65535 * 16, "product: empty or too large");
+    REQUIRE(p->a && p->w && p->out && p->status, "product: missing pointers");
+    REQUIRE(p->result >= MKBH_STORE && p->result <= MKBH_SILU && (p->result != MKBH_SILU || (!f32 && p->w2)), "product: result %d", p->result);
+    REQUIRE(p->result != MKBH_GLU || p->features % 2 == 0, "product: %d features are no pairs", p->features);
+    REQUIRE(p->lda % unit == 0 && p->ldw % unit == 0 && p->lda >= p->inner && p->ldw >= p->inner &&
+                p->ldo >= (p->result == MKBH_GLU ? p->features / 2 : p->features),
+            "product: rows");
+    REQUIRE(((uintptr_t)p->a & 15) == 0 && ((uintptr_t)p->w & 15) == 0 && ((uintptr_t)p->w2 & 15) == 0 && ((uintptr_t)p->out & 3) == 0,
+            "product: alignment");
+    // bf16 results leave in pairs
+    REQUIRE(f32 || p->result < MKBH_CAST || p->result == MKBH_GLU || p->ldo % 2 == 0, "product: rows of an odd length");
+    GemmEpilogue e = GemmEpilogue::store(static_cast<float*>(p->out), p->ldo, p->bias);
+    if (p->result == MKBH_ADD) e = GemmEpilogue::add(static_cast<float*>(p->out), p->ldo, p->scale);
+    if (p->result == MKBH_CAST) e = GemmEpilogue::to(p->out, p->ldo);
+    if (p->result == MKBH_GLU) e = GemmEpilogue::glu(p->out, p->ldo, p->limit, p->alpha);
+    if (p->result == MKBH_SILU) e = GemmEpilogue::silu(p->out, p->ldo);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (f32) MKBH_TRY(gemm_f32(static_cast<const float*>(p->a), p->lda, static_cast<const float*>(p->w), p->ldw, p->tokens, p->features, p->inner, e, s));
+    else MKBH_TRY(gemm_bf16(static_cast<const bf16*>(p->a), p->lda, static_cast<const bf16*>(p->w), p->ldw, p->tokens, p->features, p->inner, e,
+                            p->status, s, static_cast<const bf16*>(p->w2)));
+    return MKBH_OK;
+}
+
 int mkb_hybrid_validate(const MkbhGlobals* gp, const int32_t* ins) {
     if (int rc = check_globals(gp)) return rc;
     const MkbhGlobals& g = *gp;

@@ -102,6 +102,27 @@ def load_library() -> ctypes.CDLL:
     return lib
 
 
+class MkbhProduct(ctypes.Structure):
+    _fields_ = (
+        [("struct_bytes", ctypes.c_uint32)]
+        + [(n, ctypes.c_int32) for n in ("dtype", "result", "tokens", "features", "inner")]
+        + [(n, ctypes.c_int64) for n in ("lda", "ldw", "ldo")]
+        + [(n, ctypes.c_void_p) for n in ("a", "w", "w2", "bias", "scale")]
+        + [("limit", ctypes.c_float), ("alpha", ctypes.c_float), ("out", ctypes.c_void_p), ("status", ctypes.c_void_p)]
+    )
+
+
+RESULTS = ("store", "add", "cast", "glu", "silu")
+
+
+def product(result: str, a, w, out, status, inner: int, w2=None, bias=None, scale=None, limit=0.0, alpha=0.0) -> None:
+    """One matrix product of the prefill on the current stream (``mkb_hybrid_product``): ``a`` [tokens, lda],
+    ``w`` [features, ldw], the first ``inner`` columns of both."""
+    p = MkbhProduct(ctypes.sizeof(MkbhProduct), 1 if a.dtype == torch.float32 else 0, RESULTS.index(result), a.shape[0], w.shape[0], inner,
+                    a.stride(0), w.stride(0), out.stride(0), _p(a), _p(w), _p(w2), _p(bias), _p(scale), limit, alpha, _p(out), _p(status))
+    _raise(load_library().mkb_hybrid_product(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+
+
 def _raise(code: int) -> None:
     if code:
         raise HybridKernelError(code, load_library().mkb_hybrid_last_error().decode())
