@@ -33,19 +33,59 @@ struct Geo {
 };
 
 struct Shape {
-    int T, N, K, tiles_m, tiles;
+    int T, N, K, tiles_m, tiles, parts;  // parts: CTAs that share a tile's inner dimension
     unsigned long long timeout_ns;
     int* status;
 };
 
 // What the epilogue can do: a build per group of results, so that one group's code does not cost the others registers.
 enum class Group { kPlain, kSilu, kRope };  // kSilu: two weight matrices, kBN / 2 columns of each per tile
+template <int kBN> constexpr int kPartRow = kBN + 4;  // floats of a row of partial sums
 constexpr Group group_of(Result r) { return r == Result::kSilu ? Group::kSilu : r == Result::kRope ? Group::kRope : Group::kPlain; }
 
-template <int kBN, int kPair, Group kGroup>
+// columns n (even) and n + 1 of token t, where a thread has just these
+template <Group kGroup>
+__device__ __forceinline__ void put(const GemmEpilogue& e, int N, int t, int n, float x, float y) {
+    if (n >= N) return;
+    if constexpr (kGroup == Group::kRope) {
+        const RopeTarget& p = e.rope;
+        const int at = n - p.q_cols;  // column of [keys | values]
+        if (at < p.k_cols) {
+            const size_t z = (size_t)(p.pos0 + t) * p.dim + n % p.dim;
+            const float2 c = __ldg(reinterpret_cast<const float2*>(p.cos + z)), d = __ldg(reinterpret_cast<const float2*>(p.sin + z));
+            const float turned = x * c.x - y * d.x;
+            y = y * c.y + x * d.y;
+            x = turned;
+        }
+        bf16* o = at < 0 ? p.q + (size_t)t * p.q_cols + n : (at < p.k_cols ? p.k + at : p.v + (at - p.k_cols)) + (size_t)(p.pos0 + t) * p.k_cols;
+        *reinterpret_cast<uint32_t*>(o) = mkb::pack_bf16x2(x, y);
+    } else if (kGroup == Group::kSilu || e.what == Result::kCast) {
+        bf16* o = static_cast<bf16*>(e.cast) + (size_t)t * e.ld + n;
+        if (n + 1 < N) *reinterpret_cast<uint32_t*>(o) = mkb::pack_bf16x2(x, y);
+        else *o = __float2bfloat16_rn(x);
+    } else if (e.what == Result::kGlu) {  // (N is even)
+        static_cast<bf16*>(e.cast)[(size_t)t * e.ld + n / 2] = __float2bfloat16_rn(clamped_glu(x, y, e.limit, e.alpha));
+    } else {
+        float* o = e.out + (size_t)t * e.ld + n;
+        const bool two = n + 1 < N;
+        if (e.what == Result::kAdd) {  // (no other thread writes these)
+            o[0] += (e.scale ? __ldg(e.scale + n) : 1.f) * x;
+            if (two) o[1] += (e.scale ? __ldg(e.scale + n + 1) : 1.f) * y;
+        } else {
+            o[0] = x + (e.bias ? __ldg(e.bias + n) : 0.f);
+            if (two) o[1] = y + (e.bias ? __ldg(e.bias + n + 1) : 0.f);
+        }
+    }
+}
+
+// kMode 1: a CTA per tile; 2: a pair of CTAs (cta_group::2) per tile; 0: s.parts CTAs, a cluster, share a tile's
+// inner dimension and add up their accumulators through distributed shared memory, always in the same order.
+template <int kBN, int kMode, Group kGroup>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap wmap,
                  const __grid_constant__ CUtensorMap wmap2, const Shape s, const GemmEpilogue e) {
+    constexpr int kPair = kMode == 2 ? 2 : 1;
+    constexpr bool kShare = kMode == 0;
     using G = Geo<kBN, kPair>;
     extern __shared__ uint8_t raw[];
     const uint32_t raw32 = mkb::smem_u32(raw), base = (raw32 + 1023u) & ~1023u;
@@ -53,7 +93,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     volatile int* ctl = reinterpret_cast<volatile int*>(gbase + G::kCtl);  // [0] dead, [1] tensor-memory base
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = kPair == 2 ? tc_rank() : 0u;
-    const int worker = blockIdx.x / kPair, workers = gridDim.x / kPair;  // (a pair's CTAs are neighbours)
+    const int worker = blockIdx.x / (kShare ? s.parts : kPair), workers = gridDim.x / (kShare ? s.parts : kPair);  // (a pair's CTAs are neighbours)
     auto full = [&](int i) { return base + G::kBars + i * 8; };
     auto empty = [&](int i) { return base + G::kBars + (G::kStages + i) * 8; };
     auto acc_full = [&](int i) { return base + G::kBars + (2 * G::kStages + i) * 8; };
@@ -92,7 +132,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     const uint32_t tmem = (uint32_t)ctl[1];
     constexpr bool kDual = kGroup == Group::kSilu;
     constexpr int wide = kDual ? kBN / 2 : kBN;
-    const int ksteps = (s.K + kBK - 1) / kBK;
+    int ksteps = (s.K + kBK - 1) / kBK, kfirst = 0;
+    if constexpr (kShare) {
+        const int r = (int)tc_rank(), end = ksteps * (r + 1) / s.parts;  // (at least one step: parts <= steps)
+        kfirst = ksteps * r / s.parts;
+        ksteps = end - kfirst;
+    }
 
     if (warp == 0 && lane == 0) {
         uint32_t it = 0;
@@ -113,9 +158,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                     if (kDual) tc_tma_2d_pair(dw, rank ? &wmap2 : &wmap, k * kBK, n0, bar);
                     else tc_tma_2d_pair(dw, &wmap, k * kBK, n0 + rank * G::kRowsW, bar);
                 } else {
-                    tc_tma_2d(dst, &amap, k * kBK, m0, full(st));
-                    tc_tma_2d(dw, &wmap, k * kBK, n0, full(st));
-                    if (kDual) tc_tma_2d(dw + kBN / 2 * kBK * 2, &wmap2, k * kBK, n0, full(st));
+                    const int kx = (kfirst + k) * kBK;
+                    tc_tma_2d(dst, &amap, kx, m0, full(st));
+                    tc_tma_2d(dw, &wmap, kx, n0, full(st));
+                    if (kDual) tc_tma_2d(dw + kBN / 2 * kBK * 2, &wmap2, kx, n0, full(st));
                 }
             }
         }
@@ -162,7 +208,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             if (!__all_sync(0xffffffffu, ok)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int rows = min(32, s.T - m0);
-            for (int c0 = 0; c0 < wide; c0 += 32) {
+            if constexpr (kShare) {  // the ring's copies have arrived and been read: the accumulators take its place
+                for (int c0 = 0; c0 < kBN; c0 += 32) {
+                    uint32_t r[32];
+                    tc_load32(tmem + ((uint32_t)(q * 32) << 16) + c0, r);
+                    float4* o = reinterpret_cast<float4*>(gbase) + ((q * 32 + lane) * kPartRow<kBN> + c0) / 4;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        o[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                                           __uint_as_float(r[4 * j + 3]));
+                }
+            } else for (int c0 = 0; c0 < wide; c0 += 32) {
                 if (n0 + c0 >= s.N || rows <= 0) break;  // uniform over the warp
                 uint32_t r[32];
                 tc_load32(tmem + ((uint32_t)(q * 32) << 16) + buf * kBN + c0, r);
@@ -239,6 +295,31 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (kShare) {
+        tc_cluster_sync();
+        const int m0 = (worker % s.tiles_m) * kBM, n0 = (worker / s.tiles_m) * wide, rows = min(kBM, s.T - m0);
+        const uint32_t me = tc_rank(), parts = s.parts;
+        for (int i = (int)me + (int)parts * warp; i < rows; i += (int)parts * (kGemmThreads / 32))
+#pragma unroll 1
+            for (int c = 2 * lane; c < wide; c += 64) {
+                float x = 0.f, y = 0.f, ux = 0.f, uy = 0.f;
+#pragma unroll 4
+                for (uint32_t z = 0; z < parts; ++z) {
+                    const uint32_t at = tc_peer(base + (uint32_t)(i * kPartRow<kBN> + c) * 4, z);
+                    const float2 v = tc_peer_load2(at);
+                    x += v.x;
+                    y += v.y;
+                    if constexpr (kDual) {
+                        const float2 u = tc_peer_load2(at + wide * 4);
+                        ux += u.x;
+                        uy += u.y;
+                    }
+                }
+                if constexpr (kDual) x *= sigmoid_f(x) * ux, y *= sigmoid_f(y) * uy;
+                put<kGroup>(e, s.N, m0 + i, n0 + c, x, y);
+            }
+        tc_cluster_sync();
+    }
     if constexpr (kPair == 2) {
         tc_cluster_sync();
         if (warp == 1)
@@ -248,12 +329,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     }
 }
 
-template <int kBN, int kPair, Group kGroup>
+template <int kBN, int kMode, Group kGroup>
 cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, Shape s, const GemmEpilogue& e,
                    int sms, cudaStream_t st) {
+    constexpr int kPair = kMode == 2 ? 2 : 1;
     using G = Geo<kBN, kPair>;
+    static_assert(kMode != 0 || kBM * kPartRow<kBN> * 4 <= G::kEpi, "");
     static bool set[64] = {};
-    const auto kernel = gemm_bf16_kernel<kBN, kPair, kGroup>;
+    const auto kernel = gemm_bf16_kernel<kBN, kMode, kGroup>;
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess) return err;
@@ -271,37 +354,60 @@ cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
     if (kDual && (err = tc_map(&wmap2, W2, s.K, s.N, ldw, kBK, box)) != cudaSuccess) return err;
     s.tiles_m = (s.T + kPair * kBM - 1) / (kPair * kBM);
     s.tiles = s.tiles_m * ((s.N + wide - 1) / wide);
-    const int workers = s.tiles < sms / kPair ? s.tiles : sms / kPair;
+    const int workers = kMode == 0 || s.tiles < sms / kPair ? s.tiles : sms / kPair, ctas = kMode == 0 ? s.parts : kPair;
     cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(workers * kPair);
+    c.gridDim = dim3(workers * ctas);
     c.blockDim = dim3(kGemmThreads);
     c.dynamicSmemBytes = G::kAlloc;
     c.stream = st;
     cudaLaunchAttribute cluster;
     cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = kPair;
+    cluster.val.clusterDim.x = ctas;
     cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
     c.attrs = &cluster;
-    c.numAttrs = kPair > 1 ? 1 : 0;
+    c.numAttrs = ctas > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&c, kernel, amap, wmap, wmap2, s, e);
 }
 
 template <Group kGroup>
-cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, const Shape& s, const GemmEpilogue& e, int sms,
+cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, Shape s, const GemmEpilogue& e, int sms,
                    cudaStream_t st) {
-    // the tile with the shortest estimated time: full waves of tiles, wide tiles being cheaper per column
-    auto cost = [&](int bn, int pair, float per_tile) {
-        const int wide = kGroup == Group::kSilu ? bn / 2 : bn, tm = (s.T + pair * kBM - 1) / (pair * kBM);
-        const int tiles = tm * ((s.N + wide - 1) / wide), workers = sms / pair;
-        return ((tiles + workers - 1) / workers) * per_tile;
+    // The tile with the shortest estimated time, in us, fitted to 60 shapes of 16..2048 tokens x 2048..28672 features x
+    // 512..14336 (cold caches): waves of tiles, each so many steps of the inner dimension, and the last epilogue.  A step
+    // of a narrow tile costs nearly what a wide one does, so few narrow tiles with a long inner dimension are shared:
+    // 61 x 2048 x 8192 takes 45 us as 32 tiles of 64 and 21 us as 32 clusters of four; a cluster's exchange costs what
+    // its rows do, and clusters beyond one wave wait for whole groups of SMs (16 x 16384 x 2048: 25 us as 128 tiles of
+    // 128, 31 us as 128 clusters of two), as do clusters of eight.
+    const int steps = (s.K + kBK - 1) / kBK;
+    auto tiles_of = [&](int bn, int pair) {
+        const int wide = kGroup == Group::kSilu ? bn / 2 : bn;
+        return ((s.T + pair * kBM - 1) / (pair * kBM)) * ((s.N + wide - 1) / wide);
     };
-    const float p256 = cost(256, 2, 0.7f), p128 = cost(128, 2, 0.46f);
-    const float c256 = cost(256, 1, 1.f), c128 = cost(128, 1, 0.56f), c64 = cost(64, 1, 0.36f), least = fminf(fminf(c256, c128), c64);
-    if (p256 <= p128 && p256 <= least) return launch<256, 2, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
-    if (p128 <= least) return launch<128, 2, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
-    if (c256 <= c128 && c256 <= c64) return launch<256, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
-    if (c128 <= c64) return launch<128, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
-    return launch<64, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    auto alone = [&](int bn, int pair, float step, float epilogue) {
+        const int workers = sms / pair;
+        return epilogue + (tiles_of(bn, pair) + workers - 1) / workers * steps * step;
+    };
+    auto shared = [&](int bn, int parts, float step, float epilogue) {
+        if (tiles_of(bn, 1) * parts > sms || steps < 2 * parts) return INFINITY;
+        return epilogue + (steps + parts - 1) / parts * step + 1.5f + (s.T < kBM ? s.T : kBM) * bn * 0.00035f;
+    };
+    const float costs[] = {alone(256, 2, 0.37f, 4.5f),  alone(128, 2, 0.305f, 3.f), alone(256, 1, 0.41f, 4.5f), alone(128, 1, 0.3f, 1.5f),
+                           alone(64, 1, 0.295f, 0.f),   shared(128, 2, 0.3f, 1.5f), shared(128, 4, 0.3f, 1.5f), shared(64, 2, 0.295f, 0.f),
+                           shared(64, 4, 0.295f, 0.f)};
+    int best = 0;
+    for (int i = 1; i < 9; ++i)
+        if (costs[i] < costs[best]) best = i;
+    s.parts = best == 5 || best == 7 ? 2 : 4;
+    switch (best) {
+        case 0: return launch<256, 2, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+        case 1: return launch<128, 2, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+        case 2: return launch<256, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+        case 3: return launch<128, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+        case 4: return launch<64, 1, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+        case 5:
+        case 6: return launch<128, 0, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+        default: return launch<64, 0, kGroup>(A, lda, W, W2, ldw, s, e, sms, st);
+    }
 }
 
 }  // namespace
@@ -315,7 +421,7 @@ cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, in
         if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (err != cudaSuccess) return err;
     }
-    const Shape s{T, N, K, 0, 0, 2000000000ull, status};
+    const Shape s{T, N, K, 0, 0, 1, 2000000000ull, status};
     switch (group_of(e.what)) {
         case Group::kSilu: return choose<Group::kSilu>(A, lda, W, W2, ldw, s, e, sms, st);
         case Group::kRope: return choose<Group::kRope>(A, lda, W, W2, ldw, s, e, sms, st);

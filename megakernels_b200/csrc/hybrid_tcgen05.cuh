@@ -12,12 +12,14 @@ namespace {
 // Bounded wait; on expiry records the fault, marks the CTA as dead and returns false.
 __device__ __noinline__ bool tc_wait_slow(uint32_t bar, uint32_t parity, volatile int* dead, unsigned long long timeout_ns, int* status,
                                           int role) {
-    const unsigned long long t0 = mkb::globaltimer_ns();
+    unsigned long long t0 = 0;  // (the timer is read only when a wait has gone on for a while)
     for (uint32_t spins = 1;; ++spins) {
         if (mkb::mbar_try_wait(bar, parity)) return true;
         if ((spins & 63u) == 0) {
             if (dead != nullptr && *dead) return false;
-            if (mkb::globaltimer_ns() - t0 > timeout_ns) {
+            const unsigned long long now = mkb::globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > timeout_ns) {
                 if (status != nullptr && atomicCAS(&status[0], 0, (int)MKBH_ERR_DEVICE_TIMEOUT) == 0) {
                     status[1] = blockIdx.x;
                     status[2] = -1;
@@ -110,6 +112,11 @@ __device__ __forceinline__ void tc_arrive_cluster(uint32_t bar) {
 __device__ __forceinline__ void tc_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float2 tc_peer_load2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ void tc_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
