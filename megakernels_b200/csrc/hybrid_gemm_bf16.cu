@@ -33,7 +33,7 @@ struct Geo {
 };
 
 struct Shape {
-    int T, N, K, tiles_m, tiles, parts;  // parts: CTAs that share a tile's inner dimension
+    int T, N, K, tiles_m, tiles, parts, a_rows;  // parts: CTAs that share a tile's inner dimension; a_rows: tokens of a copy
     unsigned long long timeout_ns;
     int* status;
 };
@@ -91,7 +91,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     const uint32_t raw32 = mkb::smem_u32(raw), base = (raw32 + 1023u) & ~1023u;
     uint8_t* gbase = raw + (base - raw32);
     volatile int* ctl = reinterpret_cast<volatile int*>(gbase + G::kCtl);  // [0] dead, [1] tensor-memory base
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (uniform, and known to be: the roles' loops then run on the uniform datapath, which the copies and MMAs read from)
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t rank = kPair == 2 ? tc_rank() : 0u;
     const int worker = blockIdx.x / (kShare ? s.parts : kPair), workers = gridDim.x / (kShare ? s.parts : kPair);  // (a pair's CTAs are neighbours)
     auto full = [&](int i) { return base + G::kBars + i * 8; };
@@ -139,19 +140,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         ksteps = end - kfirst;
     }
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+        const bool chosen = tc_elect();
         uint32_t it = 0;
         bool ok = true;
         for (int tile = worker; tile < s.tiles && ok; tile += workers) {
             const int m0 = ((tile % s.tiles_m) * kPair + rank) * kBM, n0 = (tile / s.tiles_m) * wide;
             for (int k = 0; k < ksteps; ++k, ++it) {
                 const int st = it % G::kStages;
-                if (!tc_wait(empty(st), ((it / G::kStages) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 0)) {
-                    ok = false;
-                    break;
-                }
+                ok = __all_sync(0xffffffffu, tc_wait(empty(st), ((it / G::kStages) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 0));
+                if (!ok) break;
+                if (!chosen) continue;
                 const uint32_t dst = base + st * G::kStageBytes, dw = dst + kBM * kBK * 2;
-                if (rank == 0) mkb::mbar_expect_tx(full(st), kPair * G::kStageBytes);
+                if (rank == 0) mkb::mbar_expect_tx(full(st), kPair * (s.a_rows + G::kRowsW) * kBK * 2);
                 if constexpr (kPair == 2) {  // both CTAs' copies count on the first one's barrier
                     const uint32_t bar = tc_peer(full(st), 0);
                     tc_tma_2d_pair(dst, &amap, k * kBK, m0, bar);
@@ -171,20 +172,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
             if (ok) tc_wait(empty(i % G::kStages), (i / G::kStages) & 1u, ctl, s.timeout_ns, s.status, 0);
             else if (rank == 0) tc_wait(full(i % G::kStages), (i / G::kStages) & 1u, nullptr, s.timeout_ns, s.status, 0);
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0) {
+        const bool chosen = tc_elect();
         const uint32_t idesc = tc_idesc(kPair * kBM, kBN);
         uint32_t it = 0, acc = 0;
         bool ok = true;
         for (int tile = worker; tile < s.tiles && ok; tile += workers, ++acc) {
             const uint32_t buf = acc & 1u;
-            ok = tc_wait(acc_empty(buf), ((acc >> 1) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 1);
+            ok = __all_sync(0xffffffffu, tc_wait(acc_empty(buf), ((acc >> 1) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 1));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int k = 0; k < ksteps; ++k, ++it) {
                 const int st = it % G::kStages;
-                ok = tc_wait(full(st), (it / G::kStages) & 1u, ctl, s.timeout_ns, s.status, 1);
+                ok = __all_sync(0xffffffffu, tc_wait(full(st), (it / G::kStages) & 1u, ctl, s.timeout_ns, s.status, 1));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!chosen) continue;
                 const uint32_t a = base + st * G::kStageBytes, w = a + kBM * kBK * 2;
 #pragma unroll
                 for (int kk = 0; kk < kBK / 16; ++kk)
@@ -194,6 +197,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                 else tc_commit(empty(st));
             }
             if (!ok) break;
+            if (!chosen) continue;
             if constexpr (kPair == 2) tc_commit_pair(acc_full(buf));
             else tc_commit(acc_full(buf));
         }
@@ -348,7 +352,9 @@ cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
     CUtensorMap amap, wmap, wmap2;
     constexpr bool kDual = kGroup == Group::kSilu;
     constexpr int wide = kDual ? kBN / 2 : kBN, box = kPair == 2 ? kBN / 2 : wide;
-    if ((err = tc_map(&amap, A, s.K, s.T, lda, kBK, kBM)) != cudaSuccess) return err;
+    // (rows of the tile that no copy fills hold anything: they only reach accumulators that nobody reads)
+    s.a_rows = s.T < kBM ? (s.T + 7) / 8 * 8 : kBM;
+    if ((err = tc_map(&amap, A, s.K, s.T, lda, kBK, s.a_rows)) != cudaSuccess) return err;
     if ((err = tc_map(&wmap, W, s.K, s.N, ldw, kBK, box)) != cudaSuccess) return err;
     wmap2 = wmap;
     if (kDual && (err = tc_map(&wmap2, W2, s.K, s.N, ldw, kBK, box)) != cudaSuccess) return err;
@@ -372,12 +378,11 @@ cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
 template <Group kGroup>
 cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, int64_t ldw, Shape s, const GemmEpilogue& e, int sms,
                    cudaStream_t st) {
-    // The tile with the shortest estimated time, in us, fitted to 60 shapes of 16..2048 tokens x 2048..28672 features x
+    // The tile with the shortest estimated time, in us, fitted to 48 shapes of 16..2048 tokens x 2048..28672 features x
     // 512..14336 (cold caches): waves of tiles, each so many steps of the inner dimension, and the last epilogue.  A step
-    // of a narrow tile costs nearly what a wide one does, so few narrow tiles with a long inner dimension are shared:
-    // 61 x 2048 x 8192 takes 45 us as 32 tiles of 64 and 21 us as 32 clusters of four; a cluster's exchange costs what
-    // its rows do, and clusters beyond one wave wait for whole groups of SMs (16 x 16384 x 2048: 25 us as 128 tiles of
-    // 128, 31 us as 128 clusters of two), as do clusters of eight.
+    // costs what an SM takes in from L2 (24 KB: 0.19 us, 32 KB: 0.23 us), so few narrow tiles with a long inner dimension
+    // are shared: 61 x 2048 x 8192 takes 32 us as 32 tiles of 64 and 18.5 us as 32 clusters of four; a cluster's exchange
+    // costs what its rows do, and clusters beyond one wave wait for whole groups of SMs, as do clusters of eight.
     const int steps = (s.K + kBK - 1) / kBK;
     auto tiles_of = [&](int bn, int pair) {
         const int wide = kGroup == Group::kSilu ? bn / 2 : bn;
@@ -389,11 +394,11 @@ cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
     };
     auto shared = [&](int bn, int parts, float step, float epilogue) {
         if (tiles_of(bn, 1) * parts > sms || steps < 2 * parts) return INFINITY;
-        return epilogue + (steps + parts - 1) / parts * step + 1.5f + (s.T < kBM ? s.T : kBM) * bn * 0.00035f;
+        return epilogue + (steps + parts - 1) / parts * step + 2.7f + (s.T < kBM ? s.T : kBM) * bn * 0.00027f;
     };
-    const float costs[] = {alone(256, 2, 0.37f, 4.5f),  alone(128, 2, 0.305f, 3.f), alone(256, 1, 0.41f, 4.5f), alone(128, 1, 0.3f, 1.5f),
-                           alone(64, 1, 0.295f, 0.f),   shared(128, 2, 0.3f, 1.5f), shared(128, 4, 0.3f, 1.5f), shared(64, 2, 0.295f, 0.f),
-                           shared(64, 4, 0.295f, 0.f)};
+    const float costs[] = {alone(256, 2, 0.35f, 5.f),   alone(128, 2, 0.205f, 3.5f), alone(256, 1, 0.38f, 3.6f), alone(128, 1, 0.232f, 1.f),
+                           alone(64, 1, 0.19f, 1.f),    shared(128, 2, 0.232f, 1.f), shared(128, 4, 0.232f, 1.f), shared(64, 2, 0.19f, 1.f),
+                           shared(64, 4, 0.19f, 1.f)};
     int best = 0;
     for (int i = 1; i < 9; ++i)
         if (costs[i] < costs[best]) best = i;
@@ -421,7 +426,7 @@ cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, in
         if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (err != cudaSuccess) return err;
     }
-    const Shape s{T, N, K, 0, 0, 1, 2000000000ull, status};
+    const Shape s{T, N, K, 0, 0, 1, 0, 2000000000ull, status};
     switch (group_of(e.what)) {
         case Group::kSilu: return choose<Group::kSilu>(A, lda, W, W2, ldw, s, e, sms, st);
         case Group::kRope: return choose<Group::kRope>(A, lda, W, W2, ldw, s, e, sms, st);
