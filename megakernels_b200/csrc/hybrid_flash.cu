@@ -12,6 +12,8 @@
 // without a value that is there from the start.  Outputs of rotated values are turned back at the end.
 // Keys may come in two pieces (a latent's expanded part per head, its rotated part for all heads).
 // A tile never crosses the point where a ring of cache rows wraps.
+// Few queries over many keys leave SMs without a block: then a cluster of CTAs shares a block's tiles, and each
+// merges a share of the rows from all parts' maxima, sums and outputs, read through distributed shared memory.
 #include "hybrid_kernels.h"
 #include "hybrid_tcgen05.cuh"
 
@@ -26,11 +28,12 @@ constexpr int kSoftWarps = 8, kHalf = kTile / 2;
 constexpr int kFlashThreads = 64 + 32 * kSoftWarps;
 constexpr int kP = 2 * kTile, kOut = kP + kTile;  // tensor-memory columns: scores, weights (two buffers), output
 constexpr float kSlack = 8.f;
+template <int kE> constexpr int kShareRow = kE + 4;  // floats of a row of partial output, behind it its maximum and sum
 
 struct FlashShape {
     int n, pos0, heads, per, split_slabs, rest_slabs, v_slabs, stages;
     int key_x, value_x, value_x0, key_y, value_y;  // columns of a head, first value column; rows of a head
-    int window, chunk, ring, vdim;
+    int window, chunk, ring, vdim, parts;
     float scale;
     const float *temp, *sink, *value_rope;
     bf16* out;
@@ -55,15 +58,21 @@ struct FlashSmem {  // byte offsets
 };
 // Tiles of the keys that some query of a block sees.
 struct Tiles {
-    int lo, hi, ring;
+    int lo, hi, ring, before, count;  // tiles before the wrap (there is at most one), and in all
     __device__ __forceinline__ int first_key(const FlashShape& s, int p) const { return s.chunk > 0 ? p - p % s.chunk : max(0, p - s.window + 1); }
-    __device__ __forceinline__ Tiles(const FlashShape& s, int p0, int p1) : hi(p1), ring(s.ring) { lo = first_key(s, p0); }
+    __device__ __forceinline__ Tiles(const FlashShape& s, int p0, int p1) : hi(p1), ring(s.ring) {
+        lo = first_key(s, p0);
+        const int keys = hi + 1 - lo, head = min(keys, ring - row(lo));
+        before = (head + kTile - 1) / kTile;
+        count = before + (keys - head + kTile - 1) / kTile;
+    }
+    __device__ __forceinline__ int key(int i) const { return i < before ? lo + i * kTile : lo + ring - row(lo) + (i - before) * kTile; }
     __device__ __forceinline__ int row(int j) const { return j % ring; }
     __device__ __forceinline__ int len(int j) const { return min(min(kTile, hi - j + 1), ring - row(j)); }
 };
 
 // kE: value columns, in whole slabs
-template <int kE>
+template <int kE, bool kShare>
 __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid_constant__ FlashMaps maps, const FlashShape s) {
     extern __shared__ uint8_t raw[];
     const uint32_t raw32 = mkb::smem_u32(raw), base = (raw32 + 1023u) & ~1023u;
@@ -80,9 +89,12 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
     auto p_full = [&](int i) { return bars + (3 + 4 * S + i) * 8; };
     auto o_done = [&](int i) { return bars + (5 + 4 * S + i) * 8; };
     auto meeting = [&](int i) { return bars + (7 + 4 * S + i) * 8; };
-    const int h = blockIdx.x, g = h / s.per, t0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRows;
+    const int part = kShare ? (int)tc_rank() : 0, parts = kShare ? s.parts : 1;
+    const int h = blockIdx.x / parts, g = h / s.per, t0 = ((int)gridDim.y - 1 - (int)blockIdx.y) * kRows;
     const int nq = min(kRows, s.n - t0), p0 = s.pos0 + t0, p1 = p0 + nq - 1;
     const Tiles tiles(s, p0, p1);
+    const int tile0 = tiles.count * part / parts, count = tiles.count * (part + 1) / parts - tile0;  // (may be none)
+    const int j0 = tiles.key(tile0);
     auto wait = [&](uint32_t bar, uint32_t parity, int role) { return tc_wait(bar, parity & 1u, ctl, s.timeout_ns, s.status, role); };
 
     if (threadIdx.x == 0) {
@@ -117,7 +129,7 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
         for (int i = 0; i < slabs; ++i) tc_tma_2d(base + sm.q + i * kSlab, &maps.q, (h * slabs + i) * 64, t0, q_full);
         int issued = 0;
         bool ok = true;
-        for (int j = tiles.lo; j <= tiles.hi && ok; j += tiles.len(j), ++issued) {
+        for (int j = j0; issued < count && ok; j += tiles.len(j), ++issued) {
             const int st = issued % S, row = tiles.row(j);
             const uint32_t parity = (uint32_t)(issued / S) ^ 1u;
             ok = wait(k_empty(st), parity, 0);
@@ -162,8 +174,6 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
             tc_commit(s_full(t & 1));
             return true;
         };
-        int count = 0;
-        for (int j = tiles.lo; j <= tiles.hi; j += tiles.len(j)) ++count;
         bool ok = wait(q_full, 0, 1);
         for (int t = 0; t < 2 && t < count && ok; ++t) ok = scores(t);
         for (int t = 0; t < count && ok; ++t) {
@@ -195,10 +205,11 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
         const float log2e = 1.4426950408889634f, scale = s.scale * (s.temp ? __ldg(s.temp + h) : 1.f) * log2e;
         const int pos = p0 + min(r, nq - 1), row_lo = tiles.first_key(s, pos);
         const int warp_p0 = p0 + quarter * 32, warp_last_lo = tiles.first_key(s, min(warp_p0 + 31, p1));
-        float top = s.sink ? __ldg(s.sink + h) * log2e : -INFINITY, sum = s.sink && half == 0 ? 1.f : 0.f;
+        const bool sink = s.sink != nullptr && part == 0;
+        float top = sink ? __ldg(s.sink + h) * log2e : -INFINITY, sum = sink && half == 0 ? 1.f : 0.f;
         bool ok = true;
         int t = 0;
-        for (int j = tiles.lo; j <= tiles.hi; j += tiles.len(j), ++t) {
+        for (int j = j0; t < count; j += tiles.len(j), ++t) {
             const int len = tiles.len(j);
             ok = __all_sync(0xffffffffu, wait(s_full(t & 1), (uint32_t)(t >> 1), 2));
             if (!ok) break;
@@ -289,18 +300,36 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
             __syncwarp();
             if (lane == 0) mkb::mbar_arrive(p_full(t & 1));
         }
-        if (ok) ok = __all_sync(0xffffffffu, wait(o_done((t - 1) & 1), (uint32_t)((t - 1) >> 1), 2));
+        if (ok && t > 0) ok = __all_sync(0xffffffffu, wait(o_done((t - 1) & 1), (uint32_t)((t - 1) >> 1), 2));
         if (ok) {
             tc_after_sync();
             const int parity = (t & 1) * 2 * kRows;
             mine[parity] = sum;
             ok = meet(t);
             if (ok) sum += other[parity];
+            if constexpr (kShare) {  // keys and values have been read: the output takes their place
+                float* row = reinterpret_cast<float*>(raw + (base - raw32) + sm.k) + r * kShareRow<kE>;
+                if (half == 0) *reinterpret_cast<float2*>(row + kE) = make_float2(top, sum);
+#pragma unroll 1
+                for (int c = half * kE / 2; c < (half + 1) * kE / 2; c += 32) {
+                    uint32_t o[32];
+                    if (t > 0) {
+                        tc_load32(lanes + kOut + c, o);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = 0u;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4)
+                        *reinterpret_cast<float4*>(row + c + i) = make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]),
+                                                                              __uint_as_float(o[i + 2]), __uint_as_float(o[i + 3]));
+                }
+            }
             const float inv = sum > 0.f ? 1.f / sum : 0.f;
             const float2* turn = s.value_rope ? reinterpret_cast<const float2*>(s.value_rope) + (size_t)pos * (s.vdim / 2) : nullptr;
             bf16* dst = s.out + (size_t)(t0 + r) * s.ldo + h * s.vdim;
 #pragma unroll 1
-            for (int c = half * kE / 2; c < (half + 1) * kE / 2; c += 32) {
+            for (int c = half * kE / 2; !kShare && c < (half + 1) * kE / 2; c += 32) {
                 uint32_t o[32];
                 tc_load32(lanes + kOut + c, o);
                 if (r >= nq) continue;
@@ -326,6 +355,39 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
     }
     tc_before_sync();
     __syncthreads();
+    if constexpr (kShare) {
+        tc_cluster_sync();
+        for (int i = part + parts * warp; i < nq; i += parts * (kFlashThreads / 32)) {
+            const uint32_t row = base + sm.k + i * kShareRow<kE> * 4;
+            float best = -INFINITY, sum = 0.f;
+            for (int z = 0; z < parts; ++z) best = fmaxf(best, tc_peer_load2(tc_peer(row + kE * 4, z)).x);
+            if (best == -INFINITY) best = 0.f;
+            for (int z = 0; z < parts; ++z) {
+                const float2 ts = tc_peer_load2(tc_peer(row + kE * 4, z));
+                sum = fmaf(ts.y, exp2f(ts.x - best), sum);
+            }
+            const float inv = sum > 0.f ? 1.f / sum : 0.f;
+            for (int c = 2 * lane; c < s.vdim; c += 64) {
+                float a = 0.f, b = 0.f;
+                for (int z = 0; z < parts; ++z) {
+                    const float f = exp2f(tc_peer_load2(tc_peer(row + kE * 4, z)).x - best);
+                    const float2 v = tc_peer_load2(tc_peer(row + c * 4, z));
+                    a = fmaf(v.x, f, a);
+                    b = fmaf(v.y, f, b);
+                }
+                a *= inv;
+                b *= inv;
+                if (s.value_rope != nullptr) {
+                    const float2 z = __ldg(reinterpret_cast<const float2*>(s.value_rope) + (size_t)(p0 + i) * (s.vdim / 2) + c / 2);
+                    const float y = a * z.x + b * z.y;
+                    b = b * z.x - a * z.y;
+                    a = y;
+                }
+                *reinterpret_cast<uint32_t*>(s.out + (size_t)(t0 + i) * s.ldo + h * s.vdim + c) = mkb::pack_bf16x2(a, b);
+            }
+        }
+        tc_cluster_sync();
+    }
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
@@ -337,20 +399,46 @@ int stages_for(int slabs, int v_slabs) {
     return 0;
 }
 
-template <int kE>
+template <int kE, bool kShare>
 cudaError_t launch(const FlashMaps& maps, const FlashShape& s, cudaStream_t stream) {
     static bool set[64] = {};
+    const auto kernel = flash_tc_kernel<kE, kShare>;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (!set[dev & 63]) {
-        e = cudaFuncSetAttribute(flash_tc_kernel<kE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit + 1024);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit + 1024);
         if (e != cudaSuccess) return e;
         set[dev & 63] = true;
     }
-    const int bytes = FlashSmem(s.split_slabs + s.rest_slabs, s.v_slabs, s.stages).total + 1024;
-    flash_tc_kernel<kE><<<dim3(s.heads, (s.n + kRows - 1) / kRows), kFlashThreads, bytes, stream>>>(maps, s);
-    return cudaGetLastError();
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(s.heads * s.parts, (s.n + kRows - 1) / kRows);
+    c.blockDim = dim3(kFlashThreads);
+    c.dynamicSmemBytes = FlashSmem(s.split_slabs + s.rest_slabs, s.v_slabs, s.stages).total + 1024;
+    c.stream = stream;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = s.parts;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    c.attrs = &cluster;
+    c.numAttrs = kShare ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, maps, s);
+}
+cudaError_t choose(const FlashMaps& maps, FlashShape s, cudaStream_t stream) {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+    }
+    // as many parts as there are SMs for, each with two tiles or more of the longest block (61 queries over 1561 keys,
+    // 16 heads of 192 / 128: 27 us with one part, 18 with four)
+    const int blocks = s.heads * ((s.n + kRows - 1) / kRows), last = s.pos0 + s.n - 1;
+    const int64_t keys = s.chunk > 0 ? last % s.chunk + 1 : last + 1 < s.window ? last + 1 : s.window;
+    for (s.parts = 1; s.parts < 8 && 2 * s.parts * blocks <= sms && keys >= (int64_t)4 * s.parts * kTile;) s.parts *= 2;
+    if (s.v_slabs == 1) return s.parts > 1 ? launch<64, true>(maps, s, stream) : launch<64, false>(maps, s, stream);
+    return s.parts > 1 ? launch<128, true>(maps, s, stream) : launch<128, false>(maps, s, stream);
 }
 
 }  // namespace
@@ -378,9 +466,9 @@ cudaError_t flash_tc(const MkbhGlobals& g, const MkbhLayer& L, bf16* out, int64_
     if (B > 0 && (e = tc_map(&m.k_rest, src.shared, B, rows, src.shared_ld, 64, kTile)) != cudaSuccess) return e;
     FlashShape s{g.num_tokens, g.pos0, H, src.per, slabs_of(A), B > 0 ? slabs_of(B) : 0, slabs_of(L.vdim), 0,
                  latent ? A : 0, latent ? L.vdim : 0, latent ? H * A : 0, latent ? 0 : rows, latent ? 0 : rows,
-                 L.window, L.chunk, rows, L.vdim, L.scale, L.temp, L.sink, L.value_rope, out, ldo, 2000000000ull, g.status};
+                 L.window, L.chunk, rows, L.vdim, 1, L.scale, L.temp, L.sink, L.value_rope, out, ldo, 2000000000ull, g.status};
     s.stages = stages_for(s.split_slabs + s.rest_slabs, s.v_slabs);
-    return s.v_slabs == 1 ? launch<64>(m, s, stream) : launch<128>(m, s, stream);
+    return choose(m, s, stream);
 }
 
 cudaError_t flash_cache(const CacheAttention& a, cudaStream_t stream) {
@@ -394,8 +482,8 @@ cudaError_t flash_cache(const CacheAttention& a, cudaStream_t stream) {
     m.k_rest = m.k;
     constexpr int kAll = 1 << 30;
     FlashShape s{a.n, a.pos0, a.heads, a.heads / a.kv_heads, slabs, 0, slabs, stages_for(slabs, slabs), a.dim, a.dim, 0, 0, 0, kAll, 0, kAll,
-                 a.dim, a.scale, nullptr, nullptr, nullptr, a.out, (int64_t)a.heads * a.dim, 2000000000ull, a.status};
-    return slabs == 1 ? launch<64>(m, s, stream) : launch<128>(m, s, stream);
+                 a.dim, 1, a.scale, nullptr, nullptr, nullptr, a.out, (int64_t)a.heads * a.dim, 2000000000ull, a.status};
+    return choose(m, s, stream);
 }
 
 }  // namespace mkbh

@@ -246,6 +246,17 @@ def test_many_tiles_of_queries_and_keys(bench):
 
 
 @pytest.mark.parametrize("dtype,tol", DTYPES)
+def test_few_queries_over_many_keys(bench, dtype, tol):
+    """Short portions after long ones: attention whose tiles of keys are shared out, blocks with fewer tiles than
+    parts, a chunk edge inside a portion, a ring that wraps."""
+    raw = model_config([chunked(2, 1, 64, 64, size=1500, ff=64), latent(2, 64, 32, 64, 64), chunked(2, 2, 32, 128, size=900)], width=128)
+    raw, w, path, toks, want = bench("many", raw, n=1300, qk_gain=2.0)
+    gen = start(path, dtype, max_len=1400, portion=200)
+    for cuts in ([200] * 5 + [61, 2, 37, 200], [130] * 7 + [3, 190, 197]):
+        assert rel(run_cut(gen, toks, cuts), want) < tol, cuts
+
+
+@pytest.mark.parametrize("dtype,tol", DTYPES)
 def test_requests_in_turn_and_slots_used_again(bench, dtype, tol):
     """Requests of unequal length, interleaved over all slots, then their slots again."""
     raw, w, path, toks, _ = bench("odd")
