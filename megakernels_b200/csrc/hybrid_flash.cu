@@ -123,6 +123,8 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
     __syncthreads();
     tc_after_sync();
     const uint32_t tmem = (uint32_t)ctl[1];
+    let_next();
+    after_previous();
 
     if (warp == 0 && lane == 0) {
         mkb::mbar_expect_tx(q_full, slabs * kSlab);
@@ -416,12 +418,12 @@ cudaError_t launch(const FlashMaps& maps, const FlashShape& s, cudaStream_t stre
     c.blockDim = dim3(kFlashThreads);
     c.dynamicSmemBytes = FlashSmem(s.split_slabs + s.rest_slabs, s.v_slabs, s.stages).total + 1024;
     c.stream = stream;
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = s.parts;
-    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-    c.attrs = &cluster;
-    c.numAttrs = kShare ? 1 : 0;
+    cudaLaunchAttribute attrs[2] = {may_begin_early()};
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = s.parts;
+    attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+    c.attrs = attrs;
+    c.numAttrs = kShare ? 2 : 1;
     return cudaLaunchKernelEx(&c, kernel, maps, s);
 }
 cudaError_t choose(const FlashMaps& maps, FlashShape s, cudaStream_t stream) {

@@ -131,6 +131,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     if constexpr (kPair == 2) tc_cluster_sync();  // (the other CTA's barriers are there)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = (uint32_t)ctl[1];
+    let_next();
+    after_previous();
     constexpr bool kDual = kGroup == Group::kSilu;
     constexpr int wide = kDual ? kBN / 2 : kBN;
     int ksteps = (s.K + kBK - 1) / kBK, kfirst = 0;
@@ -366,12 +368,12 @@ cudaError_t launch(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
     c.blockDim = dim3(kGemmThreads);
     c.dynamicSmemBytes = G::kAlloc;
     c.stream = st;
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = ctas;
-    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-    c.attrs = &cluster;
-    c.numAttrs = ctas > 1 ? 1 : 0;
+    cudaLaunchAttribute attrs[2] = {may_begin_early()};
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = ctas;
+    attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
+    c.attrs = attrs;
+    c.numAttrs = ctas > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&c, kernel, amap, wmap, wmap2, s, e);
 }
 

@@ -15,9 +15,11 @@ using mkbh::GemmEpilogue;
 constexpr int kNormThreads = 256, kKept = 8;  // float4s of a row per thread: widths up to 8192
 
 // out = x / rms(x) * w, a block per row.  `first`: the rows of x are taken from the embeddings and stored.
-__global__ void __launch_bounds__(kNormThreads) prompt_norm_kernel(const bf16* __restrict__ first, float* __restrict__ x, int width, float eps,
-                                                                   const bf16* __restrict__ w, bf16* __restrict__ out) {
+__global__ void __launch_bounds__(kNormThreads) prompt_norm_kernel(const bf16* first, float* x, int width, float eps, const bf16* __restrict__ w,
+                                                                   bf16* out) {
     __shared__ float red[kNormThreads / 32];
+    mkbh::let_next();
+    mkbh::after_previous();
     const size_t row = (size_t)blockIdx.x * width;
     float4 v[kKept];
     float s[1] = {0.f};
@@ -60,8 +62,14 @@ cudaError_t prompt_launch(const MkbGlobals& g, const MkbPrompt& p, int* status, 
     const int n = p.tokens, H = g.hidden_size, F = g.intermediate_size, D = g.head_dim, Q = g.num_attention_heads * D, KV = g.num_kv_heads * D;
     auto at = [](const void* w, size_t elements) { return static_cast<const bf16*>(w) + elements; };
     auto norm = [&](const bf16* first, int rows, const bf16* w, float* x) {
-        prompt_norm_kernel<<<rows, kNormThreads, 0, s>>>(first, x, H, g.rms_norm_eps, w, b.act);
-        return cudaGetLastError();
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3(rows);
+        c.blockDim = dim3(kNormThreads);
+        c.stream = s;
+        cudaLaunchAttribute early = mkbh::may_begin_early();
+        c.attrs = &early;
+        c.numAttrs = 1;
+        return cudaLaunchKernelEx(&c, prompt_norm_kernel, first, x, H, g.rms_norm_eps, w, b.act);
     };
     auto gemm = [&](const bf16* A, const bf16* W, int rows, int N, int K, const GemmEpilogue& e, const bf16* W2 = nullptr) {
         return mkbh::gemm_bf16(A, K, W, K, rows, N, K, e, status, s, W2);
