@@ -114,6 +114,9 @@ inline int query_head(const MkbhLayer& L) {
     const int rest = L.mixer == MKBH_LATENT_ATTENTION ? L.rot_dim : 0;
     return query_rest<T>(L) + (sizeof(T) == 2 && flash_tc_supported(L) ? (rest + 63) / 64 * 64 : rest);
 }
+// attention in 32 bits: the float build's, and the bf16 build's for sizes the others do not take
+template <typename T>
+cudaError_t plain_attention(const MkbhGlobals& g, const MkbhLayer& L, T* out, int64_t ldo, cudaStream_t s);
 cudaError_t flash_tc(const MkbhGlobals& g, const MkbhLayer& L, bf16* out, int64_t ldo, cudaStream_t s);
 bool rotary_flash_supported(const MkbhLayer& L);
 cudaError_t rotary_flash(const MkbhGlobals& g, const MkbhLayer& L, bf16* out, int64_t ldo, cudaStream_t s);

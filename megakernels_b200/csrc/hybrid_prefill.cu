@@ -138,15 +138,16 @@ template <> struct Quad<bf16> {
         *reinterpret_cast<uint2*>(o) = make_uint2(mkb::pack_bf16x2(v.x, v.y), mkb::pack_bf16x2(v.z, v.w));
     }
 };
+// A block takes kTokens tokens: fewer where there are not enough blocks for the SMs.
 constexpr int kCanonTaps = 4;
-template <typename T, int kT>
+template <typename T, int kT, int kTokens>
 __global__ void __launch_bounds__(kThreads) canon_norm4_kernel(const float* __restrict__ x, int n, int pos0, int width,
                                                                const float* __restrict__ w1, const float* __restrict__ w2, float eps,
                                                                const float* __restrict__ taps_w, const float* __restrict__ hist,
                                                                float* __restrict__ tail, T* __restrict__ out, T* __restrict__ out2, int64_t ld) {
-    constexpr int kBack = kT > 1 ? kT - 1 : 0, kRowsHere = kNormTokens + kBack;
+    constexpr int kBack = kT > 1 ? kT - 1 : 0, kRowsHere = kTokens + kBack;
     __shared__ float inv[kRowsHere];
-    const int t0 = blockIdx.x * kNormTokens, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = blockIdx.x * kTokens, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = warp; i < kRowsHere; i += kThreads / 32) {
         const int t = t0 - kBack + i;
         if (t < 0 || t >= n) continue;
@@ -311,45 +312,92 @@ __global__ void __launch_bounds__(kThreads) delta_keys_kernel(float* __restrict_
     }
 }
 
-// Decays w = exp(-decay_scale * sigmoid(w2 tanh(w1) + w0)): a tile of 64 tokens x 64 channels of one head.
+// Two neighbouring values in a register pair: one instruction for both, rounded like two.
+__device__ __forceinline__ uint64_t pair_of(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 halves(uint64_t x) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Decays w = exp(-decay_scale * sigmoid(w2 tanh(w1) + w0)): a tile of 64 tokens x 64 channels of one head, kTokens x 4
+// per thread, two tokens per instruction.  Bound by shared-memory reads: one channel x 16 tokens per thread read five
+// 16-byte words per 16 products (2048 tokens, 64 heads of 64, rank 128: 174 us), 8 x 4 read three per 32 (122 us).
+// Few tokens take 4 x 4, twice the warps.  A block keeps its tokens' tanh(w1) for `heads_per` heads.
 constexpr int kDecayTile = 64, kDecayStride = kDecayTile + 4;
-__host__ __device__ inline int decay_smem(int rank) { return (kDecayTile * (rank | 1) + rank * kDecayStride) * 4; }
-template <typename T>
-__global__ void __launch_bounds__(kThreads) delta_decay_kernel(const float* __restrict__ proj, int64_t ld, int n, int HD,
-                                                               int dim, int rank, const T* __restrict__ w2,
-                                                               const float* __restrict__ w0, float decay_scale,
-                                                               float* __restrict__ decay) {
+__host__ __device__ inline int decay_smem(int rank) { return 2 * rank * kDecayStride * 4; }
+template <typename T, int kTokens>
+__global__ void __launch_bounds__(kDecayTile / kTokens * 16) delta_decay_kernel(const float* __restrict__ proj, int64_t ld, int n, int heads,
+                                                                    int dim, int rank, const T* __restrict__ w2,
+                                                                    const float* __restrict__ w0, float decay_scale,
+                                                                    float* __restrict__ decay, int heads_per) {
+    constexpr int kDecayThreads = kDecayTile / kTokens * 16, kPairs = kTokens / 2;
     extern __shared__ __align__(16) float sm[];
     float* inner = sm;                         // [rank][64 tokens]
-    float* wt = sm + rank * kDecayStride;      // [64 channels][rank | 1]
-    const int t0 = blockIdx.x * kDecayTile, nt = min(kDecayTile, n - t0), ws = rank | 1;
-    const int c0 = blockIdx.z * kDecayTile, nc = min(kDecayTile, dim - c0), col0 = blockIdx.y * dim + c0;
-    for (int i = threadIdx.x; i < kDecayTile * rank; i += kThreads) {
-        const int t = i / rank, r = i % rank;
-        inner[r * kDecayStride + t] = t < nt ? tanhf(proj[(size_t)(t0 + t) * ld + 5 * HD + r]) : 0.f;
-        wt[t * ws + r] = t < nc ? to_f(w2[(size_t)(col0 + t) * rank + r]) : 0.f;
-    }
-    __syncthreads();
-    const int ch = threadIdx.x & 63, tg = (threadIdx.x >> 6) * 16;
-    float acc[16];
+    float* wt = sm + rank * kDecayStride;      // [rank][64 channels]
+    const int HD = heads * dim, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = blockIdx.x * kDecayTile, nt = min(kDecayTile, n - t0);
+    const int c0 = blockIdx.z * kDecayTile, nc = min(kDecayTile, dim - c0);
+    for (int t = warp; t < kDecayTile; t += kDecayThreads / 32)
+        for (int r = lane; r < rank; r += 32) inner[r * kDecayStride + t] = t < nt ? tanhf(proj[(size_t)(t0 + t) * ld + 5 * HD + r]) : 0.f;
+    const int ch = (threadIdx.x & 15) * 4, tg = (threadIdx.x >> 4) * kTokens;
+    for (int h = blockIdx.y * heads_per; h < min(heads, ((int)blockIdx.y + 1) * heads_per); ++h) {
+        const int col0 = h * dim + c0;
+        __syncthreads();  // the tokens are there, the head before has been read
+        for (int c = warp; c < kDecayTile; c += kDecayThreads / 32)
+            for (int r = lane; r < rank; r += 32) wt[r * kDecayStride + c] = c < nc ? to_f(w2[(size_t)(col0 + c) * rank + r]) : 0.f;
+        __syncthreads();
+        uint64_t acc[4][kPairs] = {};  // [channel][pair of tokens]
+#pragma unroll 4
+        for (int r = 0; r < rank; ++r) {
+            const float4 w = *reinterpret_cast<const float4*>(wt + r * kDecayStride + ch);
+            uint64_t f[kPairs];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-    for (int r = 0; r < rank; ++r) {
-        const float w = wt[ch * ws + r];
+            for (int j = 0; j < kPairs; j += 2) {
+                const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(inner + r * kDecayStride + tg + 2 * j);
+                f[j] = u.x; f[j + 1] = u.y;
+            }
+            const float ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int j = 0; j < 16; j += 4) {
-            const float4 f = *reinterpret_cast<const float4*>(inner + r * kDecayStride + tg + j);
-            acc[j] = fmaf(w, f.x, acc[j]);
-            acc[j + 1] = fmaf(w, f.y, acc[j + 1]);
-            acc[j + 2] = fmaf(w, f.z, acc[j + 2]);
-            acc[j + 3] = fmaf(w, f.w, acc[j + 3]);
+            for (int c = 0; c < 4; ++c) {
+                const uint64_t x = pair_of(ws[c], ws[c]);
+#pragma unroll
+                for (int j = 0; j < kPairs; ++j) acc[c][j] = fma2(x, f[j], acc[c][j]);
+            }
+        }
+        const bool wide = (HD & 3) == 0 && (col0 & 3) == 0 && ch + 4 <= nc;  // (a row's four channels in one store)
+        float bias[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) bias[c] = ch + c < nc ? w0[col0 + ch + c] : 0.f;
+#pragma unroll
+        for (int j = 0; j < kTokens; ++j) {
+            if (tg + j >= nt) break;
+            float v[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float2 x = halves(acc[c][j >> 1]);
+                v[c] = expf(-decay_scale * sigmoid_f((j & 1 ? x.y : x.x) + bias[c]));
+            }
+            float* o = decay + (size_t)(t0 + tg + j) * HD + col0 + ch;
+            if (wide) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+            else
+                for (int c = 0; c < 4 && ch + c < nc; ++c) o[c] = v[c];
         }
     }
-    if (ch >= nc) return;
-    const float bias = w0[col0 + ch];
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-        if (tg + j < nt) decay[(size_t)(t0 + tg + j) * HD + col0 + ch] = expf(-decay_scale * sigmoid_f(acc[j] + bias));
 }
 
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
@@ -377,23 +425,24 @@ constexpr int kScanCols = 16;
 constexpr int kScanThreads = 256;
 template <int M>
 __host__ __device__ constexpr int scan_tokens() { return M <= 2 ? 32 : M <= 4 ? 16 : 8; }
-template <int M>
+template <int M, int C>
 __host__ __device__ constexpr int scan_buf() {  // floats of one buffer
-    return (scan_tokens<M>() + 1) * 4 * 32 * M + scan_tokens<M>() * (kScanCols + 2);
+    return (scan_tokens<M>() + 1) * 4 * 32 * M + scan_tokens<M>() * (kScanCols * C + 2);
 }
-template <int M>
-__host__ __device__ constexpr int scan_smem() { return 2 * scan_buf<M>() * 4; }
+template <int M, int C>
+__host__ __device__ constexpr int scan_smem() { return 2 * scan_buf<M, C>() * 4; }
 
 // A token's vectors as one lane needs them: decay, the NEXT token's key, removal rate, read vector.
-template <int M>
+template <int M, int C>
 struct ScanToken {
-    float w[4 * M], kn[4 * M], c[4 * M], r[4 * M], v;
+    uint64_t w[2 * M], kn[2 * M], c[2 * M], r[2 * M];
+    float v[C];
     float2 ab;
-    __device__ __forceinline__ static void rows(float (&x)[4 * M], const float4* base) {
+    __device__ __forceinline__ static void rows(uint64_t (&x)[2 * M], const float4* base) {
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-            const float4 f = base[8 * m];
-            x[4 * m] = f.x; x[4 * m + 1] = f.y; x[4 * m + 2] = f.z; x[4 * m + 3] = f.w;
+            const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(base + 8 * m);
+            x[2 * m] = f.x; x[2 * m + 1] = f.y;
         }
     }
     __device__ __forceinline__ void load(const float4* base, const float* vals, const float* abs_) {
@@ -402,18 +451,20 @@ struct ScanToken {
         rows(kn, base + 5 * Q);
         rows(c, base + 2 * Q);
         rows(r, base);
-        v = *vals;
+#pragma unroll
+        for (int u = 0; u < C; ++u) v[u] = vals[u * kScanCols];
         ab = *reinterpret_cast<const float2*>(abs_);
     }
 };
 
-template <int M>
-__global__ void __launch_bounds__(kScanThreads, M <= 2 ? 2 : 1)
+// C: columns of a lane group, kScanCols apart (a CTA has kScanCols * C)
+template <int M, int C>
+__global__ void __launch_bounds__(kScanThreads, M <= 2 && C == 1 ? 2 : 1)
 delta_scan_kernel(const float* __restrict__ proj, int64_t ld, int n, int heads, int dim, const float* __restrict__ decay,
                   const float* __restrict__ ab, float* __restrict__ state, int fresh, float* __restrict__ out) {
-    constexpr int DP = 32 * M, TC = scan_tokens<M>(), BUF = scan_buf<M>();
-    extern __shared__ __align__(16) float sm[];  // two of: [TC + 1][r k c w][DP], [TC][kScanCols], [TC][alpha beta]
-    const int head = blockIdx.y, col0 = blockIdx.x * kScanCols, HD = heads * dim;
+    constexpr int DP = 32 * M, TC = scan_tokens<M>(), BUF = scan_buf<M, C>(), W = kScanCols * C;
+    extern __shared__ __align__(16) float sm[];  // two of: [TC + 1][r k c w][DP], [TC][W], [TC][alpha beta]
+    const int head = blockIdx.y, col0 = blockIdx.x * W, HD = heads * dim;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     for (int i = tid; i < 2 * BUF; i += kScanThreads) sm[i] = 0.f;  // padding channels stay zero
     __syncthreads();
@@ -427,7 +478,7 @@ delta_scan_kernel(const float* __restrict__ proj, int64_t ld, int n, int heads, 
         const int units = wide ? dim / 4 : dim;               // copies per vector
         const int side = units < 32 ? 32 / units : 1;         // tokens side by side in a warp
         const int first = units < 32 ? lane / units : 0, u0 = units < 32 ? lane % units : lane;
-        const int nc = min(kScanCols, dim - col0);
+        const int nc = min(W, dim - col0);
         for (int t0 = 0, buf = 0; t0 < n; t0 += TC, buf ^= 1) {
             if (t0 >= 2 * TC) __syncthreads();  // the buffer has been consumed
             float* b = sm + buf * BUF;
@@ -441,9 +492,9 @@ delta_scan_kernel(const float* __restrict__ proj, int64_t ld, int n, int heads, 
                     }
             for (int t = lim; t < TC + (q == 1); ++t)  // beyond the portion: steps that change nothing
                 for (int c = lane; c < dim; c += 32) b[(t * 4 + q) * DP + c] = q == 3 ? 1.f : 0.f;
-            float *vals = b + (TC + 1) * 4 * DP, *abs_ = vals + TC * kScanCols;
-            for (int i = ptid; i < TC * kScanCols; i += 128) {
-                const int t = i / kScanCols, c = i % kScanCols;
+            float *vals = b + (TC + 1) * 4 * DP, *abs_ = vals + TC * W;
+            for (int i = ptid; i < TC * W; i += 128) {
+                const int t = i / W, c = i % W;
                 if (t < nt && c < nc) cp_async4(mkb::smem_u32(vals + i), vsrc + (t0 + t) * ld + c);
                 else vals[i] = 0.f;
             }
@@ -460,78 +511,113 @@ delta_scan_kernel(const float* __restrict__ proj, int64_t ld, int n, int heads, 
 
     // Barriers of both sides, in order: chunk 0 there, chunk 1 there, chunk 0 consumed, chunk 2 there,
     // chunk 1 consumed, ...
-    const int grp = lane & 7, lcol = warp * 4 + (lane >> 3), col = col0 + lcol, chunks = (n + TC - 1) / TC;
-    const bool live = col < dim;
-    float* S0 = state + ((size_t)head * dim + (live ? col : 0)) * dim;
-    float S[4 * M];
+    const int grp = lane & 7, lcol = warp * 4 + (lane >> 3), chunks = (n + TC - 1) / TC;
+    uint64_t S[C][2 * M], k[2 * M];
+    float q[C];
 #pragma unroll
-    for (int i = 0; i < 4 * M; ++i) {
-        const int ch = 32 * (i >> 2) + 4 * grp + (i & 3);
-        S[i] = (!fresh && live && ch < dim) ? S0[ch] : 0.f;
+    for (int u = 0; u < C; ++u) {
+        const int col = col0 + lcol + u * kScanCols;
+        const bool old = !fresh && col < dim;
+        const float* S0 = state + ((size_t)head * dim + (old ? col : 0)) * dim;
+#pragma unroll
+        for (int i = 0; i < 2 * M; ++i) {
+            const int ch = 32 * (i >> 1) + 4 * grp + 2 * (i & 1);
+            S[u][i] = pair_of(old && ch < dim ? S0[ch] : 0.f, old && ch + 1 < dim ? S0[ch + 1] : 0.f);
+        }
+        q[u] = 0.f;
     }
-    float k[4 * M], q = 0.f;
     __syncthreads();  // chunk 0 is there
     for (int ci = 0; ci < chunks; ++ci) {
         const float* b = sm + (ci & 1) * BUF;
         const float4* vecs = reinterpret_cast<const float4*>(b) + grp;
-        const float *vals = b + (TC + 1) * 4 * DP + lcol, *abs_ = b + (TC + 1) * 4 * DP + TC * kScanCols;
+        const float *vals = b + (TC + 1) * 4 * DP + lcol, *abs_ = b + (TC + 1) * 4 * DP + TC * W;
         if (ci == 0) {
-            ScanToken<M>::rows(k, vecs + 8 * M);
+            ScanToken<M, C>::rows(k, vecs + 8 * M);
 #pragma unroll
-            for (int i = 0; i < 4 * M; ++i) q = fmaf(k[i], S[i], q);
+            for (int u = 0; u < C; ++u) {
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+                for (int i = 0; i < 2 * M; ++i) {
+                    const float2 x = halves(k[i]), y = halves(S[u][i]);
+                    q[u] = fmaf(x.x, y.x, q[u]);
+                    q[u] = fmaf(x.y, y.y, q[u]);
+                }
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) q[u] += __shfl_xor_sync(0xffffffffu, q[u], o);
+            }
         }
-        ScanToken<M> now, next;
+        ScanToken<M, C> now, next;
         now.load(vecs, vals, abs_);
 #pragma unroll 1
         for (int t8 = 0; t8 < TC; t8 += 8) {
-            float op[8];
+            float op[C][8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int tn = j < 7 || t8 + 8 < TC ? t8 + j + 1 : 0;  // (the chunk's last token loads a dummy)
-                next.load(vecs + tn * DP, vals + tn * kScanCols, abs_ + 2 * tn);
-                float d[4] = {0.f, 0.f, 0.f, 0.f}, o[4] = {0.f, 0.f, 0.f, 0.f}, x[4 * M];
+                next.load(vecs + tn * DP, vals + tn * W, abs_ + 2 * tn);
+                float dd[C];
 #pragma unroll
-                for (int i = 0; i < 4 * M; ++i) {
-                    S[i] *= now.w[i];
-                    d[i & 3] = fmaf(now.kn[i], S[i], d[i & 3]);
+                for (int u = 0; u < C; ++u) {
+                    uint64_t d[2] = {0, 0};  // (two zeros)
+#pragma unroll
+                    for (int i = 0; i < 2 * M; ++i) {
+                        S[u][i] = mul2(S[u][i], now.w[i]);
+                        d[i & 1] = fma2(now.kn[i], S[u][i], d[i & 1]);
+                    }
+                    const float2 d0 = halves(d[0]), d1 = halves(d[1]);
+                    dd[u] = (d0.x + d0.y) + (d1.x + d1.y);
                 }
-                float dd = (d[0] + d[1]) + (d[2] + d[3]);
-                dd += __shfl_xor_sync(0xffffffffu, dd, 1);
 #pragma unroll
-                for (int i = 0; i < 4 * M; ++i) x[i] = fmaf(-now.c[i], q, now.v);
-                dd += __shfl_xor_sync(0xffffffffu, dd, 2);
+                for (int o = 1; o < 8; o <<= 1)
 #pragma unroll
-                for (int i = 0; i < 4 * M; ++i) S[i] = fmaf(k[i], x[i], S[i]);
-                dd += __shfl_xor_sync(0xffffffffu, dd, 4);
+                    for (int u = 0; u < C; ++u) dd[u] += __shfl_xor_sync(0xffffffffu, dd[u], o);
 #pragma unroll
-                for (int i = 0; i < 4 * M; ++i) o[i & 3] = fmaf(now.r[i], S[i], o[i & 3]);
-                op[j] = (o[0] + o[1]) + (o[2] + o[3]);
-                q = fmaf(now.ab.y, now.v, fmaf(-now.ab.x, q, dd));
+                for (int u = 0; u < C; ++u) {
+                    const uint64_t minus_q = pair_of(-q[u], -q[u]), v = pair_of(now.v[u], now.v[u]);
+                    uint64_t o[2] = {0, 0};
 #pragma unroll
-                for (int i = 0; i < 4 * M; ++i) k[i] = now.kn[i];
+                    for (int i = 0; i < 2 * M; ++i) {
+                        S[u][i] = fma2(k[i], fma2(now.c[i], minus_q, v), S[u][i]);
+                        o[i & 1] = fma2(now.r[i], S[u][i], o[i & 1]);
+                    }
+                    const float2 o0 = halves(o[0]), o1 = halves(o[1]);
+                    op[u][j] = (o0.x + o0.y) + (o1.x + o1.y);
+                    q[u] = fmaf(now.ab.y, now.v[u], fmaf(-now.ab.x, q[u], dd[u]));
+                }
+#pragma unroll
+                for (int i = 0; i < 2 * M; ++i) k[i] = now.kn[i];
                 now = next;
             }
             // eight sums over eight lanes in seven shuffles: lane j of a column ends up with token j
-#pragma unroll
-            for (int h = 4; h; h >>= 1)
-#pragma unroll
-                for (int j = 0; j < h; ++j) {
-                    const bool up = grp & h;
-                    const float keep = up ? op[j + h] : op[j], send = up ? op[j] : op[j + h];
-                    op[j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
-                }
             const int t = ci * TC + t8 + grp;
-            if (live && t < n) out[(size_t)t * HD + head * dim + col] = op[0];
+#pragma unroll
+            for (int u = 0; u < C; ++u) {
+#pragma unroll
+                for (int h = 4; h; h >>= 1)
+#pragma unroll
+                    for (int j = 0; j < h; ++j) {
+                        const bool up = grp & h;
+                        const float keep = up ? op[u][j + h] : op[u][j], send = up ? op[u][j] : op[u][j + h];
+                        op[u][j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+                    }
+                const int col = col0 + lcol + u * kScanCols;
+                if (col < dim && t < n) out[(size_t)t * HD + head * dim + col] = op[u][0];
+            }
         }
         if (ci + 1 < chunks) __syncthreads();  // chunk ci + 1 is there
         if (ci + 2 < chunks) __syncthreads();  // chunk ci has been consumed
     }
 #pragma unroll
-    for (int i = 0; i < 4 * M; ++i) {
-        const int ch = 32 * (i >> 2) + 4 * grp + (i & 3);
-        if (live && ch < dim) S0[ch] = S[i];
+    for (int u = 0; u < C; ++u) {
+        const int col = col0 + lcol + u * kScanCols;
+        if (col >= dim) break;
+        float* S0 = state + ((size_t)head * dim + col) * dim;
+#pragma unroll
+        for (int i = 0; i < 2 * M; ++i) {
+            const int ch = 32 * (i >> 1) + 4 * grp + 2 * (i & 1);
+            const float2 x = halves(S[u][i]);
+            if (ch < dim) S0[ch] = x.x;
+            if (ch + 1 < dim) S0[ch + 1] = x.y;
+        }
     }
 }
 
@@ -590,93 +676,13 @@ __global__ void kv_append_kernel(const float* __restrict__ proj, int64_t ld, int
     }
 }
 
-// One CTA per (token, query head): scores of 128 keys at a time, both maps, online softmax.  The
-// float build's attention, and the bf16 build's for head sizes hybrid_attention.cu does not take.
-constexpr int kAttnThreads = 128;
-constexpr int kAttnMaxE = 4;  // vdim <= 512
-template <typename T>
-__global__ void __launch_bounds__(kAttnThreads) attention_kernel(const float* __restrict__ proj, int64_t ld, int pos0,
-                                                                 MkbhLayer L, const T* __restrict__ kc,
-                                                                 const T* __restrict__ vc, float eps, T* __restrict__ out,
-                                                                 int64_t ldo) {
-    extern __shared__ float sm[];  // q [2 dim], p [2][128]
-    __shared__ float red[2 * kAttnThreads / 32];
-    const int D = L.dim, E = L.vdim, G = L.kv_heads, H = L.heads;
-    const int t = blockIdx.x, h = blockIdx.y, g = h / (H / G), tid = threadIdx.x;
-    float* q = sm;
-    float* p = sm + 2 * D;
-    const float* row = proj + (size_t)t * ld;
-    // (q takes the precision of the activations it would have had as a stored tensor)
-    for (int i = tid; i < 2 * D; i += kAttnThreads) q[i] = to_f(from_f<T>(row[h * 2 * D + i]));
-    __syncthreads();
-    const KeyRange keys(pos0 + t, L.window, L.keep_first, L.chunk);
-    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, acc[2][kAttnMaxE] = {};
-    for (int c0 = 0; c0 < keys.count; c0 += kAttnThreads) {
-        const int nk = min(kAttnThreads, keys.count - c0);
-        float s[2] = {-INFINITY, -INFINITY};
-        if (tid < nk) {
-            const T* k = kc + ((size_t)cache_row(keys.key(c0 + tid), L.cache_keep, L.cache_ring) * G + g) * 2 * D;
-            for (int b = 0; b < 2; ++b) {
-                float d = 0.f;
-                for (int i = 0; i < D; ++i) d = fmaf(q[b * D + i], to_f(k[b * D + i]), d);
-                s[b] = d * L.scale;
-            }
-        }
-        for (int b = 0; b < 2; ++b) {
-            float x = warp_max(s[b]);
-            if ((tid & 31) == 0) red[b * (kAttnThreads / 32) + (tid >> 5)] = x;
-        }
-        __syncthreads();
-        float f[2];
-        for (int b = 0; b < 2; ++b) {
-            float x = m[b];
-            for (int w = 0; w < kAttnThreads / 32; ++w) x = fmaxf(x, red[b * (kAttnThreads / 32) + w]);
-            f[b] = expf(m[b] - x);
-            m[b] = x;
-            s[b] = tid < nk ? expf(s[b] - x) : 0.f;
-            p[b * kAttnThreads + tid] = s[b];
-        }
-        __syncthreads();
-        float ps[2] = {s[0], s[1]};
-        block_sum<2, kAttnThreads>(ps, red);
-        for (int b = 0; b < 2; ++b) l[b] = l[b] * f[b] + ps[b];
-        for (int ei = 0; ei < kAttnMaxE; ++ei) {
-            const int e = tid + ei * kAttnThreads;
-            if (e >= E) break;
-            float a0 = acc[0][ei] * f[0], a1 = acc[1][ei] * f[1];
-            for (int j = 0; j < nk; ++j) {
-                const float v = to_f(vc[((size_t)cache_row(keys.key(c0 + j), L.cache_keep, L.cache_ring) * G + g) * E + e]);
-                a0 = fmaf(p[j], v, a0);
-                a1 = fmaf(p[kAttnThreads + j], v, a1);
-            }
-            acc[0][ei] = a0;
-            acc[1][ei] = a1;
-        }
-        __syncthreads();
-    }
-    float sq[1] = {0.f};
-    for (int ei = 0; ei < kAttnMaxE; ++ei) {
-        const float o = tid + ei * kAttnThreads < E ? acc[0][ei] / l[0] - L.lambda * (acc[1][ei] / l[1]) : 0.f;
-        acc[0][ei] = o;
-        sq[0] += o * o;
-    }
-    block_sum<1, kAttnThreads>(sq, red);
-    const float f = (1.f - L.diff) / sqrtf(sq[0] / E + eps);
-    const float* gate = row + H * 2 * D + h * E;
-    T* dst = out + (size_t)t * ldo + h * E;
-    for (int ei = 0; ei < kAttnMaxE; ++ei) {
-        const int e = tid + ei * kAttnThreads;
-        if (e < E) dst[e] = from_f<T>(acc[0][ei] * f * sigmoid_f(gate[e]));
-    }
-    if (h == 0)
-        for (int i = H * E + tid; i < pad8(H * E); i += kAttnThreads) out[(size_t)t * ldo + i] = from_f<T>(0.f);
-}
-
 // ---- rotary and latent attention ------------------------------------------------------------- //
 // Operands of a portion.  A warp takes one vector (a query, key or value head; the latent, its
-// rotated part) of kOpTokens tokens: convolution over time, norm, rotation of neighbours, and
+// rotated part) of a run of tokens: convolution over time, norm, rotation of neighbours, and
 // stores it as an element of the query buffer or as a cache row.
-constexpr int kOpTokens = 8;
+// Eight tokens share a vector's weights; short portions, where the SMs wait for a warp's chain of tokens, take two:
+// 61 tokens of the 1B-class widths 17 us -> 8.
+inline int run_of(int n) { return n <= 512 ? 2 : 8; }
 struct OperandArgs {
     const float* proj;
     int64_t ld, ldq;
@@ -686,6 +692,7 @@ struct OperandArgs {
     float eps;
     void *query, *kc, *vc;  // (cache bases of the slot)
     int qhead, qrest;       // entries of a query head, start of its rotated part
+    int run;                // tokens of a warp
 };
 template <typename T, int J>
 __device__ __forceinline__ void operand_vector(const OperandArgs& a, int t, int col, int len, const float* w, const float2* rope,
@@ -826,7 +833,7 @@ __global__ void __launch_bounds__(kThreads) rotary_operands_kernel(const Operand
     const MkbhLayer& L = a.L;
     const int task = blockIdx.y * (kThreads / 32) + (threadIdx.x >> 5), H = L.heads, G = L.kv_heads;
     if (task >= (kLatent ? H + 2 : H + 2 * G)) return;
-    const int t0 = blockIdx.x * kOpTokens, t1 = min(a.n, t0 + kOpTokens);
+    const int t0 = blockIdx.x * a.run, t1 = min(a.n, t0 + a.run);
     const size_t rows = L.cache_keep + L.cache_ring;
     auto query = [&](int h, int off) { return [=](int t) { return static_cast<T*>(a.query) + (size_t)t * a.ldq + h * a.qhead + off; }; };
     auto cache = [&](void* base, size_t first, int len, int off) {
@@ -860,88 +867,30 @@ __global__ void __launch_bounds__(kThreads) rotary_operands_kernel(const Operand
     }
 }
 
-// One CTA per (token, query head), 128 keys at a time, online softmax.  The float build's
-// attention, and the bf16 build's for head sizes hybrid_attention.cu does not take.
-template <typename T>
-__global__ void __launch_bounds__(kAttnThreads) rotary_attention_kernel(const T* __restrict__ query, int64_t ldq, int pos0, const MkbhLayer L,
-                                                                        const KeySource<T> src, T* __restrict__ out, int64_t ldo) {
-    extern __shared__ float sm[];  // q [split + rest], p [128], o [vdim]
-    __shared__ float red[kAttnThreads / 32];
-    const int A = src.split, B = src.rest, E = L.vdim, H = L.heads;
-    const int t = blockIdx.x, h = blockIdx.y, g = h / src.per, tid = threadIdx.x, pos = pos0 + t;
-    float *q = sm, *p = sm + A + B, *o = p + kAttnThreads;
-    for (int i = tid; i < A + B; i += kAttnThreads) q[i] = to_f(query[(size_t)t * ldq + h * (A + B) + i]);
-    __syncthreads();
-    const KeyRange keys(pos, L.window, L.keep_first, L.chunk);
-    const float scale = L.scale * (L.temp ? L.temp[h] : 1.f);
-    float m = L.sink ? L.sink[h] : -INFINITY, l = L.sink ? 1.f : 0.f, acc[kAttnMaxE] = {};
-    for (int c0 = 0; c0 < keys.count; c0 += kAttnThreads) {
-        const int nk = min(kAttnThreads, keys.count - c0);
-        float s = -INFINITY;
-        if (tid < nk) {
-            const size_t row = cache_row(keys.key(c0 + tid), src.keep, src.ring);
-            const T *k = src.keys + row * src.key_ld + g * src.key_head, *r = src.shared + row * src.shared_ld;
-            float d = 0.f;
-            for (int i = 0; i < A; ++i) d = fmaf(q[i], to_f(k[i]), d);
-            for (int i = 0; i < B; ++i) d = fmaf(q[A + i], to_f(r[i]), d);
-            s = d * scale;
-        }
-        float x = warp_max(s);
-        if ((tid & 31) == 0) red[tid >> 5] = x;
-        __syncthreads();
-        x = m;
-        for (int w = 0; w < kAttnThreads / 32; ++w) x = fmaxf(x, red[w]);
-        const float f = expf(m - x);
-        m = x;
-        s = tid < nk ? expf(s - x) : 0.f;
-        p[tid] = s;
-        __syncthreads();
-        float ps[1] = {s};
-        block_sum<1, kAttnThreads>(ps, red);
-        l = l * f + ps[0];
-        for (int ei = 0; ei < kAttnMaxE; ++ei) {
-            const int e = tid + ei * kAttnThreads;
-            if (e >= E) break;
-            float y = acc[ei] * f;
-            for (int j = 0; j < nk; ++j)
-                y = fmaf(p[j], to_f(src.values[(size_t)cache_row(keys.key(c0 + j), src.keep, src.ring) * src.value_ld + g * src.value_head + e]), y);
-            acc[ei] = y;
-        }
-        __syncthreads();
-    }
-    for (int ei = 0; ei < kAttnMaxE; ++ei)
-        if (tid + ei * kAttnThreads < E) o[tid + ei * kAttnThreads] = acc[ei] / l;
-    __syncthreads();
-    const float2* turn = L.value_rope ? reinterpret_cast<const float2*>(L.value_rope) + (size_t)pos * (E / 2) : nullptr;
-    T* dst = out + (size_t)t * ldo + h * E;
-    for (int e = tid; e < E; e += kAttnThreads) {
-        float y = o[e];
-        if (turn != nullptr) {  // back by the query's angle
-            const float2 r = turn[e >> 1];
-            y = y * r.x + (e & 1 ? -r.y : r.y) * o[e ^ 1];
-        }
-        dst[e] = from_f<T>(y);
-    }
-    if (h == 0)
-        for (int i = H * E + tid; i < pad8(H * E); i += kAttnThreads) out[(size_t)t * ldo + i] = from_f<T>(0.f);
-}
-
-template <int M>
-cudaError_t launch_scan(const MkbhGlobals& g, const MkbhLayer& L, int64_t ld, float* state, cudaStream_t s) {
+template <int M, int C>
+cudaError_t launch_scan_columns(const MkbhGlobals& g, const MkbhLayer& L, int64_t ld, float* state, cudaStream_t s) {
     static bool set[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (!set[dev & 63]) {
-        e = cudaFuncSetAttribute(delta_scan_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem<M>());
+        e = cudaFuncSetAttribute(delta_scan_kernel<M, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem<M, C>());
         if (e != cudaSuccess) return e;
         set[dev & 63] = true;
     }
-    dim3 grid((L.dim + kScanCols - 1) / kScanCols, L.heads);
-    delta_scan_kernel<M><<<grid, kScanThreads, scan_smem<M>(), s>>>(
+    dim3 grid((L.dim + kScanCols * C - 1) / (kScanCols * C), L.heads);
+    delta_scan_kernel<M, C><<<grid, kScanThreads, scan_smem<M, C>(), s>>>(
         g.proj, ld, g.num_tokens, L.heads, L.dim, g.decay, g.decay + (size_t)g.num_tokens * L.heads * L.dim, state,
         g.pos0 == 0, g.mixed);
     return cudaGetLastError();
+}
+// Two columns per lane group halve the reads of a token's vectors, which bound an SM with two CTAs (64 heads of 64, 2048
+// tokens: 394 us, 267 with two columns and one CTA); with SMs to spare one column is the shorter chain (32 heads: 237).
+template <int M>
+cudaError_t launch_scan(const MkbhGlobals& g, const MkbhLayer& L, int64_t ld, float* state, cudaStream_t s) {
+    if constexpr (M <= 2)
+        if ((L.dim + kScanCols - 1) / kScanCols * L.heads > 148) return launch_scan_columns<M, 2>(g, L, ld, state, s);
+    return launch_scan_columns<M, 1>(g, L, ld, state, s);
 }
 
 }  // namespace
@@ -968,9 +917,12 @@ cudaError_t Prefill<T>::canon_norm(const MkbhGlobals& g, const MkbhLayer& L, T* 
     const int n = g.num_tokens, smem = max(1, L.canon_taps) * g.width * 4;
     const float* hist = L.canon_hist + (L.canon_taps > 1 ? (size_t)g.slot * (L.canon_taps - 1) * g.width : 0);
     if (g.norm_kind == MKBH_RMS_NORM && g.width % 4 == 0 && L.canon_taps <= kCanonTaps) {
+        const bool few = n <= 512;  // (8 us at 61 tokens and 1B-class widths with eight tokens per block, 6 with two)
         auto go = [&](auto taps) {
-            canon_norm4_kernel<T, decltype(taps)::value><<<(n + kNormTokens - 1) / kNormTokens, kThreads, 0, s>>>(
-                g.x, n, g.pos0, g.width, L.norm1, L.norm2, g.eps, L.canon_w, hist, g.tail, out, out2, ld);
+            const auto kernel = few ? canon_norm4_kernel<T, decltype(taps)::value, 2> : canon_norm4_kernel<T, decltype(taps)::value, kNormTokens>;
+            const int tokens = few ? 2 : kNormTokens;
+            kernel<<<(n + tokens - 1) / tokens, kThreads, 0, s>>>(g.x, n, g.pos0, g.width, L.norm1, L.norm2, g.eps, L.canon_w, hist, g.tail, out,
+                                                                 out2, ld);
         };
         switch (L.canon_taps) {
             case 0: go(std::integral_constant<int, 0>{}); break;
@@ -1008,8 +960,8 @@ cudaError_t Prefill<T>::rotary_operands(const MkbhGlobals& g, const MkbhLayer& L
     OperandArgs a{g.proj, pad8(L.in_rows), pad8(L.heads * query_head<T>(L)), n, g.pos0, L,
                   L.conv_hist + (L.conv_taps > 1 ? (size_t)g.slot * (L.conv_taps - 1) * L.in_rows : 0), g.eps, g.query,
                   static_cast<T*>(L.k_cache) + rows * (latent ? latent_row(L) : L.kv_heads * L.dim),
-                  latent ? nullptr : static_cast<T*>(L.v_cache) + rows * L.kv_heads * L.vdim, query_head<T>(L), query_rest<T>(L)};
-    const dim3 grid((n + kOpTokens - 1) / kOpTokens, (tasks + kThreads / 32 - 1) / (kThreads / 32));
+                  latent ? nullptr : static_cast<T*>(L.v_cache) + rows * L.kv_heads * L.vdim, query_head<T>(L), query_rest<T>(L), run_of(n)};
+    const dim3 grid((n + a.run - 1) / a.run, (tasks + kThreads / 32 - 1) / (kThreads / 32));
     if (latent) rotary_operands_kernel<T, true><<<grid, kThreads, 0, s>>>(a);
     else rotary_operands_kernel<T, false><<<grid, kThreads, 0, s>>>(a);
     return cudaGetLastError();
@@ -1021,11 +973,7 @@ cudaError_t Prefill<T>::rotary_attention(const MkbhGlobals& g, const MkbhLayer& 
         if (flash_tc_supported(L)) return flash_tc(g, L, out, ldo, s);
         if (rotary_flash_supported(L)) return rotary_flash(g, L, out, ldo, s);
     }
-    const KeySource<T> src = key_source<T>(g, L);
-    const int q = src.split + src.rest;
-    rotary_attention_kernel<T><<<dim3(g.num_tokens, L.heads), kAttnThreads, (q + kAttnThreads + L.vdim) * 4, s>>>(
-        static_cast<const T*>(g.query), pad8(L.heads * q), g.pos0, L, src, out, ldo);
-    return cudaGetLastError();
+    return plain_attention<T>(g, L, out, ldo, s);
 }
 template <typename T>
 cudaError_t Prefill<T>::poly_norm(const float* z, int64_t ldz, int n, int ff, const float* c, float eps, T* out,
@@ -1045,15 +993,19 @@ cudaError_t Prefill<T>::delta(const MkbhGlobals& g, const MkbhLayer& L, T* out, 
     else delta_keys_kernel<8><<<pairs, kThreads, 0, s>>>(g.proj, ld, n, L.heads, L.dim, L.unit_eps, ab);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const int smem = decay_smem(L.rank);
-    if (smem > 48 * 1024) {
-        e = cudaFuncSetAttribute(delta_decay_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-    }
-    delta_decay_kernel<T><<<dim3((n + kDecayTile - 1) / kDecayTile, L.heads, (L.dim + kDecayTile - 1) / kDecayTile), kThreads,
-                            smem, s>>>(g.proj, ld, n, HD, L.dim, L.rank, static_cast<const T*>(L.decay_w2), L.decay_w0,
-                                       L.decay_scale, g.decay);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    // 8 tokens a thread where that fills the SMs with three blocks each, in one wave of as many heads as that takes
+    const int dt = (n + kDecayTile - 1) / kDecayTile, dc = (L.dim + kDecayTile - 1) / kDecayTile, smem = decay_smem(L.rank);
+    const int64_t tiles = (int64_t)dt * dc * L.heads;
+    const auto decay = [&](auto kernel, int threads, int heads_per) {
+        if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return;
+        kernel<<<dim3(dt, (L.heads + heads_per - 1) / heads_per, dc), threads, smem, s>>>(
+            g.proj, ld, n, L.heads, L.dim, L.rank, static_cast<const T*>(L.decay_w2), L.decay_w0, L.decay_scale, g.decay, heads_per);
+        e = cudaGetLastError();
+    };
+    if (tiles >= 444) decay(delta_decay_kernel<T, 8>, 128, (int)((tiles + 443) / 444));
+    else decay(delta_decay_kernel<T, 4>, 256, 1);
+    if (e != cudaSuccess) return e;
     float* state = L.state + (size_t)g.slot * HD * L.dim;
     switch ((L.dim + 31) / 32) {
         case 1: e = launch_scan<1>(g, L, ld, state, s); break;
@@ -1085,9 +1037,7 @@ cudaError_t Prefill<T>::attention(const MkbhGlobals& g, const MkbhLayer& L, T* o
     }
     if constexpr (sizeof(T) == 2)
         if (flash_supported(L)) return flash_attention(g, L, kc, vc, out, ldo, s);
-    attention_kernel<T><<<dim3(n, L.heads), kAttnThreads, (2 * L.dim + 2 * kAttnThreads) * 4, s>>>(
-        g.proj, ld, g.pos0, L, kc, vc, g.eps, out, ldo);
-    return cudaGetLastError();
+    return plain_attention<T>(g, L, out, ldo, s);
 }
 
 template struct Prefill<float>;
