@@ -17,7 +17,9 @@ constexpr int kBM = 128, kBK = 64;
 constexpr int kGemmThreads = 192;
 constexpr int kEpiStride = 33;  // floats per row of a warp's 32 x 32 transpose buffer
 
-// kPair CTAs work on one tile: 128 tokens each, the features' operand halved between them.
+// kPair CTAs work on one tile: 128 tokens each, the features' operand halved between them.  One CTA's
+// 128 x 256 tile takes in 94 bytes a cycle of MMA, more than L2 gives an SM (64); a pair's 256 x 256 takes 63 per SM:
+// 2048 x 28672 x 4096 in 330 us alone, 307 in pairs.
 template <int kBN, int kPair>
 struct Geo {
     static constexpr int kRowsW = kBN / kPair;

@@ -1,6 +1,7 @@
 // 32-bit matrix product of the hybrid models' float build (true fp32 FMA, no reduced-precision matrix mode).
 //
-// Bound by the FMA rate (74 TFLOP/s at 1.96 GHz): tiles of 16, 32 or 64 tokens x 128 features, 128 threads with up to
+// Bound by the FMA rate (74 TFLOP/s at 1.96 GHz) and by shared-memory reads, four cycles per 16-byte read of a warp (300 x
+// 8192 x 2048: 283 us, 36 TFLOP/s; 388 us with 64 x 64 tiles of 4 x 4 outputs): tiles of 16, 32 or 64 tokens x 128 features, 128 threads with up to
 // 8 x 8 outputs each, two neighbouring features per instruction (fma.rn.f32x2, rounded like two fmaf), so that issue
 // slots are left for the shared-memory reads; the next slice of operands is in registers while this one is multiplied.
 // Where the tiles do not fill the SMs evenly, a cluster of up to eight CTAs shares a tile's inner dimension and adds

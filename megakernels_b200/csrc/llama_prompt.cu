@@ -1,7 +1,7 @@
 // A prompt of a llama model, all tokens at once: the layers' matrix products on the 5th-generation tensor
 // cores with the rotation, the cache append and the gated unit as epilogues, attention over the cache.
 // Seven launches a layer.  501 tokens at the 1B widths (16 layers): 354.6 ms as a decode step per token, bound by the
-// weights that every token streams again; 2.9 ms at once, bound by the products.  The residual stream is 32-bit; operands of the products are bf16, as in decoding.
+// weights that every token streams again; 2.1 ms at once, bound by the products and the 118 launches' hand-over.  The residual stream is 32-bit; operands of the products are bf16, as in decoding.
 #include "llama_prompt.h"
 
 #include "hybrid_kernels.h"
