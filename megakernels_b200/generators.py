@@ -241,8 +241,9 @@ class MK_Generator(Generator):
             and interp.mk_func is interp.module.mk_llama
         )
 
-    # A step per token costs what the weights' traffic costs, the layers at once that and their launches.
-    shortest_prompt = 4
+    # A step per token costs what the weights' traffic costs, the layers at once that and their launches, once: two tokens
+    # take 1,132 us at once and 1,289 us as steps (1B widths, 16 layers), 729 and 1,041 us (8B widths, 4 layers).
+    shortest_prompt = 2
 
     def _prompt(self, ids: Tensor) -> Tensor:
         globs, count = self.schedule.globs, ids.shape[1]
