@@ -14,6 +14,8 @@
 // A tile never crosses the point where a ring of cache rows wraps.
 // Few queries over many keys leave SMs without a block: then a cluster of CTAs shares a block's tiles, and each
 // merges a share of the rows from all parts' maxima, sums and outputs, read through distributed shared memory.
+// Over a llama cache (kOwn) the query's own key keeps its 32-bit weight, as in the decode kernel: what the rounding to
+// bf16 took off it times the row's own value is added to the output in fp32.
 #include "hybrid_kernels.h"
 #include "hybrid_tcgen05.cuh"
 
@@ -40,6 +42,8 @@ struct FlashShape {
     int64_t ldo;
     unsigned long long timeout_ns;
     int* status;
+    const bf16* own;  // kOwn: value rows by position, own_ld apart, value_x columns per head
+    int64_t own_ld;
 };
 struct FlashMaps {
     CUtensorMap q, k, k_rest, v;
@@ -72,7 +76,7 @@ struct Tiles {
 };
 
 // kE: value columns, in whole slabs
-template <int kE, bool kShare>
+template <int kE, bool kShare, bool kOwn>
 __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid_constant__ FlashMaps maps, const FlashShape s) {
     extern __shared__ uint8_t raw[];
     const uint32_t raw32 = mkb::smem_u32(raw), base = (raw32 + 1023u) & ~1023u;
@@ -209,6 +213,8 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
         const int warp_p0 = p0 + quarter * 32, warp_last_lo = tiles.first_key(s, min(warp_p0 + 31, p1));
         const bool sink = s.sink != nullptr && part == 0;
         float top = sink ? __ldg(s.sink + h) * log2e : -INFINITY, sum = sink && half == 0 ? 1.f : 0.f;
+        float own = 0.f;  // what the own key's weight lost (its tile is the last that raises this row's maximum)
+        const bf16* own_value = kOwn ? s.own + (size_t)pos * s.own_ld + g * s.value_x : nullptr;
         bool ok = true;
         int t = 0;
         for (int j = j0; t < count; j += tiles.len(j), ++t) {
@@ -297,6 +303,15 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
                 tc_store8(lanes + kP + (t & 1) * (kTile / 2) + (half * kHalf + c) / 2, w);
             }
             sum += (part[0] + part[1]) + (part[2] + part[3]);
+            if (kOwn && j <= warp_p0 + 31 && j + len > warp_p0) {  // (uniform over the warp)
+                const int at_own = pos - j - half * kHalf;
+                float z = -INFINITY;
+#pragma unroll
+                for (int i = 0; i < kHalf; ++i)
+                    if (i == at_own) z = __uint_as_float(x[i]);
+                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(z) : "f"(fmaf(z, mul, -off)));
+                if (at_own >= 0 && at_own < kHalf) own = z - mkb::bf16_round(z);
+            }
             tc_stored();
             tc_before_sync();
             __syncwarp();
@@ -307,8 +322,19 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
             tc_after_sync();
             const int parity = (t & 1) * 2 * kRows;
             mine[parity] = sum;
+            if (kOwn) mine[parity ^ 2 * kRows] = own;  // (the maxima there were read before that tile's weights were complete)
             ok = meet(t);
             if (ok) sum += other[parity];
+            if (kOwn && ok) own += other[parity ^ 2 * kRows];  // (zero in one of them)
+            auto add_own = [&](int c, float (&v)[8]) {  // columns c .. c + 7
+                const uint4 w = *reinterpret_cast<const uint4*>(own_value + c);
+                const uint32_t words[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    v[2 * i] = fmaf(own, mkb::bf16_lo(words[i]), v[2 * i]);
+                    v[2 * i + 1] = fmaf(own, mkb::bf16_hi(words[i]), v[2 * i + 1]);
+                }
+            };
             if constexpr (kShare) {  // keys and values have been read: the output takes their place
                 float* row = reinterpret_cast<float*>(raw + (base - raw32) + sm.k) + r * kShareRow<kE>;
                 if (half == 0) *reinterpret_cast<float2*>(row + kE) = make_float2(top, sum);
@@ -322,9 +348,14 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
                         for (int i = 0; i < 32; ++i) o[i] = 0u;
                     }
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<float4*>(row + c + i) = make_float4(__uint_as_float(o[i]), __uint_as_float(o[i + 1]),
-                                                                              __uint_as_float(o[i + 2]), __uint_as_float(o[i + 3]));
+                    for (int e = 0; e < 32; e += 8) {
+                        float v[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[e + i]);
+                        if (kOwn && own != 0.f) add_own(c + e, v);  // (nothing in the parts without the own key)
+#pragma unroll
+                        for (int i = 0; i < 8; i += 4) *reinterpret_cast<float4*>(row + c + e + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                    }
                 }
             }
             const float inv = sum > 0.f ? 1.f / sum : 0.f;
@@ -339,9 +370,13 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
                 for (int e = 0; e < 32; e += 8) {
                     if (c + e >= s.vdim) break;  // (a multiple of 8)
                     uint32_t w[4];
+                    float v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[e + i]);
+                    if (kOwn && own != 0.f) add_own(c + e, v);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        float a = __uint_as_float(o[e + 2 * i]) * inv, b = __uint_as_float(o[e + 2 * i + 1]) * inv;
+                        float a = v[2 * i] * inv, b = v[2 * i + 1] * inv;
                         if (turn != nullptr) {
                             const float2 z = __ldg(turn + (c + e) / 2 + i);
                             const float y = a * z.x + b * z.y;
@@ -401,10 +436,10 @@ int stages_for(int slabs, int v_slabs) {
     return 0;
 }
 
-template <int kE, bool kShare>
+template <int kE, bool kShare, bool kOwn>
 cudaError_t launch(const FlashMaps& maps, const FlashShape& s, cudaStream_t stream) {
     static bool set[64] = {};
-    const auto kernel = flash_tc_kernel<kE, kShare>;
+    const auto kernel = flash_tc_kernel<kE, kShare, kOwn>;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -426,6 +461,7 @@ cudaError_t launch(const FlashMaps& maps, const FlashShape& s, cudaStream_t stre
     c.numAttrs = kShare ? 2 : 1;
     return cudaLaunchKernelEx(&c, kernel, maps, s);
 }
+template <bool kOwn>
 cudaError_t choose(const FlashMaps& maps, FlashShape s, cudaStream_t stream) {
     static int sms = 0;
     if (sms == 0) {
@@ -439,8 +475,8 @@ cudaError_t choose(const FlashMaps& maps, FlashShape s, cudaStream_t stream) {
     const int blocks = s.heads * ((s.n + kRows - 1) / kRows), last = s.pos0 + s.n - 1;
     const int64_t keys = s.chunk > 0 ? last % s.chunk + 1 : last + 1 < s.window ? last + 1 : s.window;
     for (s.parts = 1; s.parts < 8 && 2 * s.parts * blocks <= sms && keys >= (int64_t)4 * s.parts * kTile;) s.parts *= 2;
-    if (s.v_slabs == 1) return s.parts > 1 ? launch<64, true>(maps, s, stream) : launch<64, false>(maps, s, stream);
-    return s.parts > 1 ? launch<128, true>(maps, s, stream) : launch<128, false>(maps, s, stream);
+    if (s.v_slabs == 1) return s.parts > 1 ? launch<64, true, kOwn>(maps, s, stream) : launch<64, false, kOwn>(maps, s, stream);
+    return s.parts > 1 ? launch<128, true, kOwn>(maps, s, stream) : launch<128, false, kOwn>(maps, s, stream);
 }
 
 }  // namespace
@@ -468,9 +504,9 @@ cudaError_t flash_tc(const MkbhGlobals& g, const MkbhLayer& L, bf16* out, int64_
     if (B > 0 && (e = tc_map(&m.k_rest, src.shared, B, rows, src.shared_ld, 64, kTile)) != cudaSuccess) return e;
     FlashShape s{g.num_tokens, g.pos0, H, src.per, slabs_of(A), B > 0 ? slabs_of(B) : 0, slabs_of(L.vdim), 0,
                  latent ? A : 0, latent ? L.vdim : 0, latent ? H * A : 0, latent ? 0 : rows, latent ? 0 : rows,
-                 L.window, L.chunk, rows, L.vdim, 1, L.scale, L.temp, L.sink, L.value_rope, out, ldo, 2000000000ull, g.status};
+                 L.window, L.chunk, rows, L.vdim, 1, L.scale, L.temp, L.sink, L.value_rope, out, ldo, 2000000000ull, g.status, nullptr, 0};
     s.stages = stages_for(s.split_slabs + s.rest_slabs, s.v_slabs);
-    return choose(m, s, stream);
+    return choose<false>(m, s, stream);
 }
 
 cudaError_t flash_cache(const CacheAttention& a, cudaStream_t stream) {
@@ -484,8 +520,9 @@ cudaError_t flash_cache(const CacheAttention& a, cudaStream_t stream) {
     m.k_rest = m.k;
     constexpr int kAll = 1 << 30;
     FlashShape s{a.n, a.pos0, a.heads, a.heads / a.kv_heads, slabs, 0, slabs, stages_for(slabs, slabs), a.dim, a.dim, 0, 0, 0, kAll, 0, kAll,
-                 a.dim, 1, a.scale, nullptr, nullptr, nullptr, a.out, (int64_t)a.heads * a.dim, 2000000000ull, a.status};
-    return choose(m, s, stream);
+                 a.dim, 1, a.scale, nullptr, nullptr, nullptr, a.out, (int64_t)a.heads * a.dim, 2000000000ull, a.status,
+                 a.v, (int64_t)a.kv_heads * a.dim};
+    return choose<true>(m, s, stream);
 }
 
 }  // namespace mkbh

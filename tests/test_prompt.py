@@ -5,6 +5,7 @@ import torch
 
 from megakernels_b200.demos.latency.scheduler import LatencyScheduleOptions, covers_model
 from megakernels_b200.llama import LlamaConfig
+from megakernels_b200.scheduler import assign_to_sms, tensorize_instructions
 from oracle.llama_ref import TorchReferenceModel, assert_logits_parity
 from tests.gpu_utils import interpreter, make_pair, rel_err
 from tests.oracle_utils import build_model, build_schedule, seeded_tokens
@@ -93,3 +94,73 @@ def test_calls_that_stay_a_step_per_token():
     assert int(replayed) == int(torch.argmax(schedule.globs.logits)) == int(token)
     gen.replace_with_noops()
     assert not gen._takes_prompts(12)
+
+
+def own_weight_model(seed):
+    """One layer at the 1B widths in which head j's attention leaves ``p_j sum |v_j| - h_j`` in element j of the residual
+    stream and then in logit j, exact but for the attention's own rounding: other positions' values and the
+    feed-forward are zero, ``h_j`` (the last token's embedding) takes off nearly all of it."""
+    model = build_model(CONFIGS["1b"](num_hidden_layers=1), 700, device="cuda")
+    globs = build_schedule(model).globs
+    tensorize_instructions(globs, assign_to_sms("rr", instructions=[], sm_count=globs.sm_count()))
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    draw = lambda *shape: torch.randn(*shape, generator=gen, device="cuda")  # noqa: E731
+    H, D, Hq, Hkv = 2048, 64, 32, 8
+    for name in ("qkv_proj_weights", "o_proj_weights", "down_proj_weights"):
+        getattr(globs, name).zero_()
+    for w in (globs.attn_ln_weights, globs.mlp_ln_weights, globs.lm_head_norm_weights):
+        w.fill_(1.0)
+    wk = draw(Hkv, D, H) * (2.0 * (H / 2)) ** -0.5
+    wk[:, :, :Hq] = 0
+    gain = torch.tensor([0.125, 0.25, 0.09, 0.19], device="cuda")  # own scores of about -8 gain: never a row's maximum
+    wq = -(gain.view(1, 4, 1, 1) * wk.view(Hkv, 1, D, H)).reshape(Hq * D, H)
+    wv = draw(Hkv * D, H) * 3e-4  # (so that h_j hardly counts in the row's norm)
+    wv[:, : H // 2] = 0  # only the last token's embedding lies there
+    globs.qkv_proj_weights[0] = torch.cat([wq, wk.view(-1, H), wv])
+    globs.lm_head_weights.zero_()
+    globs.lm_head_weights[:Hq, :Hq].fill_diagonal_(1.0)
+    return model, globs, draw
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count,cached", [(2, 0), (3, 0), (130, 0), (2, 640), (40, 600)])
+def test_own_key_keeps_its_32_bit_weight(count, cached):
+    """A query's softmax weight of its own position is 32-bit, as in the step per token.  Rounding it to bf16 (up to 2^-8,
+    0.4 of that in the mean square) would move all entries of a head alike; the attention output's own rounding to bf16,
+    of that size too, moves each by itself, and the mean over 64 entries weighted by |v| (as good as 41 equal
+    ones) moves by 0.4 2^-8 / 6.4."""
+    model, globs, draw = own_weight_model(seed=count + cached)
+    H, D, Hq, Hkv = 2048, 64, 32, 8
+    for c in model.stacked_kv_cache:
+        c.zero_()
+    hidden = torch.zeros(count, H, device="cuda", dtype=torch.bfloat16)
+    hidden[:-1, Hq : H // 2] = draw(count - 1, H // 2 - Hq).bfloat16()
+    hidden[-1, H // 2 :] = draw(H // 2).bfloat16()
+    at = cached + torch.arange(count, device="cuda")
+    cos, sin = globs.rope_cos[at].double(), globs.rope_sin[at].double()
+    rounded = lambda x: x.to(torch.bfloat16).double()  # noqa: E731
+    w = globs.qkv_proj_weights[0].double()
+    for _ in range(3):  # (h_j changes the row's norm a little)
+        x = hidden.double()
+        act = rounded(x / (x.pow(2).mean(-1, keepdim=True) + globs.rms_norm_eps).sqrt())
+        q, k, v = (act @ w.T).split([Hq * D, Hkv * D, Hkv * D], dim=-1)
+        turned = []
+        for y, heads in ((q, Hq), (k, Hkv)):
+            y = y.view(count, heads, D // 2, 2)
+            c, s = cos.view(count, 1, D // 2, 2), sin.view(count, 1, D // 2, 2)
+            turned.append(rounded(torch.stack([y[..., 0] * c[..., 0] - y[..., 1] * s[..., 0],
+                                               y[..., 1] * c[..., 1] + y[..., 0] * s[..., 1]], -1)).view(count, heads, D))
+        q, k, v = turned[0][-1], turned[1].repeat_interleave(Hq // Hkv, 1), rounded(v[-1]).view(Hkv, D).repeat_interleave(Hq // Hkv, 0)
+        score = torch.cat([torch.zeros(Hq, cached, device="cuda", dtype=torch.float64), torch.einsum("hd,thd->ht", q, k) * globs.attn_scale], 1)
+        p = torch.softmax(score, -1)[:, -1]
+        assert (score[:, -1] < score.amax(-1)).all()
+        signs = v.sign()
+        globs.o_proj_weights[0, :Hq] = torch.block_diag(*signs.float().unsqueeze(1)).bfloat16()
+        whole = p * (signs * v).sum(-1)
+        hidden[-1, :Hq] = -whole.bfloat16()
+    x = hidden[-1].double()
+    x[:Hq] += whole
+    logits_scale = 1 / (x.pow(2).mean() + globs.rms_norm_eps).sqrt()
+    interpreter().module.sync_status(interpreter().prompt(globs, hidden, cached, True))
+    error = (globs.logits[:Hq].double().view(-1) / logits_scale - x[:Hq]) / whole
+    assert float(error.pow(2).mean().sqrt()) < 2 * 0.4 * 2.0**-8 / 6.4, error
