@@ -6,7 +6,7 @@
 // accumulators back while the other is being filled.  The epilogue goes through shared memory so
 // that stores are row segments: plus the bias, times the layer scale into the 32-bit residual stream,
 // in bf16, the gated unit of neighbouring columns in bf16, the gated unit of two matrices (a tile is then
-// as many rows of either), or rotated into the queries and the key/value cache.
+// as many rows of either), rotated into the queries and the key/value cache, or into a fixed-point residual stream.
 #include "hybrid_kernels.h"
 #include "hybrid_tcgen05.cuh"
 
@@ -41,9 +41,12 @@ struct Shape {
 };
 
 // What the epilogue can do: a build per group of results, so that one group's code does not cost the others registers.
-enum class Group { kPlain, kSilu, kRope };  // kSilu: two weight matrices, kBN / 2 columns of each per tile
+enum class Group { kPlain, kSilu, kRope, kFixed };  // kSilu: two weight matrices, kBN / 2 columns of each per tile
 template <int kBN> constexpr int kPartRow = kBN + 4;  // floats of a row of partial sums
-constexpr Group group_of(Result r) { return r == Result::kSilu ? Group::kSilu : r == Result::kRope ? Group::kRope : Group::kPlain; }
+constexpr Group group_of(Result r) {
+    return r == Result::kSilu ? Group::kSilu : r == Result::kRope ? Group::kRope : r == Result::kFixed ? Group::kFixed : Group::kPlain;
+}
+__device__ __forceinline__ long long fixed_of(float x) { return __float2ll_rn(x * mkb::kResidualScale); }
 
 // columns n (even) and n + 1 of token t, where a thread has just these
 template <Group kGroup>
@@ -61,6 +64,10 @@ __device__ __forceinline__ void put(const GemmEpilogue& e, int N, int t, int n, 
         }
         bf16* o = at < 0 ? p.q + (size_t)t * p.q_cols + n : (at < p.k_cols ? p.k + at : p.v + (at - p.k_cols)) + (size_t)(p.pos0 + t) * p.k_cols;
         *reinterpret_cast<uint32_t*>(o) = mkb::pack_bf16x2(x, y);
+    } else if constexpr (kGroup == Group::kFixed) {  // (no other thread writes these)
+        longlong2* o = reinterpret_cast<longlong2*>(static_cast<long long*>(e.cast) + (size_t)t * e.ld + n);
+        const longlong2 v = *o;
+        *o = make_longlong2(v.x + fixed_of(x), v.y + fixed_of(y));
     } else if (kGroup == Group::kSilu || e.what == Result::kCast) {
         bf16* o = static_cast<bf16*>(e.cast) + (size_t)t * e.ld + n;
         if (n + 1 < N) *reinterpret_cast<uint32_t*>(o) = mkb::pack_bf16x2(x, y);
@@ -288,6 +295,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                     }
                 }
                 const int n = n0 + c0 + lane;
+                if (kGroup == Group::kFixed && n < s.N) {
+                    long long* o = static_cast<long long*>(e.cast) + (size_t)m0 * e.ld + n;
+                    for (int i = 0; i < rows; ++i) mkb::red_add_u64(o + (size_t)i * e.ld, (unsigned long long)fixed_of(tr[i * kEpiStride + lane]));
+                }
                 if (kGroup == Group::kPlain && n < s.N && e.what <= Result::kAdd) {
                     float* o = e.out + (size_t)m0 * e.ld + n;
                     if (e.what == Result::kAdd) {
@@ -444,6 +455,7 @@ cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, in
     switch (group_of(e.what)) {
         case Group::kSilu: return choose<Group::kSilu>(A, lda, W, W2, ldw, s, e, sms, st);
         case Group::kRope: return choose<Group::kRope>(A, lda, W, W2, ldw, s, e, sms, st);
+        case Group::kFixed: return choose<Group::kFixed>(A, lda, W, W2, ldw, s, e, sms, st);
         default: return choose<Group::kPlain>(A, lda, W, W2, ldw, s, e, sms, st);
     }
 }

@@ -12,6 +12,7 @@ enum class Result {
     kGlu,    // cast[t, n / 2] = clamped gated unit of columns n (gate) and n + 1
     kSilu,   // cast[t, n] = silu(gate[n]) * up[n], two weight matrices (bf16 only)
     kRope,   // queries, keys and values to their places, the first two rotated (bf16 only)
+    kFixed,  // sums[t, n] += acc in the decode kernel's fixed-point format of the residual stream (bf16 only, N even)
 };
 // Where kRope puts a row of [queries | keys | values]: the keys and values of token t are row pos0 + t of
 // caches [position, key columns].  Neighbours (2i, 2i + 1) of a head are turned by the tables [position, dim].
@@ -34,6 +35,7 @@ struct GemmEpilogue {
     static GemmEpilogue to(void* out, int64_t ld) { return {Result::kCast, nullptr, out, ld, nullptr, nullptr, 0.f, 0.f}; }
     static GemmEpilogue glu(void* out, int64_t ld, float limit, float alpha) { return {Result::kGlu, nullptr, out, ld, nullptr, nullptr, limit, alpha}; }
     static GemmEpilogue silu(void* out, int64_t ld) { return {Result::kSilu, nullptr, out, ld, nullptr, nullptr, 0.f, 0.f}; }
+    static GemmEpilogue add_fixed(long long* sums, int64_t ld) { return {Result::kFixed, nullptr, sums, ld, nullptr, nullptr, 0.f, 0.f}; }
     static GemmEpilogue rotate(const RopeTarget& r) { return {Result::kRope, nullptr, nullptr, 0, nullptr, nullptr, 0.f, 0.f, r}; }
 };
 

@@ -6,7 +6,7 @@ namespace mkb {
 
 // Layout of a prompt's workspace, every part 256-byte aligned.
 struct PromptBuffers {
-    float* x;  // residual stream
+    long long* sums;  // what the layers have added to the embeddings, in the decode kernel's fixed-point format
     __nv_bfloat16 *act, *q, *ffn;
     size_t total = 0;
     PromptBuffers(const MkbGlobals& g, int tokens, void* base) {
@@ -17,7 +17,7 @@ struct PromptBuffers {
             return at;
         };
         const size_t heads = (size_t)g.num_attention_heads * g.head_dim, hidden = g.hidden_size;
-        x = reinterpret_cast<float*>(take(hidden * 4));
+        sums = reinterpret_cast<long long*>(take(hidden * 8));
         act = reinterpret_cast<__nv_bfloat16*>(take((hidden > heads ? hidden : heads) * 2));
         q = reinterpret_cast<__nv_bfloat16*>(take(heads * 2));
         ffn = reinterpret_cast<__nv_bfloat16*>(take((size_t)g.intermediate_size * 2));

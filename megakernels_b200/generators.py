@@ -209,7 +209,7 @@ class MK_Generator(Generator):
             output_ids = self.run(input_ids, pos_id=pos_id)
             output_tokens[:, in_pos + 1] = output_ids.reshape(-1)
 
-    # Tokens of a prompt that go through the layers together: the activations of a portion, 60 KB a token
+    # Tokens of a prompt that go through the layers together: the activations of a portion, 76 KB a token
     # at the 8B widths, are a workspace of this many tokens.
     prompt_portion = 2048
 

@@ -483,9 +483,12 @@ def mk_llama_prompt(*args, hidden, pos0, want_logits, stream=None, **kw):
     """Enqueue a prompt's tokens at once (``mkb_prompt``); other arguments as :func:`mk_llama`.
 
     ``hidden`` holds their embeddings ``[tokens, H]``, the first of position ``pos0``; ``pos_id`` is the
-    last one's position.  Keys and values go to the caches, the last token's logits (``want_logits``) to ``logits``.
+    last one's position.  Keys and values go to the caches, the last token's logits and what the layers added to its
+    embedding (``want_logits``) to ``logits`` and ``residual_acc``.
     """
     lib = load_library()
+    if kw.get("residual_acc") is None and kw.get("tp") is None:
+        kw["residual_acc"] = _own_residual_acc(args[16], stream)
     g = pack_globals(*args, **kw)
     p = MkbPrompt()
     p.struct_bytes = ctypes.sizeof(MkbPrompt)

@@ -164,3 +164,28 @@ def test_own_key_keeps_its_32_bit_weight(count, cached):
     interpreter().module.sync_status(interpreter().prompt(globs, hidden, cached, True))
     error = (globs.logits[:Hq].double().view(-1) / logits_scale - x[:Hq]) / whole
     assert float(error.pow(2).mean().sqrt()) < 2 * 0.4 * 2.0**-8 / 6.4, error
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,count,portion", [("1b", 2, 2048), ("8b", 61, 2048), ("1b", 300, 128), ("1b", 400, 2048)])
+def test_residual_stream_of_the_last_token(shape, count, portion):
+    """As after a step: embedding plus the exact sum, in steps of 2^-32, of what the layers added (fp32 sums would
+    have lost the low bits of the smaller terms)."""
+    from megakernels_b200.generators import MK_Generator
+
+    _, _, model, schedule = make_pair(CONFIGS[shape](), count, 0)
+    globs = schedule.globs
+    ids = torch.tensor(seeded_tokens(globs.vocab_size, count, seed=6)).cuda()
+    gen = MK_Generator(model, interpreter(), schedule)
+    gen.prompt_portion = portion
+    for pos in range(count):
+        gen.run(ids[pos].view(1, 1), pos)
+    gen.check()
+    want, hidden = globs.residual_stream(), globs.hidden_states.clone()
+    globs.residual_acc.fill_(1 << 40)
+    gen.prefill(ids)
+    gen.check()
+    assert torch.equal(globs.hidden_states, hidden)
+    assert rel_err(globs.residual_stream(), want) <= 2e-2
+    sums = globs.residual_acc.double() * 2.0**-32
+    assert (sums.float().double() != sums).float().mean() > 0.25
