@@ -24,6 +24,7 @@ import math
 from dataclasses import dataclass
 
 import torch
+from torch import Tensor
 
 from megakernels_b200.demos.latency.instructions import (
     AttentionReduction,
@@ -513,25 +514,64 @@ def split_at_collectives(instructions: list[Instruction]) -> list[tuple[list[Ins
     return segments
 
 
-def covers_model(globs: Globals, instructions: list[Instruction]) -> bool:
-    """Whether a single-sequence instruction list is the model's whole step: every block of every layer and the head."""
-    blocks: dict[tuple[int, int], int] = {}
-    for ins in instructions:
-        op, layer = ins.opcode(), getattr(ins, "layer_idx", 0)
-        if isinstance(ins, LayerNormDoubleMatVecSiLU):
-            n = len(ins.block_idxs)
-        elif isinstance(ins, (O_ProjResidual, DownProjResidual)):
-            n = ins.end_block_idx - ins.start_block_idx
-        elif isinstance(ins, (LayerNorm_QKV_MatVecRopeAppend, RMS_LM_Head)):
-            n = ins.end_output_block_idx - ins.start_output_block_idx
+def covers_model(globs: Globals, instructions: list[Instruction] | Tensor) -> bool:
+    """Whether single-sequence instructions are the model's whole step and nothing else: every block of every layer once,
+    every key/value head's attention and the head.  ``instructions`` may be the tensor that the kernel reads."""
+    if isinstance(instructions, Tensor):
+        words = instructions.reshape(-1, instructions.shape[-1])
+        words = words[words[:, 0] != 0].tolist()
+    else:
+        words = [ins.serialize() for ins in instructions if not isinstance(ins, NoOp)]
+    blocks: dict[tuple, list[tuple[int, int]]] = {}  # (opcode, layer, column slice): ranges of blocks
+    partials: dict[tuple, list[int]] = {}  # (layer, key/value head, count): partial indices
+    merges: dict[tuple, list[tuple]] = {}  # (layer, first head): (count, terminal, merged partials)
+    for op, *a in words:
+        if op == LayerNorm_QKV_MatVecRopeAppend.opcode():
+            blocks.setdefault((op, a[0], 0), []).append((a[1], a[2]))
+        elif op in (O_ProjResidual.opcode(), DownProjResidual.opcode()):
+            blocks.setdefault((op, a[0], a[3]), []).append((a[1], a[2]))
+        elif op == LayerNormDoubleMatVecSiLU.opcode():
+            blocks.setdefault((op, a[0], 0), []).extend((b, b + 1) for b in a[2 : 2 + a[1]])
+        elif op == RMS_LM_Head.opcode():
+            blocks.setdefault((op, 0, 0), []).append((a[0], a[1]))
+        elif op == PartialAttention.opcode() and not any(a[4:5]):  # (sequence 0)
+            partials.setdefault((a[0], a[1], a[2]), []).append(a[3])
+        elif op == AttentionReduction.opcode() and not any(a[5 + a[4] : 7 + a[4]]):  # (into the output, sequence 0)
+            merges.setdefault((a[0], a[1]), []).append((a[2], a[3], a[5 : 5 + a[4]]))
         else:
-            continue
-        blocks[op, layer] = blocks.get((op, layer), 0) + n
-    rows = (globs.num_attention_heads + 2 * globs.num_kv_heads) * globs.head_dim
-    want = {(RMS_LM_Head.opcode(), 0): globs.vocab_size // globs.lm_head_block_size}
+            return False
+
+    want = {(RMS_LM_Head.opcode(), 0, 0): globs.vocab_size // globs.lm_head_block_size}
+    count_of = {(layer, kv): count for layer, kv, count in partials}  # (a second count of a head is caught by the lengths)
+    want_merges: dict[tuple, list[tuple]] = {}
+    gqa = globs.num_attention_heads // globs.num_kv_heads
     for layer in range(globs.num_hidden_layers):
-        want[LayerNorm_QKV_MatVecRopeAppend.opcode(), layer] = rows // globs.qkv_block_size
-        want[O_ProjResidual.opcode(), layer] = globs.hidden_size // globs.o_proj_block_size * globs.num_o_proj_col_splits()
-        want[LayerNormDoubleMatVecSiLU.opcode(), layer] = globs.intermediate_size // globs.up_gate_proj_block_size
-        want[DownProjResidual.opcode(), layer] = globs.hidden_size // globs.down_proj_block_size * globs.num_down_proj_col_splits()
-    return blocks == want
+        want[LayerNorm_QKV_MatVecRopeAppend.opcode(), layer, 0] = globs.num_total_heads() * globs.head_dim // globs.qkv_block_size
+        want[LayerNormDoubleMatVecSiLU.opcode(), layer, 0] = globs.intermediate_size // globs.up_gate_proj_block_size
+        for split in range(globs.num_o_proj_col_splits()):
+            want[O_ProjResidual.opcode(), layer, split] = globs.hidden_size // globs.o_proj_block_size
+        for split in range(globs.num_down_proj_col_splits()):
+            want[DownProjResidual.opcode(), layer, split] = globs.hidden_size // globs.down_proj_block_size
+        for kv in range(globs.num_kv_heads):
+            count = count_of.get((layer, kv), 0)
+            if count < 1 or (count > 1 and globs.skip_attn_reduction and not globs.merge_in_last_partial):
+                return False
+            if not (globs.skip_attn_reduction or globs.merge_in_last_partial):
+                for head in range(kv * gqa, (kv + 1) * gqa, globs.attn_reduction_size):
+                    want_merges[layer, head] = [(count, 1, list(range(count)))]
+
+    def once(ranges: list[tuple[int, int]], count: int) -> bool:
+        ends = [0]
+        for start, end in sorted(ranges):
+            if start != ends[-1] or end <= start:
+                return False
+            ends.append(end)
+        return ends[-1] == count
+
+    return (
+        blocks.keys() == want.keys()
+        and all(once(ranges, want[key]) for key, ranges in blocks.items())
+        and len(partials) == len(count_of) == globs.num_hidden_layers * globs.num_kv_heads
+        and all(sorted(parts) == list(range(key[2])) for key, parts in partials.items())
+        and merges == want_merges
+    )

@@ -19,6 +19,11 @@ from megakernels_b200.model_types import BatchState
 from megakernels_b200.scheduler import Schedule
 
 
+def _edits(t: Tensor) -> int:
+    """How often a tensor was written in place (torch does not count that for tensors made in inference mode)."""
+    return 0 if t.is_inference() else t._version
+
+
 class Generator:
     def generate(
         self,
@@ -94,8 +99,9 @@ class MK_Generator(Generator):
                 globs.batch_size, dtype=torch.int32, device=globs.hidden_states.device
             )
 
-        # prompts need not go token by token when the schedule is the model's whole step
-        self._whole = has_head and globs.batch_size == 1 and covers_model(globs, schedule.get_linear_instructions())
+        # prompts need not go token by token when the instructions are the model's whole step
+        whole = has_head and globs.batch_size == 1 and globs.tp is None and covers_model(globs, globs.instructions)
+        self._whole = (globs.instructions, _edits(globs.instructions)) if whole else None
 
     def fill(self):
         """Reset the per-token VM state: barrier counters and residual accumulators."""
@@ -109,7 +115,7 @@ class MK_Generator(Generator):
 
     def replace_with_noops(self):
         self.schedule.globs.instructions.zero_()
-        self._whole = False
+        self._whole = None
 
     # -- CUDA-graph replay of one decode step -------------------------------- #
     def enable_cuda_graph(self, warmup_pos: int = 0):
@@ -216,15 +222,17 @@ class MK_Generator(Generator):
     def _takes_prompts(self, count: int) -> bool:
         """Whether a prompt of ``count`` tokens goes through the layers at once (``mkb_prompt``).
 
-        Only where that is the same as a step per token: the whole model's schedule on the library's own
-        interpreter, one sequence on one GPU, no part of a step left out or replaced, every position inside
-        cache and tables.  Shorter prompts cost less as steps.
+        Only where that is the same as a step per token: the whole model's instructions (those that were looked at when
+        the generator was made, not edited since) on the library's own interpreter, one sequence on one GPU, no part of a
+        step left out or replaced, every position inside cache and tables.
         """
         globs, interp = self.schedule.globs, self.interpreter
         own = lambda f, cls, name: getattr(f, "__func__", None) is getattr(cls, name)  # noqa: E731
         return (
             count >= self.shortest_prompt
-            and self._whole
+            and self._whole is not None
+            and globs.instructions is self._whole[0]
+            and _edits(globs.instructions) == self._whole[1]
             and not (self.skip_mk or self.skip_rest)
             and self.barrier_fill_val == 0
             and globs.tp is None
@@ -305,7 +313,7 @@ class Hybrid_Generator(MK_Generator):
         self.model, self.interpreter, self.schedule = model, interpreter, schedule
         self.skip_mk, self.skip_rest = kw.get("skip_mk", False), kw.get("skip_rest", False)
         self.last_call = None
-        self._whole = False  # (prefill and feed are this class's own)
+        self._whole = None  # (prefill and feed are this class's own)
 
     def fill(self):
         """Nothing to reset: counters are cleared by the launch, recurrent state at position 0."""

@@ -19,14 +19,26 @@ CONFIGS = {
 
 def test_only_whole_schedules_count_as_the_model():
     model = build_model(CONFIGS["1b"](), 64)
-    for options in (None, LatencyScheduleOptions(num_attention_partitions=3, coalesce_o_proj=True, merge_in_last_partial=True)):
+    for options in (None, LatencyScheduleOptions(num_attention_partitions=3, coalesce_o_proj=True, merge_in_last_partial=True),
+                    LatencyScheduleOptions(num_attention_partitions=2)):
         schedule = build_schedule(model, options)
         instructions = schedule.get_linear_instructions()
         assert covers_model(schedule.globs, instructions)
-        for dropped in (0, len(instructions) // 2, -1):
-            rest = [x for i, x in enumerate(instructions) if i != dropped % len(instructions)]
-            kind = type(instructions[dropped]).__name__
-            assert covers_model(schedule.globs, rest) == (kind in ("PartialAttention", "AttentionReduction")), kind
+        tensorize_instructions(schedule.globs, assign_to_sms("rr", schedule=schedule))
+        assert covers_model(schedule.globs, schedule.globs.instructions)
+        of_kind = {type(x): i for i, x in enumerate(instructions)}  # the last one of each
+        assert len(of_kind) == 6 + (not schedule.globs.skip_attn_reduction and not schedule.globs.merge_in_last_partial)
+        for kind, at in [*of_kind.items(), (None, 0), (None, len(instructions) // 2)]:
+            rest = instructions[:at] + instructions[at + 1 :]
+            assert not covers_model(schedule.globs, rest), kind
+            # one twice, also in another's place: as many blocks as before
+            assert not covers_model(schedule.globs, instructions + [instructions[at]]), kind
+            other = next(i for i, x in enumerate(instructions) if type(x) is type(instructions[at]) and i != at)
+            assert not covers_model(schedule.globs, rest + [instructions[other]]), kind
+        edited = schedule.globs.instructions.clone()
+        sm, place = (edited[:, :, 0] == 2).nonzero()[0].tolist()
+        edited[sm, place] = 0  # a no-op where attention was
+        assert not covers_model(schedule.globs, edited)
     for kw in (dict(layer_limit=1), dict(stop_after_op="oproj")):
         schedule = build_schedule(model, **kw)
         assert not covers_model(schedule.globs, schedule.get_linear_instructions())
@@ -189,3 +201,20 @@ def test_residual_stream_of_the_last_token(shape, count, portion):
     assert rel_err(globs.residual_stream(), want) <= 2e-2
     sums = globs.residual_acc.double() * 2.0**-32
     assert (sums.float().double() != sums).float().mean() > 0.25
+
+
+@pytest.mark.gpu
+def test_edited_or_replaced_instructions_run_as_steps():
+    from megakernels_b200.generators import MK_Generator
+
+    _, _, model, schedule = make_pair(CONFIGS["1b"](), 40, 0)
+    globs = schedule.globs
+    gen = MK_Generator(model, interpreter(), schedule)
+    assert gen._takes_prompts(8)
+    whole, globs.instructions = globs.instructions, globs.instructions.clone()
+    assert not gen._takes_prompts(8)
+    globs.instructions = whole
+    assert gen._takes_prompts(8)
+    globs.instructions[globs.instructions[:, :, 0] == 2] = 0
+    assert not gen._takes_prompts(8)
+    assert not MK_Generator(model, interpreter(), schedule)._takes_prompts(8)
