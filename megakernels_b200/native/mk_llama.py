@@ -421,6 +421,15 @@ def _stream_handle(stream) -> int:
     return int(stream.cuda_stream)
 
 
+def _as_stream(stream, device) -> torch.cuda.Stream:
+    """The stream object of ``stream`` (a stream, a handle, or None for the current one)."""
+    if stream is None:
+        return torch.cuda.current_stream(device)
+    if isinstance(stream, int):  # (an external stream of handle 0 would be another one from torch's pool)
+        return torch.cuda.ExternalStream(stream, device=device) if stream else torch.cuda.default_stream(device)
+    return stream
+
+
 def mk_llama(
     *args,
     stream=None,
@@ -497,8 +506,11 @@ def mk_llama_prompt(*args, hidden, pos0, want_logits, stream=None, **kw):
         raise ValueError(f"hidden must be [tokens, {g.hidden_size}], got {tuple(hidden.shape)}")
     p.tokens, p.pos0, p.want_logits = hidden.shape[0], pos0, int(want_logits)
     p.workspace_bytes = lib.mkb_prompt_bytes(ctypes.byref(g), p.tokens)
-    # (allocated on the current stream, which has to be the one that is launched on)
-    workspace = torch.empty(p.workspace_bytes, dtype=torch.uint8, device=hidden.device)
+    stream = _as_stream(stream, hidden.device)
+    with torch.cuda.stream(stream):  # (given back when this returns, to that stream alone: later work on it runs after the kernels)
+        workspace = torch.empty(p.workspace_bytes, dtype=torch.uint8, device=hidden.device)
+    if stream != torch.cuda.current_stream(hidden.device):
+        hidden.record_stream(stream)
     p.workspace = workspace.data_ptr()
     rc = lib.mkb_prompt(ctypes.byref(g), ctypes.byref(p), ctypes.c_void_p(_stream_handle(stream)))
     if rc != 0:

@@ -3,6 +3,7 @@
 import pytest
 import torch
 
+from megakernels_b200.demos.latency.mk import interpret_with_mk
 from megakernels_b200.demos.latency.scheduler import LatencyScheduleOptions, covers_model
 from megakernels_b200.llama import LlamaConfig
 from megakernels_b200.scheduler import assign_to_sms, tensorize_instructions
@@ -218,3 +219,38 @@ def test_edited_or_replaced_instructions_run_as_steps():
     globs.instructions[globs.instructions[:, :, 0] == 2] = 0
     assert not gen._takes_prompts(8)
     assert not MK_Generator(model, interpreter(), schedule)._takes_prompts(8)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("as_handle", [False, True])
+def test_prompt_on_another_stream_keeps_its_workspace(as_handle):
+    """The launches wait on a busy stream; what the current stream allocates and fills meanwhile is other memory."""
+    from megakernels_b200.generators import MK_Generator
+
+    count = 200
+    _, _, model, schedule = make_pair(CONFIGS["1b"](), count, 0)
+    globs = schedule.globs
+    MK_Generator(model, interpreter(), schedule)
+    module = interpreter().module
+    embed = model.model.embed_tokens.embed_tokens.weight
+    ids = torch.tensor(seeded_tokens(globs.vocab_size, count, seed=7)).cuda()
+    globs.pos_id = count - 1
+
+    def prompt(hidden, stream):
+        return interpret_with_mk(globs, lambda *args, **kw: module.mk_llama_prompt(
+            *args, hidden=hidden, pos0=0, want_logits=True, **{**kw, "stream": stream}))
+
+    module.sync_status(prompt(embed[ids], None))
+    want = globs.logits.clone()
+    globs.logits.zero_()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)  # some 50 ms
+    call = prompt(embed[ids], side.cuda_stream if as_handle else side)
+    assert not side.query()
+    junk = [torch.full((1 << k,), 255, dtype=torch.uint8, device="cuda") for k in range(16, 25) for _ in range(4)]  # every size up to 16 MB
+    torch.cuda.current_stream().synchronize()
+    module.sync_status(call, stream=side)
+    assert torch.equal(globs.logits, want)
+    del junk
