@@ -160,10 +160,6 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
                 drain(k_full(i % S), (uint32_t)(i / S));
                 drain(v_full(i % S), (uint32_t)(i / S));
             }
-        } else {  // a bounded time for whatever was issued
-            const unsigned long long end = mkb::globaltimer_ns() + 1000000ull;
-            while (mkb::globaltimer_ns() < end) {
-            }
         }
     } else if (warp == 1 && lane == 0) {
         const uint32_t s_desc = tc_idesc(kRows, kTile), o_desc = tc_idesc(kRows, kE, true);
@@ -392,6 +388,7 @@ __global__ void __launch_bounds__(kFlashThreads, 1) flash_tc_kernel(const __grid
     }
     tc_before_sync();
     __syncthreads();
+    if (*ctl) tc_settle();
     if constexpr (kShare) {
         tc_cluster_sync();
         for (int i = part + parts * warp; i < nq; i += parts * (kFlashThreads / 32)) {

@@ -324,6 +324,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*ctl) tc_settle();  // (the roles leave one by one then, the drain above too)
     if constexpr (kShare) {
         tc_cluster_sync();
         const int m0 = (worker % s.tiles_m) * kBM, n0 = (worker / s.tiles_m) * wide, rows = min(kBM, s.T - m0);

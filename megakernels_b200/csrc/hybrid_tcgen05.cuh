@@ -36,6 +36,14 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile 
     return mkb::mbar_try_wait(bar, parity) || tc_wait_slow(bar, parity, dead, timeout_ns, status, role);
 }
 
+// A CTA in which a wait has given up: a bounded time in which the copies and MMAs that were issued end (they take
+// microseconds), before shared memory and tensor memory go away.
+__device__ __noinline__ void tc_settle() {
+    const unsigned long long end = mkb::globaltimer_ns() + 1000000ull;
+    while (mkb::globaltimer_ns() < end) {
+    }
+}
+
 // one lane of a converged warp, always the same one
 __device__ __forceinline__ bool tc_elect() {
     uint32_t r;
