@@ -311,9 +311,10 @@ int mkb_launch(const MkbGlobals *g, void *cuda_stream);
  * A prompt's tokens at once (no counterpart in the reference, whose prompts go through its torch model,
  * scripts/generate.py:125-137): `tokens` rows of embeddings, the first at position `pos0` of sequence 0, whose
  * earlier positions are in the caches.  Writes their keys and values into the caches and, with `want_logits`, the
- * last token's logits and, in `residual_acc`, what the layers added to its embedding.  `g` is that of mkb_launch; batch and tensor-parallel launches, residual_scale > 1 and a
- * head_dim other than 64 or 128 are MKB_ERR_UNSUPPORTED.  Instructions, barriers and the activation
- * vectors of `g` are not touched.  `workspace`: mkb_prompt_bytes(g, tokens) bytes, 256-byte aligned.
+ * last token's logits and, in `residual_acc`, what the layers added to its embedding.  `g` is that of mkb_launch
+ * (`wait_timeout_ms` holds for every wait of these kernels too); batch and tensor-parallel launches, residual_scale > 1,
+ * MKB_FLAG_RECORD_TIMINGS and a head_dim other than 64 or 128 are MKB_ERR_UNSUPPORTED.  Instructions, barriers and the
+ * activation vectors of `g` are not touched.  `workspace`: mkb_prompt_bytes(g, tokens) bytes, 256-byte aligned.
  */
 typedef struct MkbPrompt {
     uint32_t struct_bytes;

@@ -544,6 +544,8 @@ size_t mkb_prompt_bytes(const MkbGlobals* g, int32_t tokens) { return g && token
 
 int mkb_prompt(const MkbGlobals* g, const MkbPrompt* p, void* cuda_stream) {
     if (!p || p->struct_bytes != sizeof(MkbPrompt)) return fail(MKB_ERR_INVALID_ARGUMENT, "prompt: NULL or another struct size");
+    if (g && (g->flags & MKB_FLAG_RECORD_TIMINGS))
+        return fail(MKB_ERR_UNSUPPORTED, "prompt: no instructions run, so there are no timings to record");
     int* status = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_mutex);

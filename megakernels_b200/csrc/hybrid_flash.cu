@@ -501,7 +501,7 @@ cudaError_t flash_tc(const MkbhGlobals& g, const MkbhLayer& L, bf16* out, int64_
     if (B > 0 && (e = tc_map(&m.k_rest, src.shared, B, rows, src.shared_ld, 64, kTile)) != cudaSuccess) return e;
     FlashShape s{g.num_tokens, g.pos0, H, src.per, slabs_of(A), B > 0 ? slabs_of(B) : 0, slabs_of(L.vdim), 0,
                  latent ? A : 0, latent ? L.vdim : 0, latent ? H * A : 0, latent ? 0 : rows, latent ? 0 : rows,
-                 L.window, L.chunk, rows, L.vdim, 1, L.scale, L.temp, L.sink, L.value_rope, out, ldo, 2000000000ull, g.status, nullptr, 0};
+                 L.window, L.chunk, rows, L.vdim, 1, L.scale, L.temp, L.sink, L.value_rope, out, ldo, kWaitNs, g.status, nullptr, 0};
     s.stages = stages_for(s.split_slabs + s.rest_slabs, s.v_slabs);
     return choose<false>(m, s, stream);
 }
@@ -517,7 +517,7 @@ cudaError_t flash_cache(const CacheAttention& a, cudaStream_t stream) {
     m.k_rest = m.k;
     constexpr int kAll = 1 << 30;
     FlashShape s{a.n, a.pos0, a.heads, a.heads / a.kv_heads, slabs, 0, slabs, stages_for(slabs, slabs), a.dim, a.dim, 0, 0, 0, kAll, 0, kAll,
-                 a.dim, 1, a.scale, nullptr, nullptr, nullptr, a.out, (int64_t)a.heads * a.dim, 2000000000ull, a.status,
+                 a.dim, 1, a.scale, nullptr, nullptr, nullptr, a.out, (int64_t)a.heads * a.dim, a.timeout_ns, a.status,
                  a.v, (int64_t)a.kv_heads * a.dim};
     return choose<true>(m, s, stream);
 }

@@ -4,6 +4,8 @@
 
 namespace mkbh {
 
+constexpr unsigned long long kWaitNs = 2000000000ull;  // how long a kernel's waits go on before they give up
+
 // What a matrix product does with its result.
 enum class Result {
     kStore,  // out[t, n] = acc + bias[n]
@@ -43,7 +45,8 @@ struct GemmEpilogue {
 cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int T, int N, int K,
                      const GemmEpilogue& e, cudaStream_t s);
 cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, int T, int N, int K,
-                      const GemmEpilogue& e, int* status, cudaStream_t s, const bf16* W2 = nullptr);  // W2: kSilu's up rows
+                      const GemmEpilogue& e, int* status, cudaStream_t s, const bf16* W2 = nullptr,  // W2: kSilu's up rows
+                      unsigned long long timeout_ns = kWaitNs);
 
 // Causal attention of `n` queries from position pos0 on over a cache [position, kv head, dim] that holds
 // their own rows too; dim 64 or 128.  Nothing beyond row pos0 + n - 1 is read.
@@ -53,6 +56,7 @@ struct CacheAttention {
     int n, pos0, heads, kv_heads, dim;
     float scale;
     int* status;
+    unsigned long long timeout_ns;
 };
 cudaError_t flash_cache(const CacheAttention& a, cudaStream_t s);
 

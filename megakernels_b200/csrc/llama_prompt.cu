@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kNormThreads) prompt_norm_kernel(const bf16* h
 cudaError_t prompt_launch(const MkbGlobals& g, const MkbPrompt& p, int* status, cudaStream_t s) {
     const PromptBuffers b(g, p.tokens, p.workspace);
     const int n = p.tokens, H = g.hidden_size, F = g.intermediate_size, D = g.head_dim, Q = g.num_attention_heads * D, KV = g.num_kv_heads * D;
+    const unsigned long long wait = g.wait_timeout_ms ? g.wait_timeout_ms * 1000000ull : mkbh::kWaitNs;
     auto at = [](const void* w, size_t elements) { return static_cast<const bf16*>(w) + elements; };
     auto norm = [&](int row0, int rows, bool first, long long* last, const bf16* w) {
         cudaLaunchConfig_t c = {};
@@ -84,7 +85,7 @@ cudaError_t prompt_launch(const MkbGlobals& g, const MkbPrompt& p, int* status, 
                                   H, g.rms_norm_eps, w, b.act);
     };
     auto gemm = [&](const bf16* A, const bf16* W, int rows, int N, int K, const GemmEpilogue& e, const bf16* W2 = nullptr) {
-        return mkbh::gemm_bf16(A, K, W, K, rows, N, K, e, status, s, W2);
+        return mkbh::gemm_bf16(A, K, W, K, rows, N, K, e, status, s, W2, wait);
     };
     for (size_t i = 0; i < (size_t)g.num_layers; ++i) {
         const size_t cache = i * g.kv_batch * g.kv_max_len * KV;
@@ -92,7 +93,7 @@ cudaError_t prompt_launch(const MkbGlobals& g, const MkbPrompt& p, int* status, 
         MKB_TRY(norm(0, n, i == 0, nullptr, at(g.attn_ln_weights, i * H)));
         MKB_TRY(gemm(b.act, at(g.qkv_weights, i * (Q + 2 * KV) * H), n, Q + 2 * KV, H,
                      GemmEpilogue::rotate({b.q, k, v, Q, KV, D, p.pos0, static_cast<const float*>(g.rope_cos), static_cast<const float*>(g.rope_sin)})));
-        MKB_TRY(mkbh::flash_cache({b.q, k, v, b.act, n, p.pos0, g.num_attention_heads, g.num_kv_heads, D, g.attn_scale, status}, s));
+        MKB_TRY(mkbh::flash_cache({b.q, k, v, b.act, n, p.pos0, g.num_attention_heads, g.num_kv_heads, D, g.attn_scale, status, wait}, s));
         MKB_TRY(gemm(b.act, at(g.o_proj_weights, i * H * Q), n, H, Q, GemmEpilogue::add_fixed(b.sums, H)));
         MKB_TRY(norm(0, n, false, nullptr, at(g.mlp_ln_weights, i * H)));
         MKB_TRY(gemm(b.act, at(g.gate_proj_weights, i * F * H), n, F, H, GemmEpilogue::silu(b.ffn, F), at(g.up_proj_weights, i * F * H)));

@@ -1,5 +1,7 @@
 """Prompts of llama models: all tokens at once against one decode step per token and the oracle."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -7,6 +9,7 @@ from megakernels_b200.demos.latency.mk import interpret_with_mk
 from megakernels_b200.demos.latency.scheduler import LatencyScheduleOptions, covers_model
 from megakernels_b200.llama import LlamaConfig
 from megakernels_b200.scheduler import assign_to_sms, tensorize_instructions
+from megakernels_b200.native import mk_llama
 from oracle.llama_ref import TorchReferenceModel, assert_logits_parity
 from tests.gpu_utils import interpreter, make_pair, rel_err
 from tests.oracle_utils import build_model, build_schedule, seeded_tokens
@@ -254,3 +257,37 @@ def test_prompt_on_another_stream_keeps_its_workspace(as_handle):
     module.sync_status(call, stream=side)
     assert torch.equal(globs.logits, want)
     del junk
+
+
+def test_prompts_record_no_timings():
+    lib = mk_llama.load_library()
+    g, p = mk_llama.MkbGlobals(), mk_llama.MkbPrompt(struct_bytes=ctypes.sizeof(mk_llama.MkbPrompt))
+    g.flags = mk_llama.MKB_FLAG_RECORD_TIMINGS
+    assert lib.mkb_prompt(ctypes.byref(g), ctypes.byref(p), None) == 5  # MKB_ERR_UNSUPPORTED
+    assert "timings" in lib.mkb_last_error().decode()
+
+
+@pytest.mark.gpu
+def test_prompt_honours_the_wait_limit():
+    """A tile whose inner dimension takes longer than the limit: the epilogue's wait for it gives up and the status says so."""
+    model = build_model(CONFIGS["1b"](num_hidden_layers=1), 2048, device="cuda")
+    globs = build_schedule(model).globs
+    tensorize_instructions(globs, assign_to_sms("rr", instructions=[], sm_count=globs.sm_count()))
+    wide = 200 * 2048  # 6,400 steps of at least 0.26 us (the tensor cores' rate) where the feed-forward comes back
+    up = torch.zeros(1, wide, 2048, device="cuda", dtype=torch.bfloat16)
+    globs.up_proj_weights = globs.gate_proj_weights = up
+    globs.down_proj_weights = up.view(1, 2048, wide)
+    globs.silu_out = torch.zeros(wide, device="cuda", dtype=torch.bfloat16)
+    globs.barriers = torch.zeros(1, globs.barriers.shape[1], 256, device="cuda", dtype=torch.int32)
+    hidden = torch.randn(2048, 2048, device="cuda").bfloat16()
+    module, globs.pos_id = interpreter().module, 2047
+
+    def prompt(**kw):
+        call = interpret_with_mk(globs, lambda *args, **rest: module.mk_llama_prompt(
+            *args, hidden=hidden, pos0=0, want_logits=True, **rest, **kw))
+        return module.sync_status(call)
+
+    prompt()
+    with pytest.raises(RuntimeError, match="TIMEOUT"):
+        prompt(wait_timeout_ms=1)
+    prompt()  # the device and the status record are as before
