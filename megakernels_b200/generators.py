@@ -255,9 +255,12 @@ class MK_Generator(Generator):
 
     def _prompt(self, ids: Tensor) -> Tensor:
         globs, count = self.schedule.globs, ids.shape[1]
+        if getattr(self, "_graph", None) is not None:  # (a captured step takes any whole numbers, from any device)
+            ids = ids.to(self._graph_tok)
         for a in range(0, count, self.prompt_portion):
             b = min(count, a + self.prompt_portion)
-            hidden = self.model.model.embed_tokens(BatchState(input_ids=ids[:, a:b])).hidden_states.reshape(b - a, -1)
+            post = self.model.model.embed_tokens(BatchState(input_ids=ids[:, a:b]))
+            hidden = post.hidden_states.reshape(b - a, -1).to(globs.hidden_states)
             self.last_call = self.interpreter.prompt(globs, hidden, a, b == count)
         globs.hidden_states[:] = hidden[-1]
         if globs.pos_id_device is not None:

@@ -291,3 +291,21 @@ def test_prompt_honours_the_wait_limit():
     with pytest.raises(RuntimeError, match="TIMEOUT"):
         prompt(wait_timeout_ms=1)
     prompt()  # the device and the status record are as before
+
+
+@pytest.mark.gpu
+def test_prompt_takes_what_steps_take():
+    """Whole numbers of any type into a captured step's generator, embeddings kept in another type than the kernel's."""
+    from megakernels_b200.generators import MK_Generator
+
+    _, _, model, schedule = make_pair(CONFIGS["1b"](), 40, 0)
+    gen = MK_Generator(model, interpreter(), schedule)
+    ids = torch.tensor(seeded_tokens(4096, 12))
+    want = gen.prefill(ids.cuda())
+    embed = model.model.embed_tokens.embed_tokens
+    embed.weight = embed.weight.float()
+    assert torch.equal(gen.prefill(ids.cuda()), want)
+    gen.enable_cuda_graph(warmup_pos=3)
+    assert gen._takes_prompts(12)
+    assert torch.equal(gen.prefill(ids.to(torch.int16)), want)
+    gen.check()
