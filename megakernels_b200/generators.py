@@ -259,9 +259,12 @@ class MK_Generator(Generator):
             ids = ids.to(self._graph_tok)
         for a in range(0, count, self.prompt_portion):
             b = min(count, a + self.prompt_portion)
-            post = self.model.model.embed_tokens(BatchState(input_ids=ids[:, a:b]))
-            hidden = post.hidden_states.reshape(b - a, -1).to(globs.hidden_states)
-            self.last_call = self.interpreter.prompt(globs, hidden, a, b == count)
+            try:
+                post = self.model.model.embed_tokens(BatchState(input_ids=ids[:, a:b]))
+                hidden = post.hidden_states.reshape(b - a, -1).to(globs.hidden_states)
+                self.last_call = self.interpreter.prompt(globs, hidden, a, b == count)
+            except torch.OutOfMemoryError:  # steps need no workspace
+                return self._steps(ids, a)
         globs.hidden_states[:] = hidden[-1]
         if globs.pos_id_device is not None:
             globs.pos_id_device.fill_(count - 1)
@@ -274,14 +277,17 @@ class MK_Generator(Generator):
         """Fill the KV cache with a prompt; returns the first generated token ``[1]``.
 
         The reference prefills with its torch model (scripts/generate.py:125-137).  Here the tokens go
-        through the layers at once, in portions, or where that does not apply (``_takes_prompts``) through
-        the decode kernel one at a time.
+        through the layers at once, in portions, or where that does not apply (``_takes_prompts``) or memory
+        for a portion is lacking, through the decode kernel one at a time.
         """
         ids = prompt_ids.reshape(1, -1)
         if self._takes_prompts(ids.shape[1]):
             return self._prompt(ids)
+        return self._steps(ids, 0)
+
+    def _steps(self, ids: Tensor, first: int) -> Tensor:
         out = None
-        for pos in range(ids.shape[1]):
+        for pos in range(first, ids.shape[1]):
             out = self.run(ids[:, pos : pos + 1], pos_id=pos)
         return out.reshape(-1)
 

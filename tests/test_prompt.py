@@ -309,3 +309,28 @@ def test_prompt_takes_what_steps_take():
     assert gen._takes_prompts(12)
     assert torch.equal(gen.prefill(ids.to(torch.int16)), want)
     gen.check()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fits", [0, 1])
+def test_prompt_without_memory_for_a_portion_goes_by_steps(fits, monkeypatch):
+    from megakernels_b200.generators import MK_Generator
+
+    _, _, model, schedule = make_pair(CONFIGS["1b"](), 40, 0)
+    gen = MK_Generator(model, interpreter(), schedule)
+    gen.prompt_portion = 16
+    ids = torch.tensor(seeded_tokens(4096, 40)).cuda()
+    want = [gen.prefill(ids).clone(), schedule.globs.logits.clone()]
+    calls, prompt = [], interpreter().prompt
+
+    def short(*args):
+        calls.append(args)
+        if len(calls) > fits:
+            raise torch.OutOfMemoryError("no room")
+        return prompt(*args)
+
+    monkeypatch.setattr(interpreter(), "prompt", short)
+    assert torch.equal(gen.prefill(ids), want[0])
+    gen.check()
+    assert len(calls) == fits + 1 and schedule.globs.pos_id == 39
+    assert rel_err(schedule.globs.logits, want[1]) <= 2e-2
