@@ -460,13 +460,8 @@ cudaError_t launch(const FlashMaps& maps, const FlashShape& s, cudaStream_t stre
 }
 template <bool kOwn>
 cudaError_t choose(const FlashMaps& maps, FlashShape s, cudaStream_t stream) {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-    }
+    int sms = 0;
+    if (const cudaError_t e = sm_count(&sms); e != cudaSuccess) return e;
     // as many parts as there are SMs for, each with two tiles or more of the longest block (61 queries over 1561 keys,
     // 16 heads of 192 / 128: 27 us with one part, 18 with four)
     const int blocks = s.heads * ((s.n + kRows - 1) / kRows), last = s.pos0 + s.n - 1;

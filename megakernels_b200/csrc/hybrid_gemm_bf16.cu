@@ -445,13 +445,8 @@ cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
 
 cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, int T, int N, int K, const GemmEpilogue& e,
                       int* status, cudaStream_t st, const bf16* W2, unsigned long long timeout_ns) {
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaError_t err = cudaGetDevice(&dev);
-        if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (err != cudaSuccess) return err;
-    }
+    int sms = 0;
+    if (const cudaError_t err = sm_count(&sms); err != cudaSuccess) return err;
     const Shape s{T, N, K, 0, 0, 1, 0, timeout_ns, status};
     switch (group_of(e.what)) {
         case Group::kSilu: return choose<Group::kSilu>(A, lda, W, W2, ldw, s, e, sms, st);

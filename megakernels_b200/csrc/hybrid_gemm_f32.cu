@@ -220,13 +220,8 @@ cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, i
         else gemv_f32_kernel<2><<<blocks, 256, 0, s>>>(A, lda, W, ldw, N, K, e);
         return cudaGetLastError();
     }
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaError_t err = cudaGetDevice(&dev);
-        if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (err != cudaSuccess) return err;
-    }
+    int sms = 0;
+    if (const cudaError_t err = sm_count(&sms); err != cudaSuccess) return err;
     const int rows = T <= 16 ? 16 : T <= 32 ? 32 : 64, tiles = ((T + rows - 1) / rows) * ((N + kCols - 1) / kCols);
     // An SM works off its CTAs at one rate: the share of the inner dimension that leaves the fullest SM the least
     // work, a share's own cost (filling the pipeline, the exchange) counted as 64 of the inner dimension.

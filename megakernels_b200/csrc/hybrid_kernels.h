@@ -1,8 +1,22 @@
 // Host-callable launchers of the hybrid models' kernels (one translation unit per group).
 #pragma once
+#include <atomic>
+
 #include "hybrid_common.cuh"
 
 namespace mkbh {
+
+// SMs of the current device (a process's devices are alike)
+inline cudaError_t sm_count(int* sms) {
+    static std::atomic<int> known{0};
+    *sms = known.load(std::memory_order_relaxed);
+    if (*sms) return cudaSuccess;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) known.store(*sms, std::memory_order_relaxed);
+    return e;
+}
 
 constexpr unsigned long long kWaitNs = 2000000000ull;  // how long a kernel's waits go on before they give up
 

@@ -888,8 +888,11 @@ cudaError_t launch_scan_columns(const MkbhGlobals& g, const MkbhLayer& L, int64_
 // tokens: 394 us, 267 with two columns and one CTA); with SMs to spare one column is the shorter chain (32 heads: 237).
 template <int M>
 cudaError_t launch_scan(const MkbhGlobals& g, const MkbhLayer& L, int64_t ld, float* state, cudaStream_t s) {
-    if constexpr (M <= 2)
-        if ((L.dim + kScanCols - 1) / kScanCols * L.heads > 148) return launch_scan_columns<M, 2>(g, L, ld, state, s);
+    if constexpr (M <= 2) {
+        int sms = 0;
+        if (const cudaError_t e = sm_count(&sms); e != cudaSuccess) return e;
+        if ((L.dim + kScanCols - 1) / kScanCols * L.heads > sms) return launch_scan_columns<M, 2>(g, L, ld, state, s);
+    }
     return launch_scan_columns<M, 1>(g, L, ld, state, s);
 }
 

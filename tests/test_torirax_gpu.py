@@ -139,6 +139,18 @@ def test_one_outstanding_key_just_inside_and_outside(tmp_path, distance, decoded
 
 
 @pytest.mark.parametrize("dtype,tol", DTYPES)
+def test_recurrences_of_many_heads(bench, dtype, tol):
+    """More blocks of columns than SMs: the scan takes two columns per lane group (the second group partly or wholly
+    beyond the head); more tiles than the SMs hold: the decays of several heads per block, the last block's heads
+    fewer.  Portions carry the state; most are no multiple of a chunk."""
+    raw = model_config([delta(75, 24, ff=20), delta(50, 41), delta(40, 64)], max_positions=400)
+    raw, w, path, toks, want = bench("heads", raw, n=397)
+    gen = load(path, dtype)
+    for cuts in ([397], [330, 2, 65], [63, 334]):
+        assert rel(run_cut(gen, toks, cuts), want) < tol, cuts
+
+
+@pytest.mark.parametrize("dtype,tol", DTYPES)
 def test_far_kept_keys_and_long_decoding(bench, dtype, tol):
     """250 decoded tokens after a short prompt: kept positions hundreds of tokens back, rings that
     wrap under single tokens, recurrent state that is carried all the way."""
