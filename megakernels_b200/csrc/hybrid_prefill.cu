@@ -334,69 +334,61 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
     return r;
 }
 
-// Decays w = exp(-decay_scale * sigmoid(w2 tanh(w1) + w0)): a tile of 64 tokens x 64 channels of one head, kTokens x 4
-// per thread, two tokens per instruction.  Bound by shared-memory reads: one channel x 16 tokens per thread read five
-// 16-byte words per 16 products (2048 tokens, 64 heads of 64, rank 128: 174 us), 8 x 4 read three per 32 (122 us).
-// Few tokens take 4 x 4, twice the warps.  A block keeps its tokens' tanh(w1) for `heads_per` heads.
-constexpr int kDecayTile = 64, kDecayStride = kDecayTile + 4;
+// Decays w = exp(-decay_scale * sigmoid(w2 tanh(w1) + w0)): a tile of 64 tokens x 64 channels of one head, 4 x 4 per thread,
+// two tokens per instruction.  Bound by shared-memory reads and the latency of a block's loads: one channel x 16 tokens per
+// thread read five 16-byte words per 16 products (2048 tokens, 64 heads of 64, rank 128: 174 us); this reads two, 103 us.
+// 8 x 4 reads three per 32, but with half the warps, and keeping tanh(w1) for several heads takes blocks away: 121 us, and
+// slower at 512 and 1024 tokens and at ranks 64 and 256 too.
+constexpr int kDecayTile = 64, kDecayStride = kDecayTile + 4, kDecayThreads = 256;
+constexpr int kMaxRank = 256;  // (checked on the host)
 __host__ __device__ inline int decay_smem(int rank) { return 2 * rank * kDecayStride * 4; }
-template <typename T, int kTokens>
-__global__ void __launch_bounds__(kDecayTile / kTokens * 16) delta_decay_kernel(const float* __restrict__ proj, int64_t ld, int n, int heads,
-                                                                    int dim, int rank, const T* __restrict__ w2,
-                                                                    const float* __restrict__ w0, float decay_scale,
-                                                                    float* __restrict__ decay, int heads_per) {
-    constexpr int kDecayThreads = kDecayTile / kTokens * 16, kPairs = kTokens / 2;
+template <typename T>
+__global__ void __launch_bounds__(kDecayThreads) delta_decay_kernel(const float* __restrict__ proj, int64_t ld, int n, int HD, int dim, int rank,
+                                                                    const T* __restrict__ w2, const float* __restrict__ w0, float decay_scale,
+                                                                    float* __restrict__ decay) {
     extern __shared__ __align__(16) float sm[];
     float* inner = sm;                         // [rank][64 tokens]
     float* wt = sm + rank * kDecayStride;      // [rank][64 channels]
-    const int HD = heads * dim, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = blockIdx.x * kDecayTile, nt = min(kDecayTile, n - t0);
-    const int c0 = blockIdx.z * kDecayTile, nc = min(kDecayTile, dim - c0);
-    for (int t = warp; t < kDecayTile; t += kDecayThreads / 32)
-        for (int r = lane; r < rank; r += 32) inner[r * kDecayStride + t] = t < nt ? tanhf(proj[(size_t)(t0 + t) * ld + 5 * HD + r]) : 0.f;
-    const int ch = (threadIdx.x & 15) * 4, tg = (threadIdx.x >> 4) * kTokens;
-    for (int h = blockIdx.y * heads_per; h < min(heads, ((int)blockIdx.y + 1) * heads_per); ++h) {
-        const int col0 = h * dim + c0;
-        __syncthreads();  // the tokens are there, the head before has been read
-        for (int c = warp; c < kDecayTile; c += kDecayThreads / 32)
-            for (int r = lane; r < rank; r += 32) wt[r * kDecayStride + c] = c < nc ? to_f(w2[(size_t)(col0 + c) * rank + r]) : 0.f;
-        __syncthreads();
-        uint64_t acc[4][kPairs] = {};  // [channel][pair of tokens]
+    const int c0 = blockIdx.z * kDecayTile, nc = min(kDecayTile, dim - c0), col0 = blockIdx.y * dim + c0;
+    for (int i = warp; i < kDecayTile; i += kDecayThreads / 32)
+        for (int r = lane; r < rank; r += 32) {
+            inner[r * kDecayStride + i] = i < nt ? tanhf(proj[(size_t)(t0 + i) * ld + 5 * HD + r]) : 0.f;
+            wt[r * kDecayStride + i] = i < nc ? to_f(w2[(size_t)(col0 + i) * rank + r]) : 0.f;
+        }
+    __syncthreads();
+    const int ch = (threadIdx.x & 15) * 4, tg = (threadIdx.x >> 4) * 4;
+    uint64_t acc[4][2] = {};  // [channel][pair of tokens]
 #pragma unroll 4
-        for (int r = 0; r < rank; ++r) {
-            const float4 w = *reinterpret_cast<const float4*>(wt + r * kDecayStride + ch);
-            uint64_t f[kPairs];
+    for (int r = 0; r < rank; ++r) {
+        const float4 w = *reinterpret_cast<const float4*>(wt + r * kDecayStride + ch);
+        const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(inner + r * kDecayStride + tg);
+        const float ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int j = 0; j < kPairs; j += 2) {
-                const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(inner + r * kDecayStride + tg + 2 * j);
-                f[j] = u.x; f[j + 1] = u.y;
-            }
-            const float ws[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const uint64_t x = pair_of(ws[c], ws[c]);
-#pragma unroll
-                for (int j = 0; j < kPairs; ++j) acc[c][j] = fma2(x, f[j], acc[c][j]);
-            }
+        for (int c = 0; c < 4; ++c) {
+            const uint64_t x = pair_of(ws[c], ws[c]);
+            acc[c][0] = fma2(x, f.x, acc[c][0]);
+            acc[c][1] = fma2(x, f.y, acc[c][1]);
         }
-        const bool wide = (HD & 3) == 0 && (col0 & 3) == 0 && ch + 4 <= nc;  // (a row's four channels in one store)
-        float bias[4];
+    }
+    const bool wide = (HD & 3) == 0 && (col0 & 3) == 0 && ch + 4 <= nc;  // (a row's four channels in one store)
+    float bias[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) bias[c] = ch + c < nc ? w0[col0 + ch + c] : 0.f;
+    for (int c = 0; c < 4; ++c) bias[c] = ch + c < nc ? w0[col0 + ch + c] : 0.f;
 #pragma unroll
-        for (int j = 0; j < kTokens; ++j) {
-            if (tg + j >= nt) break;
-            float v[4];
+    for (int j = 0; j < 4; ++j) {
+        if (tg + j >= nt) break;
+        float v[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const float2 x = halves(acc[c][j >> 1]);
-                v[c] = expf(-decay_scale * sigmoid_f((j & 1 ? x.y : x.x) + bias[c]));
-            }
-            float* o = decay + (size_t)(t0 + tg + j) * HD + col0 + ch;
-            if (wide) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
-            else
-                for (int c = 0; c < 4 && ch + c < nc; ++c) o[c] = v[c];
+        for (int c = 0; c < 4; ++c) {
+            const float2 x = halves(acc[c][j >> 1]);
+            v[c] = expf(-decay_scale * sigmoid_f((j & 1 ? x.y : x.x) + bias[c]));
         }
+        float* o = decay + (size_t)(t0 + tg + j) * HD + col0 + ch;
+        if (wide) *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        else
+            for (int c = 0; c < 4 && ch + c < nc; ++c) o[c] = v[c];
     }
 }
 
@@ -996,19 +988,15 @@ cudaError_t Prefill<T>::delta(const MkbhGlobals& g, const MkbhLayer& L, T* out, 
     else delta_keys_kernel<8><<<pairs, kThreads, 0, s>>>(g.proj, ld, n, L.heads, L.dim, L.unit_eps, ab);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    // 8 tokens a thread where that fills the SMs with three blocks each, in one wave of as many heads as that takes
-    const int dt = (n + kDecayTile - 1) / kDecayTile, dc = (L.dim + kDecayTile - 1) / kDecayTile, smem = decay_smem(L.rank);
-    const int64_t tiles = (int64_t)dt * dc * L.heads;
-    const auto decay = [&](auto kernel, int threads, int heads_per) {
-        if (smem > 48 * 1024) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return;
-        kernel<<<dim3(dt, (L.heads + heads_per - 1) / heads_per, dc), threads, smem, s>>>(
-            g.proj, ld, n, L.heads, L.dim, L.rank, static_cast<const T*>(L.decay_w2), L.decay_w0, L.decay_scale, g.decay, heads_per);
-        e = cudaGetLastError();
-    };
-    if (tiles >= 444) decay(delta_decay_kernel<T, 8>, 128, (int)((tiles + 443) / 444));
-    else decay(delta_decay_kernel<T, 4>, 256, 1);
-    if (e != cudaSuccess) return e;
+    const int smem = decay_smem(L.rank);
+    if (smem > 48 * 1024) {
+        // (the same for every rank: another thread's call in between must not lower it)
+        e = cudaFuncSetAttribute(delta_decay_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, decay_smem(kMaxRank));
+        if (e != cudaSuccess) return e;
+    }
+    delta_decay_kernel<T><<<dim3((n + kDecayTile - 1) / kDecayTile, L.heads, (L.dim + kDecayTile - 1) / kDecayTile), kDecayThreads, smem, s>>>(
+        g.proj, ld, n, HD, L.dim, L.rank, static_cast<const T*>(L.decay_w2), L.decay_w0, L.decay_scale, g.decay);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     float* state = L.state + (size_t)g.slot * HD * L.dim;
     switch ((L.dim + 31) / 32) {
         case 1: e = launch_scan<1>(g, L, ld, state, s); break;
