@@ -232,7 +232,8 @@ cudaError_t launch(const PlainArgs<T>& a, cudaStream_t s) {
     int floats = kRows * (dim + kThreads);
     if (floats < kQueries * a.L.vdim) floats = kQueries * a.L.vdim;
     if (floats * 4 > 47 * 1024) {  // (the kernel's own arrays are another kilobyte)
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, floats * 4);
+        // (the most there is, whatever this layer takes: another thread's call in between must not lower it)
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
         if (e != cudaSuccess) return e;
     }
     kernel<<<dim3((a.n + kQueries - 1) / kQueries, a.L.heads), kThreads, floats * 4, s>>>(a);
