@@ -673,7 +673,7 @@ __global__ void kv_append_kernel(const float* __restrict__ proj, int64_t ld, int
 // rotated part) of a run of tokens: convolution over time, norm, rotation of neighbours, and
 // stores it as an element of the query buffer or as a cache row.
 // Eight tokens share a vector's weights; short portions, where the SMs wait for a warp's chain of tokens, take two (61
-// tokens of the 1B-class widths 17 us -> 8).  A prompt of 24 runs of layers of these widths, two against eight: 61 tokens
+// tokens of the 1B-class widths 17 us -> 8).  A prompt of 16 runs of layers of these widths, two against eight: 61 tokens
 // 1,668 and 1,793 us, 512 2,725 and 2,777, 768 3,109 and 3,158, 1,024 3,516 and 3,523, 1,536 5,016 and 4,997.
 inline int run_of(int n) { return n <= 1024 ? 2 : 8; }
 struct OperandArgs {
@@ -913,7 +913,7 @@ cudaError_t Prefill<T>::canon_norm(const MkbhGlobals& g, const MkbhLayer& L, T* 
     const int n = g.num_tokens, smem = max(1, L.canon_taps) * g.width * 4;
     const float* hist = L.canon_hist + (L.canon_taps > 1 ? (size_t)g.slot * (L.canon_taps - 1) * g.width : 0);
     if (g.norm_kind == MKBH_RMS_NORM && g.width % 4 == 0 && L.canon_taps <= kCanonTaps) {
-        // (8 us at 61 tokens and 1B-class widths with eight tokens per block, 6 with two; a prompt of 24 runs of layers, two
+        // (8 us at 61 tokens and 1B-class widths with eight tokens per block, 6 with two; a prompt of 16 runs of layers, two
         // against eight: 384 tokens 2,555 and 2,710 us, 512 2,741 and 2,777, 640 2,926 and 2,917)
         const bool few = n <= 512;
         auto go = [&](auto taps) {

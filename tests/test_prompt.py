@@ -48,10 +48,12 @@ def test_only_whole_schedules_count_as_the_model():
         assert not covers_model(schedule.globs, schedule.get_linear_instructions())
 
 
-# portions of 1 (a lone last token), rows of a 128-row tile and their remainders, keys over several tiles
+# portions of 1 (a lone last token), rows of a 128-row tile and their remainders, keys over several tiles; short last
+# portions over 512 keys and more, whose tiles a cluster shares
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape,count,portion", [
     ("1b", 2, 2048), ("1b", 4, 2048), ("1b", 128, 2048), ("1b", 129, 128), ("1b", 300, 2048), ("8b", 61, 2048), ("8b", 257, 100), ("70b", 130, 2048),
+    ("1b", 620, 560), ("1b", 700, 100), ("1b", 561, 560), ("8b", 641, 100), ("70b", 530, 520),
 ])
 def test_prompt_equals_a_step_per_token(shape, count, portion):
     """Caches and logits within the decode path's own distance from the oracle (2e-2, two layers);
