@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "hybrid_kernels.h"
+#include "hybrid_product.h"
 
 namespace {
 

@@ -116,8 +116,8 @@ RESULTS = ("store", "add", "cast", "glu", "silu")
 
 
 def product(result: str, a, w, out, status, inner: int, w2=None, bias=None, scale=None, limit=0.0, alpha=0.0) -> None:
-    """One matrix product of the prefill on the current stream (``mkb_hybrid_product``): ``a`` [tokens, lda],
-    ``w`` [features, ldw], the first ``inner`` columns of both."""
+    """One matrix product of the prefill on the current stream: ``a`` [tokens, lda], ``w`` [features, ldw], the first
+    ``inner`` columns of both.  For the tests; not part of the library's interface (``csrc/hybrid_product.h``)."""
     p = MkbhProduct(ctypes.sizeof(MkbhProduct), 1 if a.dtype == torch.float32 else 0, RESULTS.index(result), a.shape[0], w.shape[0], inner,
                     a.stride(0), w.stride(0), out.stride(0), _p(a), _p(w), _p(w2), _p(bias), _p(scale), limit, alpha, _p(out), _p(status))
     _raise(load_library().mkb_hybrid_product(ctypes.byref(p), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
