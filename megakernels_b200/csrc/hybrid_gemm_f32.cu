@@ -6,7 +6,7 @@
 // slots are left for the shared-memory reads; the next slice of operands is in registers while this one is multiplied.
 // Where the tiles do not fill the SMs evenly, a cluster of up to eight CTAs shares a tile's inner dimension and adds
 // the partial tiles through distributed shared memory, always in the same order.
-// One or a few tokens (the head): a warp per feature, bound by the weights' traffic.
+// One or two tokens (the head): a warp per pair of features, bound by the weights' traffic.
 #include "hybrid_kernels.h"
 
 namespace mkbh {

@@ -130,6 +130,13 @@ def prefill_ms(gen, n: int, reps: int) -> float:
     return ms
 
 
+def llama_prompt_ms(gen, n: int, reps: int) -> float:
+    toks = torch.randint(0, gen.model.config.vocab_size, (n,), generator=torch.Generator().manual_seed(1), device="cpu").to(gen.model.device)
+    ms = timed(lambda: gen.prefill(toks), reps)
+    gen.check()
+    return ms
+
+
 def layer_parts(cfg: HybridConfig, tokens: int) -> dict:
     """Milliseconds of one layer of each kind at ``tokens`` tokens: stacks of eight, minus stacks of
     two (embedding, head of one row)."""
@@ -201,7 +208,7 @@ def run(args, sampler_cls, peaks: dict) -> None:
         Hq, Hk, L = lcfg.num_attention_heads, lcfg.num_key_value_heads, lcfg.num_hidden_layers
         nbytes = 2 * (L * ((Hq + 2 * Hk) * D * H + H * Hq * D + 3 * I * H) + lcfg.vocab_size * H) + 4 * ATTENDED * Hk * D * L
         line["closest"] = {"model": close, "layers": L, "decode": decode_row(kernel, step, nbytes, hbm),
-                           "prefill_tokens_per_s": round(1e3 / step)}  # its prompts go through the decode kernel token by token
+                           "prefill_tokens_per_s": round(2048e3 / llama_prompt_ms(gen, 2048, 5))}
         if close_list:
             del gen, model
             torch.cuda.empty_cache()
