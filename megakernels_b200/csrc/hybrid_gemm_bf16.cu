@@ -407,12 +407,13 @@ cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
     // The kind of tile with the smallest estimate, fitted in us to 48 shapes of 16..2048 tokens x 2048..28672 features x
     // 512..14336 (cold caches): waves of tiles, each so many steps of the inner dimension, and the last epilogue.  It ranks the
     // kinds and is no time: what all kinds pay alike (the launch, the weights' way from memory) is left out.  One row of
-    // a head of 128256 x 2048 takes 101 - 108 us whatever the kind (80 us of bytes), 61 x 16384 x 2048 27.5 - 27.6 in six
-    // of the nine.  A step costs what an SM takes in from L2 (24 KB: 0.19 us, 32 KB: 0.23 us), so few narrow tiles with a long
-    // inner dimension are shared, 61 x 2048 x 8192 in us: 38.0 as 16 tiles of 128, 33.8 as 32 of 64, 23.6 with two CTAs on
-    // each of these, 19.5 with four.  A cluster's exchange costs what its rows do, and clusters
-    // beyond one wave wait for whole groups of SMs, as do clusters of eight.  Of 25 shapes of 1 to 2048 tokens the choice missed
-    // the fastest kind by more than 5 % in two: 61 x 3072 x 2048 (17.4 us, 15.4) and 200 x 16384 x 2048 (33.8, 31.7).
+    // a head of 128256 x 2048 takes 101 - 108 us whatever the kind (80 us of bytes), 61 x 16384 x 2048 27.6 us as tiles of 128
+    // and of 64 and 29.8 - 33.8 as wider ones or pairs.  A step costs what an SM takes in from L2 (24 KB: 0.19 us, 32 KB:
+    // 0.23 us), so few narrow tiles with a long inner dimension are shared, 61 x 2048 x 8192 in us: 38.0 as 16 tiles of
+    // 128, 33.8 as 32 of 64, 23.6 with two CTAs on each of these, 19.5 with four.  A cluster's exchange costs what its rows
+    // do, and clusters beyond one wave wait for whole groups of SMs, as do clusters of eight.  Of 25 shapes of 1 to 2048 tokens
+    // the choice missed the fastest kind by more than 5 % in two: 61 x 3072 x 2048 (17.4 us, 15.4) and 200 x 16384 x 2048
+    // (33.8, 31.7).
     const int steps = (s.K + kBK - 1) / kBK;
     auto tiles_of = [&](int bn, int pair) {
         const int wide = kGroup == Group::kSilu ? bn / 2 : bn;
