@@ -336,3 +336,26 @@ def test_prompt_without_memory_for_a_portion_goes_by_steps(fits, monkeypatch):
     gen.check()
     assert len(calls) == fits + 1 and schedule.globs.pos_id == 39
     assert rel_err(schedule.globs.logits, want[1]) <= 2e-2
+
+
+@pytest.mark.gpu
+def test_prompt_under_capture():
+    """Captured into a graph, a prompt's launches (which may begin early) give the same bits on replay with other tokens."""
+    from megakernels_b200.generators import MK_Generator
+
+    _, _, model, schedule = make_pair(CONFIGS["1b"](), 300, 0)
+    globs = schedule.globs
+    gen = MK_Generator(model, interpreter(), schedule)
+    first, second = (torch.tensor(seeded_tokens(globs.vocab_size, 300, seed=s)).cuda() for s in (8, 9))
+    want = [gen.prefill(second).clone(), globs.logits.clone(), *(c.clone() for c in model.stacked_kv_cache)]
+    ids = first.clone()
+    gen.prefill(ids)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        token = gen.prefill(ids)
+    ids.copy_(second)
+    graph.replay()
+    gen.check()
+    for got, w in zip([token, globs.logits, *model.stacked_kv_cache], want):
+        assert torch.equal(got, w)
