@@ -23,6 +23,7 @@ from __future__ import annotations
 import math
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 from torch import Tensor
 
@@ -40,7 +41,7 @@ from megakernels_b200.demos.latency.instructions import (
     TP_AllReduce,
 )
 from megakernels_b200.instructions import NoOp, TensorParallelState
-from megakernels_b200.scheduler import DAG_Node, ScheduleBuilder
+from megakernels_b200.scheduler import DAG_Node, ScheduleBuilder, serialize_and_pad
 from megakernels_b200.utils import assert_div, get_sm_count
 
 MAX_REDUCTION_LIST = 24  # idx list + 7 fixed words must fit the 32-word instruction
@@ -518,60 +519,61 @@ def covers_model(globs: Globals, instructions: list[Instruction] | Tensor) -> bo
     """Whether single-sequence instructions are the model's whole step and nothing else: every block of every layer once,
     every key/value head's attention and the head.  ``instructions`` may be the tensor that the kernel reads."""
     if isinstance(instructions, Tensor):
-        words = instructions.reshape(-1, instructions.shape[-1])
-        words = words[words[:, 0] != 0].tolist()
+        words = instructions.reshape(-1, instructions.shape[-1]).cpu().numpy()
     else:
-        words = [ins.serialize() for ins in instructions if not isinstance(ins, NoOp)]
-    blocks: dict[tuple, list[tuple[int, int]]] = {}  # (opcode, layer, column slice): ranges of blocks
-    partials: dict[tuple, list[int]] = {}  # (layer, key/value head, count): partial indices
-    merges: dict[tuple, list[tuple]] = {}  # (layer, first head): (count, terminal, merged partials)
-    for op, *a in words:
-        if op == LayerNorm_QKV_MatVecRopeAppend.opcode():
-            blocks.setdefault((op, a[0], 0), []).append((a[1], a[2]))
-        elif op in (O_ProjResidual.opcode(), DownProjResidual.opcode()):
-            blocks.setdefault((op, a[0], a[3]), []).append((a[1], a[2]))
-        elif op == LayerNormDoubleMatVecSiLU.opcode():
-            blocks.setdefault((op, a[0], 0), []).extend((b, b + 1) for b in a[2 : 2 + a[1]])
-        elif op == RMS_LM_Head.opcode():
-            blocks.setdefault((op, 0, 0), []).append((a[0], a[1]))
-        elif op == PartialAttention.opcode() and not any(a[4:5]):  # (sequence 0)
-            partials.setdefault((a[0], a[1], a[2]), []).append(a[3])
-        elif op == AttentionReduction.opcode() and not any(a[5 + a[4] : 7 + a[4]]):  # (into the output, sequence 0)
-            merges.setdefault((a[0], a[1]), []).append((a[2], a[3], a[5 : 5 + a[4]]))
-        else:
+        words = np.array([serialize_and_pad(ins) for ins in instructions])
+    op = words[:, 0]
+    of = {kind: words[op == kind.opcode(), 1:] for kind in (
+        NoOp, LayerNorm_QKV_MatVecRopeAppend, PartialAttention, AttentionReduction, O_ProjResidual, LayerNormDoubleMatVecSiLU,
+        DownProjResidual, RMS_LM_Head)}
+    if sum(len(rows) for rows in of.values()) != len(words):  # (other instructions)
+        return False
+    L, heads, kv_heads = globs.num_hidden_layers, globs.num_attention_heads, globs.num_kv_heads
+
+    def once(layer, start, end, count: int, split=0, splits: int = 1, layers: int = L) -> bool:
+        """Ranges of blocks that make up ``0 .. count`` in each layer and column slice, without overlap."""
+        inside = (layer >= 0) & (layer < layers) & (start >= 0) & (start < end) & (end <= count) & (split >= 0) & (split < splits)
+        if not np.all(inside):
             return False
+        steps = np.zeros((layers * splits, count + 1), dtype=np.int64)
+        np.add.at(steps, (layer * splits + split, start), 1)
+        np.add.at(steps, (layer * splits + split, end), -1)
+        return bool((steps.cumsum(1)[:, :count] == 1).all())
 
-    want = {(RMS_LM_Head.opcode(), 0, 0): globs.vocab_size // globs.lm_head_block_size}
-    count_of = {(layer, kv): count for layer, kv, count in partials}  # (a second count of a head is caught by the lengths)
-    want_merges: dict[tuple, list[tuple]] = {}
-    gqa = globs.num_attention_heads // globs.num_kv_heads
-    for layer in range(globs.num_hidden_layers):
-        want[LayerNorm_QKV_MatVecRopeAppend.opcode(), layer, 0] = globs.num_total_heads() * globs.head_dim // globs.qkv_block_size
-        want[LayerNormDoubleMatVecSiLU.opcode(), layer, 0] = globs.intermediate_size // globs.up_gate_proj_block_size
-        for split in range(globs.num_o_proj_col_splits()):
-            want[O_ProjResidual.opcode(), layer, split] = globs.hidden_size // globs.o_proj_block_size
-        for split in range(globs.num_down_proj_col_splits()):
-            want[DownProjResidual.opcode(), layer, split] = globs.hidden_size // globs.down_proj_block_size
-        for kv in range(globs.num_kv_heads):
-            count = count_of.get((layer, kv), 0)
-            if count < 1 or (count > 1 and globs.skip_attn_reduction and not globs.merge_in_last_partial):
+    qkv, up, head = of[LayerNorm_QKV_MatVecRopeAppend], of[LayerNormDoubleMatVecSiLU], of[RMS_LM_Head]
+    listed = np.arange(up.shape[1] - 2) < up[:, 1:2]
+    blocks, layer_of = up[:, 2:][listed], np.broadcast_to(up[:, :1], listed.shape)[listed]
+    o, down = of[O_ProjResidual], of[DownProjResidual]
+    if not (
+        once(qkv[:, 0], qkv[:, 1], qkv[:, 2], globs.num_total_heads() * globs.head_dim // globs.qkv_block_size)
+        and once(layer_of, blocks, blocks + 1, globs.intermediate_size // globs.up_gate_proj_block_size)
+        and once(o[:, 0], o[:, 1], o[:, 2], globs.hidden_size // globs.o_proj_block_size, o[:, 3], globs.num_o_proj_col_splits())
+        and once(down[:, 0], down[:, 1], down[:, 2], globs.hidden_size // globs.down_proj_block_size, down[:, 3],
+                 globs.num_down_proj_col_splits())
+        and once(np.zeros(len(head), dtype=int), head[:, 0], head[:, 1], globs.vocab_size // globs.lm_head_block_size, layers=1)
+    ):
+        return False
+
+    merging = not (globs.skip_attn_reduction or globs.merge_in_last_partial)  # by instructions of their own
+    gqa = heads // kv_heads
+    partials: dict[tuple, list[int]] = {}
+    for layer, kv, count, part, sequence in of[PartialAttention][:, :5].tolist():
+        if sequence:
+            return False
+        partials.setdefault((layer, kv), []).append((count, part))
+    merges: dict[tuple, list] = {}
+    for layer, first, count, last, n, *rest in of[AttentionReduction].tolist():
+        merges.setdefault((layer, first), []).append((count, last, rest[:n], any(rest[n:])))  # (into the output, sequence 0)
+    want_merges: dict[tuple, list] = {}
+    for layer in range(L):
+        for kv in range(kv_heads):
+            parts = partials.pop((layer, kv), [])
+            count = len(parts)
+            if count == 0 or sorted(parts) != [(count, part) for part in range(count)]:
                 return False
-            if not (globs.skip_attn_reduction or globs.merge_in_last_partial):
-                for head in range(kv * gqa, (kv + 1) * gqa, globs.attn_reduction_size):
-                    want_merges[layer, head] = [(count, 1, list(range(count)))]
-
-    def once(ranges: list[tuple[int, int]], count: int) -> bool:
-        ends = [0]
-        for start, end in sorted(ranges):
-            if start != ends[-1] or end <= start:
+            if count > 1 and globs.skip_attn_reduction and not globs.merge_in_last_partial:
                 return False
-            ends.append(end)
-        return ends[-1] == count
-
-    return (
-        blocks.keys() == want.keys()
-        and all(once(ranges, want[key]) for key, ranges in blocks.items())
-        and len(partials) == len(count_of) == globs.num_hidden_layers * globs.num_kv_heads
-        and all(sorted(parts) == list(range(key[2])) for key, parts in partials.items())
-        and merges == want_merges
-    )
+            if merging:
+                for first in range(kv * gqa, (kv + 1) * gqa, globs.attn_reduction_size):
+                    want_merges[layer, first] = [(count, 1, list(range(count)), False)]
+    return not partials and merges == want_merges
