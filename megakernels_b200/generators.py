@@ -250,7 +250,7 @@ class MK_Generator(Generator):
         )
 
     # A step per token costs what the weights' traffic costs, the layers at once that and their launches, once: two tokens
-    # take 1,132 us at once and 1,289 us as steps (1B widths, 16 layers), 729 and 1,041 us (8B widths, 4 layers).
+    # take 1,153 us at once and 1,290 us as steps (1B widths, 16 layers), 743 and 1,033 us (8B widths, 4 layers).
     shortest_prompt = 2
 
     def _prompt(self, ids: Tensor) -> Tensor:
