@@ -53,6 +53,11 @@ enum {
      * counts into barriers[layer][MKB_BARRIER_ROW_RMS_NORM][which]; the RMS + matvec
      * opcodes 1, 5 and 7 then wait for `batch` arrivals there instead of normalising. */
     MKB_OP_RMS_NORM = 9,
+    /* Batched launches only: one of `ranks` equal shares of a layer's attention over all sequences, cut
+     * by the cached positions of this launch; in place of every MKB_OP_PARTIAL_ATTENTION and
+     * MKB_OP_ATTENTION_REDUCTION of the layer.  All shares of a layer must be there.
+     * words: [10, layer, rank, ranks] */
+    MKB_OP_BATCH_ATTENTION = 10,
 };
 
 /* Barrier rows: opcode k counts into row k - 1 (rows 0..6), as in the reference.  Row 8 has

@@ -85,6 +85,9 @@ int l2_window_from_env(const char* name, int default_kb) {
     return kb == 0 ? 0 : kNumStages + kb * 1024 / kStageBytes;
 }
 const int g_l2_window_stages = l2_window_from_env("MKB_L2_WINDOW_KB", 64);
+// (several sequences: their activations pass through L2 as well, 7 and 64 sequences in us without and with 64 KB: 1176 and
+// 1214, 2187 and 2234)
+const int g_l2_window_batched = l2_window_from_env("MKB_L2_WINDOW_KB", 0);
 const int g_l2_stall_window_stages = l2_window_from_env("MKB_L2_STALL_WINDOW_KB", 1024);
 
 std::mutex g_mutex;
@@ -103,8 +106,9 @@ int get_encode_fn() {
 }
 
 // 4-D view [D, Hkv, T, L*B] of a KV cache; one box is TS positions of one head.
-int kv_tensor_map(DeviceState* ds, const void* ptr, int D, int Hkv, int T, int LB, CUtensorMap* out) {
-    KvMapKey key{ptr, D, Hkv, T, LB};
+// (attention by shares: half a stage's positions of two heads, or a quarter of four)
+int kv_tensor_map(DeviceState* ds, const void* ptr, int D, int Hkv, int T, int LB, CUtensorMap* out, int heads = 1) {
+    KvMapKey key{ptr, D, Hkv, T, LB, heads - 1};
     if (ds)
         for (auto& e : ds->maps)
             if (e.key == key) {
@@ -118,10 +122,10 @@ int kv_tensor_map(DeviceState* ds, const void* ptr, int D, int Hkv, int T, int L
     // side by side (16 bytes each, same column) fall into 8 different bank groups.  With whole
     // 256-byte rows in shared memory they all hit the same banks (8-way conflicts, the attention
     // stages then cost 1.7 us each).
-    const int ts = (kStageBytes / 4) / D;
+    const int ts = (kStageBytes / 4) / D / heads;
     cuuint64_t dims[5] = {64, (cuuint64_t)T, (cuuint64_t)D / 64, (cuuint64_t)Hkv, (cuuint64_t)LB};
     cuuint64_t strides[4] = {(cuuint64_t)Hkv * D * 2, 128, (cuuint64_t)D * 2, (cuuint64_t)T * Hkv * D * 2};
-    cuuint32_t box[5] = {64, (cuuint32_t)ts, (cuuint32_t)D / 64, 1, 1};
+    cuuint32_t box[5] = {64, (cuuint32_t)ts, (cuuint32_t)D / 64, (cuuint32_t)heads, 1};
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     CUtensorMap m;
     CUresult r = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(ptr), dims,
@@ -443,15 +447,22 @@ int prepare_launch(const MkbGlobals* g, DeviceState* ds, int* status, int sm_cou
     if (gemm) p.argmax_out = nullptr;  // no fused argmax in this build: the host reduces the logits
     const unsigned ms = g->wait_timeout_ms ? g->wait_timeout_ms : 2000u;
     p.timeout_ns = (unsigned long long)ms * 1000000ull;
-    p.l2_window_stages = g_l2_window_stages;
-    p.l2_stall_window_stages = g_l2_stall_window_stages > g_l2_window_stages ? g_l2_stall_window_stages
-                                                                             : g_l2_window_stages;
+    p.l2_window_stages = p.batch > 1 ? g_l2_window_batched : g_l2_window_stages;
+    p.l2_stall_window_stages = g_l2_stall_window_stages > p.l2_window_stages ? g_l2_stall_window_stages
+                                                                             : p.l2_window_stages;
     p.poll_sleep_ns = 20;
 
     rc = kv_tensor_map(ds, g->k_cache, p.D, p.Hkv, p.T, p.L * p.B, &p.k_map);
     if (rc) return rc;
     rc = kv_tensor_map(ds, g->v_cache, p.D, p.Hkv, p.T, p.L * p.B, &p.v_map);
     if (rc) return rc;
+    if (p.batch > 1) {
+        p.share_heads = p.Hkv % 4 == 0 ? 4 : p.Hkv % 2 == 0 ? 2 : 1;
+        rc = kv_tensor_map(ds, g->k_cache, p.D, p.Hkv, p.T, p.L * p.B, &p.k_share_map, p.share_heads);
+        if (rc) return rc;
+        rc = kv_tensor_map(ds, g->v_cache, p.D, p.Hkv, p.T, p.L * p.B, &p.v_share_map, p.share_heads);
+        if (rc) return rc;
+    }
 
     const struct {
         const void* ptr;
@@ -655,6 +666,11 @@ int mkb_validate_instructions(const MkbGlobals* g, const int32_t* host_instructi
                     if (w[1] < 0 || w[1] >= L) return bad("layer out of range");
                     if (w[2] < 0 || w[2] > 2) return bad("which must be 0, 1 or 2");
                     if (w[3] < 0 || w[3] >= g->batch) return bad("sequence outside the batch");
+                    break;
+                case MKB_OP_BATCH_ATTENTION:
+                    if (g->batch <= 1) return bad("attention by shares in a single-sequence launch");
+                    if (w[1] < 0 || w[1] >= L) return bad("layer out of range");
+                    if (w[2] < 0 || w[2] >= w[3]) return bad("share outside their number");
                     break;
                 case MKB_OP_TP_ALL_REDUCE:
                     if (g->tp.size <= 1) return bad("all-reduce instruction without tensor parallelism");

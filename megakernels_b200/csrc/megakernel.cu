@@ -305,6 +305,110 @@ __device__ __forceinline__ AttnRange attn_range(const KParams& p, int pos, int n
     return r;
 }
 
+#if MKB_BATCH > 1
+// --------------------------------------------------------------------------- //
+// attention by shares (batched builds)
+// --------------------------------------------------------------------------- //
+// MKB_OP_BATCH_ATTENTION: a layer's attention over all sequences, cut into `ranks` equal shares of cached
+// positions, whatever the sequences' lengths are in this launch.  (One instruction per sequence and head, dealt
+// to the SMs in turn: 64 sequences of 256..4096 positions took 290 us a layer, in which the SMs were busy for 149 on average.)
+// A unit is `share_heads` neighbouring key/value heads of a sequence; a ring stage is a run of `stage_pos` positions of
+// these heads, so that a copy reads whole runs of a position's row.  A unit is as long as its stages
+// and kUnitCost more, for what it costs besides them.  Shares are cut anywhere in the line-up
+// (sequence, heads, stage); what is cut has partial rows, which the last of its parts to arrive merges.
+constexpr int kUnitCost = 3;
+struct AttnPiece {
+    int seq, kvh0;   // first key/value head
+    int lo, hi, n;   // stages of this piece, stages of the unit
+    int np, pi;      // parts of the unit, and which one this is
+};
+struct AttnShares {
+    uint32_t b0, b1, S, R, rank;  // this share's extent of the line-up; its length, the number of shares
+    uint32_t u0;                  // start of the next unit
+    int seq, sub;                 // the next unit
+
+    // control words: starts of the sequences, the length of the line-up behind them, and the largest number of shares
+    static __device__ __forceinline__ const volatile int* table(const Ctx& c) { return c.cta_abort + kCtlShares; }
+    static __device__ __forceinline__ int stage_pos(const KParams& p) { return (kStageBytes / 4) / p.D / p.share_heads; }
+    static __device__ __forceinline__ int stages(const Ctx& c, const KParams& p, int seq) {
+        const int sp = stage_pos(p);
+        return (c.pos_of(seq) + sp - 1) / sp;
+    }
+    // false: nothing for this rank
+    __device__ __forceinline__ bool begin(const Ctx& c, const KParams& p, int rank_, int ranks) {
+        const volatile int* tab = table(c);
+        S = (uint32_t)tab[p.batch];
+        R = min((uint32_t)ranks, (uint32_t)tab[kBatch + 1]);
+        rank = (uint32_t)rank_;
+        seq = p.batch;
+        b0 = b1 = u0 = 0;
+        sub = 0;
+        if (rank >= R) return false;
+        b0 = (uint32_t)((unsigned long long)S * rank / R);
+        b1 = (uint32_t)((unsigned long long)S * (rank + 1) / R);
+        int lo = 0, hi = p.batch;  // the sequence that b0 lies in
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if ((uint32_t)tab[mid] <= b0) lo = mid;
+            else hi = mid;
+        }
+        seq = lo;
+        const uint32_t len = (uint32_t)(stages(c, p, seq) + kUnitCost);
+        sub = (int)((b0 - (uint32_t)tab[lo]) / len);
+        u0 = (uint32_t)tab[lo] + sub * len;
+        return true;
+    }
+    __device__ __forceinline__ bool next(const Ctx& c, const KParams& p, AttnPiece& a) {
+        if (seq >= p.batch || u0 >= b1) return false;
+        a.n = stages(c, p, seq);
+        const uint32_t len = (uint32_t)(a.n + kUnitCost);
+        // cuts at or before x0 leave the unit whole behind them: it belongs to the last share that starts there
+        const uint32_t x0 = u0 + min((uint32_t)kUnitCost, len - 1), base = u0 + kUnitCost;
+        if (b1 <= x0) return false;
+        a.seq = seq;
+        a.kvh0 = sub * p.share_heads;
+        a.lo = b0 <= x0 ? 0 : (int)(b0 - base);
+        a.hi = min(a.n, (int)(b1 - base));
+        const uint32_t first = (uint32_t)(((unsigned long long)(x0 + 1) * R - 1) / S);
+        const uint32_t last = (uint32_t)(((unsigned long long)(u0 + len) * R - 1) / S);
+        a.np = (int)(last - first) + 1;
+        a.pi = (int)(rank - first);
+        u0 += len;
+        if (++sub == p.Hkv / p.share_heads) {
+            sub = 0;
+            ++seq;
+        }
+        return true;
+    }
+};
+// By one warp, before the roles start: the line-up of this launch's positions.
+__device__ __forceinline__ void attn_shares_table(const Ctx& c, const KParams& p, int lane) {
+    const uint32_t units = (uint32_t)(p.Hkv / p.share_heads);
+    uint32_t start = 0, longest = 1;
+    volatile int* tab = c.cta_abort + kCtlShares;
+    for (int s0 = 0; s0 < p.batch; s0 += 32) {
+        const int s = s0 + lane;
+        const uint32_t len = s < p.batch ? (uint32_t)(AttnShares::stages(c, p, s) + kUnitCost) : 0u;
+        uint32_t sum = units * len, most = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+            most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+        }
+        if (s < p.batch) tab[s] = (int)(start + sum - units * len);
+        start += __shfl_sync(0xffffffffu, sum, 31);
+        longest = max(longest, most);
+    }
+    if (lane == 0) {
+        tab[p.batch] = (int)start;
+        // every share holds something, and no unit falls into more parts than there are rows for
+        const unsigned long long rows = (unsigned long long)(p.max_partials - 1 < 23 ? p.max_partials - 1 : 23) * start / longest;
+        tab[kBatch + 1] = (int)max(1ull, min((unsigned long long)start, rows));
+    }
+}
+#endif  // MKB_BATCH > 1
+
 __device__ __forceinline__ void prefetch_l2_bulk(const void* src, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
@@ -315,6 +419,7 @@ struct StageDesc {
     int c1, c2, c3;          // weights: row, 64-column chunk, layer
     uint32_t bytes;
     int kvh, t, lb;          // K/V tile coordinates
+    bool share;              // K/V tile of an attention share
 };
 
 // Walks the instruction queue and yields its ring stages in consumption order.
@@ -334,6 +439,24 @@ struct StreamCursor {
     uint32_t bytes = 0;
     int kvh = 0, t0 = 0, lb = 0, ts = 0;
     const Ctx* ctx = nullptr;  // positions of the tokens being decoded
+
+#if MKB_BATCH > 1
+    AttnShares shares;         // attention by shares: b, eb are stages of the current piece
+
+    // the next piece with cached positions; b == eb: there is none
+    __device__ __forceinline__ void next_piece(const KParams& p) {
+        AttnPiece a;
+        while (shares.next(*ctx, p, a)) {
+            if (a.lo == a.hi) continue;
+            b = a.lo;
+            eb = a.hi;
+            kvh = a.kvh0;
+            lb = layer * p.B + a.seq;
+            return;
+        }
+        b = eb = 0;
+    }
+#endif
 
     __device__ __forceinline__ void set_matrix(const CUtensorMap* m, int kc, int chunk0_, int layer_) {
         map = m;
@@ -384,6 +507,13 @@ struct StreamCursor {
                 ts = (kStageBytes / 4) / p.D;
                 eb = r.n_stages;
             } break;
+#if MKB_BATCH > 1
+            case MKB_OP_BATCH_ATTENTION:
+                layer = __ldg(w + 1);
+                ts = AttnShares::stage_pos(p);
+                if (shares.begin(*ctx, p, __ldg(w + 2), __ldg(w + 3))) next_piece(p);
+                break;
+#endif
             default:
                 break;
         }
@@ -395,6 +525,18 @@ struct StreamCursor {
             if (++i >= p.queue_len) return false;
             decode(p, queue);
         }
+#if MKB_BATCH > 1
+        d.share = op == MKB_OP_BATCH_ATTENTION;
+        if (d.share) {
+            d.map = nullptr;
+            d.kvh = kvh;
+            d.t = b * ts;
+            d.lb = lb;
+            d.bytes = kStageBytes;
+            if (++b == eb) next_piece(p);
+            return true;
+        }
+#endif
         if (op == MKB_OP_PARTIAL_ATTENTION) {
             d.map = nullptr;
             d.kvh = kvh;
@@ -463,6 +605,7 @@ __device__ void loader_main(Ctx c, const int which) {
     StreamCursor issue, ahead;  // `ahead` is never behind `issue`
     issue.ctx = ahead.ctx = &c;
     StageDesc d, da;
+    d.share = da.share = false;
     uint32_t stage = 0;       // stages of the sequence walked so far (all loaders' stages)
     uint32_t ahead_stage = 0; // stages the look-ahead cursor has passed
     uint32_t own_issued = 0;  // one past the last stage this loader copied into the ring
@@ -490,7 +633,10 @@ __device__ void loader_main(Ctx c, const int which) {
                 // stalls of this SM's consumers cannot stop HBM from streaming
                 // while the consumers sit in a barrier wait the ring cannot drain, so the
                 // look-ahead may run deeper than in steady state
-                const int window = c.cta_abort[4] ? p.l2_stall_window_stages : p.l2_window_stages;
+                // (the GEMM build's flag is up during attention as well, whose own copies keep memory busy: no deeper look
+                // past them, 64 sequences 2248 -> 2187 us)
+                const bool stalled = c.cta_abort[4] && !(kGemm && da.share);
+                const int window = stalled ? p.l2_stall_window_stages : p.l2_window_stages;
                 if (ahead_more && (int)(ahead_stage - stage) < window) {
                     ahead_more = ahead.next(p, queue, da);
                     // skip what the ring already holds or is about to receive, and the other loaders'
@@ -510,8 +656,9 @@ __device__ void loader_main(Ctx c, const int which) {
             const uint32_t dst = c.stage_addr(slot);
             mbar_expect_tx(bar, d.bytes);
             if (d.map == nullptr) {
-                tma_tile5_g2s(dst, &p.k_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
-                tma_tile5_g2s(dst + kStageBytes / 2, &p.v_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
+                const bool share = kBatch > 1 && d.share;
+                tma_tile5_g2s(dst, share ? &p.k_share_map : &p.k_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
+                tma_tile5_g2s(dst + kStageBytes / 2, share ? &p.v_share_map : &p.v_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
             } else {
                 tma_tile4_g2s(dst, d.map, 0, d.c1, d.c2, d.c3, bar, policy);
             }
@@ -1428,6 +1575,348 @@ __device__ bool consumer_attention(const Ctx& c, ConsumerState& cs, const int* w
     return true;
 }
 
+#if MKB_BATCH > 1
+template <int N>  // 2 or 4 neighbouring floats
+__device__ __forceinline__ void load_vec(const float* src, float (&v)[N]) {
+    if constexpr (N == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(src);
+        v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    } else {
+        const float2 x = *reinterpret_cast<const float2*>(src);
+        v[0] = x.x, v[1] = x.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_vec_cg(const float* src, float (&v)[N]) {
+    if constexpr (N == 4) {
+        const uint4 x = ld_cg_v4(src);
+        v[0] = __uint_as_float(x.x), v[1] = __uint_as_float(x.y), v[2] = __uint_as_float(x.z), v[3] = __uint_as_float(x.w);
+    } else {
+        const uint2 x = ld_cg_v2(src);
+        v[0] = __uint_as_float(x.x), v[1] = __uint_as_float(x.y);
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_vec(float* dst, const float (&v)[N]) {
+    if constexpr (N == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
+}
+template <int N>
+__device__ __forceinline__ void store_bf16(__nv_bfloat16* dst, const float (&v)[N]) {
+    if constexpr (N == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+    else *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(v[0], v[1]);
+}
+
+// (row g, elements 2t and 2t + 1) -> (row 2t and 2t + 1, element g) of an 8 x 8 matrix over a warp
+__device__ __forceinline__ uint32_t transpose8(uint32_t x) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
+    return r;
+}
+
+// MKB_OP_BATCH_ATTENTION: one share of a layer's attention (geometry: AttnShares).
+// A ring slot belongs to a group of four warps, which work on four stages side by side: a stage's chain of
+// scores, softmax and values (about 0.5 us) then hides behind the other groups' and behind the copies.  With all 16 warps on
+// one stage after the other, a stage took 1.27 us in the GEMM build and 1.06 us for up to 8 sequences; an SM's
+// share of the memory rate is 0.74 us; now 0.84 us, and a layer's attention 125 us instead of 290 (64 sequences of 256..4096
+// positions), 27 us instead of 37 (7 sequences).  K/V look-ahead in L2 beyond the ring changed nothing.  A warp has 16 positions of one key/value head: scores S = K Q^T with the
+// positions as the M side and the head's queries as N, then O^T = V^T P^T with the head's dimensions as M, so that no side of an MMA
+// is padding but the queries' (4 of 8).  The warps' sums are merged once per piece, in shared memory.
+template <int D, int GQA>
+__device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const int* w) {
+    constexpr int TS = (kStageBytes / 4) / D;  // positions x heads of a stage
+    constexpr int SUB = TS / 64;               // runs of 16 positions per warp
+    constexpr int KP = D / 32, DT = D / 16, VEC = D / 32;
+    static_assert(kNumStages == 4, "a group of warps per ring slot");
+    const KParams& p = *c.p;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;
+    const int layer = __ldg(w + 1);
+    AttnShares shares;
+    if (!shares.begin(c, p, __ldg(w + 2), __ldg(w + 3))) return true;
+
+    {  // the layer's queries, keys and values of all heads are there
+        volatile int* verdict = verdict_word(c, cs);
+        if (warp == 0) {
+            const int row = MKB_OP_RMS_QKV_ROPE_APPEND - 1, slots = p.Hq + 2 * p.Hkv;
+            bool ok = __shfl_sync(0xffffffffu, *c.cta_abort, 0) == 0;  // uniform over the warp
+            for (int s0 = 0; ok && s0 < slots; s0 += 32) {
+                const int slot = s0 + lane;
+                ok = warp_wait_counters(c, slot < slots ? bar_addr(p, layer, row, slot) : nullptr, p.thr_attn_waits_qkv, layer, row, slot,
+                                        (unsigned)p.poll_sleep_ns);
+            }
+            if (lane == 0) {
+                rec(c, MKB_T_CONSUMER_WAIT_DONE);
+                *verdict = ok ? 1 : 0;
+            }
+        }
+        consumer_sync();
+        if (*verdict == 0) return false;
+    }
+
+    const int HP = p.share_heads, PS = TS / HP;
+    const int hd = (warp & 3) % HP, un = (warp & 3) / HP, grp = warp >> 2;
+    float* sml = reinterpret_cast<float*>(__cvta_shared_to_generic(c.base + kSmemAttn));  // (m, l) of [warp][query head]
+    volatile int* merged = c.cta_abort + kCtlShares + kBatch + 2;                          // verdicts of the two cut units
+    int done = 0, ncut = 0, cut_seq[2] = {0, 0}, cut_kvh[2] = {0, 0}, cut_np[2] = {0, 0};
+    AttnPiece a;
+    while (shares.next(c, p, a)) {
+        const int pos_tok = c.pos_of(a.seq), head0 = (a.kvh0 + hd) * GQA;
+        const __nv_bfloat16* q_rope = p.q_rope + (size_t)a.seq * p.o_in;
+        __nv_bfloat16* attn_out = p.attn_out + (size_t)a.seq * p.o_in;
+        float* attn_o = p.attn_o + (size_t)a.seq * p.Hq * p.max_partials * D;
+        float* attn_lse = p.attn_lse + (size_t)a.seq * p.Hq * p.max_partials;
+        const size_t tok = (((size_t)layer * p.B + a.seq) * p.T + pos_tok) * p.Hkv * D;  // the token's own row
+        if (a.n == 0) {  // nothing cached: the token's own value
+            for (int idx = 2 * tid; idx < HP * GQA * D; idx += 2 * kConsumerThreads) {
+                const int h = a.kvh0 * GQA + idx / D;
+                *reinterpret_cast<uint32_t*>(attn_out + (size_t)h * D + idx % D) = ld_cg_u32(p.v_cache + tok + (size_t)(h / GQA) * D + idx % D);
+            }
+            consumer_sync();
+            ++done;
+            continue;
+        }
+        // Q as B operand: column g = query g, chunk (t + 4 j) of the head dimension
+        uint4 qa[KP];
+#pragma unroll
+        for (int j = 0; j < KP; ++j) {
+            qa[j] = make_uint4(0, 0, 0, 0);
+            if (g < GQA) qa[j] = ld_cg_v4(q_rope + (size_t)(head0 + g) * D + (t + 4 * j) * 8);
+        }
+        // queries 2t and 2t + 1: maximum (log2 domain), this lane's part of the sum; dimensions 16 i + g and + 8
+        float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+        float o[DT][4];
+#pragma unroll
+        for (int i = 0; i < DT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+        if (a.hi == a.n && grp == 0 && un == 0) {  // the token's own key and value come first (written by another SM in this launch)
+            const __nv_bfloat16 *kc = p.k_cache + tok + (size_t)(a.kvh0 + hd) * D, *vc = p.v_cache + tok + (size_t)(a.kvh0 + hd) * D;
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < KP; ++j) {
+                float x[8], y[8];
+                unpack8(ld_cg_v4(kc + (t + 4 * j) * 8), x);
+                unpack8(qa[j], y);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
+            }
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            s += __shfl_xor_sync(0xffffffffu, s, 2);
+            s *= p.attn_scale_log2e;
+            m[0] = __shfl_sync(0xffffffffu, s, 8 * t);
+            m[1] = __shfl_sync(0xffffffffu, s, 8 * t + 4);
+            l[0] = l[1] = g == 0 ? 1.f : 0.f;
+#pragma unroll
+            for (int i = 0; i < DT; ++i) {
+                const uint32_t v0 = ld_cg_u32(vc + 16 * i + (g & 6)), v1 = ld_cg_u32(vc + 16 * i + 8 + (g & 6));
+                o[i][0] = o[i][1] = (g & 1) ? bf16_hi(v0) : bf16_lo(v0);
+                o[i][2] = o[i][3] = (g & 1) ? bf16_hi(v1) : bf16_lo(v1);
+            }
+        }
+        for (int s = a.lo; s < a.hi; ++s) {
+            const bool last = s + 1 == a.hi;
+            if ((int)cs.slot == grp) {
+                const uint32_t kbase = consumer_wait_stage(c, cs);
+#pragma unroll 1
+                for (int r = 0; r < SUB; ++r) {
+                    const int in = (un * SUB + r) * 16, pos0 = s * PS + in;
+                    if (pos0 >= pos_tok) break;
+                    const uint32_t tile = kbase + (uint32_t)(hd * (D / 64) * PS + in) * 128u;
+                    float sa[4] = {0.f, 0.f, 0.f, 0.f}, sb[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int j = 0; j < KP; ++j) {
+                        const uint32_t at = tile + (uint32_t)((j >> 1) * PS + g) * 128u + (uint32_t)(((t + 4 * (j & 1)) ^ g) << 4);
+                        const uint4 k0 = lds_v4(at), k1 = lds_v4(at + 8 * 128);
+                        mma_16816(sa, k0.x, k1.x, k0.y, k1.y, qa[j].x, qa[j].y);
+                        mma_16816(sb, k0.z, k1.z, k0.w, k1.w, qa[j].z, qa[j].w);
+                    }
+                    // positions g and g + 8 of queries 2t and 2t + 1
+                    float x[4], mn[2];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        x[e] = pos0 + g + 8 * (e >> 1) < pos_tok ? (sa[e] + sb[e]) * p.attn_scale_log2e : -INFINITY;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        mn[e] = fmaxf(x[e], x[e + 2]);
+                        mn[e] = fmaxf(mn[e], __shfl_xor_sync(0xffffffffu, mn[e], 4));
+                        mn[e] = fmaxf(mn[e], __shfl_xor_sync(0xffffffffu, mn[e], 8));
+                        mn[e] = fmaxf(mn[e], __shfl_xor_sync(0xffffffffu, mn[e], 16));
+                        mn[e] = fmaxf(mn[e], m[e]);
+                    }
+                    if (__any_sync(0xffffffffu, mn[0] != m[0] || mn[1] != m[1])) {
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const float f = exp2f(m[e] - (mn[e] == -INFINITY ? 0.f : mn[e]));
+                            m[e] = mn[e];
+                            l[e] *= f;
+#pragma unroll
+                            for (int i = 0; i < DT; ++i) {
+                                o[i][e] *= f;
+                                o[i][e + 2] *= f;
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        x[e] = exp2f(x[e] - (m[e & 1] == -INFINITY ? 0.f : m[e & 1]));
+                        l[e & 1] += x[e];
+                    }
+                    const uint32_t pb0 = transpose8(pack_bf16x2(x[0], x[1])), pb1 = transpose8(pack_bf16x2(x[2], x[3]));
+                    const int rr = lane & 7, mat = lane >> 3;
+                    const uint32_t vrow = tile + kStageBytes / 2 + (uint32_t)((mat >> 1) * 8 + rr) * 128u;
+#pragma unroll
+                    for (int i = 0; i < DT; ++i) {
+                        uint32_t a0, a1, a2, a3;
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                     : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
+                                     : "r"(vrow + (uint32_t)(i >> 2) * (PS * 128) + (uint32_t)(((2 * (i & 3) + (mat & 1)) ^ rr) << 4)));
+                        mma_16816(o[i], a0, a1, a2, a3, pb0, pb1);
+                    }
+                }
+                if (!last) {  // (the last stage stays ours: the merge below takes place there)
+                    if constexpr (kGemm) {
+                        asm volatile("bar.sync %0, 128;" ::"r"(3 + grp) : "memory");
+                        if ((tid & 127) == 0) mbar_arrive(c.empty_bar(cs.slot));
+                    } else {
+                        __syncwarp();
+                        if (lane == 0)
+                            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], 4;" ::"r"(c.empty_bar(cs.slot)) : "memory");
+                    }
+                }
+            }
+            if (!last && ++cs.slot == kNumStages) {
+                cs.slot = 0;
+                cs.phase ^= 1u;
+            }
+        }
+        if (tid == 0) rec(c, MKB_T_ATTN_STAGES_DONE);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int x = 4; x <= 16; x <<= 1) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
+        float* so = reinterpret_cast<float*>(__cvta_shared_to_generic(c.stage_addr(cs.slot)));  // [warp][4 query heads][D]
+#pragma unroll 1
+        for (int h0 = 0; h0 < GQA; h0 += 4) {  // four query heads of each key/value head at a time
+            consumer_sync();  // every warp is done with the stage (or with the four heads before)
+            if (2 * t >= h0 && 2 * t < h0 + 4) {
+                const int q = 2 * t - h0;
+#pragma unroll
+                for (int i = 0; i < DT; ++i) {
+                    float* dst = so + (size_t)(warp * 4 + q) * D + 16 * i + g;
+                    dst[0] = o[i][0];
+                    dst[D] = o[i][1];
+                    dst[8] = o[i][2];
+                    dst[D + 8] = o[i][3];
+                }
+                if (g == 0) {
+                    float* ml = sml + (warp * 4 + q) * 2;
+                    ml[0] = m[0];
+                    ml[1] = l[0];
+                    ml[2] = m[1];
+                    ml[3] = l[1];
+                }
+            }
+            consumer_sync();
+            for (int hh = warp; hh < HP * 4; hh += kConsumerWarps) {  // a warp per head, VEC dimensions per lane
+                const int h = hh / 4, q = hh % 4, head = (a.kvh0 + h) * GQA + h0 + q;
+                float mx = -INFINITY, den = 0.f, num[VEC] = {};
+                for (int e = h; e < kConsumerWarps; e += HP) mx = fmaxf(mx, sml[(e * 4 + q) * 2]);
+                const float ms = mx == -INFINITY ? 0.f : mx;
+                for (int e = h; e < kConsumerWarps; e += HP) {
+                    const float f = exp2f(sml[(e * 4 + q) * 2] - ms);
+                    den = fmaf(f, sml[(e * 4 + q) * 2 + 1], den);
+                    float v[VEC];
+                    load_vec<VEC>(so + (size_t)(e * 4 + q) * D + lane * VEC, v);
+#pragma unroll
+                    for (int i = 0; i < VEC; ++i) num[i] = fmaf(f, v[i], num[i]);
+                }
+                const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) num[i] *= inv;
+                if (a.np == 1) {
+                    store_bf16<VEC>(attn_out + (size_t)head * D + lane * VEC, num);
+                } else {
+                    const size_t row = (size_t)head * p.max_partials + a.pi;
+                    store_vec<VEC>(attn_o + row * D + lane * VEC, num);
+                    if (lane == 0) attn_lse[row] = den > 0.f ? mx + log2f(den) : -INFINITY;
+                }
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the next copy into the stage follows these writes
+        consumer_sync();  // scratch reads and global stores of all threads are done
+        if constexpr (kGemm) {
+            if (tid == 0) mbar_arrive(c.empty_bar(cs.slot));
+        } else if (lane == 0) {
+            mbar_arrive(c.empty_bar(cs.slot));
+        }
+        if (++cs.slot == kNumStages) {
+            cs.slot = 0;
+            cs.phase ^= 1u;
+        }
+        if (a.np == 1) {
+            ++done;
+        } else {  // (a share cuts its first and its last unit, no others)
+            if (tid == 0) {
+                int old;
+                asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;"
+                             : "=r"(old)
+                             : "l"(bar_addr(p, layer, MKB_OP_PARTIAL_ATTENTION - 1, a.seq * p.Hq + a.kvh0 * GQA))
+                             : "memory");
+                merged[ncut] = old == a.np - 1;
+            }
+            if (ncut == 0) cut_seq[0] = a.seq, cut_kvh[0] = a.kvh0, cut_np[0] = a.np;
+            else cut_seq[1] = a.seq, cut_kvh[1] = a.kvh0, cut_np[1] = a.np;
+            ++ncut;
+        }
+    }
+    if (ncut > 0) {
+        consumer_sync();
+        int merges = 0;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (k >= ncut || merged[k] == 0) continue;
+            ++merges;
+            const int np = cut_np[k], seq = cut_seq[k];
+            const float* attn_lse = p.attn_lse + (size_t)seq * p.Hq * p.max_partials;
+            const float* attn_o = p.attn_o + (size_t)seq * p.Hq * p.max_partials * D;
+            for (int hh = warp; hh < HP * GQA; hh += kConsumerWarps) {  // a warp per head, VEC dimensions per lane
+                const int head = cut_kvh[k] * GQA + hh;
+                const float lse = lane < np ? ld_cg_f32(attn_lse + (size_t)head * p.max_partials + lane) : -INFINITY;
+                const float* base = attn_o + (size_t)head * p.max_partials * D + lane * VEC;
+                constexpr int NB = 6;  // rows on their way together
+                float acc[VEC] = {}, f = 0.f, den = 0.f;
+                for (int j0 = 0; j0 < np; j0 += NB) {
+                    float part[NB][VEC];
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) load_vec_cg<VEC>(base + (size_t)min(j0 + j, np - 1) * D, part[j]);
+                    if (j0 == 0) {
+                        float mx = lse;
+#pragma unroll
+                        for (int x = 16; x >= 1; x >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+                        den = f = exp2f(lse - (mx == -INFINITY ? 0.f : mx));
+#pragma unroll
+                        for (int x = 16; x >= 1; x >>= 1) den += __shfl_xor_sync(0xffffffffu, den, x);
+                    }
+#pragma unroll
+                    for (int j = 0; j < NB; ++j) {
+                        const float wj = __shfl_sync(0xffffffffu, f, (j0 + j) & 31);  // (0 from np on)
+#pragma unroll
+                        for (int i = 0; i < VEC; ++i) acc[i] = fmaf(j0 + j < np ? wj : 0.f, part[j][i], acc[i]);
+                    }
+                }
+                const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) acc[i] *= inv;
+                store_bf16<VEC>(p.attn_out + (size_t)seq * p.o_in + (size_t)head * D + lane * VEC, acc);
+            }
+        }
+        consumer_sync();  // every thread's stores precede the signal
+        done += merges;
+    }
+    if (tid == 0 && done > 0 && !cs.dead) red_release_gpu_add(bar_addr(p, layer, MKB_OP_ATTENTION_REDUCTION - 1, 0), done * HP * GQA);
+    return true;
+}
+#endif  // MKB_BATCH > 1
+
 // AttentionReduction: merge `n` partial (O, LSE) pairs for 4 consecutive heads.
 // One output element per thread (thread = head * D + dim), so a batch of 12 partial rows costs 12
 // registers and all its loads are in flight together: one L2 round trip for up to 12 partials.
@@ -2021,6 +2510,13 @@ __device__ void consumer_main(Ctx c) {
                 else if (gqa == 4) ok = consumer_attention<128, 4>(c, cs, w);
                 else ok = consumer_attention<128, 8>(c, cs, w);
             } break;
+#if MKB_BATCH > 1
+            case MKB_OP_BATCH_ATTENTION:
+                if (p.D == 64) ok = consumer_batch_attention<64, 4>(c, cs, w);
+                else if (p.Hq / p.Hkv == 4) ok = consumer_batch_attention<128, 4>(c, cs, w);
+                else ok = consumer_batch_attention<128, 8>(c, cs, w);
+                break;
+#endif
             case MKB_OP_ATTENTION_REDUCTION:
                 if (p.D == 64) ok = consumer_attn_reduction<64>(c, cs, w);
                 else ok = consumer_attn_reduction<128>(c, cs, w);
@@ -2550,6 +3046,10 @@ __device__ __forceinline__ void megakernel_body(const KParams& p) {
     }
 
     const int warp = threadIdx.x >> 5;
+#if MKB_BATCH > 1
+    if (warp == 1) attn_shares_table(c, p, threadIdx.x & 31);
+    __syncthreads();
+#endif
 #if MKB_BATCH > 8
     // tensor memory for the two accumulators: allocated and freed by warp 0, address through shared memory
     if (warp == 0) {

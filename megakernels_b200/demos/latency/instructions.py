@@ -16,6 +16,7 @@ Reference: megakernels/demos/latency/instructions.py.  Word layouts (after
  7    RMS_LM_Head                     [7, start_blk, end_blk]
  8    TP_AllReduce                    [8, layer, which, chunk, num_chunks]
  9    RMS_Norm                        [9, layer, which, sequence]
+10    BatchAttention                  [10, layer, rank, ranks]
 ====  ==============================  ==========================================
 
 Batched decode (``Globals.batch_size`` > 1, no counterpart in the reference's latency
@@ -23,7 +24,8 @@ kernel): opcode 2 carries the sequence as a sixth word, opcode 3 as the word aft
 ``out_idx`` (both 0 for a single sequence, where the padded words equal the reference's),
 and opcode 9 normalises one sequence's residual stream for all SMs (``which`` 0: attention
 norm, 1: MLP norm, 2: final norm); opcodes 1, 5 and 7 then wait for one arrival per sequence
-in barrier row 9 instead of normalising themselves.
+in barrier row 9 instead of normalising themselves.  Opcode 10 is one of ``ranks`` equal shares of a
+layer's attention over all sequences, in place of its opcodes 2 and 3.
 
 Opcode 8 has no counterpart in the reference: it is one chunk of the in-kernel
 tensor-parallel all-reduce of the residual stream (``which`` 0: after the
@@ -268,6 +270,31 @@ class RMS_Norm(Instruction):
 
     def cost(self, globs: Globals):
         return globs.hidden_size * 8
+
+
+@dataclass
+class BatchAttention(Instruction):
+    """Batched decode only: a share of a layer's attention over all sequences.
+
+    The kernel cuts the cached positions that the sequences have in a launch into ``num_ranks`` equal shares, so
+    the SMs are busy for the same time however ragged the lengths are.
+    """
+
+    layer_idx: int
+    rank: int
+    num_ranks: int
+
+    @classmethod
+    def opcode(cls) -> int:
+        return 10
+
+    @classmethod
+    def prev_opcode(cls) -> int:
+        return LayerNorm_QKV_MatVecRopeAppend.opcode()
+
+    def cost(self, globs: Globals):
+        positions = sum(globs.pos_ids) + globs.batch_size if globs.pos_ids else globs.batch_size
+        return positions * globs.num_kv_heads * globs.head_dim * 2 / self.num_ranks
 
 
 @dataclass

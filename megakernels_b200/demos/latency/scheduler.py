@@ -29,6 +29,7 @@ from torch import Tensor
 
 from megakernels_b200.demos.latency.instructions import (
     AttentionReduction,
+    BatchAttention,
     DownProjResidual,
     Globals,
     Instruction,
@@ -405,11 +406,14 @@ def make_batched_dag(globs: Globals, options: LatencyScheduleOptions, layer_limi
         norm = emit([RMS_Norm(layer, 0, b) for b in range(B)], last)
         qkv = emit(schedule_qkv(globs, layer), norm)
         attn_out: list[DAG_Node] = []
-        for b in range(B):
+        if options.merge_in_last_partial:  # equal shares of whatever the sequences hold
+            ranks = globs.sm_count()
+            attn_out = emit([BatchAttention(layer, r, ranks) for r in range(ranks)], qkv)
+        for b in range(0 if options.merge_in_last_partial else B):
             for kv in range(globs.num_kv_heads):
                 parts = emit([PartialAttention(layer, kv, n_part, p, b) for p in range(n_part)], qkv)
-                if globs.skip_attn_reduction or globs.merge_in_last_partial:
-                    attn_out.extend(parts)  # (the last partial to arrive merges the rows)
+                if globs.skip_attn_reduction:
+                    attn_out.extend(parts)
                     continue
                 for h0 in range(kv * gqa, (kv + 1) * gqa, globs.attn_reduction_size):
                     attn_out.extend(

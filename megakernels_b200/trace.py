@@ -27,6 +27,7 @@ OP_NAMES = {
     7: "lm_head",
     8: "tp_all_reduce",
     9: "rms_norm",
+    10: "batch_attention",
 }
 
 
@@ -71,7 +72,7 @@ def summarize(globs) -> dict:
                 d["stream"].append(us(T_CONSUMER_DONE) - us(T_FIRST_STAGE))
                 d["loader_lead"].append(us(T_CONSUMER_START) - us(T_LOADER_START))
                 d["storer_tail"].append(us(T_STORER_DONE) - us(T_CONSUMER_DONE))
-            elif op == 2:
+            elif op in (2, 10):
                 d["stages"].append(us(5) - us(T_WAIT_DONE))
                 d["merge_store"].append(us(T_CONSUMER_DONE) - us(5))
             elif op == 8:

@@ -137,3 +137,45 @@ def test_batched_decode_matches_independent_sequences(shape, batch, parts, merge
             assert int(out[b]) == int(torch.argmax(g.logits[b])), f"fused argmax, sequence {b}"
             # the appended K/V row, and nothing beyond it
             assert torch.equal(g.k_cache[:, b, pos[b] + 1 :].cpu(), ref.k_cache[:, 0, pos[b] + 1 :])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize(
+    "heads,kv_heads,head_dim,lens",
+    # around a run of 16 positions, a stage and a warp's share of it; nothing cached; one sequence that most shares work on
+    # (its parts are as many as there are rows for); two heads and one per stage; both builds
+    [(32, 8, 128, [0, 1, 2]), (32, 8, 128, [15, 16, 17, 63, 64, 65, 7]), (32, 8, 128, [3000, 0, 40]), (32, 8, 64, [31, 32, 33, 500, 0]),
+     (32, 4, 128, [400, 129]), (16, 2, 128, [700, 33, 0]), (8, 1, 128, [1500, 100]), (32, 8, 128, [(37 * i * i) % 900 for i in range(9)]),
+     (32, 8, 128, [(131 * i) % 1100 for i in range(64)]), (16, 2, 128, [(53 * i) % 300 for i in range(12)])],
+)
+def test_attention_by_shares_matches_attention_by_sequence(heads, kv_heads, head_dim, lens):
+    """What a layer's attention leaves, by shares and by an instruction per sequence and head.  Softmax weights are
+    rounded to bf16 on either side, relative to other running maxima, and so are the results: three roundings of 2^-9."""
+    from megakernels_b200.generators import MK_Generator
+    from tests.gpu_utils import interpreter
+
+    dev, batch = "cuda:0", len(lens)
+    cfg = LlamaConfig.llama_3_1_8b(
+        num_hidden_layers=1, vocab_size=4096, hidden_size=2048, intermediate_size=2048, num_attention_heads=heads,
+        num_key_value_heads=kv_heads, head_dim=head_dim)
+    extra = ExtraModelConfig(interleave_rope=True, max_len_override=max(lens) + 8, max_batch_size=batch)
+    model = LlamaForCausalLM.from_random(cfg, extra, device=dev, seed=0, draw_on="device")
+    gen = torch.Generator(device=dev).manual_seed(2)
+    ids = torch.randint(0, cfg.vocab_size, (batch, 1), generator=torch.Generator().manual_seed(3)).to(dev)
+    prefix = [torch.randn(c.shape, generator=gen, device=dev).to(c.dtype) for c in model.stacked_kv_cache]
+    outs = []
+    for merge in (True, False):
+        for c, x in zip(model.stacked_kv_cache, prefix):
+            c.copy_(x)
+        opts = LatencyScheduleOptions(coalesce_o_proj=True, batch_size=batch, merge_in_last_partial=merge)
+        schedule = LatencyScheduleBuilder(opts).build(model)
+        kinds = {type(i).__name__ for i in schedule.get_linear_instructions()}
+        assert ("BatchAttention" in kinds, "PartialAttention" in kinds) == (merge, not merge)
+        tensorize_instructions(schedule.globs, assign_to_sms("rr", schedule=schedule))
+        mk = MK_Generator(model, interpreter(), schedule)
+        for _ in range(2):
+            mk.run(ids, lens)
+        mk.check()
+        outs.append(schedule.globs.attn_out.float().clone())
+    for b in range(batch):
+        assert float((outs[0][b] - outs[1][b]).norm() / outs[1][b].norm()) < 3 * 2.0**-9, f"sequence {b} of length {lens[b]}"
