@@ -2312,6 +2312,69 @@ __device__ __forceinline__ bool gemm_wait(const Ctx& c, ConsumerState& cs, uint3
     return !cs.dead;
 }
 
+// What a thread, row r of a block, does with its columns c_lo .. c_hi of finished accumulators (columns are
+// sequences).  Out of line and on scalars: within the consumers' loop the compiler has no registers left for it, and what should be on
+// its way together (the angles of eight sequences) went one by one: 23 us a QKV block of 64 sequences, 10 - 12 us the others'.
+struct GemmOut {
+    char* base;        // this row's place for sequence 0
+    size_t stride;     // bytes from a sequence to the next
+    int batch;
+    const float *cos, *sin;  // QKV: this row's column of the tables; null for values
+    uint32_t pos_addr;       // shared memory: the sequences' positions
+    int table_ld;            // floats of a table's row
+    size_t row;              // bytes of a position's row in the cache, 0 for queries
+    long long mult;
+};
+template <int OP>
+__device__ __noinline__ void gemm_epilogue(const uint32_t t0, const uint32_t t1, const int c_lo, const int c_hi, const GemmOut e) {
+    const int lane = threadIdx.x & 31;
+    for (int c0 = c_lo; c0 < c_hi; c0 += 8) {
+        float v[8], v2[8];
+        [[maybe_unused]] int ps[8];
+        if constexpr (OP == MKB_OP_RMS_QKV_ROPE_APPEND) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) asm volatile("ld.shared.s32 %0, [%1];" : "=r"(ps[j]) : "r"(e.pos_addr + (uint32_t)min(c0 + j, e.batch - 1) * 4));
+            if (e.cos != nullptr) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    v[j] = __ldg(e.cos + (size_t)ps[j] * e.table_ld);
+                    v2[j] = __ldg(e.sin + (size_t)ps[j] * e.table_ld);
+                }
+                float x[8];
+                tmem_ld8(t0 + c0, x);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    x[j] = bf16_round(x[j]);
+                    const float other = __shfl_xor_sync(0xffffffffu, x[j], 1);
+                    v[j] = x[j] * v[j] + ((lane & 1) ? other : -other) * v2[j];
+                }
+            } else {
+                tmem_ld8(t0 + c0, v);
+            }
+        } else {
+            tmem_ld8(t0 + c0, v);
+            if constexpr (OP == MKB_OP_RMS_UPGATE_SILU) tmem_ld8(t1 + c0, v2);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (c0 + j >= e.batch) break;
+            char* dst = e.base + (size_t)(c0 + j) * e.stride;
+            if constexpr (OP == MKB_OP_RMS_QKV_ROPE_APPEND) {
+                *reinterpret_cast<__nv_bfloat16*>(dst + (size_t)ps[j] * e.row) = __float2bfloat16_rn(v[j]);
+            } else if constexpr (OP == MKB_OP_O_PROJ_RESIDUAL) {
+                long long x = __float2ll_rn(v[j] * kResidualScale);
+                if (e.mult != 1) x *= e.mult;
+                red_add_u64(dst, (unsigned long long)x);
+            } else if constexpr (OP == MKB_OP_RMS_UPGATE_SILU) {
+                const float up = bf16_round(v[j]), gate = bf16_round(v2[j]);
+                *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(bf16_round(gate / (1.f + __expf(-gate))) * up);
+            } else {
+                *reinterpret_cast<__nv_bfloat16*>(dst) = __float2bfloat16_rn(v[j]);
+            }
+        }
+    }
+}
+
 // One GEMM instruction.  Consumer warp 0 (one lane) issues the MMAs, warps 4..15 are the
 // epilogue (tensor-memory lane quarter = warp % 4, thread = weight row; the three groups of four
 // warps split the sequences), the others only keep their ring bookkeeping in step.
@@ -2375,55 +2438,34 @@ __device__ bool gemm_instruction(const Ctx& c, ConsumerState& cs, const int* w) 
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16);
             const int grow = blk * kBlockRows + r;  // row of the projection's output
-            for (uint32_t c0 = c_lo; c0 < c_hi; c0 += 8) {
-                float v[8], v2[8];
-                tmem_ld8(lane_addr + buf * kBatch + c0, v);
-                if (pair) tmem_ld8(lane_addr + buf2 * kBatch + c0, v2);
-                if (cs.dead) continue;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int s = (int)c0 + j;  // sequence
-                    const bool live = s < p.batch;
-                    switch (g.op) {
-                        case MKB_OP_RMS_QKV_ROPE_APPEND: {
-                            float x = bf16_round(v[j]);
-                            const int k_start = p.Hq * p.D, v_start = (p.Hq + p.Hkv) * p.D;
-                            const int start = blk * kBlockRows;
-                            const int ps = live ? c.pos_of(s) : 0;
-                            if (start < v_start) {  // head_dim == 128 == block: the block is one head
-                                const float cs_ = __ldg(p.rope_cos + (size_t)ps * p.D + r);
-                                const float sn = __ldg(p.rope_sin + (size_t)ps * p.D + r);
-                                const float other = __shfl_xor_sync(0xffffffffu, x, 1);
-                                x = x * cs_ + ((r & 1) ? other : -other) * sn;
-                            }
-                            if (live) {
-                                __nv_bfloat16* dst;
-                                if (start < k_start) {
-                                    dst = p.q_rope + (size_t)s * p.o_in + start;
-                                } else {
-                                    const size_t tok = (((size_t)g.layer * p.B + s) * p.T + ps) * p.Hkv * p.D;
-                                    dst = (start < v_start) ? p.k_cache + tok + (start - k_start)
-                                                            : p.v_cache + tok + (start - v_start);
-                                }
-                                dst[r] = __float2bfloat16_rn(x);
-                            }
-                        } break;
-                        case MKB_OP_O_PROJ_RESIDUAL:
-                        case MKB_OP_DOWN_PROJ_RESIDUAL:
-                            if (live)
-                                red_add_u64(p.residual_acc + (size_t)s * p.H + grow,
-                                            (unsigned long long)(__float2ll_rn(v[j] * kResidualScale) * p.residual_mult));
-                            break;
-                        case MKB_OP_RMS_UPGATE_SILU: {
-                            const float up = bf16_round(v[j]), gate = bf16_round(v2[j]);
-                            const float x = bf16_round(gate / (1.f + __expf(-gate))) * up;
-                            if (live) p.silu_out[(size_t)s * p.I + grow] = __float2bfloat16_rn(x);
-                        } break;
-                        default:  // MKB_OP_RMS_LM_HEAD
-                            if (live) p.logits[(size_t)s * p.V + grow] = __float2bfloat16_rn(v[j]);
-                            break;
-                    }
+            const uint32_t t0 = lane_addr + buf * kBatch, t1 = lane_addr + buf2 * kBatch;
+            GemmOut e{nullptr, 0, p.batch, nullptr, nullptr, c.base + kSmemCtl + 8 * 4, p.D, 0, p.residual_mult};
+            if (cs.dead) {
+            } else if (g.op == MKB_OP_RMS_QKV_ROPE_APPEND) {  // head_dim == 128 == block: the block is one head
+                const int start = blk * kBlockRows, k_start = p.Hq * p.D, v_start = (p.Hq + p.Hkv) * p.D;
+                if (start < v_start) e.cos = p.rope_cos + r, e.sin = p.rope_sin + r;
+                if (start < k_start) {
+                    e.base = reinterpret_cast<char*>(p.q_rope + grow);
+                    e.stride = (size_t)p.o_in * 2;
+                } else {
+                    e.row = (size_t)p.Hkv * p.D * 2;
+                    e.stride = p.T * e.row;
+                    __nv_bfloat16* cache = start < v_start ? p.k_cache + (grow - k_start) : p.v_cache + (grow - v_start);
+                    e.base = reinterpret_cast<char*>(cache) + (size_t)g.layer * p.B * e.stride;
                 }
+                gemm_epilogue<MKB_OP_RMS_QKV_ROPE_APPEND>(t0, t1, c_lo, c_hi, e);
+            } else if (pair) {
+                e.base = reinterpret_cast<char*>(p.silu_out + grow);
+                e.stride = (size_t)p.I * 2;
+                gemm_epilogue<MKB_OP_RMS_UPGATE_SILU>(t0, t1, c_lo, c_hi, e);
+            } else if (g.op == MKB_OP_RMS_LM_HEAD) {
+                e.base = reinterpret_cast<char*>(p.logits + grow);
+                e.stride = (size_t)p.V * 2;
+                gemm_epilogue<MKB_OP_RMS_LM_HEAD>(t0, t1, c_lo, c_hi, e);
+            } else {
+                e.base = reinterpret_cast<char*>(p.residual_acc + grow);
+                e.stride = (size_t)p.H * 8;
+                gemm_epilogue<MKB_OP_O_PROJ_RESIDUAL>(t0, t1, c_lo, c_hi, e);
             }
             // hand the accumulator(s) back, then publish what this block wrote
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
