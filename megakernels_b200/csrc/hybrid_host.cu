@@ -125,7 +125,7 @@ int check_globals(const MkbhGlobals* gp) {
 
 template <typename T>
 cudaError_t gemm(const MkbhGlobals& g, const T* A, int64_t lda, const void* W, int T_, int N, int K, const GemmEpilogue& e, cudaStream_t s) {
-    if constexpr (sizeof(T) == 4) return gemm_f32(A, lda, static_cast<const float*>(W), pad8(K), T_, N, K, e, s);
+    if constexpr (sizeof(T) == 4) return gemm_f32(A, lda, static_cast<const float*>(W), pad8(K), T_, N, K, e, g.status, s);
     else return gemm_bf16(A, lda, static_cast<const bf16*>(W), pad8(K), T_, N, K, e, g.status, s);
 }
 
@@ -278,7 +278,7 @@ int mkb_hybrid_product(const MkbhProduct* p, void* stream) {
     if (p->result == MKBH_GLU) e = GemmEpilogue::glu(p->out, p->ldo, p->limit, p->alpha);
     if (p->result == MKBH_SILU) e = GemmEpilogue::silu(p->out, p->ldo);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (f32) MKBH_TRY(gemm_f32(static_cast<const float*>(p->a), p->lda, static_cast<const float*>(p->w), p->ldw, p->tokens, p->features, p->inner, e, s));
+    if (f32) MKBH_TRY(gemm_f32(static_cast<const float*>(p->a), p->lda, static_cast<const float*>(p->w), p->ldw, p->tokens, p->features, p->inner, e, p->status, s));
     else MKBH_TRY(gemm_bf16(static_cast<const bf16*>(p->a), p->lda, static_cast<const bf16*>(p->w), p->ldw, p->tokens, p->features, p->inner, e,
                             p->status, s, static_cast<const bf16*>(p->w2)));
     return MKBH_OK;

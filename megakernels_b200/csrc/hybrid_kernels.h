@@ -57,7 +57,7 @@ struct GemmEpilogue {
 
 // out[T, N] from A [T, lda] and W [N, ldw], K columns of both (rows 16-byte aligned)
 cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int T, int N, int K,
-                     const GemmEpilogue& e, cudaStream_t s);
+                     const GemmEpilogue& e, int* status, cudaStream_t s, unsigned long long timeout_ns = kWaitNs);
 cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, int T, int N, int K,
                       const GemmEpilogue& e, int* status, cudaStream_t s, const bf16* W2 = nullptr,  // W2: kSilu's up rows
                       unsigned long long timeout_ns = kWaitNs);

@@ -176,8 +176,9 @@ typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void
                              const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// Map of a row-major bf16 matrix; what lies outside it reads as zero.
-inline cudaError_t tc_map(CUtensorMap* map, const bf16* ptr, int cols, int rows, int64_t ld, int box_cols, int box_rows) {
+// Map of a row-major bf16 or float matrix; what lies outside it reads as zero.
+template <typename T>
+inline cudaError_t tc_map(CUtensorMap* map, const T* ptr, int cols, int rows, int64_t ld, int box_cols, int box_rows) {
     static EncodeFn encode = nullptr;
     if (encode == nullptr) {
         void* fn = nullptr;
@@ -188,9 +189,9 @@ inline cudaError_t tc_map(CUtensorMap* map, const bf16* ptr, int cols, int rows,
         encode = reinterpret_cast<EncodeFn>(fn);
     }
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(T)};
     const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, elem[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(ptr), dims, strides, box, elem,
+    const CUresult r = encode(map, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<T*>(ptr), dims, strides, box, elem,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;

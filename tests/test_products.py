@@ -91,3 +91,24 @@ def test_float32_products(result, T, N, K):
     out, want, wrong = product(result, torch.float32, T, N, K)
     assert ((out - want).abs() <= wrong + 2.0**-24 * want.abs()).all()
     assert float((out - want).norm() / want.norm()) < 2e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,N,K", [(3, 260, 40), (16, 256, 8), (17, 1000, 2048), (96, 384, 520), (97, 300, 64), (160, 512, 2048), (161, 2048, 328), (320, 257, 1000)])
+def test_float32_products_of_odd_operands(T, N, K):
+    """Infinite operands, one that rounds to infinity where it is split, and no numbers: results are infinite or no numbers where
+    64-bit sums are, the others within the bound of fp32 sums."""
+    mk = get_mk_module(name="mk_hybrid")
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    a = torch.randn(T, K, generator=gen, device="cuda")
+    w = (torch.randn(N, K, generator=gen, device="cuda") / K**0.5).bfloat16().float()  # (no remainders)
+    a[0, 5], a[1, 7], a[2, 3] = float("inf"), torch.finfo(torch.float32).max, float("nan")
+    w[3, 1], w[200, 4] = float("-inf"), float("nan")
+    out, status = torch.full((T, N), 7.0, device="cuda"), torch.zeros(16, dtype=torch.int32, device="cuda")
+    mk.product("store", a, w, out, status, K)
+    want = a.double() @ w.double().T
+    assert int(status[0]) == 0
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.float().isinf())
+    finite = out.isfinite()
+    size = a.abs().double().nan_to_num(0, 0) @ w.abs().double().nan_to_num(0, 0).T
+    assert ((out.double() - want).abs() <= (K + 1) * 2.0**-24 * size)[finite].all()
