@@ -64,10 +64,10 @@ __device__ __forceinline__ void put(const GemmEpilogue& e, int N, int t, int n, 
         }
         bf16* o = at < 0 ? p.q + (size_t)t * p.q_cols + n : (at < p.k_cols ? p.k + at : p.v + (at - p.k_cols)) + (size_t)(p.pos0 + t) * p.k_cols;
         *reinterpret_cast<uint32_t*>(o) = mkb::pack_bf16x2(x, y);
-    } else if constexpr (kGroup == Group::kFixed) {  // (no other thread writes these)
-        longlong2* o = reinterpret_cast<longlong2*>(static_cast<long long*>(e.cast) + (size_t)t * e.ld + n);
-        const longlong2 v = *o;
-        *o = make_longlong2(v.x + fixed_of(x), v.y + fixed_of(y));
+    } else if constexpr (kGroup == Group::kFixed) {
+        long long* o = static_cast<long long*>(e.cast) + (size_t)t * e.ld + n;
+        mkb::red_add_u64(o, (unsigned long long)fixed_of(x));
+        mkb::red_add_u64(o + 1, (unsigned long long)fixed_of(y));
     } else if (kGroup == Group::kSilu || e.what == Result::kCast) {
         bf16* o = static_cast<bf16*>(e.cast) + (size_t)t * e.ld + n;
         if (n + 1 < N) *reinterpret_cast<uint32_t*>(o) = mkb::pack_bf16x2(x, y);
@@ -77,9 +77,9 @@ __device__ __forceinline__ void put(const GemmEpilogue& e, int N, int t, int n, 
     } else {
         float* o = e.out + (size_t)t * e.ld + n;
         const bool two = n + 1 < N;
-        if (e.what == Result::kAdd) {  // (no other thread writes these)
-            o[0] += (e.scale ? __ldg(e.scale + n) : 1.f) * x;
-            if (two) o[1] += (e.scale ? __ldg(e.scale + n + 1) : 1.f) * y;
+        if (e.what == Result::kAdd) {  // (no other thread writes these: one addition each, in L2)
+            asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o), "f"((e.scale ? __ldg(e.scale + n) : 1.f) * x) : "memory");
+            if (two) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + 1), "f"((e.scale ? __ldg(e.scale + n + 1) : 1.f) * y) : "memory");
         } else {
             o[0] = x + (e.bias ? __ldg(e.bias + n) : 0.f);
             if (two) o[1] = y + (e.bias ? __ldg(e.bias + n + 1) : 0.f);
@@ -329,24 +329,44 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         tc_cluster_sync();
         const int m0 = (worker % s.tiles_m) * kBM, n0 = (worker / s.tiles_m) * wide, rows = min(kBM, s.T - m0);
         const uint32_t me = tc_rank(), parts = s.parts;
-        for (int i = (int)me + (int)parts * warp; i < rows; i += (int)parts * (kGemmThreads / 32))
+        // Four rows of a warp at a time: a row's parts, another SM's shared memory, take most of a microsecond to arrive.
+        constexpr int kRowsAtOnce = 4, kWarps = kGemmThreads / 32;
+        const int next = (int)parts * kWarps;
+        for (int i0 = (int)me + (int)parts * warp; i0 < rows; i0 += kRowsAtOnce * next)
 #pragma unroll 1
             for (int c = 2 * lane; c < wide; c += 64) {
-                float x = 0.f, y = 0.f, ux = 0.f, uy = 0.f;
-#pragma unroll 4
-                for (uint32_t z = 0; z < parts; ++z) {
-                    const uint32_t at = tc_peer(base + (uint32_t)(i * kPartRow<kBN> + c) * 4, z);
-                    const float2 v = tc_peer_load2(at);
-                    x += v.x;
-                    y += v.y;
-                    if constexpr (kDual) {
-                        const float2 u = tc_peer_load2(at + wide * 4);
-                        ux += u.x;
-                        uy += u.y;
-                    }
+                float2 sum[kRowsAtOnce], up[kRowsAtOnce];
+#pragma unroll
+                for (int r = 0; r < kRowsAtOnce; ++r) sum[r] = up[r] = make_float2(0.f, 0.f);
+                for (uint32_t z = 0; z < parts; z += 2) {  // (two or four parts)
+                    float2 v[2][kRowsAtOnce], u[2][kRowsAtOnce];
+#pragma unroll
+                    for (int y = 0; y < 2; ++y)
+#pragma unroll
+                        for (int r = 0; r < kRowsAtOnce; ++r) {
+                            const uint32_t at = tc_peer(base + (uint32_t)(min(i0 + r * next, rows - 1) * kPartRow<kBN> + c) * 4, z + y);
+                            v[y][r] = tc_peer_load2(at);
+                            if constexpr (kDual) u[y][r] = tc_peer_load2(at + wide * 4);
+                        }
+#pragma unroll
+                    for (int y = 0; y < 2; ++y)
+#pragma unroll
+                        for (int r = 0; r < kRowsAtOnce; ++r) {
+                            sum[r].x += v[y][r].x;
+                            sum[r].y += v[y][r].y;
+                            if constexpr (kDual) {
+                                up[r].x += u[y][r].x;
+                                up[r].y += u[y][r].y;
+                            }
+                        }
                 }
-                if constexpr (kDual) x *= sigmoid_f(x) * ux, y *= sigmoid_f(y) * uy;
-                put<kGroup>(e, s.N, m0 + i, n0 + c, x, y);
+#pragma unroll
+                for (int r = 0; r < kRowsAtOnce; ++r) {
+                    if (i0 + r * next >= rows) break;
+                    float x = sum[r].x, y = sum[r].y;
+                    if constexpr (kDual) x *= sigmoid_f(x) * up[r].x, y *= sigmoid_f(y) * up[r].y;
+                    put<kGroup>(e, s.N, m0 + i0 + r * next, n0 + c, x, y);
+                }
             }
         tc_cluster_sync();
     }

@@ -104,6 +104,9 @@ __device__ __forceinline__ void split4(float4& x, float4& r, float& odd) {
 __device__ __forceinline__ bool infinite(float h) { return (__float_as_uint(h) & 0x7fffffffu) == 0x7f800000u; }
 __device__ __forceinline__ bool infinite4(const float4& h) { return infinite(h.x) | infinite(h.y) | infinite(h.z) | infinite(h.w); }
 
+// (no other thread writes these: one addition each, in L2, and nobody waits for it)
+__device__ __forceinline__ void add_once(float* o, float x) { asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o), "f"(x) : "memory"); }
+
 // columns n (even) and n + 1 of token t
 __device__ __forceinline__ void put(const GemmEpilogue& e, int t, int n, int N, float x, float y) {
     if (n >= N) return;
@@ -113,8 +116,8 @@ __device__ __forceinline__ void put(const GemmEpilogue& e, int t, int n, int N, 
     }
     float* o = (e.what == Result::kCast ? static_cast<float*>(e.cast) : e.out) + (size_t)t * e.ld + n;
     if (e.what == Result::kAdd) {
-        o[0] += (e.scale ? e.scale[n] : 1.f) * x;
-        if (n + 1 < N) o[1] += (e.scale ? e.scale[n + 1] : 1.f) * y;
+        add_once(o, (e.scale ? e.scale[n] : 1.f) * x);
+        if (n + 1 < N) add_once(o + 1, (e.scale ? e.scale[n + 1] : 1.f) * y);
     } else {
         o[0] = x + (e.bias ? e.bias[n] : 0.f);
         if (n + 1 < N) o[1] = y + (e.bias ? e.bias[n + 1] : 0.f);
@@ -398,7 +401,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_kernel(const __grid_cons
 #pragma unroll
                 for (int j = 0; j < C; ++j)
                     if (tt + j < end) {
-                        if (e.what == Result::kAdd) o[(size_t)j * e.ld] += f * sum[j];
+                        if (e.what == Result::kAdd) add_once(o + (size_t)j * e.ld, f * sum[j]);
                         else o[(size_t)j * e.ld] = sum[j] + b;
                     }
             }
