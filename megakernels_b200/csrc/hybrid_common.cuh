@@ -26,7 +26,10 @@ template <> __device__ __forceinline__ bf16 from_f<bf16>(float v) { return __flo
 
 // Launches that may begin while the one before them on the stream still runs (programmatic dependent launch): a kernel
 // launched this way touches nothing that an earlier launch writes or reads before `after_previous`; the next one's
-// blocks may be placed as soon as all of this one's have called `let_next` (or left).
+// blocks may be placed as soon as all of this one's have called `let_next` (or left).  Weights are no launch's result:
+// the first launch of a prompt is an ordinary one, so whatever wrote them before has ended.  Kernels whose pointers are
+// __restrict__ call both in front of a body of their own, so that no read of what is another launch's result can be moved
+// before the wait.
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 inline cudaLaunchAttribute may_begin_early() {

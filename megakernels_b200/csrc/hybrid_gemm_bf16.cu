@@ -38,6 +38,7 @@ struct Shape {
     int T, N, K, tiles_m, tiles, parts, a_rows;  // parts: CTAs that share a tile's inner dimension; a_rows: tokens of a copy
     unsigned long long timeout_ns;
     int* status;
+    bool early;  // begins before the launch before it has ended: weights may be read until then
 };
 
 // What the epilogue can do: a build per group of results, so that one group's code does not cost the others registers.
@@ -141,7 +142,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = (uint32_t)ctl[1];
     let_next();
-    after_previous();
+    if (warp != 0) after_previous();
     constexpr bool kDual = kGroup == Group::kSilu;
     constexpr int wide = kDual ? kBN / 2 : kBN;
     int ksteps = (s.K + kBK - 1) / kBK, kfirst = 0;
@@ -155,6 +156,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         const bool chosen = tc_elect();
         uint32_t it = 0;
         bool ok = true;
+        auto weights = [&](int st, int k, int n0) {
+            const uint32_t dw = base + st * G::kStageBytes + kBM * kBK * 2;
+            if (rank == 0) mkb::mbar_expect_tx(full(st), kPair * (s.a_rows + G::kRowsW) * kBK * 2);
+            if constexpr (kPair == 2) {  // both CTAs' copies count on the first one's barrier
+                const uint32_t bar = tc_peer(full(st), 0);
+                if (kDual) tc_tma_2d_pair(dw, rank ? &wmap2 : &wmap, k * kBK, n0, bar);
+                else tc_tma_2d_pair(dw, &wmap, k * kBK, n0 + rank * G::kRowsW, bar);
+            } else {
+                tc_tma_2d(dw, &wmap, (kfirst + k) * kBK, n0, full(st));
+                if (kDual) tc_tma_2d(dw + kBN / 2 * kBK * 2, &wmap2, (kfirst + k) * kBK, n0, full(st));
+            }
+        };
+        // a ring of weights is on its way while the launch before this one ends (if it has ended, the tokens' copies
+        // would only wait behind them)
+        const int before = s.early ? min(ksteps, G::kStages) : 0;
+        if (chosen)
+            for (int k = 0; k < before; ++k) weights(k, k, (worker / s.tiles_m) * wide);
+        after_previous();
         for (int tile = worker; tile < s.tiles && ok; tile += workers) {
             const int m0 = ((tile % s.tiles_m) * kPair + rank) * kBM, n0 = (tile / s.tiles_m) * wide;
             for (int k = 0; k < ksteps; ++k, ++it) {
@@ -162,19 +181,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                 ok = __all_sync(0xffffffffu, tc_wait(empty(st), ((it / G::kStages) & 1u) ^ 1u, ctl, s.timeout_ns, s.status, 0));
                 if (!ok) break;
                 if (!chosen) continue;
-                const uint32_t dst = base + st * G::kStageBytes, dw = dst + kBM * kBK * 2;
-                if (rank == 0) mkb::mbar_expect_tx(full(st), kPair * (s.a_rows + G::kRowsW) * kBK * 2);
-                if constexpr (kPair == 2) {  // both CTAs' copies count on the first one's barrier
-                    const uint32_t bar = tc_peer(full(st), 0);
-                    tc_tma_2d_pair(dst, &amap, k * kBK, m0, bar);
-                    if (kDual) tc_tma_2d_pair(dw, rank ? &wmap2 : &wmap, k * kBK, n0, bar);
-                    else tc_tma_2d_pair(dw, &wmap, k * kBK, n0 + rank * G::kRowsW, bar);
-                } else {
-                    const int kx = (kfirst + k) * kBK;
-                    tc_tma_2d(dst, &amap, kx, m0, full(st));
-                    tc_tma_2d(dw, &wmap, kx, n0, full(st));
-                    if (kDual) tc_tma_2d(dw + kBN / 2 * kBK * 2, &wmap2, kx, n0, full(st));
-                }
+                if (it >= (uint32_t)before) weights(st, k, n0);
+                const uint32_t dst = base + st * G::kStageBytes;
+                if constexpr (kPair == 2) tc_tma_2d_pair(dst, &amap, k * kBK, m0, tc_peer(full(st), 0));
+                else tc_tma_2d(dst, &amap, (kfirst + k) * kBK, m0, full(st));
             }
         }
         // no copy may be in flight when the CTA's shared memory goes away, nor an arrival from the pair's first CTA
@@ -469,10 +479,10 @@ cudaError_t choose(const bf16* A, int64_t lda, const bf16* W, const bf16* W2, in
 }  // namespace
 
 cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, int T, int N, int K, const GemmEpilogue& e,
-                      int* status, cudaStream_t st, const bf16* W2, unsigned long long timeout_ns) {
+                      int* status, cudaStream_t st, const bf16* W2, unsigned long long timeout_ns, bool early) {
     int sms = 0;
     if (const cudaError_t err = sm_count(&sms); err != cudaSuccess) return err;
-    const Shape s{T, N, K, 0, 0, 1, 0, timeout_ns, status};
+    const Shape s{T, N, K, 0, 0, 1, 0, timeout_ns, status, early};
     switch (group_of(e.what)) {
         case Group::kSilu: return choose<Group::kSilu>(A, lda, W, W2, ldw, s, e, sms, st);
         case Group::kRope: return choose<Group::kRope>(A, lda, W, W2, ldw, s, e, sms, st);

@@ -47,6 +47,7 @@ struct ShapeF {
     int T, N, K, tokens, token_tiles, parts;  // tokens of a tile (the rest of its NT are padding)
     unsigned long long timeout_ns;
     int* status;
+    bool early;
 };
 
 __device__ __forceinline__ void mma_tf32(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_kernel(const __grid_cons
     tc_after_sync();
     const uint32_t tmem = (uint32_t)ctl[1];
     let_next();
-    after_previous();
+    if (warp != 0) after_previous();
     const int tile = blockIdx.x / s.parts, part = blockIdx.x % s.parts;
     const int t0 = (tile % s.token_tiles) * s.tokens, n0 = (tile / s.token_tiles) * kFeatures;
     const int steps_all = (s.K + kStep - 1) / kStep, first = steps_all * part / s.parts, steps = steps_all * (part + 1) / s.parts - first;
@@ -248,13 +249,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_kernel(const __grid_cons
         const bool chosen = tc_elect();
         bool ok = true;
         int it = 0;
+        auto weights = [&](int i) {
+            const uint32_t b = w_full(i % G::kWStages);
+            mkb::mbar_expect_tx(b, G::kW);
+            tc_tma_2d(base + i % G::kWStages * G::kW, &wmap, (first + i) * kStep, n0, b);
+        };
+        // a ring of weights is on its way while the launch before this one ends
+        const int before = s.early ? min(steps, G::kWStages) : 0;
+        if (chosen)
+            for (int i = 0; i < before; ++i) weights(i);
+        after_previous();
         for (; it < steps; ++it) {
             const int ws = it % G::kWStages, xs = it % G::kXStages;
             ok = __all_sync(0xffffffffu, wait(w_empty(ws), it / G::kWStages + 1, 0) && wait(empty(xs), it / G::kXStages + 1, 0));
             if (!ok) break;
             if (!chosen) continue;
-            mkb::mbar_expect_tx(w_full(ws), G::kW);
-            tc_tma_2d(base + ws * G::kW, &wmap, (first + it) * kStep, n0, w_full(ws));
+            if (it >= before) weights(it);
             mkb::mbar_expect_tx(full(xs), G::kX);
             tc_tma_2d(base + G::kTokens + xs * G::kX, &amap, (first + it) * kStep, t0, full(xs));
         }
@@ -460,7 +470,7 @@ cudaError_t launch(const float* A, int64_t lda, const float* W, int64_t ldw, Sha
 }  // namespace
 
 cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int T, int N, int K,
-                     const GemmEpilogue& e, int* status, cudaStream_t st, unsigned long long timeout_ns) {
+                     const GemmEpilogue& e, int* status, cudaStream_t st, unsigned long long timeout_ns, bool early) {
     if (T <= 2) {
         const int blocks = (N + 15) / 16;
         if (T == 1) gemv_f32_kernel<1><<<blocks, 256, 0, st>>>(A, lda, W, ldw, N, K, e);
@@ -473,7 +483,7 @@ cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, i
     // and an end of its own; a cluster's exchange besides.  Clusters of eight wait for whole groups of SMs (20 x 2048 x 8192: 57 us, four
     // 49 us, when a step took as long).
     const int widths[] = {16, 32, 64, 96, 128, 160}, steps = (K + kStep - 1) / kStep, rows = (N + kFeatures - 1) / kFeatures;
-    ShapeF s{T, N, K, 0, 0, 1, timeout_ns, status};
+    ShapeF s{T, N, K, 0, 0, 1, timeout_ns, status, early};
     int width = 0;
     float least = 0.f;
     for (int w : widths) {

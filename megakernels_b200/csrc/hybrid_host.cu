@@ -123,10 +123,12 @@ int check_globals(const MkbhGlobals* gp) {
     return MKBH_OK;
 }
 
+// `early`: the launch before lets the next one begin (products, flash_tc, the launches of launch_early)
 template <typename T>
-cudaError_t gemm(const MkbhGlobals& g, const T* A, int64_t lda, const void* W, int T_, int N, int K, const GemmEpilogue& e, cudaStream_t s) {
-    if constexpr (sizeof(T) == 4) return gemm_f32(A, lda, static_cast<const float*>(W), pad8(K), T_, N, K, e, g.status, s);
-    else return gemm_bf16(A, lda, static_cast<const bf16*>(W), pad8(K), T_, N, K, e, g.status, s);
+cudaError_t gemm(const MkbhGlobals& g, const T* A, int64_t lda, const void* W, int T_, int N, int K, const GemmEpilogue& e, cudaStream_t s,
+                 bool early = false) {
+    if constexpr (sizeof(T) == 4) return gemm_f32(A, lda, static_cast<const float*>(W), pad8(K), T_, N, K, e, g.status, s, kWaitNs, early);
+    else return gemm_bf16(A, lda, static_cast<const bf16*>(W), pad8(K), T_, N, K, e, g.status, s, nullptr, kWaitNs, early);
 }
 
 template <typename T>
@@ -164,8 +166,8 @@ int prefill(const MkbhGlobals& g, cudaStream_t s) {
         }
         if (L.canon_taps || beside) MKBH_TRY(P::canon_norm(g, L, act, beside ? act2 : nullptr, ldx, s));
         else MKBH_TRY(P::norm(g, nullptr, n, L.norm1, act, ldx, s));
-        MKBH_TRY(gemm<T>(g, act, ldx, L.in_w, n, L.in_rows, width, GemmEpilogue::store(g.proj, ldp, L.in_bias), s));
-        if (beside) MKBH_TRY(gemm<T>(g, act2, ldx, L.up_w, n, up_rows(L), width, GemmEpilogue::glu(ffn, ldf, L.glu_limit, L.glu_alpha), s));
+        MKBH_TRY(gemm<T>(g, act, ldx, L.in_w, n, L.in_rows, width, GemmEpilogue::store(g.proj, ldp, L.in_bias), s, L.canon_taps || beside));
+        if (beside) MKBH_TRY(gemm<T>(g, act2, ldx, L.up_w, n, up_rows(L), width, GemmEpilogue::glu(ffn, ldf, L.glu_limit, L.glu_alpha), s, true));
         const int K = mixer_out(L);
         if (L.mixer == MKBH_DELTA_RULE) {
             MKBH_TRY(P::delta(g, L, act, pad8(K), s));
@@ -180,9 +182,10 @@ int prefill(const MkbhGlobals& g, cudaStream_t s) {
             }
             MKBH_TRY(P::rotary_attention(g, L, act, pad8(K), s));
         }
-        if (L.canon_taps > 1 || L.conv_taps > 1) MKBH_TRY(P::keep_inputs(g, L, s));
-        MKBH_TRY(gemm<T>(g, act, pad8(K), L.out_w, n, width, K, GemmEpilogue::add(g.x, width, L.ls1), s));
-        if (beside) MKBH_TRY(gemm<T>(g, ffn, ldf, L.down_w, n, width, L.ff, GemmEpilogue::add(g.x, width, L.ls2), s));
+        const bool keep = L.canon_taps > 1 || L.conv_taps > 1;
+        if (keep) MKBH_TRY(P::keep_inputs(g, L, s));
+        MKBH_TRY(gemm<T>(g, act, pad8(K), L.out_w, n, width, K, GemmEpilogue::add(g.x, width, L.ls1), s, keep));
+        if (beside) MKBH_TRY(gemm<T>(g, ffn, ldf, L.down_w, n, width, L.ff, GemmEpilogue::add(g.x, width, L.ls2), s, true));
         else if (L.ff)
             if (int rc = feed_forward<T>(g, L, s)) return rc;
         if (g.layers_out)
@@ -278,9 +281,9 @@ int mkb_hybrid_product(const MkbhProduct* p, void* stream) {
     if (p->result == MKBH_GLU) e = GemmEpilogue::glu(p->out, p->ldo, p->limit, p->alpha);
     if (p->result == MKBH_SILU) e = GemmEpilogue::silu(p->out, p->ldo);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (f32) MKBH_TRY(gemm_f32(static_cast<const float*>(p->a), p->lda, static_cast<const float*>(p->w), p->ldw, p->tokens, p->features, p->inner, e, p->status, s));
+    if (f32) MKBH_TRY(gemm_f32(static_cast<const float*>(p->a), p->lda, static_cast<const float*>(p->w), p->ldw, p->tokens, p->features, p->inner, e, p->status, s, kWaitNs, false));
     else MKBH_TRY(gemm_bf16(static_cast<const bf16*>(p->a), p->lda, static_cast<const bf16*>(p->w), p->ldw, p->tokens, p->features, p->inner, e,
-                            p->status, s, static_cast<const bf16*>(p->w2)));
+                            p->status, s, static_cast<const bf16*>(p->w2), kWaitNs, false));
     return MKBH_OK;
 }
 

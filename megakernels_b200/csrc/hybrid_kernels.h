@@ -18,6 +18,20 @@ inline cudaError_t sm_count(int* sms) {
     return e;
 }
 
+// A launch that may begin before the one before it on the stream has ended (its kernel calls `after_previous`).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute early = may_begin_early();
+    c.attrs = &early;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+}
+
 constexpr unsigned long long kWaitNs = 2000000000ull;  // how long a kernel's waits go on before they give up
 
 // What a matrix product does with its result.
@@ -55,12 +69,13 @@ struct GemmEpilogue {
     static GemmEpilogue rotate(const RopeTarget& r) { return {Result::kRope, nullptr, nullptr, 0, nullptr, nullptr, 0.f, 0.f, r}; }
 };
 
-// out[T, N] from A [T, lda] and W [N, ldw], K columns of both (rows 16-byte aligned)
+// out[T, N] from A [T, lda] and W [N, ldw], K columns of both (rows 16-byte aligned); `early`: the launch before lets this one
+// begin early, and weights are read from then on
 cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, int T, int N, int K,
-                     const GemmEpilogue& e, int* status, cudaStream_t s, unsigned long long timeout_ns = kWaitNs);
+                     const GemmEpilogue& e, int* status, cudaStream_t s, unsigned long long timeout_ns = kWaitNs, bool early = true);
 cudaError_t gemm_bf16(const bf16* A, int64_t lda, const bf16* W, int64_t ldw, int T, int N, int K,
                       const GemmEpilogue& e, int* status, cudaStream_t s, const bf16* W2 = nullptr,  // W2: kSilu's up rows
-                      unsigned long long timeout_ns = kWaitNs);
+                      unsigned long long timeout_ns = kWaitNs, bool early = true);
 
 // Causal attention of `n` queries from position pos0 on over a cache [position, kv head, dim] that holds
 // their own rows too; dim 64 or 128.  Nothing beyond row pos0 + n - 1 is read.

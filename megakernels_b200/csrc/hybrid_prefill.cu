@@ -141,10 +141,10 @@ template <> struct Quad<bf16> {
 // A block takes kTokens tokens: fewer where there are not enough blocks for the SMs.
 constexpr int kCanonTaps = 4;
 template <typename T, int kT, int kTokens>
-__global__ void __launch_bounds__(kThreads) canon_norm4_kernel(const float* __restrict__ x, int n, int pos0, int width,
-                                                               const float* __restrict__ w1, const float* __restrict__ w2, float eps,
-                                                               const float* __restrict__ taps_w, const float* __restrict__ hist,
-                                                               float* __restrict__ tail, T* __restrict__ out, T* __restrict__ out2, int64_t ld) {
+__device__ __noinline__ void canon_norm4_kernel_body(const float* __restrict__ x, int n, int pos0, int width, const float* __restrict__ w1,
+                                                     const float* __restrict__ w2, float eps, const float* __restrict__ taps_w,
+                                                     const float* __restrict__ hist, float* __restrict__ tail, T* __restrict__ out,
+                                                     T* __restrict__ out2, int64_t ld) {
     constexpr int kBack = kT > 1 ? kT - 1 : 0, kRowsHere = kTokens + kBack;
     __shared__ float inv[kRowsHere];
     const int t0 = blockIdx.x * kTokens, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -206,6 +206,14 @@ __global__ void __launch_bounds__(kThreads) canon_norm4_kernel(const float* __re
         }
     }
 }
+template <typename T, int kT, int kTokens>
+__global__ void __launch_bounds__(kThreads) canon_norm4_kernel(const float* x, int n, int pos0, int width, const float* w1, const float* w2,
+                                                               float eps, const float* taps_w, const float* hist, float* tail, T* out, T* out2,
+                                                               int64_t ld) {
+    let_next();
+    after_previous();
+    canon_norm4_kernel_body<T, kT, kTokens>(x, n, pos0, width, w1, w2, eps, taps_w, hist, tail, out, out2, ld);
+}
 
 // After a portion: the last taps - 1 inputs of a convolution by position, and the sum of the next
 // position's terms of earlier inputs.  `back(i)` is the input i tokens before the portion's end.
@@ -220,8 +228,8 @@ __device__ __forceinline__ void keep_channel(const float* w, float* hist, float*
     for (int i = 0; i < taps - 1 && i < n; ++i) hist[((end - i) % (taps - 1)) * ld] = back(i);
     *next = s;
 }
-__global__ void __launch_bounds__(kThreads) keep_inputs_kernel(const MkbhLayer L, int slot, int n, int pos0, int width,
-                                                               const float* __restrict__ tail, const float* __restrict__ proj, int64_t ld) {
+__device__ __noinline__ void keep_inputs_kernel_body(const MkbhLayer& L, int slot, int n, int pos0, int width, const float* __restrict__ tail,
+                                                     const float* __restrict__ proj, int64_t ld) {
     const int ch = blockIdx.x * kThreads + threadIdx.x, end = pos0 + n - 1;
     if (L.canon_taps > 1 && ch < width)
         keep_channel(L.canon_w + ch, L.canon_hist + (size_t)slot * (L.canon_taps - 1) * width + ch,
@@ -231,6 +239,12 @@ __global__ void __launch_bounds__(kThreads) keep_inputs_kernel(const MkbhLayer L
         keep_channel(L.conv_w + ch, L.conv_hist + (size_t)slot * (L.conv_taps - 1) * L.in_rows + ch,
                      L.conv_part + (size_t)slot * L.in_rows + ch, L.conv_taps, L.in_rows, n, end,
                      [&](int i) { return proj[(size_t)(n - 1 - i) * ld + ch]; });
+}
+__global__ void __launch_bounds__(kThreads) keep_inputs_kernel(const MkbhLayer L, int slot, int n, int pos0, int width, const float* tail,
+                                                               const float* proj, int64_t ld) {
+    let_next();
+    after_previous();
+    keep_inputs_kernel_body(L, slot, n, pos0, width, tail, proj, ld);
 }
 
 // ---- PolyNorm ----------------------------------------------------------------------------- //
@@ -919,7 +933,7 @@ cudaError_t Prefill<T>::canon_norm(const MkbhGlobals& g, const MkbhLayer& L, T* 
         auto go = [&](auto taps) {
             const auto kernel = few ? canon_norm4_kernel<T, decltype(taps)::value, 2> : canon_norm4_kernel<T, decltype(taps)::value, kNormTokens>;
             const int tokens = few ? 2 : kNormTokens;
-            kernel<<<(n + tokens - 1) / tokens, kThreads, 0, s>>>(g.x, n, g.pos0, g.width, L.norm1, L.norm2, g.eps, L.canon_w, hist, g.tail, out,
+            launch_early(kernel, (n + tokens - 1) / tokens, kThreads, 0, s, g.x, n, g.pos0, g.width, L.norm1, L.norm2, g.eps, L.canon_w, hist, g.tail, out,
                                                                  out2, ld);
         };
         switch (L.canon_taps) {
@@ -946,7 +960,7 @@ cudaError_t Prefill<T>::canon_norm(const MkbhGlobals& g, const MkbhLayer& L, T* 
 template <typename T>
 cudaError_t Prefill<T>::keep_inputs(const MkbhGlobals& g, const MkbhLayer& L, cudaStream_t s) {
     const int channels = max(L.canon_taps > 1 ? g.width : 0, L.conv_taps > 1 ? L.in_rows : 0);
-    keep_inputs_kernel<<<(channels + kThreads - 1) / kThreads, kThreads, 0, s>>>(L, g.slot, g.num_tokens, g.pos0, g.width, g.tail, g.proj,
+    launch_early(keep_inputs_kernel, (channels + kThreads - 1) / kThreads, kThreads, 0, s, L, g.slot, g.num_tokens, g.pos0, g.width, g.tail, g.proj,
                                                                                 pad8(L.in_rows));
     return cudaGetLastError();
 }

@@ -80,7 +80,7 @@ cudaError_t prompt_launch(const MkbGlobals& g, const MkbPrompt& p, int* status, 
         c.stream = s;
         cudaLaunchAttribute early = mkbh::may_begin_early();
         c.attrs = &early;
-        c.numAttrs = 1;
+        c.numAttrs = first ? 0 : 1;  // (the first launch waits for all that came before, the weights' arrival among it)
         return cudaLaunchKernelEx(&c, prompt_norm_kernel, static_cast<const bf16*>(p.hidden) + (size_t)row0 * H, b.sums + (size_t)row0 * H, first, last,
                                   H, g.rms_norm_eps, w, b.act);
     };
