@@ -41,6 +41,23 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// two floats at this shared-memory address of the cluster's CTA `rank`
+template <bool kSplit>
+__device__ __forceinline__ float2 peer_load2(uint32_t addr, uint32_t rank) {
+    uint32_t at;
+    float2 v;
+    if constexpr (!kSplit) {
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+        return v;
+    }
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at) : "memory");
+    return v;
+}
+
 struct FlashArgs {
     const float* proj;
     int64_t ld, ldo;
@@ -49,7 +66,8 @@ struct FlashArgs {
     const bf16 *kc, *vc;
     bf16* out;
     float eps;
-    int dp;  // dim padded to 16
+    int dp;     // dim padded to 16
+    int parts;  // CTAs, a cluster, that share a block's keys
 };
 
 struct FlashSmem {  // bf16 element offsets; row strides are odd multiples of 16 bytes
@@ -62,18 +80,19 @@ struct FlashSmem {  // bf16 element offsets; row strides are odd multiples of 16
         buf = 2 * kBKeys * qs + kBKeys * vs;
         v = k + 2 * kBKeys * qs;
         total = k + 2 * buf;
-        const int merge = k + kBQ * (ep + 4) * 2;  // second map's rows as floats
+        const int merge = k + 2 * 2 * kBQ * (ep + 4 + 2);  // both maps' rows as floats, their maxima and sums
         if (merge > total) total = merge;
     }
 };
 
-template <int EP>
+template <int EP, bool kSplit>
 __global__ void __launch_bounds__(kFlashThreads, EP <= 128 ? 2 : 1) flash_kernel(const FlashArgs a) {
     extern __shared__ __align__(128) bf16 sm[];
     const MkbhLayer& L = a.L;
     const int D = L.dim, E = L.vdim, G = L.kv_heads, dp = a.dp;
     const FlashSmem S(dp, EP);
-    const int h = blockIdx.y, g = h / (L.heads / G), t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kBQ;
+    const int parts = kSplit ? a.parts : 1, part = kSplit ? (int)blockIdx.x % parts : 0;
+    const int h = blockIdx.y, g = h / (L.heads / G), t0 = ((int)(gridDim.x - blockIdx.x - 1) / parts) * kBQ;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int map = warp >> 2, r0 = (warp & 3) * 16;  // this warp's query rows
     const int nq = min(kBQ, a.n - t0);
@@ -89,12 +108,17 @@ __global__ void __launch_bounds__(kFlashThreads, EP <= 128 ? 2 : 1) flash_kernel
         return keep + (r >= ring ? r - ring : r);
     };
 
-    for (int i = tid; i < S.total / 8; i += kFlashThreads) reinterpret_cast<uint4*>(sm)[i] = make_uint4(0, 0, 0, 0);
-    __syncthreads();  // padding columns stay zero
-    for (int i = tid; i < nq * 2 * D; i += kFlashThreads) {
-        const int r = i / (2 * D), c = i % (2 * D), m = c >= D;
-        sm[S.q + (m * kBQ + r) * S.qs + c - m * D] = __float2bfloat16_rn(a.proj[(size_t)(t0 + r) * a.ld + h * 2 * D + c]);
+    if (D != dp) {  // padding columns stay zero (rows beyond the portion are their own)
+        for (int i = tid; i < S.total / 8; i += kFlashThreads) reinterpret_cast<uint4*>(sm)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
     }
+#pragma unroll 4
+    for (int r = warp; r < nq; r += kFlashThreads / 32)
+        for (int c = 4 * lane; c < 2 * D; c += 128) {  // (D is a multiple of 8, rows begin at 16 bytes)
+            const float4 v = *reinterpret_cast<const float4*>(a.proj + (size_t)(t0 + r) * a.ld + h * 2 * D + c);
+            const int m = c >= D;
+            *reinterpret_cast<uint2*>(sm + S.q + (m * kBQ + r) * S.qs + c - m * D) = make_uint2(mkb::pack_bf16x2(v.x, v.y), mkb::pack_bf16x2(v.z, v.w));
+        }
     const int kunits = D / 8, vunits = E / 8;
     auto fetch = [&](int tile, int buf) {
         const uint32_t kd = mkb::smem_u32(sm + S.k + buf * S.buf), vd = mkb::smem_u32(sm + S.v + buf * S.buf);
@@ -125,9 +149,9 @@ __global__ void __launch_bounds__(kFlashThreads, EP <= 128 ? 2 : 1) flash_kernel
     const float scale = L.scale * 1.4426950408889634f;
     const int row_pos[2] = {p0 + r0 + (lane >> 2), p0 + r0 + (lane >> 2) + 8};
 
-    const int tiles = (total + kBKeys - 1) / kBKeys;
-    fetch(0, 0);
-    for (int tile = 0; tile < tiles; ++tile) {
+    const int all_tiles = (total + kBKeys - 1) / kBKeys, tile0 = all_tiles * part / parts, tiles = all_tiles * (part + 1) / parts;
+    if (tile0 < tiles) fetch(tile0, tile0 & 1);
+    for (int tile = tile0; tile < tiles; ++tile) {
         const int buf = tile & 1;
         if (tile + 1 < tiles) {
             fetch(tile + 1, buf ^ 1);
@@ -222,67 +246,103 @@ __global__ void __launch_bounds__(kFlashThreads, EP <= 128 ? 2 : 1) flash_kernel
         }
         __syncthreads();
     }
+    // Both maps' rows, maxima and sums go through shared memory (the tiles are done with); then all warps of the cluster put
+    // the parts together, combine the maps, normalise and gate, whole rows in a loop.  Unrolled in registers this was 100 KB
+    // of code that every launch fetched anew (46 us for 30 tokens in all, now 20; 2048 tokens 669 and 531 us).
+    float* rows = reinterpret_cast<float*>(sm + S.k);
+    const int os = EP + 4;
+    float2* stats = reinterpret_cast<float2*>(rows + 2 * kBQ * os);
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         l_[r] += __shfl_xor_sync(0xffffffffu, l_[r], 1);
         l_[r] += __shfl_xor_sync(0xffffffffu, l_[r], 2);
-        l_[r] = l_[r] > 0.f ? 1.f / l_[r] : 0.f;  // rows beyond the portion have no keys
+        const int at = map * kBQ + r0 + (lane >> 2) + 8 * r;
+        if ((lane & 3) == 0) stats[at] = make_float2(m_[r], l_[r]);
+#pragma unroll
+        for (int i = 0; i < EP / 8; ++i) *reinterpret_cast<float2*>(rows + at * os + i * 8 + (lane & 3) * 2) = make_float2(o[i][2 * r], o[i][2 * r + 1]);
     }
-    float* other = reinterpret_cast<float*>(sm + S.k);  // second map's rows (the tiles are done with)
-    const int os = EP + 4;
-    if (map == 1) {
+    if constexpr (kSplit) cluster_sync();
+    else __syncthreads();
+    const uint32_t rows_at = mkb::smem_u32(rows), stats_at = mkb::smem_u32(stats);
+    for (int row = part + parts * warp; row < nq; row += parts * (kFlashThreads / 32)) {
+        constexpr int N = (EP + 63) / 64;
+        float2 v[N], g2[N];
+        const float* gate = a.proj + (size_t)(t0 + row) * a.ld + L.heads * 2 * D + h * E;
+        bf16* dst = a.out + (size_t)(t0 + row) * a.ldo + h * E;
 #pragma unroll
-        for (int i = 0; i < EP / 8; ++i)
+        for (int k = 0; k < N; ++k) {
+            const int e = 64 * k + 2 * lane;  // (E is a multiple of 8)
+            v[k] = make_float2(0.f, 0.f);
+            g2[k] = e < E ? __ldg(reinterpret_cast<const float2*>(gate + e)) : make_float2(0.f, 0.f);
+        }
+#pragma unroll 1
+        for (int m = 0; m < 2; ++m) {
+            const int at = m * kBQ + row;
+            float top = -INFINITY, den = 0.f;
+            for (int z = 0; z < parts; ++z) top = fmaxf(top, peer_load2<kSplit>(stats_at + at * 8, z).x);
+            const float base = top == -INFINITY ? 0.f : top;
+            float2 sum[N];
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
-                *reinterpret_cast<float2*>(other + (r0 + (lane >> 2) + 8 * r) * os + i * 8 + (lane & 3) * 2) =
-                    make_float2(o[i][2 * r] * l_[r], o[i][2 * r + 1] * l_[r]);
-    }
-    __syncthreads();
-    if (map == 1) return;
+            for (int k = 0; k < N; ++k) sum[k] = make_float2(0.f, 0.f);
+            for (int z = 0; z < parts; ++z) {
+                const float2 ml = peer_load2<kSplit>(stats_at + at * 8, z);
+                const float w = fast_exp2(ml.x - base);
+                den = fmaf(w, ml.y, den);
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int row = r0 + (lane >> 2) + 8 * r;
+                for (int k = 0; k < N; ++k) {
+                    if (64 * k + 2 * lane >= E) break;
+                    const float2 x = peer_load2<kSplit>(rows_at + (at * os + 64 * k + 2 * lane) * 4, z);
+                    sum[k].x = fmaf(w, x.x, sum[k].x);
+                    sum[k].y = fmaf(w, x.y, sum[k].y);
+                }
+            }
+            const float f = (m ? -L.lambda : 1.f) * (den > 0.f ? 1.f / den : 0.f);
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                v[k].x = fmaf(f, sum[k].x, v[k].x);
+                v[k].y = fmaf(f, sum[k].y, v[k].y);
+            }
+        }
         float sq = 0.f;
 #pragma unroll
-        for (int i = 0; i < EP / 8; ++i) {
-            const float2 b = *reinterpret_cast<const float2*>(other + row * os + i * 8 + (lane & 3) * 2);
-            const float x = o[i][2 * r] * l_[r] - L.lambda * b.x, y = o[i][2 * r + 1] * l_[r] - L.lambda * b.y;
-            o[i][2 * r] = x;
-            o[i][2 * r + 1] = y;
-            sq += x * x + y * y;
-        }
-        sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-        sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-        if (row >= nq) continue;  // (after the shuffles)
-        const float fin = (1.f - L.diff) / sqrtf(sq / E + a.eps);
-        const float* __restrict__ gate = a.proj + (size_t)(t0 + row) * a.ld + L.heads * 2 * D + h * E;
-        bf16* __restrict__ dst = a.out + (size_t)(t0 + row) * a.ldo + h * E;
+        for (int k = 0; k < N; ++k) sq += v[k].x * v[k].x + v[k].y * v[k].y;  // (zero beyond E)
+        const float fin = (1.f - L.diff) / sqrtf(warp_sum(sq) / E + a.eps);
 #pragma unroll
-        for (int i = 0; i < EP / 8; ++i) {
-            const int e = i * 8 + (lane & 3) * 2;
-            if (e < E)  // E is a multiple of 8
-                *reinterpret_cast<uint32_t*>(dst + e) =
-                    mkb::pack_bf16x2(o[i][2 * r] * fin * sigmoid_f(__ldg(gate + e)), o[i][2 * r + 1] * fin * sigmoid_f(__ldg(gate + e + 1)));
+        for (int k = 0; k < N; ++k) {
+            const int e = 64 * k + 2 * lane;
+            if (e < E) *reinterpret_cast<uint32_t*>(dst + e) = mkb::pack_bf16x2(v[k].x * fin * sigmoid_f(g2[k].x), v[k].y * fin * sigmoid_f(g2[k].y));
         }
     }
+    if constexpr (kSplit) cluster_sync();  // (the others may still read here)
 }
 
-template <int EP>
-cudaError_t launch(const FlashArgs& a, cudaStream_t s) {
+template <int EP, bool kSplit>
+cudaError_t launch_flash(const FlashArgs& a, cudaStream_t s) {
     static int set[64] = {};
     const int bytes = FlashSmem(a.dp, EP).total * 2;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (set[dev & 63] < bytes) {
-        e = cudaFuncSetAttribute(flash_kernel<EP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        e = cudaFuncSetAttribute(flash_kernel<EP, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
         set[dev & 63] = bytes;
     }
-    flash_kernel<EP><<<dim3((a.n + kBQ - 1) / kBQ, a.L.heads), kFlashThreads, bytes, s>>>(a);
-    return cudaGetLastError();
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((a.n + kBQ - 1) / kBQ * a.parts, a.L.heads);
+    c.blockDim = dim3(kFlashThreads);
+    c.dynamicSmemBytes = bytes;
+    c.stream = s;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = a.parts;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    c.attrs = &cluster;
+    c.numAttrs = a.parts > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&c, flash_kernel<EP, kSplit>, a);
 }
+template <int EP>
+cudaError_t launch(const FlashArgs& a, cudaStream_t s) { return a.parts > 1 ? launch_flash<EP, true>(a, s) : launch_flash<EP, false>(a, s); }
 
 // ---- one map ------------------------------------------------------------------------------- //
 struct RotaryArgs {
@@ -516,7 +576,13 @@ bool flash_supported(const MkbhLayer& L) { return L.dim % 8 == 0 && L.vdim % 8 =
 
 cudaError_t flash_attention(const MkbhGlobals& g, const MkbhLayer& L, const bf16* kc, const bf16* vc, bf16* out,
                             int64_t ldo, cudaStream_t s) {
-    FlashArgs a{g.proj, pad8(L.in_rows), ldo, g.num_tokens, g.pos0, L, kc, vc, out, g.eps, (L.dim + 15) & ~15};
+    FlashArgs a{g.proj, pad8(L.in_rows), ldo, g.num_tokens, g.pos0, L, kc, vc, out, g.eps, (L.dim + 15) & ~15, 1};
+    // few queries over several tiles of keys: CTAs that would have nothing to do take a share of the tiles each (100 queries
+    // after 500 positions, 16 heads of 64: 51 us alone, 30 with four)
+    int sms = 0;
+    if (const cudaError_t e = sm_count(&sms); e != cudaSuccess) return e;
+    const int blocks = (a.n + kBQ - 1) / kBQ * L.heads, keys = min(a.pos0 + a.n, L.window + kBQ + L.keep_first);
+    while (a.parts < 8 && 2 * a.parts * blocks <= sms && 2 * a.parts * kBKeys <= keys) a.parts *= 2;
     if (L.vdim <= 32) return launch<32>(a, s);
     if (L.vdim <= 64) return launch<64>(a, s);
     if (L.vdim <= 128) return launch<128>(a, s);

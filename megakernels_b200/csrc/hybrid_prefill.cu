@@ -754,9 +754,17 @@ template <> struct Pair<bf16> {
     using type = uint32_t;
     static __device__ __forceinline__ uint32_t make(float x, float y) { return mkb::pack_bf16x2(x, y); }
 };
-template <typename T, int J, bool kConv, typename Dst>
+// where the vectors of a head go: rows of queries, or rows of a cache
+template <typename T, bool kCache>
+struct Place {
+    T* base;
+    int64_t ld;
+    int keep, ring;
+    __device__ __forceinline__ T* at(int t, int pos) const { return base + (size_t)(kCache ? cache_row(pos, keep, ring) : t) * ld; }
+};
+template <typename T, int J, bool kConv, bool kCache>
 __device__ __forceinline__ void operand_run(const OperandArgs& a, int t0, int t1, int col, int len, const float* w, const float* rope, int rot,
-                                            int end, Dst dst) {
+                                            int end, const Place<T, kCache>& place) {
     const MkbhLayer& L = a.L;
     const int lane = threadIdx.x & 31, taps = L.conv_taps;
     float2 tap[kConv ? kTaps : 1][J], norm[J], u[kConv ? kTaps : 1][J];  // tap k, u[k]: k tokens ago
@@ -806,7 +814,7 @@ __device__ __forceinline__ void operand_run(const OperandArgs& a, int t0, int t1
             s = fmaf(v[j].x, v[j].x, fmaf(v[j].y, v[j].y, s));
         }
         const float inv = w != nullptr ? 1.f / sqrtf(warp_sum(s) / len + a.eps) : 1.f;
-        T* o = dst(t);
+        T* o = place.at(t, a.pos0 + t);
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const int i = 2 * (lane + 32 * j);
@@ -816,58 +824,58 @@ __device__ __forceinline__ void operand_run(const OperandArgs& a, int t0, int t1
         for (int i = 64 * J + 2 * lane; i < end; i += 64) *reinterpret_cast<typename Pair<T>::type*>(o + i) = Pair<T>::make(0.f, 0.f);
     }
 }
-// A vector of a run of tokens, by whatever path its size allows.
-template <typename T, bool kConv, typename Dst>
+// A vector of a run of tokens, by whatever path its size allows.  (One copy for keys and values: with one each, and with
+// places as functions, the rotary kernel was 680 KB of code.)
+template <typename T, bool kConv, bool kCache>
 __device__ __forceinline__ void operand_tokens(const OperandArgs& a, int t0, int t1, int col, int len, const float* w, const float* rope, int rot,
-                                               int end, Dst dst) {
+                                               int end, const Place<T, kCache>& place) {
     const bool pairs = (col & 1) == 0 && (len & 1) == 0 && (rot == 0 || len >= rot) && (!kConv || a.L.conv_taps <= kTaps) &&
-                       (reinterpret_cast<uint64_t>(dst(t0)) & (2 * sizeof(T) - 1)) == 0 && (reinterpret_cast<uint64_t>(dst(t0 + 1)) & (2 * sizeof(T) - 1)) == 0;
-    if (pairs && len <= 64) return operand_run<T, 1, kConv>(a, t0, t1, col, len, w, rope, rot, end, dst);
-    if (pairs && len <= 128) return operand_run<T, 2, kConv>(a, t0, t1, col, len, w, rope, rot, end, dst);
+                       (reinterpret_cast<uint64_t>(place.base) & (2 * sizeof(T) - 1)) == 0 && (place.ld & 1) == 0;
+    if (pairs && len <= 64) return operand_run<T, 1, kConv, kCache>(a, t0, t1, col, len, w, rope, rot, end, place);
+    if (pairs && len <= 128) return operand_run<T, 2, kConv, kCache>(a, t0, t1, col, len, w, rope, rot, end, place);
     if constexpr (!kConv) {
-        if (pairs && len <= 256) return operand_run<T, 4, kConv>(a, t0, t1, col, len, w, rope, rot, end, dst);
-        if (pairs) return operand_run<T, 8, kConv>(a, t0, t1, col, len, w, rope, rot, end, dst);
+        if (pairs && len <= 256) return operand_run<T, 4, kConv, kCache>(a, t0, t1, col, len, w, rope, rot, end, place);
+        if (pairs) return operand_run<T, 8, kConv, kCache>(a, t0, t1, col, len, w, rope, rot, end, place);
     }
     for (int t = t0; t < t1; ++t) {
         const float2* angles = reinterpret_cast<const float2*>(rope) + (size_t)(a.pos0 + t) * (rot / 2);
-        if (len <= 256) operand_vector<T, 4>(a, t, col, len, w, angles, rot, dst(t));
-        else operand_vector<T, 8>(a, t, col, len, w, angles, rot, dst(t));
-        for (int i = len + (threadIdx.x & 31); i < end; i += 32) dst(t)[i] = from_f<T>(0.f);
+        T* o = place.at(t, a.pos0 + t);
+        if (len <= 256) operand_vector<T, 4>(a, t, col, len, w, angles, rot, o);
+        else operand_vector<T, 8>(a, t, col, len, w, angles, rot, o);
+        for (int i = len + (threadIdx.x & 31); i < end; i += 32) o[i] = from_f<T>(0.f);
     }
 }
 template <typename T, bool kLatent>
-__global__ void __launch_bounds__(kThreads) rotary_operands_kernel(const OperandArgs a) {
+__global__ void __launch_bounds__(kThreads, 3) rotary_operands_kernel(const OperandArgs a) {
     const MkbhLayer& L = a.L;
     const int task = blockIdx.y * (kThreads / 32) + (threadIdx.x >> 5), H = L.heads, G = L.kv_heads;
     if (task >= (kLatent ? H + 2 : H + 2 * G)) return;
     const int t0 = blockIdx.x * a.run, t1 = min(a.n, t0 + a.run);
     const size_t rows = L.cache_keep + L.cache_ring;
-    auto query = [&](int h, int off) { return [=](int t) { return static_cast<T*>(a.query) + (size_t)t * a.ldq + h * a.qhead + off; }; };
-    auto cache = [&](void* base, size_t first, int len, int off) {
-        return [=](int t) { return static_cast<T*>(base) + (first + cache_row(a.pos0 + t, a.L.cache_keep, a.L.cache_ring)) * len + off; };
-    };
+    const Place<T, false> query{static_cast<T*>(a.query) + task * a.qhead, a.ldq, 0, 0};
     if constexpr (kLatent) {
         const int hd = L.dim + L.rot_dim, lr = latent_row(L);
+        const Place<T, true> latent{static_cast<T*>(a.kc), lr, L.cache_keep, L.cache_ring};
         if (task < H) {
-            operand_tokens<T, false>(a, t0, t1, task * hd, L.dim, nullptr, nullptr, 0, a.qrest, query(task, 0));
-            operand_tokens<T, false>(a, t0, t1, task * hd + L.dim, L.rot_dim, nullptr, L.rope, L.rope_dims, a.qhead - a.qrest, query(task, a.qrest));
+            operand_tokens<T, false>(a, t0, t1, task * hd, L.dim, nullptr, nullptr, 0, a.qrest, query);
+            const Place<T, false> rotated{query.base + a.qrest, a.ldq, 0, 0};
+            operand_tokens<T, false>(a, t0, t1, task * hd + L.dim, L.rot_dim, nullptr, L.rope, L.rope_dims, a.qhead - a.qrest, rotated);
         } else if (task == H) {
-            operand_tokens<T, false>(a, t0, t1, H * hd, L.rank, L.k_norm, nullptr, 0, L.rank, cache(a.kc, 0, lr, 0));
+            operand_tokens<T, false>(a, t0, t1, H * hd, L.rank, L.k_norm, nullptr, 0, L.rank, latent);
         } else {
-            operand_tokens<T, false>(a, t0, t1, H * hd + L.rank, L.rot_dim, nullptr, L.rope, L.rope_dims, L.rot_dim, cache(a.kc, 0, lr, pad8(L.rank)));
+            const Place<T, true> rotated{latent.base + pad8(L.rank), lr, L.cache_keep, L.cache_ring};
+            operand_tokens<T, false>(a, t0, t1, H * hd + L.rank, L.rot_dim, nullptr, L.rope, L.rope_dims, L.rot_dim, rotated);
         }
     } else {
         auto run = [&](auto conv) {
             constexpr bool kConv = decltype(conv)::value;
-            if (task < H) {
-                operand_tokens<T, kConv>(a, t0, t1, task * L.dim, L.dim, L.q_norm, L.rope, L.rope_dims, a.qhead, query(task, 0));
-            } else if (task < H + G) {
-                operand_tokens<T, kConv>(a, t0, t1, task * L.dim, L.dim, L.k_norm, L.rope, L.rope_dims, L.dim, cache(a.kc, (task - H) * rows, L.dim, 0));
-            } else {
-                const int g = task - H - G;
-                operand_tokens<T, kConv>(a, t0, t1, (H + G) * L.dim + g * L.vdim, L.vdim, nullptr, L.value_rope, L.value_rope ? L.vdim : 0, L.vdim,
-                                         cache(a.vc, g * rows, L.vdim, 0));
-            }
+            if (task < H) return operand_tokens<T, kConv>(a, t0, t1, task * L.dim, L.dim, L.q_norm, L.rope, L.rope_dims, a.qhead, query);
+            // keys or values
+            const bool key = task < H + G;
+            const int g = key ? task - H : task - H - G, len = key ? L.dim : L.vdim, col = key ? task * L.dim : (H + G) * L.dim + g * L.vdim;
+            const float* rope = key ? L.rope : L.value_rope;
+            const Place<T, true> place{static_cast<T*>(key ? a.kc : a.vc) + g * rows * len, len, L.cache_keep, L.cache_ring};
+            operand_tokens<T, kConv>(a, t0, t1, col, len, key ? L.k_norm : nullptr, rope, key ? L.rope_dims : rope ? len : 0, len, place);
         };
         if (L.conv_taps > 0) run(std::true_type{});
         else run(std::false_type{});
