@@ -384,57 +384,43 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_kernel(const __grid_cons
         }
         if (ok) {
             add_columns<C>(at + G::kSums * NT, sum);  // (the last commit covers these too)
-            if (ctl[2]) {
+            // the ring's stages have been read: [token][feature], for the loop below (unrolled from registers, with its kinds of
+            // results, it was 100 KB of code)
+            float* o = reinterpret_cast<float*>(gbase) + half * C * kFeatures + q * 32 + lane;
 #pragma unroll
-                for (int j = 0; j < C; ++j) sum[j] = 0.f;
-                const int last = min(s.K, (first + steps) * kStep);
-                for (int k = first * kStep; n < s.N && k < last; ++k) {
-                    const float w = W[(size_t)n * ldw + k];
-#pragma unroll
-                    for (int j = 0; j < C; ++j)
-                        if (tt + j < end) sum[j] = fmaf(w, A[(size_t)(tt + j) * lda + k], sum[j]);
+            for (int j = 0; j < C; ++j) o[j * kFeatures] = sum[j];
+            if (ctl[2]) {  // with FMA
+                for (int j = 0; j < C && tt + j < end; ++j) {
+                    float x = 0.f;
+                    const float *w = W + (size_t)n * ldw, *v = A + (size_t)(tt + j) * lda;
+                    const int last = min(s.K, (first + steps) * kStep);
+                    for (int k = first * kStep; n < s.N && k < last; ++k) x = fmaf(w[k], v[k], x);
+                    o[j * kFeatures] = x;
                 }
-            }
-            if (s.parts > 1) {  // the ring's stages have been read: [token][feature]
-                float* o = reinterpret_cast<float*>(gbase) + half * C * kFeatures + q * 32 + lane;
-#pragma unroll
-                for (int j = 0; j < C; ++j) o[j * kFeatures] = sum[j];
-            } else if (e.what == Result::kGlu) {
-#pragma unroll
-                for (int j = 0; j < C; ++j) {
-                    const float up = __shfl_down_sync(0xffffffffu, sum[j], 1);
-                    if (!(lane & 1) && tt + j < end) put(e, tt + j, n, s.N, sum[j], up);
-                }
-            } else if (n < s.N) {
-                float* o = (e.what == Result::kCast ? static_cast<float*>(e.cast) : e.out) + (size_t)tt * e.ld + n;
-                const float b = e.bias ? e.bias[n] : 0.f, f = e.scale ? e.scale[n] : 1.f;
-#pragma unroll
-                for (int j = 0; j < C; ++j)
-                    if (tt + j < end) {
-                        if (e.what == Result::kAdd) add_once(o + (size_t)j * e.ld, f * sum[j]);
-                        else o[(size_t)j * e.ld] = sum[j] + b;
-                    }
             }
         }
     }
     tc_before_sync();
     __syncthreads();
     if (*ctl) tc_settle();
-    if (s.parts > 1) {
-        tc_cluster_sync();
-        const int tokens = min(s.tokens, s.T - t0), c = 4 * lane;
-        for (int t = part + s.parts * warp; t < tokens; t += s.parts * (kThreads / 32)) {
-            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (s.parts > 1) tc_cluster_sync();
+    const int tokens = min(s.tokens, s.T - t0), c = 4 * lane;
+#pragma unroll 2
+    for (int t = part + s.parts * warp; t < tokens; t += s.parts * (kThreads / 32)) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s.parts == 1) {
+            x = *reinterpret_cast<const float4*>(gbase + (t * kFeatures + c) * 4);
+        } else {
             for (int z = 0; z < s.parts; ++z) {
                 const uint32_t at = tc_peer(base + (uint32_t)(t * kFeatures + c) * 4, z);
                 const float2 u = tc_peer_load2(at), v = tc_peer_load2(at + 8);
                 x.x += u.x, x.y += u.y, x.z += v.x, x.w += v.y;
             }
-            put(e, t0 + t, n0 + c, s.N, x.x, x.y);
-            put(e, t0 + t, n0 + c + 2, s.N, x.z, x.w);
         }
-        tc_cluster_sync();
+        put(e, t0 + t, n0 + c, s.N, x.x, x.y);
+        put(e, t0 + t, n0 + c + 2, s.N, x.z, x.w);
     }
+    if (s.parts > 1) tc_cluster_sync();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)G::kTmem) : "memory");
 }
 

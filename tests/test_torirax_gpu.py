@@ -307,3 +307,18 @@ def test_trace_run(bench, tmp_path, dtype, tol):
     assert rel(read(2), want[[41, 43]]) < tol and rel(read(4), want[[45, 99]]) < tol
     for k in range(5):
         assert rel(read(5 + k), want[9 + k : 10 + k]) < tol
+
+
+@pytest.mark.parametrize(
+    "heads,kv_heads,dim,vdim,size,keep_first,earlier,count",
+    # CTAs that share a block's keys: two, four and eight of them, parts that begin inside the kept keys or a window's edge, one
+    # block of queries and two, every width of values, padded sizes
+    [(4, 2, 64, 128, 1000, 4, 130, 3), (3, 3, 16, 32, 700, 0, 300, 65), (2, 1, 128, 256, 520, 9, 600, 2), (2, 2, 24, 56, 300, 200, 640, 30),
+     (6, 3, 8, 24, 640, 3, 700, 17), (1, 1, 64, 120, 128, 0, 400, 64)],
+)
+def test_few_queries_over_many_keys(tmp_path, heads, kv_heads, dim, vdim, size, keep_first, earlier, count):
+    raw = model_config([attention(heads, kv_heads, dim, vdim, size=size, keep_first=keep_first, ff=40)], max_positions=800)
+    weights, tokens = make_weights(raw), tokens_for(raw, earlier + count)
+    gen = load(write_checkpoint(tmp_path / "m", raw, weights), dtype=torch.bfloat16)
+    got = run_cut(gen, tokens, [earlier, count])
+    assert rel(got[earlier:], oracle_logits(raw, weights, tokens)[earlier:]) < BF16_TOL
