@@ -454,7 +454,8 @@ template <> struct Chunk<bf16> {
 };
 
 // Multiply the instruction's rows with the activations in `act` (fp32, zero beyond the matrix's
-// columns); partial sums [row][group] replace them.  Ends with a consumer barrier.
+// columns); partial sums [group][row] replace them (a row's by a thread: with its groups side by side its 32 lanes' reads
+// fell into two banks).  Ends with a consumer barrier.
 template <typename T, int kPer>
 __device__ __forceinline__ bool matvec_rows(const Params& p, Cta& c, const Desc& d, float* act, uint32_t& ring_slot,
                                             uint32_t& ring_phase) {
@@ -510,7 +511,7 @@ __device__ __forceinline__ bool matvec_rows(const Params& p, Cta& c, const Desc&
             y += __shfl_xor_sync(0xffffffffu, y, 2);
             y += __shfl_xor_sync(0xffffffffu, y, 1);
             const int row = r + (lane >> 3) * nrg;
-            if ((lane & 7) == 0 && row < n) act[(r0 + row) * groups + cg] = y;
+            if ((lane & 7) == 0 && row < n) act[cg * rows + r0 + row] = y;
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(c.empty(slot));
@@ -1846,7 +1847,8 @@ __device__ __forceinline__ void consumer_main(const Params& p, Cta& c, const Sme
             unsigned long long best = 0;
             if (tid < rows) {
                 float y = 0.f;
-                for (int k = 0; k < d.groups; ++k) y += act[tid * d.groups + k];
+#pragma unroll 4
+                for (int k = 0; k < d.groups; ++k) y += act[k * rows + tid];
                 const int row = d.a0 + tid;
                 kept = y;
                 if (adds) {
@@ -1864,7 +1866,8 @@ __device__ __forceinline__ void consumer_main(const Params& p, Cta& c, const Sme
                 } else if ((F & kRotary) && op == MKBH_OP_NORM_UP && (F == kRotary || L.ff_kind == MKBH_CLAMPED_GLU)) {  // rows alternate gate, up
                     if ((tid & 1) == 0) {
                         float up = 0.f;
-                        for (int k = 0; k < d.groups; ++k) up += act[(tid + 1) * d.groups + k];
+#pragma unroll 4
+                        for (int k = 0; k < d.groups; ++k) up += act[k * rows + tid + 1];
                         side_in(g)[row >> 1] = clamped_glu(y, up, L.glu_limit, L.glu_alpha);
                     }
                 } else if (op == MKBH_OP_HEAD) {
