@@ -2304,6 +2304,12 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
 }
+// one lane of a converged warp, always the same one
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
 __device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 2, 384;" ::: "memory"); }  // warps 4..15
 __device__ __forceinline__ bool gemm_wait(const Ctx& c, ConsumerState& cs, uint32_t bar, uint32_t parity) {
     if (!cs.dead && !mbar_try_wait(bar, parity)) {
@@ -2387,10 +2393,13 @@ __device__ bool gemm_instruction(const Ctx& c, ConsumerState& cs, const int* w) 
     const uint32_t n = (uint32_t)p.gemm_n;
     const uint32_t tmem = c.tmem_base();
 
-    if (warp == 0 && lane == 0) {
+    if (__shfl_sync(0xffffffffu, warp, 0) == 0) {
+        // The warp stays converged and an elected lane issues: on one lane of a diverged warp every operand of an MMA is first
+        // moved to uniform registers, and a stage took 0.62 us whatever was copied meanwhile.
         // fp32 accumulate, bf16 x bf16, both operands K-major, N = n, M = 128
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((uint32_t)(kBlockRows >> 4) << 24);
         uint32_t slot = cs.slot, phase = cs.phase, xstage = cs.xstage, acc = cs.acc;
+        const bool chosen = elect_lane();
         for (int b = 0; b < g.nblocks; ++b) {
             const uint32_t buf = acc & 1u, use = acc >> 1;
             gemm_wait(c, cs, c.acc_empty_bar(buf), (use & 1u) ^ 1u);  // the epilogue has drained this accumulator
@@ -2399,26 +2408,29 @@ __device__ bool gemm_instruction(const Ctx& c, ConsumerState& cs, const int* w) 
                 const uint32_t xslot = xstage % kXStages;
                 gemm_wait(c, cs, c.full_bar(slot), phase);
                 gemm_wait(c, cs, c.xfull_bar(xslot), (xstage / kXStages) & 1u);
-                if (b == 0 && st == 0) rec(c, MKB_T_CONSUMER_FIRST_STAGE);
+                cs.dead = __any_sync(0xffffffffu, cs.dead);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t wb = c.stage_addr(slot), xb = c.xstage_addr(xslot);
-                if (!cs.dead) {
+                if (chosen) {
+                    if (b == 0 && st == 0) rec(c, MKB_T_CONSUMER_FIRST_STAGE);
+                    const uint32_t wb = c.stage_addr(slot), xb = c.xstage_addr(xslot);
+                    if (!cs.dead) {
 #pragma unroll
-                    for (int ch = 0; ch < kStageCols / 64; ++ch)  // one swizzle atom (64 columns) at a time
+                        for (int ch = 0; ch < kStageCols / 64; ++ch)  // one swizzle atom (64 columns) at a time
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)                // four K = 16 steps inside the 128-byte rows
-                            umma_f16(tmem + buf * kBatch, umma_smem_desc(wb + ch * (kBlockRows * 128) + k * 32),
-                                     umma_smem_desc(xb + ch * (n * 128) + k * 32), idesc, (uint32_t)((st | ch | k) != 0));
+                            for (int k = 0; k < 4; ++k)                // four K = 16 steps inside the 128-byte rows
+                                umma_f16(tmem + buf * kBatch, umma_smem_desc(wb + ch * (kBlockRows * 128) + k * 32),
+                                         umma_smem_desc(xb + ch * (n * 128) + k * 32), idesc, (uint32_t)((st | ch | k) != 0));
+                    }
+                    umma_commit(c.empty_bar(slot));    // both stages are free once these MMAs have read them
+                    umma_commit(c.xempty_bar(xslot));
+                    if (st == spb - 1) umma_commit(c.acc_full_bar(buf));
                 }
-                umma_commit(c.empty_bar(slot));    // both stages are free once these MMAs have read them
-                umma_commit(c.xempty_bar(xslot));
                 if (++slot == kNumStages) { slot = 0; phase ^= 1u; }
                 ++xstage;
             }
-            umma_commit(c.acc_full_bar(buf));
             ++acc;
         }
-        rec(c, MKB_T_ATTN_STAGES_DONE);  // (GEMM instructions: every MMA of the instruction is issued)
+        if (chosen) rec(c, MKB_T_ATTN_STAGES_DONE);  // (GEMM instructions: every MMA of the instruction is issued)
     } else if (warp >= 4) {
         // Twelve epilogue warps: warp w reads the lane quarter w % 4 of tensor memory (its rows), and
         // the three groups of four warps share the sequences (accumulator columns) of every block.
