@@ -56,7 +56,8 @@ class LatencyScheduleOptions:
     coalesce_o_proj: bool = False
     # with more than one attention partition: no AttentionReduction instructions; the partial of a
     # KV head that arrives last merges the partial rows itself and signals the o-proj (one barrier
-    # hop and one instruction less on the critical path of a layer)
+    # hop and one instruction less on the critical path of a layer).  Batched: attention in equal shares of all
+    # sequences' cached positions, whatever the number of partitions
     merge_in_last_partial: bool = False
     # > 1: batched decode, that many independent sequences per launch (at most 64; more than 8
     # switches the schedule to 128-row blocks for the tcgen05 build of the kernel); the model's
