@@ -316,7 +316,9 @@ __device__ __forceinline__ AttnRange attn_range(const KParams& p, int pos, int n
 // these heads, so that a copy reads whole runs of a position's row.  A unit is as long as its stages
 // and kUnitCost more, for what it costs besides them.  Shares are cut anywhere in the line-up
 // (sequence, heads, stage); what is cut has partial rows, which the last of its parts to arrive merges.
-constexpr int kUnitCost = 3;
+// (7 and 64 sequences, us: 3: 1154, 1720; 6: 1139, 1695; 10: 1128, 1678; 16: 1128, 1677; 40: 1137, 1752.  Besides a unit's own cost it is
+// what a cut nearby costs: those move to the unit's edge.)
+constexpr int kUnitCost = 12;
 struct AttnPiece {
     int seq, kvh0;   // first key/value head
     int lo, hi, n;   // stages of this piece, stages of the unit
