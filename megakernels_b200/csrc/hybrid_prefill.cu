@@ -819,7 +819,10 @@ __device__ __forceinline__ void operand_run(const OperandArgs& a, int t0, int t1
         for (int j = 0; j < J; ++j) {
             const int i = 2 * (lane + 32 * j);
             const float x = v[j].x * inv * norm[j].x, y = v[j].y * inv * norm[j].y;
-            if (i < end) *reinterpret_cast<typename Pair<T>::type*>(o + i) = Pair<T>::make(x * r[j].x - y * r[j].y, y * r[j].x + x * r[j].y);
+            // (which of a sum's products is rounded is written out, so that a result's last bit does not depend on how the copies of
+            // this function are merged: values of up to 64 entries differ from keys)
+            const float odd = J == 1 && w == nullptr ? fmaf(x, r[j].y, __fmul_rn(y, r[j].x)) : fmaf(y, r[j].x, __fmul_rn(x, r[j].y));
+            if (i < end) *reinterpret_cast<typename Pair<T>::type*>(o + i) = Pair<T>::make(fmaf(x, r[j].x, -__fmul_rn(y, r[j].y)), odd);
         }
         for (int i = 64 * J + 2 * lane; i < end; i += 64) *reinterpret_cast<typename Pair<T>::type*>(o + i) = Pair<T>::make(0.f, 0.f);
     }

@@ -9,6 +9,7 @@ from pathlib import Path
 import pytest
 import torch
 
+from megakernels_b200.hybrid import RopeSpec
 from tests.dumalix_utils import (
     BF16_TOL, EVEN, F32_TOL, GROUPS, MODELS, ODD, WIDE, changed, chunked, latent, load, make_weights, model_config, oracle_logits, rel,
     run_cut, tokens_for, write_checkpoint,
@@ -415,3 +416,22 @@ def test_trace_run(bench, tmp_path, dtype, tol):
     assert rel(read(2), want[[41, 43]]) < tol and rel(read(4), want[[45, 99]]) < tol
     for k in range(5):
         assert rel(read(5 + k), want[9 + k : 10 + k]) < tol
+
+
+@pytest.mark.parametrize("conv", [0, 1])
+@pytest.mark.parametrize("vdim", [10, 48, 64, 96, 128])
+def test_rotated_values_round_one_product(tmp_path, vdim, conv):
+    """One token over and over: the first position's values are not turned, the others' are these, turned.  Even entries are
+    fma(x, cos, -(y sin)); odd ones fma(x, sin, y cos) up to 64 entries, fma(y, cos, x sin) above, one rounding of a product and one of the
+    sum (64-bit sums of a 48-bit product and a float round to the same float)."""
+    raw = model_config([chunked(2, 1, 16, vdim, size=1000, base=10000.0, conv=conv)], width=64, taps=1)
+    gen = start(write_checkpoint(tmp_path / "m", raw, make_weights(raw)), torch.float32)
+    gen.feed([7] * 200, 0, [199])
+    gen.check()
+    held = gen.model.state.values[0][0, 0, :200].cpu()
+    table = gen.model.rope_table(RopeSpec(vdim, 10000.0)).cpu().view(-1, vdim // 2, 2)[:200]
+    x, y = held[0, 0::2], held[0, 1::2]
+    c, s = table[..., 0], table[..., 1]
+    fma = lambda a, b, z: (a.double() * b.double() + z.double()).float()  # noqa: E731
+    assert torch.equal(held[:, 0::2], fma(x, c, -(y * s)))
+    assert torch.equal(held[:, 1::2], fma(x, s, y * c) if vdim <= 64 else fma(y, c, x * s))
