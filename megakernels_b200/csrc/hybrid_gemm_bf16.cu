@@ -49,9 +49,19 @@ constexpr Group group_of(Result r) {
 }
 __device__ __forceinline__ long long fixed_of(float x) { return __float2ll_rn(x * mkb::kResidualScale); }
 
-// columns n (even) and n + 1 of token t, where a thread has just these
+// Columns n (even) and n + 1 of token t, where a thread has just these.  kAdd: `before` is what they are added to, fetched while the
+// sums are still on their way (as additions in L2, which nobody waits for, the scaled sum would be rounded first).
 template <Group kGroup>
-__device__ __forceinline__ void put(const GemmEpilogue& e, int N, int t, int n, float x, float y) {
+__device__ __forceinline__ float2 put_on(const GemmEpilogue& e, int N, int t, int n) {
+    float2 v = make_float2(0.f, 0.f);
+    if (kGroup != Group::kPlain || e.what != Result::kAdd || n >= N) return v;
+    const float* o = e.out + (size_t)t * e.ld + n;
+    v.x = __ldcg(o);
+    if (n + 1 < N) v.y = __ldcg(o + 1);
+    return v;
+}
+template <Group kGroup>
+__device__ __forceinline__ void put(const GemmEpilogue& e, int N, int t, int n, float x, float y, float2 before) {
     if (n >= N) return;
     if constexpr (kGroup == Group::kRope) {
         const RopeTarget& p = e.rope;
@@ -78,9 +88,9 @@ __device__ __forceinline__ void put(const GemmEpilogue& e, int N, int t, int n, 
     } else {
         float* o = e.out + (size_t)t * e.ld + n;
         const bool two = n + 1 < N;
-        if (e.what == Result::kAdd) {  // (no other thread writes these: one addition each, in L2)
-            asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o), "f"((e.scale ? __ldg(e.scale + n) : 1.f) * x) : "memory");
-            if (two) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o + 1), "f"((e.scale ? __ldg(e.scale + n + 1) : 1.f) * y) : "memory");
+        if (e.what == Result::kAdd) {  // (no other thread writes these)
+            o[0] = fmaf(e.scale ? __ldg(e.scale + n) : 1.f, x, before.x);
+            if (two) o[1] = fmaf(e.scale ? __ldg(e.scale + n + 1) : 1.f, y, before.y);
         } else {
             o[0] = x + (e.bias ? __ldg(e.bias + n) : 0.f);
             if (two) o[1] = y + (e.bias ? __ldg(e.bias + n + 1) : 0.f);
@@ -345,9 +355,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
         for (int i0 = (int)me + (int)parts * warp; i0 < rows; i0 += kRowsAtOnce * next)
 #pragma unroll 1
             for (int c = 2 * lane; c < wide; c += 64) {
-                float2 sum[kRowsAtOnce], up[kRowsAtOnce];
+                float2 sum[kRowsAtOnce], up[kRowsAtOnce], before[kRowsAtOnce];
 #pragma unroll
-                for (int r = 0; r < kRowsAtOnce; ++r) sum[r] = up[r] = make_float2(0.f, 0.f);
+                for (int r = 0; r < kRowsAtOnce; ++r) {
+                    sum[r] = up[r] = make_float2(0.f, 0.f);
+                    before[r] = put_on<kGroup>(e, s.N, m0 + min(i0 + r * next, rows - 1), n0 + c);
+                }
                 for (uint32_t z = 0; z < parts; z += 2) {  // (two or four parts)
                     float2 v[2][kRowsAtOnce], u[2][kRowsAtOnce];
 #pragma unroll
@@ -375,7 +388,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant
                     if (i0 + r * next >= rows) break;
                     float x = sum[r].x, y = sum[r].y;
                     if constexpr (kDual) x *= sigmoid_f(x) * up[r].x, y *= sigmoid_f(y) * up[r].y;
-                    put<kGroup>(e, s.N, m0 + i0 + r * next, n0 + c, x, y);
+                    put<kGroup>(e, s.N, m0 + i0 + r * next, n0 + c, x, y, before[r]);
                 }
             }
         tc_cluster_sync();

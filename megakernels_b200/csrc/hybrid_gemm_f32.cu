@@ -105,9 +105,6 @@ __device__ __forceinline__ void split4(float4& x, float4& r, float& odd) {
 __device__ __forceinline__ bool infinite(float h) { return (__float_as_uint(h) & 0x7fffffffu) == 0x7f800000u; }
 __device__ __forceinline__ bool infinite4(const float4& h) { return infinite(h.x) | infinite(h.y) | infinite(h.z) | infinite(h.w); }
 
-// (no other thread writes these: one addition each, in L2, and nobody waits for it)
-__device__ __forceinline__ void add_once(float* o, float x) { asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o), "f"(x) : "memory"); }
-
 // columns n (even) and n + 1 of token t
 __device__ __forceinline__ void put(const GemmEpilogue& e, int t, int n, int N, float x, float y) {
     if (n >= N) return;
@@ -117,8 +114,8 @@ __device__ __forceinline__ void put(const GemmEpilogue& e, int t, int n, int N, 
     }
     float* o = (e.what == Result::kCast ? static_cast<float*>(e.cast) : e.out) + (size_t)t * e.ld + n;
     if (e.what == Result::kAdd) {
-        add_once(o, (e.scale ? e.scale[n] : 1.f) * x);
-        if (n + 1 < N) add_once(o + 1, (e.scale ? e.scale[n + 1] : 1.f) * y);
+        o[0] = fmaf(e.scale ? e.scale[n] : 1.f, x, o[0]);
+        if (n + 1 < N) o[1] = fmaf(e.scale ? e.scale[n + 1] : 1.f, y, o[1]);
     } else {
         o[0] = x + (e.bias ? e.bias[n] : 0.f);
         if (n + 1 < N) o[1] = y + (e.bias ? e.bias[n + 1] : 0.f);

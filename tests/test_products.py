@@ -112,3 +112,21 @@ def test_float32_products_of_odd_operands(T, N, K):
     finite = out.isfinite()
     size = a.abs().double().nan_to_num(0, 0) @ w.abs().double().nan_to_num(0, 0).T
     assert ((out.double() - want).abs() <= (K + 1) * 2.0**-24 * size)[finite].all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,T,N,K", [(torch.bfloat16, 61, 2048, 8192), (torch.bfloat16, 20, 2045, 4096), (torch.float32, 1, 300, 64),
+                                         (torch.float32, 3, 260, 40), (torch.float32, 61, 2047, 1024), (torch.float32, 300, 512, 256)])
+def test_scaled_sums_are_added_with_one_rounding(dtype, T, N, K):
+    """Sums of products of -1, 0 and 1 are exact: what is left is the rounding of out + scale * sum (64 bits hold it but for about 2^-29 of
+    the elements), one and not two.  In bf16 where CTAs share a tile's inner dimension."""
+    mk = get_mk_module(name="mk_hybrid")
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    pad = (K + 7) // 8 * 8
+    a, w = (torch.randint(-1, 2, (rows, pad), generator=gen, device="cuda").to(dtype) for rows in (T, N))
+    scale, out = torch.randn(N, generator=gen, device="cuda"), torch.randn(T, N, generator=gen, device="cuda")
+    want = (out.double() + (a[:, :K].double() @ w[:, :K].double().T) * scale.double()).float()
+    status = torch.zeros(16, dtype=torch.int32, device="cuda")
+    mk.product("add", a, w, out, status, K, scale=scale)
+    assert int(status[0]) == 0
+    assert int((out != want).sum()) <= out.numel() * 1e-6
