@@ -366,7 +366,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_kernel(const __grid_cons
     } else {
         const int q = warp & 3, half = (warp - 2 - kSplitWarps) >> 2;  // the quarter of tensor memory's lanes this warp may read
         const uint32_t at = tmem + ((uint32_t)(q * 32) << 16) + half * C;
-        const int n = n0 + q * 32 + lane, tt = t0 + half * C, end = min(s.T, t0 + s.tokens);
         float sum[C] = {};
         bool ok = true;
         for (int chunk = 0; chunk < chunks; ++chunk) {
@@ -386,22 +385,30 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f32_kernel(const __grid_cons
             float* o = reinterpret_cast<float*>(gbase) + half * C * kFeatures + q * 32 + lane;
 #pragma unroll
             for (int j = 0; j < C; ++j) o[j * kFeatures] = sum[j];
-            if (ctl[2]) {  // with FMA
-                for (int j = 0; j < C && tt + j < end; ++j) {
-                    float x = 0.f;
-                    const float *w = W + (size_t)n * ldw, *v = A + (size_t)(tt + j) * lda;
-                    const int last = min(s.K, (first + steps) * kStep);
-                    for (int k = first * kStep; n < s.N && k < last; ++k) x = fmaf(w[k], v[k], x);
-                    o[j * kFeatures] = x;
-                }
-            }
         }
     }
     tc_before_sync();
     __syncthreads();
     if (*ctl) tc_settle();
-    if (s.parts > 1) tc_cluster_sync();
     const int tokens = min(s.tokens, s.T - t0), c = 4 * lane;
+    if (ctl[2]) {  // (behind the block's barrier: whichever warp found the operand)
+        const int last = min(s.K, (first + steps) * kStep);
+        for (int i = warp; i < tokens * kFeatures; i += kThreads / 32) {  // an element per warp, with FMA
+            const int t = i / kFeatures, n = i % kFeatures;
+            if (n0 + n >= s.N) continue;
+            const float *w = W + (size_t)(n0 + n) * ldw, *v = A + (size_t)(t0 + t) * lda;
+            float x = 0.f;
+#pragma unroll 4
+            for (int k = first * kStep + 4 * lane; k < last; k += 128) {
+                const float4 a = slice(w, true, k, last), b = slice(v, true, k, last);
+                x = fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, x))));
+            }
+            x = warp_sum(x);
+            if (lane == 0) reinterpret_cast<float*>(gbase)[t * kFeatures + n] = x;
+        }
+        __syncthreads();
+    }
+    if (s.parts > 1) tc_cluster_sync();
 #pragma unroll 2
     for (int t = part + s.parts * warp; t < tokens; t += s.parts * (kThreads / 32)) {
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -115,6 +115,29 @@ def test_float32_products_of_odd_operands(T, N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,N,K", [(61, 300, 1000), (161, 2048, 8192), (300, 260, 2048)])
+def test_infinite_operands_at_the_edges(T, N, K):
+    """One infinite operand in the last token and one in the last feature, at either end of the inner dimension (another CTA's part
+    of it): their sums are infinite, all others as before; in a bounded time (a tile is done over by all of its warps)."""
+    mk = get_mk_module(name="mk_hybrid")
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    a, w = torch.randn(T, K, generator=gen, device="cuda"), torch.randn(N, K, generator=gen, device="cuda") / K**0.5
+    a[T - 1, K - 1], w[N - 1, 0] = float("inf"), float("-inf")
+    out, status = torch.full((T, N), 7.0, device="cuda"), torch.zeros(16, dtype=torch.int32, device="cuda")
+    mk.product("store", a, w, out, status, K)  # (the first launch loads the kernel)
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    begin.record()
+    mk.product("store", a, w, out, status, K)
+    end.record()
+    torch.cuda.synchronize()
+    want = a.double() @ w.double().T
+    assert int(status[0]) == 0 and begin.elapsed_time(end) < 10
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out.isinf(), want.isinf())
+    size = a.abs().double().nan_to_num(0, 0, 0) @ w.abs().double().nan_to_num(0, 0, 0).T
+    assert ((out.double() - want).abs() <= (K + 1) * 2.0**-24 * size)[out.isfinite()].all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype,T,N,K", [(torch.bfloat16, 61, 2048, 8192), (torch.bfloat16, 20, 2045, 4096), (torch.float32, 1, 300, 64),
                                          (torch.float32, 3, 260, 40), (torch.float32, 61, 2047, 1024), (torch.float32, 300, 512, 256)])
 def test_scaled_sums_are_added_with_one_rounding(dtype, T, N, K):
