@@ -84,13 +84,57 @@ def test_bf16_products(result, T, N, K):
 @pytest.mark.parametrize("T,N,K", SHAPES)
 @pytest.mark.parametrize("result", ["store", "add", "cast", "glu"])
 def test_float32_products(result, T, N, K):
-    """fp32 FMA throughout, an error of 2^-24 of the sum so far per step: far below what bf16 or tf32 operands would give
-    (2^-9, 2^-11)."""
+    """Products are exact but for 2^-24 of them, a step of 32 of the inner dimension is cut by at most 2^-23 of its sum and added up with an error of
+    2^-24 of the sum so far; one or two tokens and an inner dimension below 16 are FMA.  Far below what bf16 or tf32 operands would give
+    (2^-9, 2^-11), and in the mean square below what two tf32 parts give (2e-7 at any length; units and their exponentials aside)."""
     if result == "glu" and N % 2:
         N += 1
     out, want, wrong = product(result, torch.float32, T, N, K)
     assert ((out - want).abs() <= wrong + 2.0**-24 * want.abs()).all()
-    assert float((out - want).norm() / want.norm()) < 2e-6
+    assert float((out - want).norm() / want.norm()) < (2e-6 if result == "glu" else most_wrong(K))
+
+
+def most_wrong(K):
+    """Largest 2-norm of the relative error of sums that stay within the size of the result: steps of 32 cut by 0 .. 2^-23 (mean square 2^-23 /
+    sqrt 3) and as many roundings of 2^-24 / sqrt 3 to sums that grow to it.  Below 16, the roundings of FMA."""
+    adds = K if K < 16 else (K + 31) // 32
+    return 2.0**-23 * (3**-0.5 + 0.29 * (adds / 2) ** 0.5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [1, 2, 5, 8, 15, 16, 17, 31, 33, 64, 200, 1024])
+@pytest.mark.parametrize("kind", ["normal", "one sign", "remainders", "dominated"])
+def test_float32_products_keep_all_bits_of_their_operands(kind, K):
+    """Short and long inner dimensions, where an operand's last bits show: sums of one sign, operands whose remainders are as large as they
+    get at 11 and at 8 bits (their products' exact sums), one column a thousand times the others (not further off than FMA in order,
+    which rounds every later sum)."""
+    mk = get_mk_module(name="mk_hybrid")
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    T, N, pad = 48, 512, (K + 7) // 8 * 8
+    a, w = torch.zeros(T, pad, device="cuda"), torch.zeros(N, pad, device="cuda")
+    for m in (a, w):
+        if kind == "one sign":
+            m[:, :K] = 1 + torch.rand(len(m), K, generator=gen, device="cuda")
+        elif kind == "remainders":
+            m[:, :K] = 1 + 2.0**-11 - 2.0**-23
+        else:
+            m[:, :K] = torch.randn(len(m), K, generator=gen, device="cuda")
+    if kind == "dominated":
+        a[:, K // 2] *= 1000
+    out, status = torch.zeros(T, N, device="cuda"), torch.zeros(16, dtype=torch.int32, device="cuda")
+    mk.product("store", a, w, out, status, K)
+    want = a.double() @ w.double().T
+    error = out.double() - want
+    assert int(status[0]) == 0
+    if kind == "remainders":
+        assert (error.abs() <= 2.0**-23 * want).all()
+    elif kind == "dominated":
+        fma = torch.zeros(T, N, device="cuda")  # (64-bit sums of a 48-bit product and a float, rounded once)
+        for k in range(K):
+            fma = (fma.double() + a[:, k, None].double() * w[None, :, k].double()).float()
+        assert float(error.norm()) <= 1.02 * float((fma.double() - want).norm())
+    else:
+        assert float(error.norm() / want.norm()) < most_wrong(K)
 
 
 @pytest.mark.gpu
