@@ -55,7 +55,9 @@ enum {
     MKB_OP_RMS_NORM = 9,
     /* Batched launches only: one of `ranks` equal shares of a layer's attention over all sequences, cut
      * by the cached positions of this launch; in place of every MKB_OP_PARTIAL_ATTENTION and
-     * MKB_OP_ATTENTION_REDUCTION of the layer.  All shares of a layer must be there.
+     * MKB_OP_ATTENTION_REDUCTION of the layer.  All shares of a layer must be there.  One to four
+     * key/value heads of a sequence fall into at most min(max_partials, 24) shares: with few long sequences
+     * fewer than 24 keep SMs idle, and max_partials = 1 leaves the layer to one SM.
      * words: [10, layer, rank, ranks] */
     MKB_OP_BATCH_ATTENTION = 10,
 };

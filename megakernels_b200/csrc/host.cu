@@ -456,11 +456,11 @@ int prepare_launch(const MkbGlobals* g, DeviceState* ds, int* status, int sm_cou
     if (rc) return rc;
     rc = kv_tensor_map(ds, g->v_cache, p.D, p.Hkv, p.T, p.L * p.B, &p.v_map);
     if (rc) return rc;
-    if (p.batch > 1) {
-        p.share_heads = p.Hkv % 4 == 0 ? 4 : p.Hkv % 2 == 0 ? 2 : 1;
-        rc = kv_tensor_map(ds, g->k_cache, p.D, p.Hkv, p.T, p.L * p.B, &p.k_share_map, p.share_heads);
+    for (int heads : {4, 2}) {
+        if (p.batch == 1 || p.Hkv % heads != 0) continue;
+        rc = kv_tensor_map(ds, g->k_cache, p.D, p.Hkv, p.T, p.L * p.B, heads == 4 ? &p.k_map4 : &p.k_map2, heads);
         if (rc) return rc;
-        rc = kv_tensor_map(ds, g->v_cache, p.D, p.Hkv, p.T, p.L * p.B, &p.v_share_map, p.share_heads);
+        rc = kv_tensor_map(ds, g->v_cache, p.D, p.Hkv, p.T, p.L * p.B, heads == 4 ? &p.v_map4 : &p.v_map2, heads);
         if (rc) return rc;
     }
 

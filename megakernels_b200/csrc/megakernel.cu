@@ -312,12 +312,12 @@ __device__ __forceinline__ AttnRange attn_range(const KParams& p, int pos, int n
 // MKB_OP_BATCH_ATTENTION: a layer's attention over all sequences, cut into `ranks` equal shares of cached
 // positions, whatever the sequences' lengths are in this launch.  (One instruction per sequence and head, dealt
 // to the SMs in turn: 64 sequences of 256..4096 positions took 290 us a layer, in which the SMs were busy for 149 on average.)
-// A unit is `share_heads` neighbouring key/value heads of a sequence; a ring stage is a run of `stage_pos` positions of
+// A unit is four, two or one neighbouring key/value heads of a sequence (`heads`); a ring stage is a run of `stage_pos` positions of
 // these heads, so that a copy reads whole runs of a position's row.  A unit is as long as its stages
 // and kUnitCost more, for what it costs besides them.  Shares are cut anywhere in the line-up
 // (sequence, heads, stage); what is cut has partial rows, which the last of its parts to arrive merges.
-// (7 and 64 sequences, us: 3: 1154, 1720; 6: 1139, 1695; 10: 1128, 1678; 16: 1128, 1677; 40: 1137, 1752.  Besides a unit's own cost it is
-// what a cut nearby costs: those move to the unit's edge.)
+// (7 and 64 sequences, us: 3: 1154, 1720; 6: 1139, 1695; 10: 1128, 1678; 16: 1128, 1677; 40: 1137, 1752; 12 was taken.  Besides a unit's own
+// cost it is what a cut nearby costs: those move to the unit's edge.)
 constexpr int kUnitCost = 12;
 struct AttnPiece {
     int seq, kvh0;   // first key/value head
@@ -329,11 +329,13 @@ struct AttnShares {
     uint32_t u0;                  // start of the next unit
     int seq, sub;                 // the next unit
 
-    // control words: starts of the sequences, the length of the line-up behind them, and the largest number of shares
+    // control words: starts of the sequences, the length of the line-up behind them, the largest number of shares; then (two
+    // verdicts of a share's merges and) a unit's heads
     static __device__ __forceinline__ const volatile int* table(const Ctx& c) { return c.cta_abort + kCtlShares; }
-    static __device__ __forceinline__ int stage_pos(const KParams& p) { return (kStageBytes / 4) / p.D / p.share_heads; }
-    static __device__ __forceinline__ int stages(const Ctx& c, const KParams& p, int seq) {
-        const int sp = stage_pos(p);
+    static __device__ __forceinline__ int heads(const Ctx& c) { return table(c)[kBatch + 4]; }
+    static __device__ __forceinline__ int stage_pos(const KParams& p, int heads) { return (kStageBytes / 4) / p.D / heads; }
+    static __device__ __forceinline__ int stages(const Ctx& c, const KParams& p, int seq, int heads) {
+        const int sp = stage_pos(p, heads);
         return (c.pos_of(seq) + sp - 1) / sp;
     }
     // false: nothing for this rank
@@ -355,20 +357,21 @@ struct AttnShares {
             else hi = mid;
         }
         seq = lo;
-        const uint32_t len = (uint32_t)(stages(c, p, seq) + kUnitCost);
+        const uint32_t len = (uint32_t)(stages(c, p, seq, heads(c)) + kUnitCost);
         sub = (int)((b0 - (uint32_t)tab[lo]) / len);
         u0 = (uint32_t)tab[lo] + sub * len;
         return true;
     }
     __device__ __forceinline__ bool next(const Ctx& c, const KParams& p, AttnPiece& a) {
         if (seq >= p.batch || u0 >= b1) return false;
-        a.n = stages(c, p, seq);
+        const int heads = this->heads(c);
+        a.n = stages(c, p, seq, heads);
         const uint32_t len = (uint32_t)(a.n + kUnitCost);
         // cuts at or before x0 leave the unit whole behind them: it belongs to the last share that starts there
         const uint32_t x0 = u0 + min((uint32_t)kUnitCost, len - 1), base = u0 + kUnitCost;
         if (b1 <= x0) return false;
         a.seq = seq;
-        a.kvh0 = sub * p.share_heads;
+        a.kvh0 = sub * heads;
         a.lo = b0 <= x0 ? 0 : (int)(b0 - base);
         a.hi = min(a.n, (int)(b1 - base));
         const uint32_t first = (uint32_t)(((unsigned long long)(x0 + 1) * R - 1) / S);
@@ -376,7 +379,7 @@ struct AttnShares {
         a.np = (int)(last - first) + 1;
         a.pi = (int)(rank - first);
         u0 += len;
-        if (++sub == p.Hkv / p.share_heads) {
+        if (++sub == p.Hkv / heads) {
             sub = 0;
             ++seq;
         }
@@ -384,29 +387,52 @@ struct AttnShares {
     }
 };
 // By one warp, before the roles start: the line-up of this launch's positions.
+// Units of four heads read the longest runs, but no unit falls into more parts than there are rows for, and two sequences of 8 such heads
+// would keep 92 of 148 SMs busy, a long one beside short ones 46: then units are of fewer heads.  A stage of them costs 1 and 5 % more (8 and 64
+// sequences).  8B widths, 4 layers, us, units of 4, 2, 1 heads: two sequences of 4096 486, 476, 478, of 16384 564, 538, 540, 16384 and 40
+// positions 568, 514, 501 (558 by an instruction per sequence and head); eight of 4096 547, 545, 551.  Instructions remain ahead where few
+// sequences are equally long and short (two of 1000: 448, shares 461) and by 3 - 7 % with equally long ones of 64 dimensions.
 __device__ __forceinline__ void attn_shares_table(const Ctx& c, const KParams& p, int lane) {
-    const uint32_t units = (uint32_t)(p.Hkv / p.share_heads);
-    uint32_t start = 0, longest = 1;
     volatile int* tab = c.cta_abort + kCtlShares;
+    const uint32_t rows = (uint32_t)min(23, p.max_partials - 1);
+    float best = 0.f;
+    uint32_t heads = 0, shares = 1;
+    for (int h = 4; h >= 1; h >>= 1) {
+        if (p.Hkv % h != 0) continue;
+        const uint32_t units = (uint32_t)(p.Hkv / h);
+        uint32_t line = 0, longest = 0;
+        for (int s = lane; s < p.batch; s += 32) {
+            const uint32_t len = (uint32_t)(AttnShares::stages(c, p, s, h) + kUnitCost);
+            line += len * units;
+            longest = max(longest, len);
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) {
+            line += __shfl_xor_sync(0xffffffffu, line, o);
+            longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+        }
+        // (every share holds something)
+        const uint32_t most = (uint32_t)max(1ull, min((unsigned long long)line, (unsigned long long)rows * line / longest));
+        const float time = (float)line * (h == 4 ? 1.f : h == 2 ? 1.01f : 1.05f) / (float)min(most, gridDim.x);
+        if (heads == 0 || time < best) best = time, heads = (uint32_t)h, shares = most;
+    }
+    uint32_t start = 0;
     for (int s0 = 0; s0 < p.batch; s0 += 32) {
         const int s = s0 + lane;
-        const uint32_t len = s < p.batch ? (uint32_t)(AttnShares::stages(c, p, s) + kUnitCost) : 0u;
-        uint32_t sum = units * len, most = len;
+        const uint32_t len = s < p.batch ? (uint32_t)p.Hkv / heads * (uint32_t)(AttnShares::stages(c, p, s, (int)heads) + kUnitCost) : 0u;
+        uint32_t sum = len;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
             if (lane >= o) sum += v;
-            most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
         }
-        if (s < p.batch) tab[s] = (int)(start + sum - units * len);
+        if (s < p.batch) tab[s] = (int)(start + sum - len);
         start += __shfl_sync(0xffffffffu, sum, 31);
-        longest = max(longest, most);
     }
     if (lane == 0) {
         tab[p.batch] = (int)start;
-        // every share holds something, and no unit falls into more parts than there are rows for
-        const unsigned long long rows = (unsigned long long)(p.max_partials - 1 < 23 ? p.max_partials - 1 : 23) * start / longest;
-        tab[kBatch + 1] = (int)max(1ull, min((unsigned long long)start, rows));
+        tab[kBatch + 1] = (int)shares;
+        tab[kBatch + 4] = (int)heads;
     }
 }
 #endif  // MKB_BATCH > 1
@@ -421,7 +447,7 @@ struct StageDesc {
     int c1, c2, c3;          // weights: row, 64-column chunk, layer
     uint32_t bytes;
     int kvh, t, lb;          // K/V tile coordinates
-    bool share;              // K/V tile of an attention share
+    int share;               // K/V tile of an attention share: heads of its unit, else 0
 };
 
 // Walks the instruction queue and yields its ring stages in consumption order.
@@ -512,7 +538,7 @@ struct StreamCursor {
 #if MKB_BATCH > 1
             case MKB_OP_BATCH_ATTENTION:
                 layer = __ldg(w + 1);
-                ts = AttnShares::stage_pos(p);
+                ts = AttnShares::stage_pos(p, AttnShares::heads(*ctx));
                 if (shares.begin(*ctx, p, __ldg(w + 2), __ldg(w + 3))) next_piece(p);
                 break;
 #endif
@@ -528,7 +554,7 @@ struct StreamCursor {
             decode(p, queue);
         }
 #if MKB_BATCH > 1
-        d.share = op == MKB_OP_BATCH_ATTENTION;
+        d.share = op == MKB_OP_BATCH_ATTENTION ? AttnShares::heads(*ctx) : 0;
         if (d.share) {
             d.map = nullptr;
             d.kvh = kvh;
@@ -607,7 +633,7 @@ __device__ void loader_main(Ctx c, const int which) {
     StreamCursor issue, ahead;  // `ahead` is never behind `issue`
     issue.ctx = ahead.ctx = &c;
     StageDesc d, da;
-    d.share = da.share = false;
+    d.share = da.share = 0;
     uint32_t stage = 0;       // stages of the sequence walked so far (all loaders' stages)
     uint32_t ahead_stage = 0; // stages the look-ahead cursor has passed
     uint32_t own_issued = 0;  // one past the last stage this loader copied into the ring
@@ -658,9 +684,9 @@ __device__ void loader_main(Ctx c, const int which) {
             const uint32_t dst = c.stage_addr(slot);
             mbar_expect_tx(bar, d.bytes);
             if (d.map == nullptr) {
-                const bool share = kBatch > 1 && d.share;
-                tma_tile5_g2s(dst, share ? &p.k_share_map : &p.k_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
-                tma_tile5_g2s(dst + kStageBytes / 2, share ? &p.v_share_map : &p.v_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
+                const int wide = kBatch > 1 ? d.share : 0;  // (a unit of one head: the tile of an instruction per head)
+                tma_tile5_g2s(dst, wide == 4 ? &p.k_map4 : wide == 2 ? &p.k_map2 : &p.k_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
+                tma_tile5_g2s(dst + kStageBytes / 2, wide == 4 ? &p.v_map4 : wide == 2 ? &p.v_map2 : &p.v_map, 0, d.t, 0, d.kvh, d.lb, bar, policy);
             } else {
                 tma_tile4_g2s(dst, d.map, 0, d.c1, d.c2, d.c3, bar, policy);
             }
@@ -1637,26 +1663,26 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
     AttnShares shares;
     if (!shares.begin(c, p, __ldg(w + 2), __ldg(w + 3))) return true;
 
-    {  // the layer's queries, keys and values of all heads are there
-        volatile int* verdict = verdict_word(c, cs);
-        if (warp == 0) {
+    {  // the layer's queries, keys and values of all heads are there (two warps: 64 counters in one round trip)
+        volatile int *first = verdict_word(c, cs), *second = c.cta_abort + kCtlShares + kBatch + 3;
+        if (warp < 2) {
             const int row = MKB_OP_RMS_QKV_ROPE_APPEND - 1, slots = p.Hq + 2 * p.Hkv;
             bool ok = __shfl_sync(0xffffffffu, *c.cta_abort, 0) == 0;  // uniform over the warp
-            for (int s0 = 0; ok && s0 < slots; s0 += 32) {
+            for (int s0 = 32 * warp; ok && s0 < slots; s0 += 64) {
                 const int slot = s0 + lane;
                 ok = warp_wait_counters(c, slot < slots ? bar_addr(p, layer, row, slot) : nullptr, p.thr_attn_waits_qkv, layer, row, slot,
                                         (unsigned)p.poll_sleep_ns);
             }
             if (lane == 0) {
-                rec(c, MKB_T_CONSUMER_WAIT_DONE);
-                *verdict = ok ? 1 : 0;
+                if (warp == 0) rec(c, MKB_T_CONSUMER_WAIT_DONE);
+                *(warp == 0 ? first : second) = ok ? 1 : 0;
             }
         }
         consumer_sync();
-        if (*verdict == 0) return false;
+        if (*first == 0 || *second == 0) return false;
     }
 
-    const int HP = p.share_heads, PS = TS / HP;
+    const int HP = AttnShares::heads(c), PS = TS / HP;
     const int hd = (warp & 3) % HP, un = (warp & 3) / HP, grp = warp >> 2;
     float* sml = reinterpret_cast<float*>(__cvta_shared_to_generic(c.base + kSmemAttn));  // (m, l) of [warp][query head]
     volatile int* merged = c.cta_abort + kCtlShares + kBatch + 2;                          // verdicts of the two cut units
@@ -1692,6 +1718,9 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
         for (int i = 0; i < DT; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
         if (a.hi == a.n && grp == 0 && un == 0) {  // the token's own key and value come first (written by another SM in this launch)
             const __nv_bfloat16 *kc = p.k_cache + tok + (size_t)(a.kvh0 + hd) * D, *vc = p.v_cache + tok + (size_t)(a.kvh0 + hd) * D;
+            uint32_t own[DT][2];  // (on its way together with the key and the queries)
+#pragma unroll
+            for (int i = 0; i < DT; ++i) own[i][0] = ld_cg_u32(vc + 16 * i + (g & 6)), own[i][1] = ld_cg_u32(vc + 16 * i + 8 + (g & 6));
             float s = 0.f;
 #pragma unroll
             for (int j = 0; j < KP; ++j) {
@@ -1709,9 +1738,8 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
             l[0] = l[1] = g == 0 ? 1.f : 0.f;
 #pragma unroll
             for (int i = 0; i < DT; ++i) {
-                const uint32_t v0 = ld_cg_u32(vc + 16 * i + (g & 6)), v1 = ld_cg_u32(vc + 16 * i + 8 + (g & 6));
-                o[i][0] = o[i][1] = (g & 1) ? bf16_hi(v0) : bf16_lo(v0);
-                o[i][2] = o[i][3] = (g & 1) ? bf16_hi(v1) : bf16_lo(v1);
+                o[i][0] = o[i][1] = (g & 1) ? bf16_hi(own[i][0]) : bf16_lo(own[i][0]);
+                o[i][2] = o[i][3] = (g & 1) ? bf16_hi(own[i][1]) : bf16_lo(own[i][1]);
             }
         }
         for (int s = a.lo; s < a.hi; ++s) {

@@ -94,7 +94,7 @@ constexpr int kNumMbars = 2 * kNumStages + 2 * kOutSlots + 2 * kXStages + (kGemm
 constexpr int kSmemCtl = kSmemBars + kNumMbars * 8;            // control words, then the positions
 // (batched builds: then where the sequences' cached positions begin in a layer's attention work, see AttnShares)
 constexpr int kCtlShares = 8 + (kBatch < 8 ? 8 : kBatch);
-constexpr int kCtlWords = kCtlShares + (kBatch == 1 ? 0 : kBatch + 4);
+constexpr int kCtlWords = kCtlShares + (kBatch == 1 ? 0 : kBatch + 5);
 // A few launch constants that out-of-line code on the critical path reads from shared memory
 // (HotConsts, 16-byte aligned) instead of chasing pointers through local and parameter memory.
 constexpr int kSmemHot = (kSmemCtl + kCtlWords * 4 + 15) & ~15;
@@ -169,9 +169,8 @@ struct KParams {
     int l2_stall_window_stages;  // the same while this SM's consumers wait on a barrier counter
     // TMA descriptors of the KV cache, 4-D [D, Hkv, T, L*B], box {D, 1, TS, 1}
     CUtensorMap k_map, v_map;
-    // batched builds, attention by shares: a box is `share_heads` key/value heads of a run of positions
-    CUtensorMap k_share_map, v_share_map;
-    int share_heads;
+    // batched builds, attention by shares: a box is four or two key/value heads of a run of positions
+    CUtensorMap k_map4, v_map4, k_map2, v_map2;
     // weight matrices as 4-D [64, rows, K/64, L] with the 128-byte swizzle; one box is a ring
     // stage: 16 rows x up to 1024 columns, stored [64-column chunk][row][128 B]
     CUtensorMap qkv_map, o_map, up_map, gate_map, down_map, lm_map;

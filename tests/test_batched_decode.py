@@ -146,7 +146,9 @@ def test_batched_decode_matches_independent_sequences(shape, batch, parts, merge
     # (its parts are as many as there are rows for); two heads and one per stage; both builds
     [(32, 8, 128, [0, 1, 2]), (32, 8, 128, [15, 16, 17, 63, 64, 65, 7]), (32, 8, 128, [3000, 0, 40]), (32, 8, 64, [31, 32, 33, 500, 0]),
      (32, 4, 128, [400, 129]), (16, 2, 128, [700, 33, 0]), (8, 1, 128, [1500, 100]), (32, 8, 128, [(37 * i * i) % 900 for i in range(9)]),
-     (32, 8, 128, [(131 * i) % 1100 for i in range(64)]), (16, 2, 128, [(53 * i) % 300 for i in range(12)])],
+     (32, 8, 128, [(131 * i) % 1100 for i in range(64)]), (16, 2, 128, [(53 * i) % 300 for i in range(12)]),
+     # units of two heads (two long sequences) and of one (a long one beside a short one), in runs and at their edges
+     (32, 8, 128, [2600, 2500]), (32, 8, 128, [3500, 20]), (32, 8, 64, [5003, 4000]), (32, 8, 64, [9001, 0]), (16, 2, 128, [4097, 64])],
 )
 def test_attention_by_shares_matches_attention_by_sequence(heads, kv_heads, head_dim, lens):
     """What a layer's attention leaves, by shares and by an instruction per sequence and head.  Softmax weights are
@@ -179,3 +181,62 @@ def test_attention_by_shares_matches_attention_by_sequence(heads, kv_heads, head
         outs.append(schedule.globs.attn_out.float().clone())
     for b in range(batch):
         assert float((outs[0][b] - outs[1][b]).norm() / outs[1][b].norm()) < 3 * 2.0**-9, f"sequence {b} of length {lens[b]}"
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_shares_cover_every_stage_once(seed):
+    """Whatever the positions, heads, rows of parts, SMs and shares: a unit's parts are its stages, numbered, no more than there are rows for; a
+    share cuts at most two units."""
+    import random
+
+    from oracle.attention_shares import LineUp
+
+    rng = random.Random(seed)
+    for _ in range(150):
+        batch, top = rng.choice([2, 2, 3, 5, 8, 9, 33, 64]), rng.choice([1, 40, 300, 4096, 20000, 131072])
+        positions = [rng.choice([0, top, rng.randint(0, top), 15, 16, 17]) for _ in range(batch)]
+        kv_heads, head_dim = rng.choice([1, 2, 4, 6, 8, 8, 12]), rng.choice([64, 128])
+        rows, sms = rng.choice([24, 24, 148, 1, 2, 10]), rng.choice([148, 148, 132, 8])
+        ranks = rng.choice([sms, sms, sms // 2, sms + 5, 1])
+        line, seen = LineUp.of(positions, kv_heads, head_dim, rows, sms), {}
+        for rank in range(ranks):
+            pieces = line.pieces(rank, ranks)
+            assert sum(p.parts > 1 for p in pieces) <= 2
+            for p in pieces:
+                assert p.parts <= max(1, min(24, rows)) and (p.last > p.first or p.stages == 0)
+                seen.setdefault((p.seq, p.head), []).append(p)
+        assert len(seen) == batch * kv_heads // line.heads
+        for parts in seen.values():
+            parts.sort(key=lambda p: p.part)
+            assert [p.part for p in parts] == list(range(len(parts))) and {p.parts for p in parts} == {len(parts)}
+            assert parts[0].first == 0 and parts[-1].last == parts[0].stages
+            assert all(a.last == b.first for a, b in zip(parts, parts[1:]))
+
+
+@pytest.mark.parametrize("positions", [[4096, 4096], [16384, 16384], [16384, 40], [16384, 40, 40], [4096] * 3, [9000, 300, 300, 300], [2000] * 8])
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_shares_of_few_sequences_reach_the_sms(positions, head_dim):
+    """Units of four heads of two equal sequences fall into 92 shares, of a long one beside short ones into 46: then units are smaller.
+    At least 85 % of 148 SMs hold cached positions (with few stages per SM some shares are a unit's own cost)."""
+    from oracle.attention_shares import LineUp
+
+    line = LineUp.of(positions, 8, head_dim, 24, 148)
+    work = [sum(p.last - p.first for p in line.pieces(r, 148)) for r in range(148)]
+    assert sum(w > 0 for w in work) >= 0.85 * 148 or max(work) <= 8
+    assert max(work) <= 1.35 * sum(work) / 148 + 12
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,positions", [(8, 2, 64, [0, 40, 700]), (8, 1, 128, [300, 17]), (32, 8, 128, [150, 0])])
+def test_attention_by_shares_is_attention(heads, kv_heads, head_dim, positions):
+    """The parts of all shares, merged by their sums of exponentials, against softmax attention in 64 bits."""
+    from oracle.attention_shares import attend
+
+    gen = torch.Generator().manual_seed(1)
+    q, T = torch.randn(len(positions), heads, head_dim, generator=gen), max(positions) + 1
+    k, v = (torch.randn(len(positions), T, kv_heads, head_dim, generator=gen) for _ in range(2))
+    got = attend(q, k, v, positions, head_dim**-0.5, 24, 148, 148)
+    for b, p in enumerate(positions):
+        for h in range(heads):
+            kv = h * kv_heads // heads
+            score = k[b, : p + 1, kv].double() @ q[b, h].double() * head_dim**-0.5
+            assert torch.allclose(got[b, h], torch.softmax(score, 0) @ v[b, : p + 1, kv].double(), rtol=1e-12, atol=1e-12)
