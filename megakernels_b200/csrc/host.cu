@@ -608,6 +608,9 @@ int mkb_validate_instructions(const MkbGlobals* g, const int32_t* host_instructi
     const int Hq = g->num_attention_heads, Hkv = g->num_kv_heads, R = g->matvec_reduction_size;
     const int br = g->batch > mkb_batched::max_batch() ? mkb_gemm::block_rows() : 16;  // rows per block
     const int qkv_blocks = (Hq + 2 * Hkv) * D / br;
+    // attention by shares: how often each share of a layer is there, and whether instructions per head are as well
+    std::vector<std::vector<int>> shares(L);
+    std::vector<char> by_head(L, 0);
     for (int sm = 0; sm < g->num_sms; ++sm) {
         for (int i = 0; i < g->queue_len; ++i) {
             const int32_t* w = host_instructions + ((size_t)sm * g->queue_len + i) * MKB_INTS_PER_INSTRUCTION;
@@ -630,11 +633,13 @@ int mkb_validate_instructions(const MkbGlobals* g, const int32_t* host_instructi
                     if (g->skip_attn_reduction == 1 && w[3] != 1) return bad("skip_attn_reduction = 1 needs num_partials == 1");
                     if (g->skip_attn_reduction == 2 && w[3] > 24) return bad("at most 24 partials can be merged by the last one");
                     if (w[5] < 0 || w[5] >= (g->batch > 1 ? g->batch : 1)) return bad("sequence outside the batch");
+                    by_head[w[1]] = 1;
                     break;
                 case MKB_OP_ATTENTION_REDUCTION: {
                     if (g->skip_attn_reduction == 2) return bad("AttentionReduction instruction although the last partial merges (skip_attn_reduction = 2)");
                     if (w[1] < 0 || w[1] >= L) return bad("layer out of range");
                     if (w[2] < 0 || w[2] + 4 > Hq) return bad("head range outside the Q heads");
+                    by_head[w[1]] = 1;
                     const int n = w[5];
                     if (n < 1 || n > 24) return bad("reduction list length must be 1..24");
                     if (w[7 + n] < 0 || w[7 + n] >= (g->batch > 1 ? g->batch : 1)) return bad("sequence outside the batch");
@@ -671,6 +676,10 @@ int mkb_validate_instructions(const MkbGlobals* g, const int32_t* host_instructi
                     if (g->batch <= 1) return bad("attention by shares in a single-sequence launch");
                     if (w[1] < 0 || w[1] >= L) return bad("layer out of range");
                     if (w[2] < 0 || w[2] >= w[3]) return bad("share outside their number");
+                    if (w[3] > g->num_sms * g->queue_len) return bad("more shares than instructions");
+                    if (shares[w[1]].empty()) shares[w[1]].resize(w[3]);
+                    if ((int)shares[w[1]].size() != w[3]) return bad("a layer's shares differ in their number");
+                    if (shares[w[1]][w[2]]++) return bad("share is there twice");
                     break;
                 case MKB_OP_TP_ALL_REDUCE:
                     if (g->tp.size <= 1) return bad("all-reduce instruction without tensor parallelism");
@@ -682,6 +691,13 @@ int mkb_validate_instructions(const MkbGlobals* g, const int32_t* host_instructi
                     return bad("unknown opcode");
             }
         }
+    }
+    for (int layer = 0; layer < L; ++layer) {
+        if (shares[layer].empty()) continue;
+        if (by_head[layer]) return fail(MKB_ERR_INVALID_ARGUMENT, "layer %d: attention by shares and by head", layer);
+        for (size_t r = 0; r < shares[layer].size(); ++r)
+            if (shares[layer][r] == 0)
+                return fail(MKB_ERR_INVALID_ARGUMENT, "layer %d: share %d of %d is not there", layer, (int)r, (int)shares[layer].size());
     }
     return MKB_OK;
 }

@@ -11,6 +11,7 @@ import torch
 
 from megakernels_b200.demos.latency.instructions import (
     AttentionReduction,
+    BatchAttention,
     PartialAttention,
     RMS_Norm,
 )
@@ -37,6 +38,29 @@ def test_single_sequence_words_are_unchanged_by_the_batch_fields():
     words = serialize_and_pad(AttentionReduction(1, 8, 3, True, [0, 1, 2], None, 5))
     assert words[:11] == [3, 1, 8, 3, 1, 3, 0, 1, 2, 0, 5]
     assert serialize_and_pad(RMS_Norm(7, 1, 3))[:5] == [9, 7, 1, 3, 0]
+
+
+@pytest.mark.parametrize("batch", [2, 8, 16])
+def test_schedule_by_shares(batch):
+    """What ``merge_in_last_partial`` schedules for a batch: every SM's share of every layer once, between its QKV and o-proj, no instruction per
+    head; the words."""
+    assert serialize_and_pad(BatchAttention(3, 17, 148))[:5] == [10, 3, 17, 148, 0]
+    set_sm_count_override(148)
+    extra = ExtraModelConfig(interleave_rope=True, max_len_override=64, max_batch_size=batch)
+    cfg = LlamaConfig.llama_3_1_8b(num_hidden_layers=2, vocab_size=4096)
+    model = LlamaForCausalLM.from_random(cfg, extra, device="cpu", seed=0, draw_on="zeros")
+    opts = LatencyScheduleOptions(num_attention_partitions=1, coalesce_o_proj=True, batch_size=batch, merge_in_last_partial=True)
+    schedule = LatencyScheduleBuilder(opts).build(model)
+    ins = schedule.get_linear_instructions()
+    assert not any(isinstance(i, (PartialAttention, AttentionReduction)) for i in ins)
+    for layer in range(2):
+        mine = [n for n, i in enumerate(ins) if isinstance(i, BatchAttention) and i.layer_idx == layer]
+        assert [(ins[n].rank, ins[n].num_ranks) for n in mine] == [(r, 148) for r in range(148)]
+        kind = lambda name: [n for n, i in enumerate(ins) if type(i).__name__ == name and i.layer_idx == layer]  # noqa: E731
+        assert max(kind("LayerNorm_QKV_MatVecRopeAppend")) < min(mine) and max(mine) < min(kind("O_ProjResidual"))
+    for mode in ("rr", "zz"):
+        queues = assign_to_sms(mode, schedule=schedule)
+        assert sorted((i.layer_idx, i.rank) for q in queues for i in q if isinstance(i, BatchAttention)) == [(m, r) for m in range(2) for r in range(148)]
 
 
 def test_more_than_eight_sequences_schedule_blocks_of_128_rows():

@@ -172,3 +172,51 @@ def test_host_validation_of_attention_reduction_modes():
     assert rc == 1 and "0, 1 or 2" in msg
     ins[0, 1].zero_()  # without the reduction instruction mode 2 is a valid stream
     assert check(2)[0] == 0
+
+
+def test_host_validation_of_attention_shares():
+    """Opcode 10: every share of a layer once, all with the same number of shares, in place of opcodes 2 and 3."""
+    import sys
+
+    import torch
+
+    sys.path.insert(0, str(ROOT / "megakernels_b200" / "native"))
+    import mk_llama
+
+    lib = mk_llama.load_library()
+    lib.mkb_validate_instructions.argtypes = [ctypes.POINTER(mk_llama.MkbGlobals), ctypes.c_void_p]
+    lib.mkb_validate_instructions.restype = ctypes.c_int
+    g = mk_llama.MkbGlobals()
+    g.abi_version, g.struct_bytes = mk_llama.MKB_ABI_VERSION, ctypes.sizeof(mk_llama.MkbGlobals)
+    for name, ctype in mk_llama.MkbGlobals._fields_:
+        if ctype is ctypes.c_void_p and name not in ("timings", "status", "pos_id_device", "argmax_out"):
+            setattr(g, name, 0x10000)
+    g.num_sms, g.queue_len, g.barrier_ops, g.barrier_width = 3, 3, 10, 128
+    g.num_layers, g.hidden_size, g.intermediate_size, g.head_dim = 2, 2048, 8192, 64
+    g.num_attention_heads, g.num_kv_heads, g.vocab_size = 32, 8, 128256
+    g.kv_max_len, g.kv_batch, g.max_partials, g.matvec_reduction_size = 128, 3, 24, 2048
+    g.batch, g.skip_attn_reduction = 3, 2
+    good = torch.zeros(3, 3, 32, dtype=torch.int32)
+    for sm in range(3):
+        for layer in range(2):
+            good[sm, layer, :4] = torch.tensor([10, layer, sm, 3])
+
+    def check(*changes):
+        ins = good.clone()
+        for sm, i, words in changes:
+            ins[sm, i] = 0
+            ins[sm, i, : len(words)] = torch.tensor(words)
+        rc = lib.mkb_validate_instructions(ctypes.byref(g), ctypes.c_void_p(ins.data_ptr()))
+        return rc, lib.mkb_last_error().decode()
+
+    assert check()[0] == 0, check()[1]
+    for changes, what in [
+        ([(1, 1, [10, 2, 1, 3])], "layer out of range"), ([(1, 1, [10, 1, 3, 3])], "outside their number"), ([(1, 1, [10, 1, 1, 1 << 30])], "more shares"),
+        ([(1, 1, [10, 1, 1, 2])], "differ in their number"), ([(1, 1, [10, 1, 2, 3])], "twice"), ([(1, 1, [0])], "share 1 of 3 is not there"),
+        ([(1, 2, [2, 1, 0, 1, 0, 0])], "by shares and by head"),
+    ]:
+        rc, msg = check(*changes)
+        assert rc == 1 and what in msg, (what, msg)
+    g.batch, g.kv_batch = 1, 1
+    rc, msg = check()
+    assert rc == 1 and "single-sequence" in msg
