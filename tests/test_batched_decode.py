@@ -264,3 +264,42 @@ def test_attention_by_shares_is_attention(heads, kv_heads, head_dim, positions):
             kv = h * kv_heads // heads
             score = k[b, : p + 1, kv].double() @ q[b, h].double() * head_dim**-0.5
             assert torch.allclose(got[b, h], torch.softmax(score, 0) @ v[b, : p + 1, kv].double(), rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv_heads,head_dim,lens,parts", [
+    (32, 8, 64, [31, 500, 0, 64, 200], 2), (32, 8, 128, [17, 900, 128, 300], 3), (16, 2, 128, [700, 33], 5), (32, 8, 128, [(37 * i) % 300 for i in range(40)], 2)])
+def test_last_partial_of_a_batch_merges(heads, kv_heads, head_dim, lens, parts):
+    """Instructions per sequence and head whose last part to arrive merges (what a caller of the C interface may still schedule with
+    skip_attn_reduction = 2) leave what reduction instructions leave: both merge in 32 bits and round to bf16 once."""
+    from megakernels_b200.generators import MK_Generator
+    from tests.gpu_utils import interpreter
+
+    dev, batch = "cuda:0", len(lens)
+    cfg = LlamaConfig.llama_3_1_8b(
+        num_hidden_layers=1, vocab_size=4096, hidden_size=2048, intermediate_size=2048, num_attention_heads=heads,
+        num_key_value_heads=kv_heads, head_dim=head_dim)
+    extra = ExtraModelConfig(interleave_rope=True, max_len_override=max(lens) + 8, max_batch_size=batch)
+    model = LlamaForCausalLM.from_random(cfg, extra, device=dev, seed=0, draw_on="device")
+    gen = torch.Generator(device=dev).manual_seed(2)
+    ids = torch.randint(0, cfg.vocab_size, (batch, 1), generator=torch.Generator().manual_seed(3)).to(dev)
+    prefix = [torch.randn(c.shape, generator=gen, device=dev).to(c.dtype) for c in model.stacked_kv_cache]
+    outs = []
+    for merge in (True, False):
+        for c, x in zip(model.stacked_kv_cache, prefix):
+            c.copy_(x)
+        opts = LatencyScheduleOptions(num_attention_partitions=parts, coalesce_o_proj=True, batch_size=batch)
+        schedule = LatencyScheduleBuilder(opts).build(model)
+        queues = assign_to_sms("rr", schedule=schedule)
+        assert any(isinstance(i, AttentionReduction) for q in queues for i in q)
+        if merge:
+            queues = [[i for i in q if not isinstance(i, AttentionReduction)] for q in queues]
+            schedule.globs.merge_in_last_partial = True
+        tensorize_instructions(schedule.globs, queues)
+        mk = MK_Generator(model, interpreter(), schedule)
+        for _ in range(2):
+            mk.run(ids, lens)
+        mk.check()
+        outs.append(schedule.globs.attn_out.float().clone())
+    for b in range(batch):
+        assert float((outs[0][b] - outs[1][b]).norm() / outs[1][b].norm()) < 2 * 2.0**-9, f"sequence {b} of length {lens[b]}"
