@@ -85,8 +85,8 @@ int l2_window_from_env(const char* name, int default_kb) {
     return kb == 0 ? 0 : kNumStages + kb * 1024 / kStageBytes;
 }
 const int g_l2_window_stages = l2_window_from_env("MKB_L2_WINDOW_KB", 64);
-// (several sequences: their activations pass through L2 as well, 7 and 64 sequences in us without and with 64 KB: 1176 and
-// 1214, 2187 and 2234)
+// (several sequences: their activations pass through L2 as well, 7 and 64 sequences in us without and with 64 KB: 1124 and
+// 1189, 1674 and 1732)
 const int g_l2_window_batched = l2_window_from_env("MKB_L2_WINDOW_KB", 0);
 const int g_l2_stall_window_stages = l2_window_from_env("MKB_L2_STALL_WINDOW_KB", 1024);
 

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kFlashThreads, EP <= 128 ? 2 : 1) flash_kernel
     }
     // Both maps' rows, maxima and sums go through shared memory (the tiles are done with); then all warps of the cluster put
     // the parts together, combine the maps, normalise and gate, whole rows in a loop.  Unrolled in registers this was 100 KB
-    // of code that every launch fetched anew (46 us for 30 tokens in all, now 20; 2048 tokens 669 and 531 us).
+    // of code that every launch fetched anew (16 heads of 128: 53 us for 30 tokens in all, now 20; 2048 tokens 634 and 526 us).
     float* rows = reinterpret_cast<float*>(sm + S.k);
     const int os = EP + 4;
     float2* stats = reinterpret_cast<float2*>(rows + 2 * kBQ * os);
@@ -578,7 +578,9 @@ cudaError_t flash_attention(const MkbhGlobals& g, const MkbhLayer& L, const bf16
                             int64_t ldo, cudaStream_t s) {
     FlashArgs a{g.proj, pad8(L.in_rows), ldo, g.num_tokens, g.pos0, L, kc, vc, out, g.eps, (L.dim + 15) & ~15, 1};
     // few queries over several tiles of keys: CTAs that would have nothing to do take a share of the tiles each (100 queries
-    // after 500 positions, 16 heads of 64: 51 us alone, 30 with four)
+    // after 500 positions, 16 heads of 64: 51 us alone, 30 with four).  Over 108 sizes it is never behind one CTA by more than 2 % of a layer; four instead of
+    // eight would be up to 1.3 times as fast with values of 256 dimensions and up to 61 queries, two waves up to 1.27 times with 200 and
+    // more queries after 1500 and more positions.
     int sms = 0;
     if (const cudaError_t e = sm_count(&sms); e != cudaSuccess) return e;
     const int blocks = (a.n + kBQ - 1) / kBQ * L.heads, keys = min(a.pos0 + a.n, L.window + kBQ + L.keep_first);

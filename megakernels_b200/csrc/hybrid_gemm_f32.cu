@@ -489,7 +489,7 @@ cudaError_t gemm_f32(const float* A, int64_t lda, const float* W, int64_t ldw, i
     int sms = 0;
     if (const cudaError_t err = sm_count(&sms); err != cudaSuccess) return err;
     // Tokens of a tile and CTAs on it: waves of tiles, each so many steps (in cycles, as measured with tf32 parts; of 78 shapes of 3 to
-    // 2048 tokens x 512 to 10304 features x 512 to 8192 the choice misses the fastest of these kinds by 2 % at most) and a beginning
+    // 2048 tokens x 512 to 10304 features x 512 to 8192 the choice misses the fastest of these kinds by more than 5 % in two, 2 us at most) and a beginning
     // and an end of its own; a cluster's exchange besides.  Clusters of eight wait for whole groups of SMs (20 x 2048 x 8192: 57 us, four
     // 49 us, when a step took as long).
     const int widths[] = {16, 32, 64, 96, 128, 160}, steps = (K + kStep - 1) / kStep, rows = (N + kFeatures - 1) / kFeatures;

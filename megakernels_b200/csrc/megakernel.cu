@@ -316,7 +316,7 @@ __device__ __forceinline__ AttnRange attn_range(const KParams& p, int pos, int n
 // these heads, so that a copy reads whole runs of a position's row.  A unit is as long as its stages
 // and kUnitCost more, for what it costs besides them.  Shares are cut anywhere in the line-up
 // (sequence, heads, stage); what is cut has partial rows, which the last of its parts to arrive merges.
-// (7 and 64 sequences, us: 3: 1154, 1720; 6: 1139, 1695; 10: 1128, 1678; 16: 1128, 1677; 40: 1137, 1752; 12 was taken.  Besides a unit's own
+// (7 and 64 sequences, us: 3: 1139, 1716; 6: 1122, 1698; 10: 1111, 1659; 12: 1111, 1648; 16: 1113, 1640; 40: 1119, 1707.  Besides a unit's own
 // cost it is what a cut nearby costs: those move to the unit's edge.)
 constexpr int kUnitCost = 12;
 struct AttnPiece {
@@ -1646,8 +1646,9 @@ __device__ __forceinline__ uint32_t transpose8(uint32_t x) {
 // A ring slot belongs to a group of four warps, which work on four stages side by side: a stage's chain of
 // scores, softmax and values (about 0.5 us) then hides behind the other groups' and behind the copies.  With all 16 warps on
 // one stage after the other, a stage took 1.27 us in the GEMM build and 1.06 us for up to 8 sequences; an SM's
-// share of the memory rate is 0.74 us; now 0.84 us, and a layer's attention 125 us instead of 290 (64 sequences of 256..4096
-// positions), 27 us instead of 37 (7 sequences).  K/V look-ahead in L2 beyond the ring changed nothing.  A warp has 16 positions of one key/value head: scores S = K Q^T with the
+// share of the memory rate is 0.74 us; now a share of 120 stages takes 87 us and what surrounds it 15: a layer's attention 102 us instead of 290
+// (64 sequences of 256..4096 positions), 22 us instead of 37 (7 sequences).  K/V look-ahead in L2 beyond the ring changed nothing.
+// A warp has 16 positions of one key/value head: scores S = K Q^T with the
 // positions as the M side and the head's queries as N, then O^T = V^T P^T with the head's dimensions as M, so that no side of an MMA
 // is padding but the queries' (4 of 8).  The warps' sums are merged once per piece, in shared memory.
 template <int D, int GQA>
