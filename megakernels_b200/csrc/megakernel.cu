@@ -390,8 +390,8 @@ struct AttnShares {
 // Units of four heads read the longest runs, but no unit falls into more parts than there are rows for, and two sequences of 8 such heads
 // would keep 92 of 148 SMs busy, a long one beside short ones 46: then units are of fewer heads.  A stage of them costs 1 and 5 % more (8 and 64
 // sequences).  8B widths, 4 layers, us, units of 4, 2, 1 heads: two sequences of 4096 486, 476, 478, of 16384 564, 538, 540, 16384 and 40
-// positions 568, 514, 501 (558 by an instruction per sequence and head); eight of 4096 547, 545, 551.  Instructions remain ahead where few
-// sequences are equally long and short (two of 1000: 448, shares 461) and by 3 - 7 % with equally long ones of 64 dimensions.
+// positions 568, 514, 501 (554 by an instruction per sequence and head); eight of 4096 547, 545, 551.  Instructions remain ahead where few
+// sequences are equally long and short (two of 1000: 448, shares 454) and by up to 5 % with equally long ones of 64 dimensions.
 __device__ __forceinline__ void attn_shares_table(const Ctx& c, const KParams& p, int lane) {
     volatile int* tab = c.cta_abort + kCtlShares;
     const uint32_t rows = (uint32_t)min(23, p.max_partials - 1);
@@ -1629,10 +1629,19 @@ __device__ __forceinline__ void store_vec(float* dst, const float (&v)[N]) {
     if constexpr (N == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
     else *reinterpret_cast<float2*>(dst) = make_float2(v[0], v[1]);
 }
+// A row of a head in shared memory, and a partial row, has dimensions 16 i + g and 16 i + 8 + g side by side, as a thread's accumulators hold
+// them: N of its floats from lane * N on.
 template <int N>
-__device__ __forceinline__ void store_bf16(__nv_bfloat16* dst, const float (&v)[N]) {
-    if constexpr (N == 4) *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
-    else *reinterpret_cast<uint32_t*>(dst) = pack_bf16x2(v[0], v[1]);
+__device__ __forceinline__ void store_pairs(__nv_bfloat16* row, int lane, const float (&v)[N]) {
+    if constexpr (N == 4) {
+        uint32_t* dst = reinterpret_cast<uint32_t*>(row + (lane >> 2) * 16 + (lane & 3) * 2);
+        dst[0] = pack_bf16x2(v[0], v[2]);
+        dst[4] = pack_bf16x2(v[1], v[3]);
+    } else {
+        __nv_bfloat16* dst = row + (lane >> 3) * 16 + (lane & 7);
+        dst[0] = __float2bfloat16_rn(v[0]);
+        dst[8] = __float2bfloat16_rn(v[1]);
+    }
 }
 
 // (row g, elements 2t and 2t + 1) -> (row 2t and 2t + 1, element g) of an 8 x 8 matrix over a warp
@@ -1662,7 +1671,9 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
     const int g = lane >> 2, t = lane & 3;
     const int layer = __ldg(w + 1);
     AttnShares shares;
-    if (!shares.begin(c, p, __ldg(w + 2), __ldg(w + 3))) return true;
+    AttnPiece a;
+    // (the first piece's divisions are done while the wait goes on)
+    if (!shares.begin(c, p, __ldg(w + 2), __ldg(w + 3)) || !shares.next(c, p, a)) return true;
 
     {  // the layer's queries, keys and values of all heads are there (two warps: 64 counters in one round trip)
         volatile int *first = verdict_word(c, cs), *second = c.cta_abort + kCtlShares + kBatch + 3;
@@ -1688,8 +1699,7 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
     float* sml = reinterpret_cast<float*>(__cvta_shared_to_generic(c.base + kSmemAttn));  // (m, l) of [warp][query head]
     volatile int* merged = c.cta_abort + kCtlShares + kBatch + 2;                          // verdicts of the two cut units
     int done = 0, ncut = 0, cut_seq[2] = {0, 0}, cut_kvh[2] = {0, 0}, cut_np[2] = {0, 0};
-    AttnPiece a;
-    while (shares.next(c, p, a)) {
+    do {
         const int pos_tok = c.pos_of(a.seq), head0 = (a.kvh0 + hd) * GQA;
         const __nv_bfloat16* q_rope = p.q_rope + (size_t)a.seq * p.o_in;
         __nv_bfloat16* attn_out = p.attn_out + (size_t)a.seq * p.o_in;
@@ -1830,13 +1840,12 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
             consumer_sync();  // every warp is done with the stage (or with the four heads before)
             if (2 * t >= h0 && 2 * t < h0 + 4) {
                 const int q = 2 * t - h0;
+                float* dst = so + (size_t)(warp * 4 + q) * D + 2 * g;  // pairs, see store_pairs
 #pragma unroll
                 for (int i = 0; i < DT; ++i) {
-                    float* dst = so + (size_t)(warp * 4 + q) * D + 16 * i + g;
-                    dst[0] = o[i][0];
-                    dst[D] = o[i][1];
-                    dst[8] = o[i][2];
-                    dst[D + 8] = o[i][3];
+                    const int at = (16 * i) ^ (8 * q);  // (q is 0 or 2: the two lie in different banks)
+                    *reinterpret_cast<float2*>(dst + at) = make_float2(o[i][0], o[i][2]);
+                    *reinterpret_cast<float2*>(dst + D + at) = make_float2(o[i][1], o[i][3]);
                 }
                 if (g == 0) {
                     float* ml = sml + (warp * 4 + q) * 2;
@@ -1856,7 +1865,7 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
                     const float f = exp2f(sml[(e * 4 + q) * 2] - ms);
                     den = fmaf(f, sml[(e * 4 + q) * 2 + 1], den);
                     float v[VEC];
-                    load_vec<VEC>(so + (size_t)(e * 4 + q) * D + lane * VEC, v);
+                    load_vec<VEC>(so + (size_t)(e * 4 + q) * D + ((lane * VEC) ^ (8 * (q & 2))), v);
 #pragma unroll
                     for (int i = 0; i < VEC; ++i) num[i] = fmaf(f, v[i], num[i]);
                 }
@@ -1864,7 +1873,7 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
 #pragma unroll
                 for (int i = 0; i < VEC; ++i) num[i] *= inv;
                 if (a.np == 1) {
-                    store_bf16<VEC>(attn_out + (size_t)head * D + lane * VEC, num);
+                    store_pairs<VEC>(attn_out + (size_t)head * D, lane, num);
                 } else {
                     const size_t row = (size_t)head * p.max_partials + a.pi;
                     store_vec<VEC>(attn_o + row * D + lane * VEC, num);
@@ -1898,7 +1907,7 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
             else cut_seq[1] = a.seq, cut_kvh[1] = a.kvh0, cut_np[1] = a.np;
             ++ncut;
         }
-    }
+    } while (shares.next(c, p, a));
     if (ncut > 0) {
         consumer_sync();
         int merges = 0;
@@ -1913,12 +1922,20 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
                 const int head = cut_kvh[k] * GQA + hh;
                 const float lse = lane < np ? ld_cg_f32(attn_lse + (size_t)head * p.max_partials + lane) : -INFINITY;
                 const float* base = attn_o + (size_t)head * p.max_partials * D + lane * VEC;
-                constexpr int NB = 6;  // rows on their way together
+                constexpr int NB = kGemm ? 6 : 12;  // rows on their way together (the GEMM build has no registers for more: 64 sequences 1,602 -> 2,150 us)
                 float acc[VEC] = {}, f = 0.f, den = 0.f;
                 for (int j0 = 0; j0 < np; j0 += NB) {
                     float part[NB][VEC];
 #pragma unroll
-                    for (int j = 0; j < NB; ++j) load_vec_cg<VEC>(base + (size_t)min(j0 + j, np - 1) * D, part[j]);
+                    for (int j = 0; j < NB; ++j) {
+                        if constexpr (kGemm) {
+                            load_vec_cg<VEC>(base + (size_t)min(j0 + j, np - 1) * D, part[j]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < VEC; ++i) part[j][i] = 0.f;
+                            if (j0 + j < np) load_vec_cg<VEC>(base + (size_t)(j0 + j) * D, part[j]);
+                        }
+                    }
                     if (j0 == 0) {
                         float mx = lse;
 #pragma unroll
@@ -1937,7 +1954,7 @@ __device__ bool consumer_batch_attention(const Ctx& c, ConsumerState& cs, const 
                 const float inv = den > 0.f ? 1.f / den : 0.f;
 #pragma unroll
                 for (int i = 0; i < VEC; ++i) acc[i] *= inv;
-                store_bf16<VEC>(p.attn_out + (size_t)seq * p.o_in + (size_t)head * D + lane * VEC, acc);
+                store_pairs<VEC>(p.attn_out + (size_t)seq * p.o_in + (size_t)head * D, lane, acc);
             }
         }
         consumer_sync();  // every thread's stores precede the signal
